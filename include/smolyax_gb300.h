@@ -187,6 +187,44 @@ size_t smx_jacobian_workspace(const smx_plan* plan_host, int64_t P);
 int smx_jacobian(const smx_plan* plan_host, const double* x, int64_t P, int64_t ldx, double* J, void* ws,
                  size_t ws_bytes, void* stream);
 
+/* Jacobian tables of the orthogonal form (Leja / Gauss-Hermite rules), all
+ * device pointers.  Slots are the (dimension, degree >= 1) pairs of the active
+ * dimensions, degrees ascending: slot soff[h] + g - 1 for degree g of dimension
+ * dim[h].  Rows are the products "entry without one of its dimensions"; terms
+ * {row, entry} are sorted by the slot of the dimension left out and cut into
+ * units {first term, end term, slot, h} of at most 128 terms. */
+typedef struct smx_jacobian64 {
+  int32_t d_in, d_out;
+  int32_t n_dims, n_slots, n_rows, n_units;
+  int32_t max_deg;             /* largest degree                                     */
+  const int32_t* dim;          /* [n_dims] active dimensions                         */
+  const int32_t* deg;          /* [n_dims] their largest degrees                     */
+  const int32_t* soff;         /* [n_dims] first slot                                */
+  const int32_t* node_off;     /* [n_dims + 1] into node                             */
+  const double* node;          /* nodes of the summands' pairs, by dimension         */
+  const int32_t* dim_index;    /* [d_in] h of a dimension, -1 without entries        */
+  const int32_t* unit_off;     /* [n_dims + 1] units of each active dimension        */
+  const int32_t* row_off;      /* [n_rows + 1] into row_slot                         */
+  const int32_t* row_slot;     /* slots of each row                                  */
+  const int32_t* unit;         /* [n_units * 4], 16-byte aligned                     */
+  const int32_t* term;         /* [n_terms * 2], 8-byte aligned                      */
+  const double* C;             /* [n_lambda * d_out] coefficients                    */
+  const double* rec;           /* [2][max_deg][2] alpha_n, beta_n of phi_{n+1} =
+                                  alpha_n z phi_n - beta_n phi_{n-1} of each family,
+                                  16-byte aligned                                    */
+  const double* fam_a;         /* [d_in] affine map to the family's variable         */
+  const double* fam_b;         /* [d_in]                                             */
+  const int32_t* fam;          /* [d_in] 0 Legendre, 1 normalised Hermite            */
+} smx_jacobian64;
+
+/* The same Jacobian as smx_jacobian through the orthogonal form: one
+ * multiply-add per (entry, active dimension), output and point.  NaN in
+ * dimension j where x_j is an interpolation node, as there
+ * (barycentric.py:126-155).  ws 16-byte aligned. */
+size_t smx_jacobian64_workspace(const smx_jacobian64* tables_host, int64_t P);
+int smx_jacobian64_eval(const smx_jacobian64* tables_host, const double* x, int64_t P, int64_t ldx, double* J,
+                        void* ws, size_t ws_bytes, void* stream);
+
 /* Integral: Q[o] = offset[o] + sum_r qw(r) F64[r, o] with qw the product of
  * the pairs' quadrature weights `qnode` ([n_values], host-computed rule
  * weights) (interpolation.py:347-390). */

@@ -141,6 +141,36 @@ class SmxSpectral64(C.Structure):
     ]
 
 
+class SmxJacobian64(C.Structure):
+    """Mirror of ``struct smx_jacobian64``."""
+
+    _fields_ = [
+        ("d_in", _i32),
+        ("d_out", _i32),
+        ("n_dims", _i32),
+        ("n_slots", _i32),
+        ("n_rows", _i32),
+        ("n_units", _i32),
+        ("max_deg", _i32),
+        ("dim", _p),
+        ("deg", _p),
+        ("soff", _p),
+        ("node_off", _p),
+        ("node", _p),
+        ("dim_index", _p),
+        ("unit_off", _p),
+        ("row_off", _p),
+        ("row_slot", _p),
+        ("unit", _p),
+        ("term", _p),
+        ("C", _p),
+        ("rec", _p),
+        ("fam_a", _p),
+        ("fam_b", _p),
+        ("fam", _p),
+    ]
+
+
 class SmxBlocked(C.Structure):
     """Mirror of ``struct smx_blocked``."""
 
@@ -225,6 +255,8 @@ SIGNATURES = {
     "smx_eval": (_int, [_p, _int, _p, _i64, _i64, _p, _p, _sz, _p]),
     "smx_jacobian_workspace": (_sz, [_p, _i64]),
     "smx_jacobian": (_int, [_p, _p, _i64, _i64, _p, _p, _sz, _p]),
+    "smx_jacobian64_workspace": (_sz, [_p, _i64]),
+    "smx_jacobian64_eval": (_int, [_p, _p, _i64, _i64, _p, _p, _sz, _p]),
     "smx_integral_workspace": (_sz, [_p]),
     "smx_integral": (_int, [_p, _p, _p, _p, _sz, _p]),
     "smx_spectral_pairs": (_int, [_int, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p]),

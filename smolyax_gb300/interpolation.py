@@ -88,6 +88,8 @@ class SmolyakBarycentricInterpolator:
         self._precision = precision
         self._spectral = None
         self._fp64_form_ok = None
+        self._coef = None  # FP64 coefficients of the orthogonal form (built on first use)
+        self._jacobian = None  # tables of the FP64 Jacobian: a plan, False (not for this interpolant) or None
         self._side_streams = {}  # device -> the two streams of chunked host-input evaluation
         self._d_in = len(k)
         self._d_out = int(d_out)
@@ -223,7 +225,7 @@ class SmolyakBarycentricInterpolator:
         self._plan = P
         self._assemble_rows(fu_d if on_device else T(fu, torch.float64))
         P.keep["ent"] = ent
-        self._spectral = None
+        self._spectral = self._coef = self._jacobian = None
         self._fp64_form_ok = None
         self._tree = tree
         self._maxdeg = maxdeg_h
@@ -255,7 +257,7 @@ class SmolyakBarycentricInterpolator:
         else:
             P.keep["center"] = torch.zeros(d_out, dtype=torch.float64, device=fu_d.device)
             P.set("offset", P.keep["offset0"].clone())
-        self._spectral = None
+        self._spectral = self._coef = None
 
     @property
     def nodal_values(self) -> torch.Tensor:
@@ -473,6 +475,14 @@ class SmolyakBarycentricInterpolator:
         lim = max(1, int(self._memory_limit * 1024**3 // max(1, bytes_per_point)))
         return lim
 
+    def _coefficients(self):
+        """FP64 coefficients of the orthogonal form (built on first use)."""
+        if self._coef is None:
+            from .spectral import Coefficients
+
+            self._coef = Coefficients(self)
+        return self._coef
+
     def spectral_plan(self):
         """The FP32 orthogonal-polynomial form of this interpolant (built on first use)."""
         assert self._plan is not None, "The operator has not yet been set up for a target function via `set_f`."
@@ -535,14 +545,37 @@ class SmolyakBarycentricInterpolator:
                                   and self.spectral_plan().fp64_form() is not None)
         return self.spectral_plan() if self._fp64_form_ok else None
 
+    def _jacobian_plan(self):
+        """Tables of the orthogonal form's Jacobian, or None where the combination
+        sum serves ``gradient``: other rules than Leja and Gauss-Hermite (their
+        polynomial families are the form's), degrees of 24 and more (the basis
+        change of the form is a host computation there), interpolants without
+        summands, and coefficient workspaces beyond 16 GB (as large as the nodal
+        values' rows, which the combination sum does not need twice)."""
+        if self._jacobian is None:
+            from .jacobian import MAX_DEGREE, JacobianPlan
+
+            c = self._plan.c
+            ok = (c.n_entries > 0 and c.n_entries * c.d_out * 8 <= 16 * 1024**3
+                  and int(np.max(self._maxdeg, initial=0)) < MAX_DEGREE
+                  and all(isinstance(g, (_nodes.Leja1D, _nodes.GaussHermite1D)) for g in self._node_gen))
+            self._jacobian = JacobianPlan(self) if ok else False
+        return self._jacobian or None
+
     def gradient(self, x: ArrayLike) -> torch.Tensor:
-        """Jacobian of the interpolant at x: (n_points, d_out, d_in) (``interpolation.py:306-345``)."""
+        """Jacobian of the interpolant at x: (n_points, d_out, d_in) (``interpolation.py:306-345``).
+        NaN in a dimension whose coordinate is an interpolation node."""
         x = self._validate_input(x)
         Pn = int(x.shape[0])
         J = torch.empty(Pn, self._d_out, self._d_in, dtype=torch.float64, device=x.device)
         if Pn == 0:
             return J
         st = _stream()
+        # (a capturing stream cannot build the tables: the combination sum there)
+        ready = (self._jacobian is not None and self._coef is not None) or not torch.cuda.is_current_stream_capturing()
+        jac = self._jacobian_plan() if ready else None
+        if jac is not None:
+            return jac.evaluate(self._coefficients(), x, J, st, self._memory_limit * 1024**3)
         pl = self._plan
         per_point = capi.size("smx_jacobian_workspace", pl.ref(), 1)
         step = self._chunk(per_point)

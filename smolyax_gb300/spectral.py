@@ -73,8 +73,11 @@ def basis_change_quadrature(pdim, pdeg, pvoff, node, fam, fa, fb):
     return np.concatenate(out) if out else np.zeros(1)
 
 
-class SpectralPlan:
-    """Device arrays and the ``smx_spectral`` struct of one interpolant."""
+class Coefficients:
+    """FP64 coefficients of an interpolant over its index set (device arrays):
+    ``C64`` [n_lambda, d_out], the basis-change matrices ``A`` / ``aoff`` and the
+    entry ``ids`` of every row (kept for the adjoint), and the polynomial family
+    and affine map of every dimension."""
 
     def __init__(self, ip):
         pl = ip._plan
@@ -83,7 +86,6 @@ class SpectralPlan:
         st = capi.stream_ptr(torch.cuda.current_stream())
         c = pl.c
         d, d_out = c.d_in, c.d_out
-        self.keep = {}
         T = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a), dtype=dt, device=dev)
 
         # per-dimension family and affine map to the family's variable
@@ -91,6 +93,7 @@ class SpectralPlan:
         for j, g in enumerate(ip._node_gen):
             name, a, b = g.spectral_map()
             fam[j], fa[j], fb[j] = FAMILIES[name], a, b
+        self.fam_h, self.fa_h, self.fb_h = fam, fa, fb
         self.fam = T(fam, torch.int32)
         self.fa64, self.fb64 = T(fa, torch.float64), T(fb, torch.float64)
 
@@ -128,6 +131,24 @@ class SpectralPlan:
         self.C64 = C.view(n_lam, d_out)
         del G
         self.A, self.aoff, self.ids = A, aoff, ids  # kept for the adjoint (backward w.r.t. nodal values)
+
+
+class SpectralPlan:
+    """Device arrays and the ``smx_spectral`` struct of one interpolant."""
+
+    def __init__(self, ip):
+        pl = ip._plan
+        tree = ip._tree
+        dev = tree.rem.device
+        st = capi.stream_ptr(torch.cuda.current_stream())
+        c = pl.c
+        d, d_out = c.d_in, c.d_out
+        self.keep = {}
+        T = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a), dtype=dt, device=dev)
+        co = ip._coefficients()
+        fam, fa, fb = co.fam_h, co.fa_h, co.fb_h
+        self.fam, self.fa64, self.fb64, self.C64 = co.fam, co.fa64, co.fb64, co.C64
+        self.A, self.aoff, self.ids = co.A, co.aoff, co.ids  # for the adjoint (backward w.r.t. nodal values)
 
         # layout for the FP32 evaluator (host construction from the device tree)
         tree_np = dict(
