@@ -260,6 +260,36 @@ int smx_spectral_coefficients(const smx_plan* plan_host, const int64_t* aoff, co
                               const int32_t* tdeg, int64_t n_lambda, double* G, int32_t* ids, double* C,
                               int32_t* flag, void* ws, size_t ws_bytes, void* stream);
 
+/* Stream tables of the orthogonal form (device pointers, int32 words), shared
+ * by the FP32 evaluator of 2..15 outputs and the FP64 evaluator: every entry of
+ * Lambda is one term (row, coefficients) of an item (a hot node or a cold
+ * (dimension, degree) pair), the items are dealt to 16 lists (one per warp of a block), and
+ * each list's terms are consecutive 16-term chunks, padded with zero
+ * coefficients on the constant row (FP32: every item to a multiple of 4 terms).
+ * Rows: n_hb hot basis values, then n_vp
+ * prefix products (the first is the empty prefix, 1).
+ *   hot[n_hot][8]    dimension, largest degree, first row, family, a, b (doubles)
+ *   vp[n_vp][4]      8 uint16 rows whose product is the prefix, 0xffff past the last
+ *   desc[items][8]   hot: number of factors (0..8), 0, start of the sum (double; FP64
+ *                    with one output, else 0), 8 uint16 rows;
+ *                    cold: 2^8 | family 2^9 | factor is x itself 2^11 | degree 2^16,
+ *                    dimension, 0, 0, a, b (doubles)
+ *   warp[34]         first item of each list and the total, first chunk and total
+ *   chunk[passes][n_chunks]  16 int32 row offsets (row * row_bytes; bit 0: last
+ *                    term of its item), then 16 x `pass` coefficients (FP32 or FP64)
+ * pass = 0: no stream tables (the tables of the containing struct are used). */
+typedef struct smx_stream {
+  int32_t pass;     /* outputs per pass: 1, 4 or 8                              */
+  int32_t row_bytes; /* of one row of a tile: points per tile x value size      */
+  int32_t n_hb, n_vp, n_rows, n_hot;
+  int32_t n_chunks; /* per pass                                                 */
+  const int32_t* hot;
+  const int32_t* vp;
+  const int32_t* desc;
+  const int32_t* warp;
+  const int32_t* chunk;
+} smx_stream;
+
 /* Evaluation layout of the orthogonal form.  "Hot" dimensions are those that
  * occur before another dimension in some multi-index; every entry of Lambda
  * is either hot (all its dimensions hot) or cold (hot prefix + one cold last
@@ -300,6 +330,7 @@ typedef struct smx_spectral {
   const float* fam_b;       /* [d_in]                                             */
   const int32_t* fam;       /* [d_in] 0 Legendre, 1 Hermite                       */
   const float* c0;          /* [d_out] coefficient of the constant                */
+  smx_stream stream;        /* d_out 2..15: evaluated through these tables when set */
 } smx_spectral;
 
 /* FP32 evaluation y[P, d_out] (x FP64 row-major, leading dimension ldx). */
@@ -348,6 +379,7 @@ typedef struct smx_spectral64 {
   const double* fam_b;      /* [d_in]                                               */
   const int32_t* fam;       /* [d_in]                                               */
   const double* c0;         /* [d_out] coefficients of the constant                 */
+  smx_stream stream;        /* evaluated through these tables when set              */
 } smx_spectral64;
 
 /* y[P, d_out] (FP64) = the interpolant at the P rows of x (FP64, leading dimension ldx). */
@@ -638,11 +670,14 @@ int smx_split_tf32(const float* src, int64_t rows, int64_t cols, int64_t lds, fl
  * reference's evaluation (interpolation.py:264-304) as the smx_spectral /
  * smx_blocked comments describe; smx_fp32_plan_create uses them.  Tables are
  * read back by name (the field names of smx_blocked / smx_spectral, plus
- * "dims", "dmax", "dsoff", "tape", "ent", "lvl1" of the tape). */
+ * "dims", "dmax", "dsoff", "tape", "ent", "lvl1" of the tape; the int32 tables
+ * "st_hot", "st_vp", "st_desc", "st_warp", "st_chunk" and the scalars "st_pass",
+ * "st_row_bytes", "st_n_hb", "st_n_vp", "st_n_rows", "st_n_hot", "st_n_chunks" of the stream). */
 #define SMX_LAYOUT_BLOCKED 0
 #define SMX_LAYOUT_PERPOINT 1
 #define SMX_LAYOUT_TAPE 2
 #define SMX_LAYOUT_BLOCKED_TC 3
+#define SMX_LAYOUT_STREAM 4
 typedef struct smx_host_tables smx_host_tables;
 int smx_layout_build(int kind, int64_t n, const int32_t* parent_host, const int32_t* dim_host,
                      const int32_t* deg_host, const int32_t* level_host, const int64_t* rank_host,
@@ -650,7 +685,7 @@ int smx_layout_build(int kind, int64_t n, const int32_t* parent_host, const int3
                      const int32_t* fam_host, const double* fam_a_host, const double* fam_b_host,
                      smx_host_tables** out);
 /* The layout of the FP64 evaluator (smx_spectral64) from FP64 coefficients
- * C[n][d_out]: kind SMX_LAYOUT_PERPOINT only (its FP64 form); tables
+ * C[n][d_out]: kind SMX_LAYOUT_PERPOINT (its FP64 form) or SMX_LAYOUT_STREAM; tables
  * "node_c", "cold_ab", "terms", "coef" are read with smx_layout_f64, the others
  * with smx_layout_i32 and smx_layout_scalar. */
 int smx_layout_build_f64(int kind, int64_t n, const int32_t* parent_host, const int32_t* dim_host,

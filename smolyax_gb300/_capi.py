@@ -70,6 +70,25 @@ class SmxTree(C.Structure):
     ]
 
 
+class SmxStream(C.Structure):
+    """Mirror of ``struct smx_stream``."""
+
+    _fields_ = [
+        ("pass_", _i32),
+        ("row_bytes", _i32),
+        ("n_hb", _i32),
+        ("n_vp", _i32),
+        ("n_rows", _i32),
+        ("n_hot", _i32),
+        ("n_chunks", _i32),
+        ("hot", _p),
+        ("vp", _p),
+        ("desc", _p),
+        ("warp", _p),
+        ("chunk", _p),
+    ]
+
+
 class SmxSpectral(C.Structure):
     """Mirror of ``struct smx_spectral``."""
 
@@ -104,6 +123,7 @@ class SmxSpectral(C.Structure):
         ("fam_b", _p),
         ("fam", _p),
         ("c0", _p),
+        ("stream", SmxStream),
     ]
 
 
@@ -138,6 +158,7 @@ class SmxSpectral64(C.Structure):
         ("fam_b", _p),
         ("fam", _p),
         ("c0", _p),
+        ("stream", SmxStream),
     ]
 
 
@@ -373,7 +394,7 @@ def stream_ptr(stream):
     return C.c_void_p(stream.cuda_stream) if stream is not None else None
 
 
-LAYOUT_KINDS = {"blocked": 0, "perpoint": 1, "tape": 2, "blocked_tc": 3}
+LAYOUT_KINDS = {"blocked": 0, "perpoint": 1, "tape": 2, "blocked_tc": 3, "stream": 4}
 
 
 def host_layout(kind, tree, coef, d_out, maxdeg, fam, fa, fb, i32=(), f32=(), scalars=(), fp64=False):

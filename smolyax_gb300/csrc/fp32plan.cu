@@ -135,6 +135,8 @@ struct smx_fp32_plan {
   DevBuf<int32_t> ti64;
   DevBuf<double> tf64, fa64, fb64;
   smx_spectral64 spectral64{};
+  // stream tables of the FP32 per-point evaluator (several outputs) and of the FP64 evaluator
+  DevBuf<int32_t> st32, st64;
 };
 
 namespace {
@@ -187,6 +189,31 @@ struct Pack {
     return nullptr;
   }
 };
+
+// The stream tables of t in one device blob (16-byte aligned each) and their struct.
+int upload_stream(const smx::layout::Tables& t, DevBuf<int32_t>& blob, smx_stream& s, cudaStream_t st) {
+  Pack<int32_t> p;
+  const char* names[] = {"st_hot", "st_vp", "st_desc", "st_warp", "st_chunk"};
+  for (const char* nm : names) p.add(nm, t.i32.at(nm));
+  int rc = blob.upload(p.v, st);
+  if (rc) return rc;
+  if (cudaStreamSynchronize(st) != cudaSuccess)  // the staging vector goes out of scope
+    return smx::set_error(SMX_ERR_CUDA, "smx_fp32_plan_create: sync failed");
+  auto at = [&](const char* nm) { return p.at(blob.p, nm, t.i32.at(nm)); };
+  s.pass = int(t.scalar.at("st_pass"));
+  s.row_bytes = int(t.scalar.at("st_row_bytes"));
+  s.n_hb = int(t.scalar.at("st_n_hb"));
+  s.n_vp = int(t.scalar.at("st_n_vp"));
+  s.n_rows = int(t.scalar.at("st_n_rows"));
+  s.n_hot = int(t.scalar.at("st_n_hot"));
+  s.n_chunks = int(t.scalar.at("st_n_chunks"));
+  s.hot = at("st_hot");
+  s.vp = at("st_vp");
+  s.desc = at("st_desc");
+  s.warp = at("st_warp");
+  s.chunk = at("st_chunk");
+  return SMX_OK;
+}
 
 size_t size_of(const smx::layout::Tables& t, const char* name) {
   auto it = t.i32.find(name);
@@ -415,6 +442,11 @@ extern "C" int smx_fp32_plan_create(const smx_plan* pl, const smx_tree* tree, co
           (rc = h->fb64.upload(fb_v, st)))
         return rc;
       smx_spectral64& s = h->spectral64;
+      smx::layout::Tables s64;
+      if (smx::layout::build_stream(tr, C64_h.data(), dout, maxdeg.data(), d, fam_v.data(), fa_v.data(), fb_v.data(),
+                                    s64) &&
+          (rc = upload_stream(s64, h->st64, s.stream, st)))
+        return rc;
       s.d_in = d;
       s.d_out = dout;
       s.dstride = int(p64.scalar["dstride"]);
@@ -532,6 +564,12 @@ extern "C" int smx_fp32_plan_create(const smx_plan* pl, const smx_tree* tree, co
       s.fam_b = h->fam_b.p;
       s.fam = h->fam.p;
       s.c0 = b.fp(h.get(), "c0");
+      smx::layout::Tables s32;
+      if (dout > 1 &&
+          smx::layout::build_stream(tr, C32.data(), dout, maxdeg.data(), d, fam_v.data(), fa_v.data(), fb_v.data(),
+                                    s32) &&
+          (rc = upload_stream(s32, h->st32, s.stream, st)))
+        return rc;
     }
     if (cudaStreamSynchronize(st) != cudaSuccess)
       return smx::set_error(SMX_ERR_CUDA, "smx_fp32_plan_create: sync failed");

@@ -20,6 +20,7 @@
 
 #include "blocked_tc.h"
 #include "layout.h"
+#include "stream_eval.cuh"
 
 namespace smx {
 namespace layout {
@@ -867,6 +868,186 @@ bool build_perpoint64(const Tree& tr, const double* C, int d_out, const int64_t*
   return true;
 }
 
+// Stream tables (stream_eval.cuh): items dealt to the warps, longest first,
+// each to the warp with the least work so far.  Hot items hold the node's own
+// coefficient (on the constant row) and its leaf children; a node that is a
+// stored prefix takes its factor from that row.  The cold dimensions of one
+// 32-byte piece of x (4 consecutive ones) go to one warp, which then reads the
+// piece from its cache.
+template <typename T>
+bool build_stream(const Tree& tr, const T* C, int d_out, const int64_t* maxdeg, int d, const int32_t* fam,
+                  const double* fa, const double* fb, Tables& out) {
+  constexpr int kTerms = smx::stream::kTerms;
+  const int kItem = sizeof(T) == 4 ? 32 : 64;  // terms per item: FP32 sums stay short
+  // Work of an item beyond its terms, in terms: FP64 is bound by multiply-adds
+  // (the item's own, and the factors' products); FP32 by issue slots (the
+  // compensated addition of the item's sums is ~6 terms' worth).
+  const double kOver = sizeof(T) == 4 ? 7.0 : 1.0;
+  const Front f = front(tr, maxdeg, d);
+  if (f.max_depth > kMaxPath || f.n_hb + f.n_vp > 0x7fff) return false;
+  const int pass = d_out == 1 ? 1 : (sizeof(T) == 4 && d_out > 4 ? 8 : 4);
+  const int one = int(f.n_hb);  // the constant row
+  const int row_bytes = 32 * smx::stream::lane_points<T>(pass) * int(sizeof(T));
+  auto put_double = [](int32_t* p, double v) { std::memcpy(p, &v, 8); };
+  auto path_rows = [&](int64_t e, uint16_t* s) {
+    int n = 0;
+    for (int64_t v = e; v != 0; v = tr.parent[v]) s[n++] = uint16_t(f.slot[v]);
+    std::reverse(s, s + n);
+    return n;
+  };
+
+  std::vector<int32_t> hot;
+  for (size_t h = 0; h < f.hot_dims.size(); ++h) {
+    int32_t w[8] = {f.hot_dims[h], f.hot_deg[h], f.hot_soff[h], fam[f.hot_dims[h]]};
+    put_double(w + 4, fa[f.hot_dims[h]]);
+    put_double(w + 6, fb[f.hot_dims[h]]);
+    hot.insert(hot.end(), w, w + 8);
+  }
+  std::vector<int32_t> vp(size_t(f.n_vp) * 4, -1);
+  for (int64_t e = 1; e < tr.n; ++e)
+    if (f.vp_row[e] >= 0) {
+      uint16_t s[kMaxPath];
+      const int n = path_rows(e, s);
+      std::memcpy(&vp[size_t(f.vp_row[e] - f.n_hb) * 4], s, n * sizeof(uint16_t));
+    }
+
+  // items: descriptor, terms (row, entry); bundles of items that stay together
+  struct Item {
+    int32_t desc[8];
+    std::vector<std::pair<int, int64_t>> terms;
+  };
+  struct Bundle {
+    std::vector<Item> items;
+    double cost = 0.0;
+  };
+  std::vector<Bundle> bundles;
+  // terms from the smallest to the largest coefficients: the running sum grows
+  // last, which keeps its rounding down
+  std::vector<double> size(tr.n, 0.0);
+  for (int64_t e = 0; e < tr.n; ++e)
+    for (int o = 0; o < d_out; ++o) size[e] = std::max(size[e], std::abs(double(C[e * d_out + o])));
+  auto by_size = [&](std::vector<std::pair<int, int64_t>>& terms) {
+    std::stable_sort(terms.begin(), terms.end(),
+                     [&](const auto& a, const auto& b) { return size[a.second] < size[b.second]; });
+  };
+  auto add = [&](Bundle& b, const int32_t* desc, const std::vector<std::pair<int, int64_t>>& terms, double over) {
+    for (size_t i = 0; i < terms.size(); i += kItem) {
+      Item it;
+      std::memcpy(it.desc, desc, sizeof(it.desc));
+      it.terms.assign(terms.begin() + i, terms.begin() + std::min(terms.size(), i + kItem));
+      b.cost += double(sizeof(T) == 4 ? round4(int64_t(it.terms.size())) : int64_t(it.terms.size())) + over;
+      b.items.push_back(std::move(it));
+    }
+  };
+  for (size_t i = 0; i < f.nodes.size(); ++i) {
+    const int64_t e = f.nodes[i];
+    std::vector<std::pair<int, int64_t>> terms;
+    // the node's own coefficient: the start of its first sum (FP64, one output),
+    // or a term on the constant row
+    const bool own_start = sizeof(T) == 8 && pass == 1 && e != 0 && f.starts[i] < f.ends[i];
+    if (e != 0 && !own_start) terms.push_back({one, e});
+    for (int64_t q = f.starts[i]; q < f.ends[i]; ++q) terms.push_back({int(f.slot[f.leaf[q]]), f.leaf[q]});
+    by_size(terms);
+    uint16_t s[kMaxPath] = {};
+    int n = 0;
+    if (e != 0 && f.vp_row[e] >= 0)
+      s[n++] = uint16_t(f.vp_row[e]);
+    else
+      n = path_rows(e, s);
+    int32_t desc[8] = {n};
+    std::memcpy(desc + 4, s, sizeof(s));
+    for (size_t t = 0; t < terms.size(); t += kItem) {  // parts of one node may go to several lists
+      Bundle b;
+      put_double(desc + 2, own_start && t == 0 ? double(C[e * d_out]) : 0.0);
+      add(b, desc,
+          std::vector<std::pair<int, int64_t>>(terms.begin() + t, terms.begin() + std::min(terms.size(), t + kItem)),
+          kOver + (n > 1 ? n - 1 : 0));
+      bundles.push_back(std::move(b));
+    }
+  }
+  std::vector<int64_t> cold = f.cold;
+  std::stable_sort(cold.begin(), cold.end(), [&](int64_t a, int64_t b) {
+    return std::make_tuple(tr.dim[a], tr.deg[a], f.vp_row[tr.parent[a]]) <
+           std::make_tuple(tr.dim[b], tr.deg[b], f.vp_row[tr.parent[b]]);
+  });
+  for (size_t i = 0; i < cold.size();) {
+    Bundle b;
+    const int piece = tr.dim[cold[i]] / 4;
+    while (i < cold.size() && tr.dim[cold[i]] / 4 == piece) {
+      const int j = tr.dim[cold[i]], g = tr.deg[cold[i]];
+      std::vector<std::pair<int, int64_t>> terms;
+      for (; i < cold.size() && tr.dim[cold[i]] == j && tr.deg[cold[i]] == g; ++i)
+        terms.push_back({int(f.vp_row[tr.parent[cold[i]]]), cold[i]});
+      by_size(terms);
+      const bool plain = g == 1 && fam[j] == 0 && fa[j] == 1.0 && fb[j] == 0.0;
+      int32_t desc[8] = {(1 << 8) | (fam[j] << 9) | (plain ? 1 << 11 : 0) | (g << 16), j};
+      put_double(desc + 4, fa[j]);
+      put_double(desc + 6, fb[j]);
+      add(b, desc, terms, kOver + 3.0 * (g - 1));
+    }
+    bundles.push_back(std::move(b));
+  }
+
+  std::vector<int64_t> order = stable_order(int64_t(bundles.size()), [&](int64_t i) { return -bundles[i].cost; });
+  std::vector<std::vector<int64_t>> lists(kWarps);
+  double load[kWarps] = {0};
+  for (int64_t i : order) {
+    const int w = argmin(load, kWarps);
+    lists[w].push_back(i);
+    load[w] += bundles[i].cost;
+  }
+  std::vector<int32_t> desc, warp(2 * (kWarps + 1), 0);
+  std::vector<std::pair<int, int64_t>> terms;  // byte offset of the row | last, entry (-1: padding)
+  for (int w = 0; w < kWarps; ++w) {
+    std::sort(lists[w].begin(), lists[w].end());  // hot nodes in pre-order, then cold dimensions ascending
+    for (int64_t b : lists[w])
+      for (const Item& it : bundles[b].items) {
+        desc.insert(desc.end(), it.desc, it.desc + 8);
+        for (const auto& tm : it.terms) terms.push_back({tm.first * row_bytes, tm.second});
+        while (sizeof(T) == 4 && terms.size() % 4) terms.push_back({one * row_bytes, -1});  // whole groups of 4
+        terms.back().first |= 1;
+      }
+    while (terms.size() % kTerms) terms.push_back({one * row_bytes, -1});
+    warp[w + 1] = int32_t(desc.size() / 8);
+    warp[kWarps + 1 + w + 1] = int32_t(terms.size() / kTerms);
+  }
+  const int64_t n_chunks = int64_t(terms.size()) / kTerms;
+  const int passes = (d_out + pass - 1) / pass;
+  const size_t words = size_t(smx::stream::chunk_bytes<T>(pass)) / 4;
+  std::vector<int32_t> chunk(size_t(passes) * n_chunks * words, 0);
+  for (int ps = 0; ps < passes; ++ps)
+    for (int64_t c = 0; c < n_chunks; ++c) {
+      uint8_t* p = reinterpret_cast<uint8_t*>(chunk.data() + (size_t(ps) * n_chunks + c) * words);
+      for (int t = 0; t < kTerms; ++t) {
+        const auto& tm = terms[c * kTerms + t];
+        const int32_t off = int32_t(tm.first);
+        std::memcpy(p + 4 * t, &off, 4);
+        if (tm.second < 0) continue;
+        for (int o = ps * pass; o < std::min(d_out, (ps + 1) * pass); ++o)
+          std::memcpy(p + 4 * kTerms + (size_t(t) * pass + (o - ps * pass)) * sizeof(T), &C[tm.second * d_out + o],
+                      sizeof(T));
+      }
+    }
+  out.i32["st_hot"] = hot;
+  out.i32["st_vp"] = vp;
+  out.i32["st_desc"] = desc;
+  out.i32["st_warp"] = warp;
+  out.i32["st_chunk"] = chunk;
+  out.scalar["st_pass"] = double(pass);
+  out.scalar["st_row_bytes"] = double(row_bytes);
+  out.scalar["st_n_hb"] = double(f.n_hb);
+  out.scalar["st_n_vp"] = double(f.n_vp);
+  out.scalar["st_n_rows"] = double(f.n_hb + f.n_vp);
+  out.scalar["st_n_hot"] = double(f.hot_dims.size());
+  out.scalar["st_n_chunks"] = double(n_chunks);
+  return true;
+}
+
+template bool build_stream<float>(const Tree&, const float*, int, const int64_t*, int, const int32_t*, const double*,
+                                  const double*, Tables&);
+template bool build_stream<double>(const Tree&, const double*, int, const int64_t*, int, const int32_t*, const double*,
+                                   const double*, Tables&);
+
 // Tape of the tensor-core panel (spectral.py build_tape): non-root entries in
 // DFS pre-order; word = basis slot | depth << 16; slots of dimension j with
 // max degree m_j > 0 are dsoff[j] .. dsoff[j] + m_j - 1.
@@ -938,6 +1119,8 @@ extern "C" int smx_layout_build(int kind, int64_t n, const int32_t* parent, cons
   } else if (kind == SMX_LAYOUT_BLOCKED_TC) {
     SMX_REQUIRE(d_out == 1, "smx_layout_build: the blocked evaluator has one output");
     ok = smx::layout::build_blocked_tc(tr, C, maxdeg, d, fam, fa, fb, h->t);
+  } else if (kind == SMX_LAYOUT_STREAM) {
+    ok = smx::layout::build_stream(tr, C, d_out, maxdeg, d, fam, fa, fb, h->t);
   } else {
     return smx::set_error(SMX_ERR_ARG, "smx_layout_build: unknown layout kind");
   }
@@ -953,11 +1136,13 @@ extern "C" int smx_layout_build_f64(int kind, int64_t n, const int32_t* parent, 
   SMX_REQUIRE(out && n >= 1 && d >= 1 && d_out >= 1 && parent && dim && deg && level && rank && rem && maxdeg && fam &&
                   fa && fb && C,
               "smx_layout_build_f64: bad arguments");
-  SMX_REQUIRE(kind == SMX_LAYOUT_PERPOINT, "smx_layout_build_f64: only the per-point layout has an FP64 form");
+  SMX_REQUIRE(kind == SMX_LAYOUT_PERPOINT || kind == SMX_LAYOUT_STREAM,
+              "smx_layout_build_f64: only the per-point and stream layouts have an FP64 form");
   *out = nullptr;
   smx::layout::Tree tr{n, parent, dim, deg, level, rank, rem};
   auto h = std::make_unique<smx_host_tables>();
-  if (!smx::layout::build_perpoint64(tr, C, d_out, maxdeg, d, fam, fa, fb, h->t))
+  if (kind == SMX_LAYOUT_STREAM ? !smx::layout::build_stream(tr, C, d_out, maxdeg, d, fam, fa, fb, h->t)
+                                : !smx::layout::build_perpoint64(tr, C, d_out, maxdeg, d, fam, fa, fb, h->t))
     return smx::set_error(SMX_ERR_UNSUPPORTED, "smx_layout_build_f64: the plan is outside this evaluator's limits");
   *out = h.release();
   return SMX_OK;

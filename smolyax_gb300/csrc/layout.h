@@ -42,6 +42,11 @@ bool build_perpoint(const Tree& tr, const float* C, int d_out, const int64_t* ma
 // one term (slot, coefficients); FP64 tables in Tables::f64.
 bool build_perpoint64(const Tree& tr, const double* C, int d_out, const int64_t* maxdeg, int d, const int32_t* fam,
                       const double* fa, const double* fb, Tables& out);
+// Stream tables (struct smx_stream) from FP32 or FP64 coefficients C[n][d_out];
+// false for hot nodes deeper than 8 or rows beyond 15 bits.
+template <typename T>
+bool build_stream(const Tree& tr, const T* C, int d_out, const int64_t* maxdeg, int d, const int32_t* fam,
+                  const double* fa, const double* fb, Tables& out);
 bool build_tape(const Tree& tr, const int64_t* maxdeg, int d, Tables& out);
 bool build_blocked_tc(const Tree& tr, const float* C, const int64_t* maxdeg, int d, const int32_t* fam,
                       const double* fa, const double* fb, Tables& out);

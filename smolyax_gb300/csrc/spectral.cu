@@ -20,6 +20,7 @@
 
 #include "common.cuh"
 #include "recurrence.cuh"
+#include "stream_eval.cuh"
 
 namespace {
 
@@ -300,6 +301,7 @@ __global__ void run_sum_kernel(int64_t R, int dout, const int32_t* __restrict__ 
 constexpr int kSeg = 4;
 constexpr int kTP = 128;
 constexpr int kThreads = kSeg * kTP;
+constexpr size_t kSmemMax = 226 * 1024;  // dynamic shared memory (227 KB less the static part)
 
 struct SpecArgs {
   int d_in, dout, dstride, row, n_hb, n_vp, n_hot_dims, n_nodes, n_cold_groups;
@@ -322,6 +324,7 @@ struct SpecArgs {
   const float* fam_b;
   const int32_t* fam;
   const float* c0;
+  smx_stream stream;  // stream.pass != 0: evaluated through these tables
 };
 
 __device__ __forceinline__ void kahan_add(float& sum, float& comp, float v) {
@@ -341,6 +344,13 @@ __device__ __forceinline__ float x32(double v) {
 
 __constant__ float c_alpha[2][kMaxRec];
 __constant__ float c_beta[2][kMaxRec];
+
+// Recurrence and conversion of the stream evaluator.
+struct Rec32 {
+  static __device__ __forceinline__ float alpha(int fm, int n) { return c_alpha[fm][n]; }
+  static __device__ __forceinline__ float beta(int fm, int n) { return c_beta[fm][n]; }
+  static __device__ __forceinline__ float convert(double v) { return x32(v); }
+};
 
 // s[q] = sum over the run's slots of coef * row value (runs are at most 32
 // slots long, so each is a short FP32 chain; callers add the run sums with
@@ -599,16 +609,29 @@ __global__ void __launch_bounds__(kThreads, 2) spectral_eval_kernel(SpecArgs a, 
   spectral_eval_tile<DO>(a, x, P, ldx, y, o0, blockIdx.x, sm);
 }
 
+template <int DO>
+__global__ void __launch_bounds__(kThreads, 1)
+    spectral_stream_kernel(SpecArgs a, const double* __restrict__ x, int64_t P, int64_t ldx, float* __restrict__ y,
+                           int64_t tile0, int parts) {
+  extern __shared__ __align__(16) float sm[];
+  smx::stream::stream_tile<float, DO, Rec32>(a.stream, a.dout, a.c0, x, P, ldx, y, blockIdx.y,
+                                             tile0 + blockIdx.x / parts, reinterpret_cast<unsigned char*>(sm),
+                                             parts > 1 ? int(smx::stream::cluster_rank()) : 0, parts);
+}
+
 // Serving: one persistent launch over a table of work items (plan, inputs,
 // outputs, output chunk) of different interpolants and batch sizes.  CTAs take
-// 128-point tiles from an atomic counter; the tile's item is found by binary
-// search over the items' first tiles.
+// tiles (128 points, or those of the plan's stream tables) from an atomic
+// counter; the tile's item is found by binary search over the items' first
+// tiles.
 struct WorkItem {
   int plan, o0;
   int64_t tile0, P, ldx;
   const double* x;
   float* y;
 };
+
+static_assert(32 * 16 == kThreads, "one block shape for both tile functions");
 
 __global__ void __launch_bounds__(kThreads, 1) spectral_eval_batch_kernel(const SpecArgs* __restrict__ plans,
                                                                            const WorkItem* __restrict__ items,
@@ -631,6 +654,12 @@ __global__ void __launch_bounds__(kThreads, 1) spectral_eval_batch_kernel(const 
     const SpecArgs& a = plans[it.plan];
     if (a.dout == 1)
       spectral_eval_tile<1>(a, it.x, it.P, it.ldx, it.y, it.o0, t - it.tile0, sm);
+    else if (a.stream.pass == 8)
+      smx::stream::stream_tile<float, 8, Rec32>(a.stream, a.dout, a.c0, it.x, it.P, it.ldx, it.y, it.o0 / 8,
+                                                   t - it.tile0, reinterpret_cast<unsigned char*>(sm));
+    else if (a.stream.pass == 4)
+      smx::stream::stream_tile<float, 4, Rec32>(a.stream, a.dout, a.c0, it.x, it.P, it.ldx, it.y, it.o0 / 4,
+                                                   t - it.tile0, reinterpret_cast<unsigned char*>(sm));
     else
       spectral_eval_tile<4>(a, it.x, it.P, it.ldx, it.y, it.o0, t - it.tile0, sm);
     __syncthreads();
@@ -758,6 +787,11 @@ int check_spec(const smx_spectral* sp, const char* who) {
     return smx::set_error(SMX_ERR_ARG, std::string(who) + ": segments do not cover the plan");
   if (sp->n_cold_blocks && (sp->d_out != 1 || !sp->blk_dims || !sp->blk_run || !sp->blk_ab))
     return smx::set_error(SMX_ERR_ARG, std::string(who) + ": cold blocks need d_out = 1");
+  if (sp->stream.pass) {
+    if (sp->d_out == 1 || sp->stream.pass == 1)
+      return smx::set_error(SMX_ERR_ARG, std::string(who) + ": FP32 stream tables need several outputs");
+    return smx::stream::check<float>(sp->stream, sp->d_out, who);
+  }
   return SMX_OK;
 }
 
@@ -793,12 +827,27 @@ SpecArgs to_args(const smx_spectral* sp) {
   a.fam_b = sp->fam_b;
   a.fam = sp->fam;
   a.c0 = sp->c0;
+  a.stream = sp->stream;
   return a;
 }
 
-size_t spec_smem(const smx_spectral* sp) {
+// Outputs per pass: those of the stream tables, else 1 or 4.
+int spec_pass(const smx_spectral* sp) { return sp->stream.pass ? sp->stream.pass : sp->d_out == 1 ? 1 : 4; }
+
+// Points per tile.
+int spec_points(const smx_spectral* sp) {
+  return sp->stream.pass ? 32 * smx::stream::lane_points<float>(sp->stream.pass) : kTP;
+}
+
+// Shared memory of the general tables; plans beyond 220 KB are refused whichever
+// tables evaluate them.
+size_t row_smem(const smx_spectral* sp) {
   const int DO = sp->d_out == 1 ? 1 : 4;
   return (size_t(sp->row) + size_t(kSeg) * DO * 2) * kTP * sizeof(float);
+}
+
+size_t spec_smem(const smx_spectral* sp) {
+  return sp->stream.pass ? smx::stream::smem_bytes<float>(sp->stream) : row_smem(sp);
 }
 
 }  // namespace
@@ -815,8 +864,20 @@ extern "C" int smx_spectral_eval(const smx_spectral* sp, const double* x, int64_
   const SpecArgs a = to_args(sp);
   const int DO = sp->d_out == 1 ? 1 : 4;
   const size_t smem = spec_smem(sp);
-  SMX_REQUIRE(smem <= 220 * 1024, "smx_spectral_eval: per-point row too large for shared memory");
+  SMX_REQUIRE(row_smem(sp) <= 220 * 1024 && smem <= kSmemMax, "smx_spectral_eval: per-point row too large for shared memory");
   cudaStream_t st = smx::as_stream(stream);
+  if (sp->stream.pass) {
+    const int passes = (sp->d_out + sp->stream.pass - 1) / sp->stream.pass;
+    SMX_REQUIRE(passes <= 65535, "smx_spectral_eval: too many outputs");
+    auto kernel = sp->stream.pass == 8 ? spectral_stream_kernel<8> : spectral_stream_kernel<4>;
+    static bool set[2] = {false, false};
+    if (!set[sp->stream.pass == 8]) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax));
+      set[sp->stream.pass == 8] = true;
+    }
+    return smx::stream::launch(kernel, kThreads, (P + spec_points(sp) - 1) / spec_points(sp), passes, sp->stream.n_chunks, smem, st,
+                               "smx_spectral_eval", a, x, P, ldx, y);
+  }
   static bool attr_set[2] = {false, false};
   for (int o0 = 0; o0 < sp->d_out; o0 += DO) {
     if (DO == 1) {
@@ -855,9 +916,10 @@ extern "C" int smx_spectral_eval_batch(const smx_spectral* plans, int n_plans, c
     if (rc) return rc;
     args[i] = to_args(&plans[i]);
     max_dout = std::max(max_dout, plans[i].d_out);
+    SMX_REQUIRE(row_smem(&plans[i]) <= 220 * 1024, "smx_spectral_eval_batch: per-point row too large for shared memory");
     smem = std::max(smem, spec_smem(&plans[i]));
   }
-  SMX_REQUIRE(smem <= 220 * 1024, "smx_spectral_eval_batch: per-point row too large for shared memory");
+  SMX_REQUIRE(smem <= kSmemMax, "smx_spectral_eval_batch: per-point row too large for shared memory");
   std::vector<WorkItem> work;
   int64_t tiles = 0;
   for (int j = 0; j < n_items; ++j) {
@@ -867,7 +929,7 @@ extern "C" int smx_spectral_eval_batch(const smx_spectral* plans, int n_plans, c
     if (w.P == 0) continue;
     SMX_REQUIRE(w.x && w.y, "smx_spectral_eval_batch: null work pointers");
     const int dout = plans[w.plan].d_out;
-    const int DO = dout == 1 ? 1 : 4;
+    const int DO = spec_pass(&plans[w.plan]), pts = spec_points(&plans[w.plan]);
     for (int o0 = 0; o0 < dout; o0 += DO) {
       WorkItem it;
       it.plan = w.plan;
@@ -878,7 +940,7 @@ extern "C" int smx_spectral_eval_batch(const smx_spectral* plans, int n_plans, c
       it.x = w.x;
       it.y = w.y;
       work.push_back(it);
-      tiles += (w.P + kTP - 1) / kTP;
+      tiles += (w.P + pts - 1) / pts;
     }
   }
   if (work.empty()) return SMX_OK;
@@ -897,7 +959,7 @@ extern "C" int smx_spectral_eval_batch(const smx_spectral* plans, int n_plans, c
   SMX_LAUNCH_CHECK("smx_spectral_eval_batch copies");
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(spectral_eval_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    cudaFuncSetAttribute(spectral_eval_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax));
     attr = true;
   }
   int dev = 0, sms = 0, per_sm = 1;

@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "recurrence.cuh"
+#include "stream_eval.cuh"
 
 namespace {
 
@@ -63,10 +64,13 @@ __constant__ double c_alpha64[2][kMaxRec];
 __constant__ double c_beta64[2][kMaxRec];
 
 // Infinite coordinates become NaN, as in the barycentric evaluation, whose
-// weights w/(x - node) vanish and normalise to 0/0 there.
+// weights w/(x - node) vanish and normalise to 0/0 there.  Integer operations
+// on the two words: a comparison of doubles would go to the FP64 pipe.
 __device__ __forceinline__ double xin(double v) {
-  const long long b = __double_as_longlong(v);
-  return (b & 0x7fffffffffffffffll) == 0x7ff0000000000000ll ? __longlong_as_double(0x7ff8000000000000ll) : v;
+  int hi = __double2hiint(v);
+  const int lo = __double2loint(v);
+  if (lo == 0 && (hi & 0x7fffffff) == 0x7ff00000) hi |= 0x00080000;  // infinity -> quiet NaN
+  return __hiloint2double(hi, lo);
 }
 
 // s[q] += sum over the terms [t0, t1) of coefficient (output o0 + q) * row
@@ -230,6 +234,23 @@ __global__ void __launch_bounds__(kSeg * kTP, kTP == 64 ? 2 : 1)
   }
 }
 
+// Recurrence and conversion of the stream evaluator.
+struct Rec64 {
+  static __device__ __forceinline__ double alpha(int fm, int n) { return c_alpha64[fm][n]; }
+  static __device__ __forceinline__ double beta(int fm, int n) { return c_beta64[fm][n]; }
+  static __device__ __forceinline__ double convert(double v) { return xin(v); }
+};
+
+template <int DO>
+__global__ void __launch_bounds__(smx::stream::kThreads, 2)
+    spectral_stream64_kernel(smx_stream a, int d_out, const double* __restrict__ c0, const double* __restrict__ x,
+                             int64_t P, int64_t ldx, double* __restrict__ y, int64_t tile0, int parts) {
+  extern __shared__ __align__(16) double sm64[];
+  smx::stream::stream_tile<double, DO, Rec64>(a, d_out, c0, x, P, ldx, y, blockIdx.y, tile0 + blockIdx.x / parts,
+                                              reinterpret_cast<unsigned char*>(sm64),
+                                              parts > 1 ? int(smx::stream::cluster_rank()) : 0, parts);
+}
+
 bool g_consts64_ready = false;
 
 int upload_consts64() {
@@ -342,6 +363,23 @@ extern "C" int smx_spectral_eval64(const smx_spectral64* sp, const double* x, in
   SMX_REQUIRE(x && y, "smx_spectral_eval64: null pointer");
   int rc = upload_consts64();
   if (rc) return rc;
+  if (sp->stream.pass) {
+    SMX_REQUIRE(sp->stream.pass == DO, "smx_spectral_eval64: stream tables of another pass width");
+    if ((rc = smx::stream::check<double>(sp->stream, sp->d_out, who))) return rc;
+    const size_t smem = smx::stream::smem_bytes<double>(sp->stream);
+    if (smem > kSmemMax)
+      return smx::set_error(SMX_ERR_UNSUPPORTED, std::string(who) + ": rows too large for shared memory");
+    const int passes = (sp->d_out + DO - 1) / DO;
+    SMX_REQUIRE(passes <= 65535, "smx_spectral_eval64: too many outputs");
+    auto kernel = DO == 1 ? spectral_stream64_kernel<1> : spectral_stream64_kernel<4>;
+    static bool set[2] = {false, false};
+    if (!set[DO == 1]) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax));
+      set[DO == 1] = true;
+    }
+    return smx::stream::launch(kernel, smx::stream::kThreads, (P + 31) / 32, passes, sp->stream.n_chunks, smem, smx::as_stream(stream), who,
+                               sp->stream, sp->d_out, sp->c0, x, P, ldx, y);
+  }
   Spec64Args a;
   a.d_in = sp->d_in;
   a.d_out = sp->d_out;

@@ -25,7 +25,30 @@ BLOCKED_TC_TABLES = dict(i32=("tc_td", "tc_row", "tc_chunk", "tc_b", "tc_box"), 
                          scalars=("tc_n_td", "tc_n_phi", "tc_n_phi_pad", "tc_n_rows", "tc_max_depth", "tc_n_agen",
                                   "tc_n_chunks", "tc_n_boxes", "tc_lin0", "tc_stages", "tc_td_col", "tc_td_bytes",
                                   "c0"))
+STREAM_TABLES = dict(i32=("st_hot", "st_vp", "st_desc", "st_warp", "st_chunk"),
+                     scalars=("st_pass", "st_row_bytes", "st_n_hb", "st_n_vp", "st_n_rows", "st_n_hot", "st_n_chunks"))
+FP64_TABLES = dict(i32=("node_seg", "cold_seg", "hot_dim", "hot_deg", "hot_soff", "node", "cold", "run"),
+                   f32=("node_c", "cold_ab", "terms", "coef"),
+                   scalars=("d_out", "dstride", "row", "n_hb", "n_vp", "n_hot_dims", "n_nodes", "n_cold_groups",
+                            "max_depth", "n_terms"))
 MAX_DEGREE = 512  # recurrence tables of the kernels
+
+
+def stream_tables(struct, tree, coef, d_out, maxdeg, fam, fa, fb, T, fp64):
+    """Fills the ``smx_stream`` member of an evaluator's struct (library builder)
+    from FP32 or FP64 coefficients; returns the device arrays to keep, or None
+    where the plan is outside the tables' limits."""
+    lay = capi.host_layout("stream", tree, coef, d_out, maxdeg, fam, fa, fb, fp64=fp64, **STREAM_TABLES)
+    if lay is None:
+        return None
+    keep = {name: T(lay["st_" + name], torch.int32) for name in ("hot", "vp", "desc", "warp", "chunk")}
+    s = struct.stream
+    s.pass_ = int(lay["st_pass"])
+    for name in ("row_bytes", "n_hb", "n_vp", "n_rows", "n_hot", "n_chunks"):
+        setattr(s, name, int(lay["st_" + name]))
+    for name, t in keep.items():
+        setattr(s, name, t.data_ptr() if t.numel() else None)
+    return keep
 
 
 def _phi_table(fam, z, n):
@@ -198,6 +221,8 @@ class SpectralPlan:
         self.blocked_tc = None
         if d_out == 1 and self.tc is None:
             self._build_blocked(tree_np, C32[:, 0], np.asarray(ip._maxdeg), d, fam, fa, fb, T)
+        if d_out > 1 and self.tc is None:
+            self.stream_keep = stream_tables(self.c, tree_np, C32, d_out, np.asarray(ip._maxdeg), fam, fa, fb, T, False)
 
     def _build_tc(self, tr, C32, maxdeg, fam, fa, fb, T, st):
         """Operands of the tensor-core contraction: tape over all non-root entries
@@ -436,9 +461,13 @@ class SpectralPlan:
             self._f64 = False
             tr, _, maxdeg, fam, fa, fb, T, _ = self._fwd_args
             d = int(self.c.d_in)
-            lay = build_layout64(tr, self.C64.cpu().numpy(), maxdeg, d, fam, fa, fb)
+            C64 = self.C64.cpu().numpy()
+            lay = capi.host_layout("perpoint", tr, C64, int(C64.shape[1]), maxdeg, fam, fa, fb, fp64=True,
+                                   **FP64_TABLES)
+            if lay is None:
+                return None
             row = int(lay["row"])
-            DO = 1 if lay["d_out"] == 1 else 4
+            DO = 1 if int(lay["d_out"]) == 1 else 4
             if (row + 4 * DO) * 64 * 8 <= 227 * 1024 and int(lay["max_depth"]) <= 8:
                 k = {}
                 for name in ("hot_dim", "hot_deg", "hot_soff", "node", "cold", "run"):
@@ -457,6 +486,7 @@ class SpectralPlan:
                 for name, t in k.items():
                     setattr(st, name, t.data_ptr() if t.numel() else None)
                 st.fam_a, st.fam_b, st.fam = self.fa64.data_ptr(), self.fb64.data_ptr(), self.fam.data_ptr()
+                k["stream"] = stream_tables(st, tr, C64, int(lay["d_out"]), maxdeg, fam, fa, fb, T, True)
                 self._f64 = (st, k)
         return self._f64 or None
 
