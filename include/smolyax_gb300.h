@@ -660,6 +660,53 @@ int smx_split_bf16(const float* src, int64_t rows, int64_t cols, int64_t lds, ui
 int smx_split_tf32(const float* src, int64_t rows, int64_t cols, int64_t lds, float* hi, float* lo, int64_t ldo,
                    void* stream);
 
+/* ---- tensor-core evaluation of many outputs -------------------------------------------
+ * y = A C + c0 with the basis products A of all non-root entries (reversed DFS
+ * pre-order) and the coefficients C, both as pairs of 16-bit values
+ * (interpolation.py:264-304 over the index set, as smx_spectral_eval).  bf16 = 0:
+ * FP16 pairs with exact power-of-two scales per output, entry, and point and
+ * 64-column group: 22 significant bits per operand, FP32 accumulation, as the
+ * 3xTF32 product.  bf16 = 1: BF16 pairs (16 bits).  All pointers are device
+ * pointers; the struct is read on the host. */
+typedef struct smx_tensor {
+  int32_t d_in, d_out;
+  int32_t n_dims, n_slots;    /* active dimensions, their (dimension, degree) slots    */
+  int32_t max_deg;
+  int32_t K, n_groups;        /* entries without the root; ceil(K / 64)                */
+  int32_t splits;             /* K slices of the contraction (smx_tensor_splits)       */
+  int32_t bf16;
+  int32_t reserved;
+  int64_t chunk;              /* points per pass (the panel of one pass: 4 ldb bytes a point) */
+  int64_t ldb;                /* row pitch of Bh, Bl and the panel: K rounded up to 64  */
+  const int32_t* dims;        /* [n_dims], with dmax (largest degree), dsoff (first slot) */
+  const int32_t* dmax;
+  const int32_t* dsoff;
+  const float* fam_a;         /* [d_in] affine map to the family's variable            */
+  const float* fam_b;
+  const int32_t* fam;         /* [d_in]                                                */
+  const float* rec;           /* [2][max_deg][2] recurrence alpha_n, beta_n per family */
+  const int32_t* tape;        /* [64 n_groups][2] smx_tensor_operands, 16-byte aligned */
+  const int32_t* path;        /* [n_groups][8] slots above each group's first entry, -1 past the last
+                                 ("path" of the tape tables)                            */
+  const uint16_t* Bh;         /* [d_out][ldb] high and low parts of the coefficients   */
+  const uint16_t* Bl;
+  const float* out_scale;     /* [d_out] (bf16 = 0)                                    */
+  const float* bias;          /* [d_out] c0                                            */
+  int32_t* err;               /* set when a pipeline wait runs out                     */
+} smx_tensor;
+int smx_tensor_splits(int d_out, int K);
+/* FP16 operands from the FP32 coefficients B[N][K] (column k = tape entry K-1-k):
+ * high and low parts, the output scales, and the padded tape: ceil(K/64)*64 - K
+ * entries of padding, then per entry {128 * slot, FP32 bits of 2^f | 128 * (depth - 1)
+ * | 1 where the parent's product is read back from the stack | 2 where the entry has
+ * children}.  smx_tensor_tape: the padded tape alone, f = 0 (bf16). */
+int smx_tensor_operands(const float* B, int N, int K, int64_t ldb, const int32_t* tape, int32_t* tape_out,
+                        uint16_t* B_hi, uint16_t* B_lo, int64_t ldh, float* out_scale, void* stream);
+int smx_tensor_tape(const int32_t* tape, int K, int32_t* tape_out, void* stream);
+size_t smx_tensor_workspace(const smx_tensor* plan_host, int64_t P);
+int smx_tensor_eval(const smx_tensor* plan_host, const double* x, int64_t P, int64_t ldx, float* y, void* ws,
+                    size_t ws_bytes, void* stream);
+
 /* ---- host-side layout builders of the FP32 evaluators ------------------------------
  * The tables of the blocked one-output evaluator (smx_blocked), of the
  * per-point evaluator (smx_spectral) and the entry tape of the tensor-core
@@ -670,7 +717,7 @@ int smx_split_tf32(const float* src, int64_t rows, int64_t cols, int64_t lds, fl
  * reference's evaluation (interpolation.py:264-304) as the smx_spectral /
  * smx_blocked comments describe; smx_fp32_plan_create uses them.  Tables are
  * read back by name (the field names of smx_blocked / smx_spectral, plus
- * "dims", "dmax", "dsoff", "tape", "ent", "lvl1" of the tape; the int32 tables
+ * "dims", "dmax", "dsoff", "tape", "ent", "lvl1", "path" of the tape; the int32 tables
  * "st_hot", "st_vp", "st_desc", "st_warp", "st_chunk" and the scalars "st_pass",
  * "st_row_bytes", "st_n_hb", "st_n_vp", "st_n_rows", "st_n_hot", "st_n_chunks" of the stream). */
 #define SMX_LAYOUT_BLOCKED 0

@@ -162,6 +162,39 @@ class SmxSpectral64(C.Structure):
     ]
 
 
+class SmxTensor(C.Structure):
+    """Mirror of ``struct smx_tensor``."""
+
+    _fields_ = [
+        ("d_in", _i32),
+        ("d_out", _i32),
+        ("n_dims", _i32),
+        ("n_slots", _i32),
+        ("max_deg", _i32),
+        ("K", _i32),
+        ("n_groups", _i32),
+        ("splits", _i32),
+        ("bf16", _i32),
+        ("reserved", _i32),
+        ("chunk", _i64),
+        ("ldb", _i64),
+        ("dims", _p),
+        ("dmax", _p),
+        ("dsoff", _p),
+        ("fam_a", _p),
+        ("fam_b", _p),
+        ("fam", _p),
+        ("rec", _p),
+        ("tape", _p),
+        ("path", _p),
+        ("Bh", _p),
+        ("Bl", _p),
+        ("out_scale", _p),
+        ("bias", _p),
+        ("err", _p),
+    ]
+
+
 class SmxJacobian64(C.Structure):
     """Mirror of ``struct smx_jacobian64``."""
 
@@ -301,6 +334,11 @@ SIGNATURES = {
     "smx_serve_poll": (_int, [_p, _i64]),
     "smx_serve_destroy": (None, [_p]),
     "smx_eval_f64_noalloc": (_int, [_p, _p, _i64, _i64, _p, _p]),
+    "smx_tensor_splits": (_int, [_int, _int]),
+    "smx_tensor_operands": (_int, [_p, _int, _int, _i64, _p, _p, _p, _p, _i64, _p, _p]),
+    "smx_tensor_tape": (_int, [_p, _int, _p, _p]),
+    "smx_tensor_workspace": (_sz, [_p, _i64]),
+    "smx_tensor_eval": (_int, [_p, _p, _i64, _i64, _p, _p, _sz, _p]),
     "smx_spectral_panel_workspace": (_sz, [_int, _i64]),
     "smx_spectral_panel_tf32": (_int, [_int, _p, _p, _p, _int, _p, _int, _p, _int, _p, _p, _p, _p, _i64, _i64, _p,
                                         _p, _i64, _p, _sz, _p]),

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "layout.h"
+#include "recurrence.cuh"
 
 namespace {
 
@@ -126,7 +127,10 @@ struct smx_fp32_plan {
   bool have_tape = false;
   int K = 0, ldk = 0, ldo = 0, n_slots = 0, n_dims = 0;
   DevBuf<int32_t> dims, dmax, dsoff, tape, ent, segs, err;
-  DevBuf<float> Bh, Bl, bias, Rh, Rl;
+  DevBuf<float> bias, Rh, Rl, out_scale, rec;
+  DevBuf<uint16_t> Bh, Bl;
+  DevBuf<int32_t> tape_pad, path;
+  smx_tensor tensor{};
   std::vector<int32_t> lvl1;
   std::vector<int> seg_off, seg_n;  // per wanted segment count: offset into segs, number of segments
   int vjp_want = 1;                 // tape segments of the gradient walk (fixed per plan)
@@ -222,27 +226,12 @@ size_t size_of(const smx::layout::Tables& t, const char* name) {
   return jt == t.f32.end() ? 0 : jt->second.size();
 }
 
-// Points per tensor-core chunk (the TF32 hi/lo panel of one chunk fits the memory limit).
+// Points per chunk of the backward (the TF32 hi/lo panel of one chunk fits the memory limit).
 int64_t tc_step(const smx_fp32_plan* h, int64_t P) {
   const int64_t per = 8 * round32(std::max(h->K, 1));
   int64_t step = int64_t(h->memory_limit * 1073741824.0 / double(per)) / 128 * 128;
   step = std::max<int64_t>(128, step);
   return std::max<int64_t>(1, std::min(step, P));
-}
-
-// K slices of the forward contraction: fixed per plan (from its full chunk),
-// as in the package, so that both give the same values.
-int tc_splits(const smx_fp32_plan* h) {
-  return smx_gemm_tf32x3_splits(tc_step(h, int64_t(1) << 40), h->d_out, h->K);
-}
-
-// Segments of one panel launch over n points (spectral.py segment_count).
-int seg_want(const smx_fp32_plan* h, int64_t n) {
-  const int64_t n_pb = std::max<int64_t>((n + 127) / 128, 1);
-  int64_t want = std::min<int64_t>(32, (12 * int64_t(h->sms) + n_pb - 1) / n_pb);
-  want = std::min<int64_t>(want, h->K / 256);
-  want = std::min<int64_t>(want, int64_t(h->lvl1.size()));
-  return int(std::max<int64_t>(1, want));
 }
 
 }  // namespace
@@ -392,9 +381,37 @@ extern "C" int smx_fp32_plan_create(const smx_plan* pl, const smx_tree* tree, co
       return rc;
     if ((rc = smx_split_tf32(Rd.p, std::max(h->K, 1), h->ldo, h->ldo, h->Rh.p, h->Rl.p, h->ldo, stream))) return rc;
     if (use_tc) {
-      if ((rc = Bd.upload(B, st)) || (rc = h->Bh.alloc(B.size())) || (rc = h->Bl.alloc(B.size())) ||
-          (rc = smx_split_tf32(Bd.p, dout, h->ldk, h->ldk, h->Bh.p, h->Bl.p, h->ldk, stream)))
+      // tensor-core operands (spectral.py _tc_struct)
+      smx_tensor& t = h->tensor;
+      t.d_in = d, t.d_out = dout, t.n_dims = h->n_dims, t.n_slots = h->n_slots;
+      t.K = h->K, t.n_groups = (h->K + 63) / 64;
+      t.ldb = std::max(64, 64 * t.n_groups);
+      t.splits = smx_tensor_splits(dout, h->K);
+      t.chunk = std::max<int64_t>(128, int64_t(memory_limit_gib * 1073741824.0 / double(4 * t.ldb)) / 128 * 128);
+      t.max_deg = 1;
+      for (int64_t m : maxdeg) t.max_deg = std::max(t.max_deg, int32_t(m));
+      std::vector<float> rec(size_t(4) * t.max_deg);
+      for (int f = 0; f < 2; ++f)
+        for (int m = 0; m < t.max_deg; ++m) {
+          double al, be;
+          smx::rec_coeffs(f, m, &al, &be);
+          rec[(size_t(f) * t.max_deg + m) * 2] = float(al);
+          rec[(size_t(f) * t.max_deg + m) * 2 + 1] = float(be);
+        }
+      const size_t nb = size_t(dout) * t.ldb;
+      if ((rc = h->rec.upload(rec, st)) || (rc = h->path.upload(tp.i32["path"], st)) ||
+          (rc = h->tape_pad.alloc(size_t(128) * t.n_groups)) || (rc = h->Bh.alloc(nb)) || (rc = h->Bl.alloc(nb)) ||
+          (rc = h->out_scale.alloc(dout)) || (rc = Bd.upload(B, st)))
         return rc;
+      cudaMemsetAsync(h->Bh.p, 0, nb * sizeof(uint16_t), st);
+      cudaMemsetAsync(h->Bl.p, 0, nb * sizeof(uint16_t), st);
+      if (h->K > 0 && (rc = smx_tensor_operands(Bd.p, dout, h->K, h->ldk, h->tape.p, h->tape_pad.p, h->Bh.p, h->Bl.p,
+                                                t.ldb, h->out_scale.p, stream)))
+        return rc;
+      t.dims = h->dims.p, t.dmax = h->dmax.p, t.dsoff = h->dsoff.p;
+      t.fam_a = h->fam_a.p, t.fam_b = h->fam_b.p, t.fam = h->fam.p, t.rec = h->rec.p;
+      t.tape = h->tape_pad.p, t.path = h->path.p, t.Bh = h->Bh.p, t.Bl = h->Bl.p;
+      t.out_scale = h->out_scale.p, t.bias = h->bias.p, t.err = h->err.p;
     }
     // segment bounds of the panel for every wanted count (spectral.py segment_bounds):
     // near-equal splits of the tape, every bound but the last at a depth-1 entry
@@ -603,10 +620,7 @@ extern "C" size_t smx_fp32_workspace(const smx_fp32_plan* h, int64_t P) {
   if (!h || P < 0) return 0;
   if (h->evaluator == SMX_FP32_BLOCKED) return smx_blocked_eval_workspace(&h->blocked, P);
   if (h->evaluator != SMX_FP32_TENSOR) return 0;
-  const int64_t step = tc_step(h, std::max<int64_t>(P, 1));
-  const size_t lda = size_t(round32(std::max(h->K, 1)));
-  return 2 * up(size_t(step) * lda * sizeof(float)) + up(smx_spectral_panel_workspace(h->n_slots, step)) +
-         (tc_splits(h) > 1 ? up(smx_gemm_tf32x3_splitk_workspace(int(step), h->d_out, h->K, tc_splits(h))) : 0);
+  return smx_tensor_workspace(&h->tensor, P);
 }
 
 extern "C" int smx_fp32_eval(const smx_fp32_plan* h, const double* x, int64_t P, int64_t ldx, float* y, void* ws,
@@ -618,33 +632,7 @@ extern "C" int smx_fp32_eval(const smx_fp32_plan* h, const double* x, int64_t P,
   SMX_REQUIRE(ws_bytes >= need && (ws || need == 0), "smx_fp32_eval: workspace too small");
   if (h->evaluator == SMX_FP32_BLOCKED) return smx_blocked_eval(&h->blocked, x, P, ldx, y, ws, ws_bytes, stream);
   if (h->evaluator == SMX_FP32_PERPOINT) return smx_spectral_eval(&h->spectral, x, P, ldx, y, stream);
-  // tensor core: per chunk of points a basis-product panel (TF32 hi/lo) and the contraction
-  const int64_t step = tc_step(h, P);
-  const int64_t lda = round32(std::max(h->K, 1));
-  uint8_t* w = static_cast<uint8_t*>(ws);
-  const size_t panel_bytes = up(size_t(step) * lda * sizeof(float));
-  float* Ah = reinterpret_cast<float*>(w);
-  float* Al = reinterpret_cast<float*>(w + panel_bytes);
-  const int splits = tc_splits(h);
-  const size_t sk_bytes = splits > 1 ? up(smx_gemm_tf32x3_splitk_workspace(int(step), h->d_out, h->K, splits)) : 0;
-  void* skws = w + 2 * panel_bytes;
-  void* pws = w + 2 * panel_bytes + sk_bytes;
-  const size_t pws_bytes = ws_bytes - 2 * panel_bytes - sk_bytes;
-  int rc;
-  for (int64_t p0 = 0; p0 < P; p0 += step) {
-    const int64_t m = std::min(step, P - p0);
-    const int want = seg_want(h, m);
-    const int n_seg = want <= 1 ? 1 : h->seg_n[want];
-    const int32_t* seg = want <= 1 ? nullptr : h->segs.p + h->seg_off[want];
-    if ((rc = smx_spectral_panel_tf32(h->n_dims, h->dims.p, h->dmax.p, h->dsoff.p, h->n_slots, h->tape.p, h->K, seg,
-                                      n_seg, h->fam_a.p, h->fam_b.p, h->fam.p, x + p0 * ldx, m, ldx, Ah, Al, lda, pws,
-                                      pws_bytes, stream)) ||
-        (rc = smx_gemm_tf32x3_splitk(Ah, Al, lda, h->Bh.p, h->Bl.p, h->ldk, int(m), h->d_out, h->K,
-                                     y + p0 * h->d_out, h->d_out, h->bias.p, 0, splits, skws, sk_bytes, h->err.p,
-                                     stream)))
-      return rc;
-  }
-  return SMX_OK;
+  return smx_tensor_eval(&h->tensor, x, P, ldx, y, ws, ws_bytes, stream);
 }
 
 extern "C" int smx_fp32_plan_check(const smx_fp32_plan* h, void* stream) {

@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "tc_util.cuh"
+#include "tensor_eval.h"
 
 namespace {
 
@@ -45,6 +46,7 @@ __device__ __forceinline__ uint64_t make_desc_k(uint32_t saddr) { return make_de
 // bound), 256 for the split-BF16 form, whose error the 16-bit split sets
 constexpr int kChunkTf32 = 64 / kBK;
 constexpr int kChunkBf16 = 256 / (2 * kBK);
+constexpr int kChunkF16 = 64 / (2 * kBK);  // scaled FP16: one row scale per 64 products
 
 template <int BN>
 struct Tile {
@@ -71,20 +73,26 @@ struct GemmArgs {
   int64_t zstride;  // split-K: floats between the slices' outputs
   uint64_t wait_ns; // bound on each pipeline wait (kWaitNs; shorter only in the self-test)
   int no_loads;     // self-test only: the producer issues no copies, so the first wait must time out
+  const float* row_scale;  // scaled FP16: [K-tile][ld_scale], by row
+  int64_t ld_scale;
+  const float* col_scale;  // scaled FP16: by column
 };
 
 constexpr int kEpiLd = 132;  // epilogue staging row stride (floats): 16-byte rows, conflict-free
 static_assert(Tile<128>::kDrainWarps * 32 * kEpiLd * 4 <= Tile<128>::kTiles, "epilogue staging must fit");
 static_assert(Tile<256>::kDrainWarps * 32 * kEpiLd * 4 <= Tile<256>::kTiles, "epilogue staging must fit");
 
-// BF16 = false: kind::tf32 on FP32 operands (32 per 128-byte slice); true:
-// kind::f16 on BF16 operands (64 per slice).  Same slices, stages and MMAs.
-template <bool BF16, int BN>
+// KIND kTf32: kind::tf32 on FP32 operands (32 per 128-byte slice); kBf16, kF16:
+// kind::f16 on 16-bit operands (64 per slice).  Same slices, stages and MMAs;
+// kF16 multiplies each drained accumulator by its row's scale of the slice and
+// the result by the column's.
+template <int KIND, int BN>
 __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                        const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, GemmArgs g) {
+  constexpr bool BF16 = KIND != kTf32;  // 16-bit operands
   constexpr int EK = BF16 ? 2 * kBK : kBK;  // elements per K-tile
-  constexpr int kChunk = BF16 ? kChunkBf16 : kChunkTf32;
+  constexpr int kChunk = KIND == kF16 ? kChunkF16 : BF16 ? kChunkBf16 : kChunkTf32;
   using L = Tile<BN>;
   constexpr int kBN = BN;
   constexpr int kStages = L::kStages;
@@ -156,7 +164,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     __syncwarp();
   } else if (warp == L::kWarpMMA) {
     if (lane == 0) {  // ---- MMA issuer
-      constexpr uint32_t idesc = idesc_mma(kBM, kBN, BF16);
+      constexpr uint32_t idesc = idesc_fmt(kBM, kBN, KIND == kTf32 ? 2u : KIND == kBf16 ? 1u : 0u);
       bool ok = true;
       int kt = 0;
       for (int c = 0; c < NCH && ok; ++c) {
@@ -217,8 +225,15 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     for (int j = 0; j < 128; ++j) acc[j] = 0.f;
     bool ok = true;
     const uint32_t lane_base = tmem + (uint32_t(quad * 32) << 16);
+    const float* rs = nullptr;  // this row's scale of the next slice
+    if constexpr (KIND == kF16) rs = g.row_scale + kt_base * g.ld_scale + min(m0 + quad * 32 + lane, g.M - 1);
     for (int c = 0; c < NCH; ++c) {
       const int b = c & 1;
+      float scale = 1.f;
+      if constexpr (KIND == kF16) {
+        scale = __ldg(rs);
+        rs += g.ld_scale;
+      }
       ok = __all_sync(0xffffffffu,
                       ok && mbar_wait(&acc_full[b], (c >> 1) & 1, abort_flag, g.wait_ns) && !*abort_flag);
       if (!ok) break;
@@ -234,7 +249,12 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
             : "r"(lane_base + uint32_t(b * kBN + cw + q)));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[q + j] += __uint_as_float(r[j]);
+        for (int j = 0; j < 16; ++j) {
+          if constexpr (KIND == kF16)
+            acc[q + j] = fmaf(scale, __uint_as_float(r[j]), acc[q + j]);
+          else
+            acc[q + j] += __uint_as_float(r[j]);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
@@ -255,11 +275,19 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
       float bv[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) bv[i] = g.bias && c0 + i < g.N ? g.bias[c0 + i] : 0.f;
+      float cs[4] = {1.f, 1.f, 1.f, 1.f};
+      if constexpr (KIND == kF16) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cs[i] = c0 + i < g.N ? g.col_scale[c0 + i] : 1.f;
+      }
       for (int r = 0; r < 32; ++r) {
         const int row = m0 + quad * 32 + r;
         if (row >= g.M) break;
         const float4 t = *reinterpret_cast<const float4*>(T + r * kEpiLd + 4 * lane);
         float v[4] = {t.x + bv[0], t.y + bv[1], t.z + bv[2], t.w + bv[3]};
+        if constexpr (KIND == kF16)
+          v[0] = fmaf(t.x, cs[0], bv[0]), v[1] = fmaf(t.y, cs[1], bv[1]), v[2] = fmaf(t.z, cs[2], bv[2]),
+          v[3] = fmaf(t.w, cs[3], bv[3]);
         float* dr = D + int64_t(row) * g.ldd + c0;
         if (vec) {
           if (g.accumulate) {
@@ -322,15 +350,18 @@ int get_encode() {
   return SMX_OK;
 }
 
-int make_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, bool bf16 = false) {
-  const int es = bf16 ? 2 : 4;
+int make_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, int kind = kTf32) {
+  const int es = kind == kTf32 ? 4 : 2;
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (ld * es) % 16)
     return smx::set_error(SMX_ERR_ARG, "tensor map: base must be 16-byte aligned and the row pitch a multiple of 16");
   cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
   cuuint64_t strides[1] = {cuuint64_t(ld * es)};
-  cuuint32_t box[2] = {cuuint32_t(bf16 ? 2 * kBK : kBK), cuuint32_t(box_rows)};
+  cuuint32_t box[2] = {cuuint32_t(kRowBytes / es), cuuint32_t(box_rows)};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+  const CUtensorMapDataType type = kind == kTf32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                   : kind == kBf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                   : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUresult r = g_encode(tm, type, 2,
                         const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         kRowBytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -338,44 +369,46 @@ int make_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64
   return SMX_OK;
 }
 
-template <bool BF16, int BN>
+template <int KIND, int BN>
 int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, const void* Bl, int64_t ldb, int M,
                 int N, int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
-                int splits, uint64_t wait_ns, int no_loads) {
+                int splits, uint64_t wait_ns, int no_loads, const SplitGemm* sc) {
   using L = Tile<BN>;
   CUtensorMap tBh, tBl;
   int rc;
-  if ((rc = make_map(&tBh, Bh, N, K, ldb, BN, BF16)) || (rc = make_map(&tBl, Bl, N, K, ldb, BN, BF16))) return rc;
+  if ((rc = make_map(&tBh, Bh, N, K, ldb, BN, KIND)) || (rc = make_map(&tBl, Bl, N, K, ldb, BN, KIND))) return rc;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(gemm_tf32x3_kernel<BF16, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
+    cudaFuncSetAttribute(gemm_tf32x3_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
     attr = true;
   }
   // split-K: slice z runs K-tiles [z * kt_per_z, ...) into D + z * zstride
-  const int EK = BF16 ? 2 * kBK : kBK;
+  const int EK = KIND != kTf32 ? 2 * kBK : kBK;
   const int KT = (K + EK - 1) / EK;
   const int kt_per_z = splits > 1 ? (KT + splits - 1) / splits : 0;
   const int nz = splits > 1 ? (KT + kt_per_z - 1) / kt_per_z : 1;
-  GemmArgs g{M, N, K, D, ldd, bias, err, accumulate, kt_per_z, int64_t(M) * ldd, wait_ns, no_loads};
+  GemmArgs g{M,       N,        K,       D,      ldd, bias, err, accumulate, kt_per_z, int64_t(M) * ldd,
+             wait_ns, no_loads, nullptr, 0,      nullptr};
+  if (sc) g.row_scale = sc->row_scale, g.ld_scale = sc->ld_scale, g.col_scale = sc->col_scale;
   dim3 grid((N + BN - 1) / BN, (M + kBM - 1) / kBM, nz);
-  gemm_tf32x3_kernel<BF16, BN><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
-  SMX_LAUNCH_CHECK(BF16 ? "smx_gemm_bf16x3" : "smx_gemm_tf32x3");
+  gemm_tf32x3_kernel<KIND, BN><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
+  SMX_LAUNCH_CHECK(KIND == kTf32 ? "smx_gemm_tf32x3" : KIND == kBf16 ? "smx_gemm_bf16x3" : "smx_tensor_eval");
   return SMX_OK;
 }
 
 // Products wider than 192 columns use 128 x 256 tiles, the others 128 x 128.
-template <bool BF16>
+template <int KIND>
 int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const void* Bl, int64_t ldb, int M, int N,
            int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
-           int splits = 1, uint64_t wait_ns = kWaitNs, int no_loads = 0) {
+           int splits = 1, uint64_t wait_ns = kWaitNs, int no_loads = 0, const SplitGemm* sc = nullptr) {
   CUtensorMap tAh, tAl;
   int rc;
-  if ((rc = make_map(&tAh, Ah, M, K, lda, kBM, BF16)) || (rc = make_map(&tAl, Al, M, K, lda, kBM, BF16))) return rc;
+  if ((rc = make_map(&tAh, Ah, M, K, lda, kBM, KIND)) || (rc = make_map(&tAl, Al, M, K, lda, kBM, KIND))) return rc;
   if (N > 192)
-    return launch_tile<BF16, 256>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
-                                  no_loads);
-  return launch_tile<BF16, 128>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
-                                no_loads);
+    return launch_tile<KIND, 256>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
+                                  no_loads, sc);
+  return launch_tile<KIND, 128>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
+                                no_loads, sc);
 }
 
 // ---- BF16 split: hi = x rounded to BF16 (round to nearest even), lo = BF16(x - hi)
@@ -418,7 +451,7 @@ extern "C" int smx_gemm_tf32x3(const float* A_hi, const float* A_lo, int64_t lda
   SMX_REQUIRE(K >= 1 && A_hi && A_lo && B_hi && B_lo && D && err, "smx_gemm_tf32x3: null pointer");
   int rc = get_encode();
   if (rc) return rc;
-  return launch<false>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, D, ldd, bias, err, accumulate,
+  return launch<kTf32>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, D, ldd, bias, err, accumulate,
                        smx::as_stream(stream));
 }
 
@@ -436,7 +469,7 @@ extern "C" int smx_gemm_tf32x3_timeout_selftest(const float* A_hi, const float* 
   SMX_REQUIRE(wait_ns <= kWaitNs, "smx_gemm_tf32x3_timeout_selftest: wait bound above the default");
   int rc = get_encode();
   if (rc) return rc;
-  return launch<false>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, D, ldd, nullptr, err, 0, smx::as_stream(stream), 1,
+  return launch<kTf32>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, D, ldd, nullptr, err, 0, smx::as_stream(stream), 1,
                        wait_ns, 1);
 }
 
@@ -448,7 +481,7 @@ extern "C" int smx_gemm_bf16x3(const uint16_t* A_hi, const uint16_t* A_lo, int64
   SMX_REQUIRE(K >= 1 && A_hi && A_lo && B_hi && B_lo && D && err, "smx_gemm_bf16x3: null pointer");
   int rc = get_encode();
   if (rc) return rc;
-  return launch<true>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, D, ldd, bias, err, accumulate,
+  return launch<kBf16>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, D, ldd, bias, err, accumulate,
                       smx::as_stream(stream));
 }
 
@@ -508,11 +541,45 @@ extern "C" int smx_gemm_tf32x3_splitk(const float* A_hi, const float* A_lo, int6
   if (rc) return rc;
   cudaStream_t st = smx::as_stream(stream);
   float* part = static_cast<float*>(ws);
-  rc = launch<false>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, part, N, nullptr, err, 0, st, splits);
+  rc = launch<kTf32>(A_hi, A_lo, lda, B_hi, B_lo, ldb, M, N, K, part, N, nullptr, err, 0, st, splits);
   if (rc) return rc;
   splitk_reduce_kernel<<<smx::grid_for(int64_t(M) * N, 256), 256, 0, st>>>(part, splitk_slices(K, splits), M, N, D,
                                                                           ldd, bias, accumulate);
   SMX_LAUNCH_CHECK("smx_gemm_tf32x3_splitk");
+  return SMX_OK;
+}
+
+int smx::tc::panel_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows,
+                       int bits) {
+  const int rc = get_encode();
+  return rc ? rc : make_map(tm, ptr, rows, cols, ld, box_rows, bits);
+}
+
+int smx::tc::split_gemm(const SplitGemm& g, cudaStream_t st) {
+  int rc = get_encode();
+  if (rc) return rc;
+  if (g.K == 0 || g.splits <= 1) {
+    if (g.K == 0) {  // the constant alone
+      splitk_reduce_kernel<<<smx::grid_for(int64_t(g.M) * g.N, 256), 256, 0, st>>>(nullptr, 0, g.M, g.N, g.D, g.ldd,
+                                                                                  g.bias, 0);
+      SMX_LAUNCH_CHECK("smx_tensor_eval");
+      return SMX_OK;
+    }
+    return g.bits == kF16 ? launch<kF16>(g.Ah, g.Al, g.lda, g.Bh, g.Bl, g.ldb, g.M, g.N, g.K, g.D, g.ldd, g.bias,
+                                         g.err, 0, st, 1, kWaitNs, 0, &g)
+                          : launch<kBf16>(g.Ah, g.Al, g.lda, g.Bh, g.Bl, g.ldb, g.M, g.N, g.K, g.D, g.ldd, g.bias,
+                                          g.err, 0, st);
+  }
+  const int kt = (g.K + 2 * kBK - 1) / (2 * kBK), per = (kt + g.splits - 1) / g.splits;
+  const int slices = (kt + per - 1) / per;
+  rc = g.bits == kF16 ? launch<kF16>(g.Ah, g.Al, g.lda, g.Bh, g.Bl, g.ldb, g.M, g.N, g.K, g.partial, g.N, nullptr,
+                                     g.err, 0, st, g.splits, kWaitNs, 0, &g)
+                      : launch<kBf16>(g.Ah, g.Al, g.lda, g.Bh, g.Bl, g.ldb, g.M, g.N, g.K, g.partial, g.N, nullptr,
+                                      g.err, 0, st, g.splits);
+  if (rc) return rc;
+  splitk_reduce_kernel<<<smx::grid_for(int64_t(g.M) * g.N, 256), 256, 0, st>>>(g.partial, slices, g.M, g.N, g.D,
+                                                                              g.ldd, g.bias, 0);
+  SMX_LAUNCH_CHECK("smx_tensor_eval");
   return SMX_OK;
 }
 

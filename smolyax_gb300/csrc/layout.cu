@@ -1077,12 +1077,23 @@ bool build_tape(const Tree& tr, const int64_t* maxdeg, int d, Tables& out) {
     ent32.push_back(int32_t(e));
     if (tr.level[e] == 1) lvl1.push_back(int32_t(i));
   }
+  // slots above the first entry of every group of 64 tape entries (the tape
+  // padded in front to whole groups)
+  const size_t pad = (64 - ent.size() % 64) % 64, n_groups = (ent.size() + 63) / 64;
+  std::vector<int32_t> path(n_groups * 8, -1), above(9, -1);
+  for (size_t i = 0; i < ent.size(); ++i) {
+    const int depth = int(tr.level[ent[i]]);
+    if ((pad + i) % 64 == 0)
+      for (int q = 1; q < depth; ++q) path[(pad + i) / 64 * 8 + q - 1] = above[q];
+    above[depth] = tape[i] & 0xffff;
+  }
   out.i32["dims"] = dims;
   out.i32["dmax"] = dmax;
   out.i32["dsoff"] = dsoff;
   out.i32["tape"] = tape;
   out.i32["ent"] = ent32;
   out.i32["lvl1"] = lvl1;
+  out.i32["path"] = path;
   out.scalar["n_slots"] = double(n_slots);
   out.scalar["K"] = double(ent.size());
   out.scalar["ldk"] = double(round32(std::max<int64_t>(int64_t(ent.size()), 1)));

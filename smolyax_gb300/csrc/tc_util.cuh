@@ -99,12 +99,12 @@ __device__ __forceinline__ uint64_t make_desc_sw(uint32_t saddr, int row_bytes) 
   return d;
 }
 
-// Instruction descriptor: D = F32, A = B = TF32 (kind::tf32, format 2) or
-// BF16 (kind::f16, format 1), both K-major, M x N.
-__host__ __device__ constexpr uint32_t idesc_mma(int M, int N, bool bf16) {
-  return (1u << 4) | ((bf16 ? 1u : 2u) << 7) | ((bf16 ? 1u : 2u) << 10) | (uint32_t(N >> 3) << 17) |
-         (uint32_t(M >> 4) << 24);
+// Instruction descriptor: D = F32, A = B = TF32 (kind::tf32, format 2), BF16
+// (kind::f16, format 1) or FP16 (kind::f16, format 0), both K-major, M x N.
+__host__ __device__ constexpr uint32_t idesc_fmt(int M, int N, uint32_t fmt) {
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
+__host__ __device__ constexpr uint32_t idesc_mma(int M, int N, bool bf16) { return idesc_fmt(M, N, bf16 ? 1u : 2u); }
 
 template <bool BF16>
 __device__ __forceinline__ void mma_op(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,

@@ -224,30 +224,79 @@ class SpectralPlan:
         if d_out > 1 and self.tc is None:
             self.stream_keep = stream_tables(self.c, tree_np, C32, d_out, np.asarray(ip._maxdeg), fam, fa, fb, T, False)
 
-    def _build_tc(self, tr, C32, maxdeg, fam, fa, fb, T, st):
-        """Operands of the tensor-core contraction: tape over all non-root entries
-        (pre-order), coefficient matrix B = C^T split into TF32 hi/lo."""
-        self.tree_np, self.maxdeg = tr, maxdeg
-        tp = build_tape(tr, maxdeg)
+    def _build_tape(self, tr, C32, maxdeg, fam, fa, fb, T, st):
+        """Tape over all non-root entries (pre-order) for the tensor-core
+        evaluation and the backward, or None (entries deeper than 8: the panel's
+        product stack)."""
+        tp = capi.host_layout("tape", tr, None, int(C32.shape[1]), maxdeg, fam, fa, fb,
+                              i32=("dims", "dmax", "dsoff", "tape", "ent", "lvl1", "path"), scalars=("n_slots",))
         if tp is None:
+            return None
+        dev = self.fam.device
+        K = int(tp["ent"].size)
+        return dict(dims=T(tp["dims"], torch.int32), dmax=T(tp["dmax"], torch.int32),
+                    dsoff=T(tp["dsoff"], torch.int32), n_slots=int(tp["n_slots"]), tape=T(tp["tape"], torch.int32),
+                    path=T(tp["path"], torch.int32), K=K, ldk=_round32(max(K, 1)),
+                    max_deg=max(1, int(np.max(tp["dmax"], initial=1))), bias=self.keep["c0"],
+                    err=torch.zeros(1, dtype=torch.int32, device=dev),
+                    ent=torch.as_tensor(tp["ent"].astype(np.int64), device=dev), ent_h=tp["ent"].astype(np.int64),
+                    # tape positions of the depth-1 entries: where independent segments may start
+                    lvl1=tp["lvl1"].astype(np.int64),
+                    sms=torch.cuda.get_device_properties(dev).multi_processor_count)
+
+    def _build_tc(self, tr, C32, maxdeg, fam, fa, fb, T, st):
+        """Operands of the tensor-core evaluation: the tape and the coefficient
+        matrix B = C^T in the panel's column order."""
+        tc = self._build_tape(tr, C32, maxdeg, fam, fa, fb, T, st)
+        if tc is None:
             return  # the FP32 stream evaluator serves this plan
-        dims, dmax, dsoff, n_slots, tape, ent = (tp[key] for key in ("dims", "dmax", "dsoff", "n_slots", "tape", "ent"))
-        K = int(ent.size)
-        ldk = _round32(max(K, 1))  # 128-byte rows: whole cache lines per TMA row of B
+        K, ldk = tc["K"], tc["ldk"]
         d_out = C32.shape[1]
         B = np.zeros((d_out, ldk), dtype=np.float32)
-        B[:, :K] = C32[ent[::-1]].T  # the panel stores the entries in reversed pre-order
-        dev = self.fam.device
-        Bd = T(B, torch.float32)
-        Bh, Bl = torch.empty_like(Bd), torch.empty_like(Bd)
-        call("smx_split_tf32", ptr(Bd), d_out, ldk, ldk, ptr(Bh), ptr(Bl), ldk, st)
-        self.tc = dict(dims=T(dims, torch.int32), dmax=T(dmax, torch.int32), dsoff=T(dsoff, torch.int32),
-                       n_slots=n_slots, tape=T(tape, torch.int32), K=K, ldk=ldk, Bh=Bh, Bl=Bl, Bd=Bd,
-                       bias=self.keep["c0"], err=torch.zeros(1, dtype=torch.int32, device=dev),
-                       ent=torch.as_tensor(ent, device=dev),
-                       # tape positions of the depth-1 entries: where independent segments may start
-                       lvl1=np.nonzero(tr["level"][ent] == 1)[0],
-                       sms=torch.cuda.get_device_properties(dev).multi_processor_count)
+        B[:, :K] = C32[tc["ent_h"][::-1]].T  # the panel stores the entries in reversed pre-order
+        tc["Bd"] = T(B, torch.float32)
+        m = np.arange(tc["max_deg"])
+        tc["rec"] = T(np.stack([np.stack([(2 * m + 1) / (m + 1), m / (m + 1)], axis=1),
+                                np.stack([np.sqrt(2.0 / (m + 1)), np.sqrt(m / (m + 1))], axis=1)]), torch.float32)
+        self.tc = tc
+
+    def _tc_struct(self, bf16=False):
+        """``smx_tensor`` of the plan: FP16 operands with scales, or the BF16
+        operands of ``mode="bf16x3"`` (each built on first use)."""
+        tc = self.tc
+        key = "bf16" if bf16 else "f16"
+        if key not in tc:
+            Bd = tc["Bd"]
+            d_out, K = int(Bd.shape[0]), tc["K"]
+            n_groups = (K + 63) // 64
+            ldb = max(64, 64 * n_groups)
+            dev = Bd.device
+            st = capi.stream_ptr(torch.cuda.current_stream())
+            k = dict(Bh=torch.zeros(d_out, ldb, dtype=torch.bfloat16 if bf16 else torch.float16, device=dev))
+            k["Bl"] = torch.zeros_like(k["Bh"])
+            k["tape"] = torch.zeros(2 * 64 * n_groups, dtype=torch.int32, device=dev)
+            if bf16:
+                if K:
+                    call("smx_tensor_tape", ptr(tc["tape"]), K, ptr(k["tape"]), st)
+                    call("smx_split_bf16", ptr(Bd), d_out, K, tc["ldk"], ptr(k["Bh"]), ptr(k["Bl"]), ldb, st)
+            else:
+                k["out_scale"] = torch.ones(d_out, dtype=torch.float32, device=dev)
+                if K:
+                    call("smx_tensor_operands", ptr(Bd), d_out, K, tc["ldk"], ptr(tc["tape"]), ptr(k["tape"]),
+                         ptr(k["Bh"]), ptr(k["Bl"]), ldb, ptr(k["out_scale"]), st)
+            s = capi.SmxTensor()
+            s.d_in, s.d_out = int(self.c.d_in), d_out
+            s.n_dims, s.n_slots, s.max_deg = int(tc["dims"].numel()), tc["n_slots"], tc["max_deg"]
+            s.K, s.n_groups, s.bf16 = K, n_groups, int(bf16)
+            s.splits, s.chunk, s.ldb = self.tc_splits(), self._tc_step(1 << 40), ldb
+            for name in ("dims", "dmax", "dsoff", "path", "rec", "bias", "err"):
+                setattr(s, name, tc[name].data_ptr())
+            for name in ("fam_a", "fam_b", "fam"):
+                setattr(s, name, self.keep[name].data_ptr())
+            for name, t in k.items():
+                setattr(s, name, t.data_ptr())
+            tc[key] = (s, k)
+        return tc[key][0]
 
     def _build_blocked(self, tr, c, maxdeg, d, fam, fa, fb, T):
         """Tables of the blocked evaluator (one output), if the plan fits it."""
@@ -309,10 +358,7 @@ class SpectralPlan:
         """Tape operands (built as for the forward tensor-core path) plus the
         coefficient rows C[K x ldo] in the panel's reversed order, TF32 hi/lo."""
         if self._bwd is None:
-            fwd_tc = self.tc
-            self._build_tc(*self._fwd_args)
-            ops = self.tc
-            self.tc = fwd_tc
+            ops = dict(self.tc) if self.tc is not None else self._build_tape(*self._fwd_args)
             if ops is None:
                 raise RuntimeError("backward needs Smolyak index depth <= 8 (register product stack)")
             T = self._fwd_args[6]
@@ -321,7 +367,7 @@ class SpectralPlan:
             K = ops["K"]
             d_out = C32.shape[1]
             ldo = _round4(d_out)
-            ent = ops["ent"].cpu().numpy()
+            ent = ops["ent_h"]
             rows = np.zeros((max(K, 1), ldo), dtype=np.float32)
             rows[:K, :d_out] = C32[ent[::-1]]
             Rd = T(rows, torch.float32)
@@ -506,17 +552,15 @@ class SpectralPlan:
         return y
 
     def _tc_step(self, P):
-        """Points per panel chunk (the hi/lo panel of one chunk fits the memory limit)."""
-        step = max(128, int(self.memory_limit * 1024**3 // (8 * ((self.tc["K"] + 31) // 32 * 32))) // 128 * 128)
+        """Points per panel chunk (the 16-bit hi/lo panel of one chunk fits the memory limit)."""
+        step = max(128, int(self.memory_limit * 1024**3 // (4 * max(64, (self.tc["K"] + 63) // 64 * 64))) // 128 * 128)
         return max(1, min(step, P))
 
     def tc_splits(self):
-        """K slices of the forward contraction (``smx_gemm_tf32x3_splits`` for a
-        full panel chunk): a plan constant, so a point's value does not depend
-        on the batch it arrives in."""
+        """K slices of the forward contraction (``smx_tensor_splits``): a plan
+        constant, so a point's value does not depend on the batch it arrives in."""
         if "splits" not in self.tc:
-            self.tc["splits"] = capi.size("smx_gemm_tf32x3_splits", self._tc_step(1 << 40),
-                                          int(self.tc["Bd"].shape[0]), self.tc["K"])
+            self.tc["splits"] = capi.size("smx_tensor_splits", int(self.tc["Bd"].shape[0]), self.tc["K"])
         return self.tc["splits"]
 
     def tc_chunks(self, P):
@@ -525,10 +569,8 @@ class SpectralPlan:
 
     def tc_launches(self, P):
         """Kernel launches of one tensor-core evaluation of P points: per chunk the
-        panel (plus its basis-row kernel when the rows go to global scratch) and
-        the GEMM."""
-        scratch = capi.size("smx_spectral_panel_workspace", self.tc["n_slots"], 1) > 0
-        return self.tc_chunks(P) * ((3 if scratch else 2) + (1 if self.tc_splits() > 1 else 0))
+        basis rows, the panel and the contraction, and the sum of its K slices."""
+        return self.tc_chunks(P) * (3 + (1 if self.tc_splits() > 1 else 0))
 
     def _segments(self, n):
         """Tape segments of one panel launch over n points (see segment_bounds).
@@ -543,70 +585,22 @@ class SpectralPlan:
         t = cache[want]
         return t, int(t.numel()) - 1
 
-    def _bf16_operands(self):
-        """Coefficient matrix B split to BF16 hi/lo (built on first use), rows
-        padded to 64 entries (128 bytes)."""
-        tc = self.tc
-        if "Bh16" not in tc:
-            d_out, K = int(tc["Bd"].shape[0]), tc["K"]
-            ld16 = (K + 63) // 64 * 64
-            Bh = torch.zeros(d_out, ld16, dtype=torch.bfloat16, device=tc["Bd"].device)
-            Bl = torch.zeros_like(Bh)
-            call("smx_split_bf16", ptr(tc["Bd"]), d_out, K, tc["ldk"], ptr(Bh), ptr(Bl), ld16,
-                 capi.stream_ptr(torch.cuda.current_stream()))
-            tc.update(Bh16=Bh, Bl16=Bl, ld16=ld16)
-        return tc["Bh16"], tc["Bl16"], tc["ld16"]
+    def tc_workspace(self, P):
+        """Device bytes of scratch of one tensor-core evaluation of P points."""
+        import ctypes
+
+        return capi.size("smx_tensor_workspace", ctypes.byref(self._tc_struct()), int(P))
 
     def _evaluate_tc(self, x, y, st, bf16=False):
-        """Tensor-core path: basis-product panel (TF32 or BF16 hi/lo) in chunks
-        of points, each contracted with the coefficient matrix by the tcgen05
-        kernel."""
-        tc = self.tc
-        k = self.keep
-        P, d = int(x.shape[0]), int(x.shape[1])
-        d_out = int(y.shape[1])
-        if bf16:
-            Bh, Bl, ld16 = self._bf16_operands()
-            step = self._tc_step(P)
-            lda = (tc["K"] + 63) // 64 * 64  # 128-byte panel rows
-            Ah = torch.empty(step, lda, dtype=torch.bfloat16, device=x.device)
-            Al = torch.empty_like(Ah)
-            for p0 in range(0, P, step):
-                p1 = min(P, p0 + step)
-                nws = capi.size("smx_spectral_panel_workspace", tc["n_slots"], p1 - p0)
-                ws = torch.empty(max(nws, 1), dtype=torch.uint8, device=x.device)
-                seg, n_seg = self._segments(p1 - p0)
-                call("smx_spectral_panel_bf16", int(tc["dims"].numel()), ptr(tc["dims"]), ptr(tc["dmax"]),
-                     ptr(tc["dsoff"]), tc["n_slots"], ptr(tc["tape"]), tc["K"], ptr(seg), n_seg, ptr(k["fam_a"]),
-                     ptr(k["fam_b"]), ptr(k["fam"]), ptr(x[p0:p1]), p1 - p0, d, ptr(Ah), ptr(Al), lda, ptr(ws), nws,
-                     st)
-                call("smx_gemm_bf16x3", ptr(Ah), ptr(Al), lda, ptr(Bh), ptr(Bl), ld16, p1 - p0, d_out, tc["K"],
-                     ptr(y[p0:p1]), d_out, ptr(tc["bias"]), 0, ptr(tc["err"]), st)
-            return y
-        ldk = tc["ldk"]
-        step = self._tc_step(P)
-        lda = (tc["K"] + 31) // 32 * 32  # 128-byte panel rows
-        Ah = torch.empty(step, lda, dtype=torch.float32, device=x.device)
-        Al = torch.empty_like(Ah)
-        splits = self.tc_splits()
-        if splits > 1:
-            nsk = capi.size("smx_gemm_tf32x3_splitk_workspace", step, d_out, tc["K"], splits)
-            skws = torch.empty(max(nsk, 1), dtype=torch.uint8, device=x.device)
-        for p0 in range(0, P, step):
-            p1 = min(P, p0 + step)
-            nws = capi.size("smx_spectral_panel_workspace", tc["n_slots"], p1 - p0)
-            ws = torch.empty(max(nws, 1), dtype=torch.uint8, device=x.device)
-            seg, n_seg = self._segments(p1 - p0)
-            call("smx_spectral_panel_tf32", int(tc["dims"].numel()), ptr(tc["dims"]), ptr(tc["dmax"]),
-                 ptr(tc["dsoff"]), tc["n_slots"], ptr(tc["tape"]), tc["K"], ptr(seg), n_seg, ptr(k["fam_a"]),
-                 ptr(k["fam_b"]), ptr(k["fam"]), ptr(x[p0:p1]), p1 - p0, d, ptr(Ah), ptr(Al), lda, ptr(ws), nws, st)
-            if splits > 1:
-                call("smx_gemm_tf32x3_splitk", ptr(Ah), ptr(Al), lda, ptr(tc["Bh"]), ptr(tc["Bl"]), ldk, p1 - p0,
-                     d_out, tc["K"], ptr(y[p0:p1]), d_out, ptr(tc["bias"]), 0, splits, ptr(skws), nsk, ptr(tc["err"]),
-                     st)
-            else:
-                call("smx_gemm_tf32x3", ptr(Ah), ptr(Al), lda, ptr(tc["Bh"]), ptr(tc["Bl"]), ldk, p1 - p0, d_out,
-                     tc["K"], ptr(y[p0:p1]), d_out, ptr(tc["bias"]), 0, ptr(tc["err"]), st)
+        """Tensor-core path: basis-product panel (16-bit hi/lo) in chunks of
+        points, each contracted with the coefficient matrix (``smx_tensor_eval``)."""
+        import ctypes
+
+        ref = ctypes.byref(self._tc_struct(bf16))
+        P = int(x.shape[0])
+        nws = capi.size("smx_tensor_workspace", ref, P)
+        ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=x.device)
+        call("smx_tensor_eval", ref, ptr(x), P, int(x.shape[1]), ptr(y), ptr(ws), nws, st)
         return y
 
 
