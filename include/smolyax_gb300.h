@@ -707,6 +707,49 @@ size_t smx_tensor_workspace(const smx_tensor* plan_host, int64_t P);
 int smx_tensor_eval(const smx_tensor* plan_host, const double* x, int64_t P, int64_t ldx, float* y, void* ws,
                     size_t ws_bytes, void* stream);
 
+/* Tables of the gradient walk (device pointers; SMX_LAYOUT_WALK, table names w_perm, w_off,
+ * ...).  With V_n the product of node n's path, G_e the adjoint of entry e's product:
+ *   bar[s] = sum over entries with last slot s of V_parent G
+ *          + sum over nodes with s on their path of S_n times the other factors
+ *   S_n    = sum over node n's children of phi G
+ * The rows of a block of 32 points (128 bytes each) are phi [n_slots], V [n_nodes], bar
+ * [n_slots], S [n_nodes] and one for padding; G comes in chunks of `chunk` entries in the
+ * order `perm` (-1: no entry).  A term {source row | destination row << 16, byte offset
+ * of the entry in the chunk} adds source * G to the destination; terms come in pairs of
+ * different destinations, at most `most` per chunk. */
+typedef struct smx_walk {
+  int32_t n_nodes, n_chunks, chunk, most;
+  const int32_t* off;        /* [n_chunks][33] first term of each warp, and the end      */
+  const int32_t* term;       /* [..][2], 16-byte aligned                                 */
+  const int32_t* node_path;  /* [n_nodes][4] 8 uint16 slots, 0xffff past the last        */
+  const int32_t* slot;       /* [n_slots][4] {slot, first, end, 0} by warp, 16-byte aligned */
+  const int32_t* warp;       /* [33] first slot entry of each warp                       */
+  const int32_t* row;        /* path factors: row of S, and 8 uint16 other slots         */
+  const int32_t* other;
+  const int32_t* dim_index;  /* [d_in] position of a dimension in smx_tensor.dims, or -1 */
+} smx_walk;
+
+/* Operands of the backward: rows of C / scale in the walk's order as FP16 pairs with a
+ * scale per row and group of 64 outputs. */
+typedef struct smx_tensor_bwd {
+  int64_t n_rows;            /* walk.n_chunks * walk.chunk                              */
+  int64_t ldo;               /* pitch of Rh, Rl: d_out rounded up to 64                 */
+  int64_t chunk;             /* points per pass: 4 (n_rows + 2 n_slots) bytes a point   */
+  const uint16_t* Rh;        /* [n_rows][ldo]                                           */
+  const uint16_t* Rl;
+  const float* row_scale;    /* [ldo / 64][n_rows]                                      */
+  const float* out_scale;    /* [d_out]                                                 */
+  smx_walk walk;
+} smx_tensor_bwd;
+/* From FP32 coefficient rows C[n_rows][d_out]. */
+int smx_tensor_bwd_operands(const float* C, int64_t n_rows, int d_out, int64_t ldo, uint16_t* R_hi, uint16_t* R_lo,
+                            float* row_scale, float* out_scale, void* stream);
+size_t smx_tensor_vjp_x_workspace(const smx_tensor* plan_host, const smx_tensor_bwd* bwd_host, int64_t P);
+/* dx[p][j] = sum_o g[p][o] dy_o/dx_j (FP64, all d_in columns written) at cotangent g [P, d_out]. */
+int smx_tensor_vjp_x(const smx_tensor* plan_host, const smx_tensor_bwd* bwd_host, const double* x, int64_t P,
+                     int64_t ldx, const float* g, int64_t ldg, double* dx, int64_t lddx, void* ws, size_t ws_bytes,
+                     void* stream);
+
 /* ---- host-side layout builders of the FP32 evaluators ------------------------------
  * The tables of the blocked one-output evaluator (smx_blocked), of the
  * per-point evaluator (smx_spectral) and the entry tape of the tensor-core
@@ -725,6 +768,7 @@ int smx_tensor_eval(const smx_tensor* plan_host, const double* x, int64_t P, int
 #define SMX_LAYOUT_TAPE 2
 #define SMX_LAYOUT_BLOCKED_TC 3
 #define SMX_LAYOUT_STREAM 4
+#define SMX_LAYOUT_WALK 5
 typedef struct smx_host_tables smx_host_tables;
 int smx_layout_build(int kind, int64_t n, const int32_t* parent_host, const int32_t* dim_host,
                      const int32_t* deg_host, const int32_t* level_host, const int64_t* rank_host,

@@ -195,6 +195,40 @@ class SmxTensor(C.Structure):
     ]
 
 
+class SmxWalk(C.Structure):
+    """Mirror of ``struct smx_walk``."""
+
+    _fields_ = [
+        ("n_nodes", _i32),
+        ("n_chunks", _i32),
+        ("chunk", _i32),
+        ("most", _i32),
+        ("off", _p),
+        ("term", _p),
+        ("node_path", _p),
+        ("slot", _p),
+        ("warp", _p),
+        ("row", _p),
+        ("other", _p),
+        ("dim_index", _p),
+    ]
+
+
+class SmxTensorBwd(C.Structure):
+    """Mirror of ``struct smx_tensor_bwd``."""
+
+    _fields_ = [
+        ("n_rows", _i64),
+        ("ldo", _i64),
+        ("chunk", _i64),
+        ("Rh", _p),
+        ("Rl", _p),
+        ("row_scale", _p),
+        ("out_scale", _p),
+        ("walk", SmxWalk),
+    ]
+
+
 class SmxJacobian64(C.Structure):
     """Mirror of ``struct smx_jacobian64``."""
 
@@ -337,6 +371,9 @@ SIGNATURES = {
     "smx_tensor_splits": (_int, [_int, _int]),
     "smx_tensor_operands": (_int, [_p, _int, _int, _i64, _p, _p, _p, _p, _i64, _p, _p]),
     "smx_tensor_tape": (_int, [_p, _int, _p, _p]),
+    "smx_tensor_bwd_operands": (_int, [_p, _i64, _int, _i64, _p, _p, _p, _p, _p]),
+    "smx_tensor_vjp_x_workspace": (_sz, [_p, _p, _i64]),
+    "smx_tensor_vjp_x": (_int, [_p, _p, _p, _i64, _i64, _p, _i64, _p, _i64, _p, _sz, _p]),
     "smx_tensor_workspace": (_sz, [_p, _i64]),
     "smx_tensor_eval": (_int, [_p, _p, _i64, _i64, _p, _p, _sz, _p]),
     "smx_spectral_panel_workspace": (_sz, [_int, _i64]),
@@ -432,7 +469,7 @@ def stream_ptr(stream):
     return C.c_void_p(stream.cuda_stream) if stream is not None else None
 
 
-LAYOUT_KINDS = {"blocked": 0, "perpoint": 1, "tape": 2, "blocked_tc": 3, "stream": 4}
+LAYOUT_KINDS = {"blocked": 0, "perpoint": 1, "tape": 2, "blocked_tc": 3, "stream": 4, "walk": 5}
 
 
 def host_layout(kind, tree, coef, d_out, maxdeg, fam, fa, fb, i32=(), f32=(), scalars=(), fp64=False):

@@ -271,6 +271,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
         *reinterpret_cast<float4*>(T + lane * kEpiLd + q) = make_float4(acc[q], acc[q + 1], acc[q + 2], acc[q + 3]);
       __syncwarp();
       const int c0 = n0 + cw + 4 * lane;
+      const bool blocked = KIND == kF16 && g.ldd == 0;  // D is [N / 32][M][32]
       const bool vec = (g.ldd % 4) == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0 && c0 + 3 < g.N;
       float bv[4];
 #pragma unroll
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
         if constexpr (KIND == kF16)
           v[0] = fmaf(t.x, cs[0], bv[0]), v[1] = fmaf(t.y, cs[1], bv[1]), v[2] = fmaf(t.z, cs[2], bv[2]),
           v[3] = fmaf(t.w, cs[3], bv[3]);
-        float* dr = D + int64_t(row) * g.ldd + c0;
+        float* dr = blocked ? D + (int64_t(c0 >> 5) * g.M + row) * 32 + (c0 & 31) : D + int64_t(row) * g.ldd + c0;
         if (vec) {
           if (g.accumulate) {
             const float4 o = *reinterpret_cast<const float4*>(dr);

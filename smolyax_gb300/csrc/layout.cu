@@ -9,6 +9,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -1048,6 +1049,169 @@ template bool build_stream<float>(const Tree&, const float*, int, const int64_t*
 template bool build_stream<double>(const Tree&, const double*, int, const int64_t*, int, const int32_t*, const double*,
                                    const double*, Tables&);
 
+// Gradient walk (tensor_vjp.cu).  With V_n the product of node n's path (nodes:
+// entries with children), G_e the adjoint of entry e's product and s(e) its
+// last slot, the adjoint of a slot's basis value is
+//   bar[s] = sum over e with s(e) = s of V_parent(e) G_e
+//          + sum over nodes n with s on their path of S_n prod of the others
+//   S_n    = sum over the children c of n of phi_s(c) G_c
+// The adjoints stream through shared memory in chunks of E entries; a term adds
+// row value * G to a destination row (bar of a slot, S of a node), and every
+// destination belongs to one of 32 warps, longest first.  The entries are dealt
+// to the chunks in turn in the order of (slot, parent), so that each chunk holds
+// its share of every destination and the warps stay together.
+bool build_walk(const Tree& tr, const int64_t* maxdeg, int d, Tables& out) {
+  constexpr int kW = 32;
+  std::vector<int64_t> idx(d, -1), dsoff;
+  int64_t n_dims = 0, n_slots = 0;
+  for (int j = 0; j < d; ++j)
+    if (maxdeg[j] > 0) {
+      idx[j] = n_dims++;
+      dsoff.push_back(n_slots);
+      n_slots += maxdeg[j];
+    }
+  std::vector<int64_t> slot(tr.n, -1), node_row(tr.n, -1), kids(tr.n, 0), nodes;
+  for (int64_t e = 1; e < tr.n; ++e) {
+    if (tr.level[e] > kMaxPath) return false;
+    slot[e] = dsoff[idx[tr.dim[e]]] + tr.deg[e] - 1;
+    ++kids[tr.parent[e]];
+  }
+  for (int64_t e = 0; e < tr.n; ++e)
+    if (kids[e]) {
+      node_row[e] = int64_t(nodes.size());
+      nodes.push_back(e);
+    }
+  const int64_t K = tr.n - 1, n_nodes = int64_t(nodes.size());
+  if (K < 1) return false;
+  if (n_slots > 0x7fff) return false;
+  const int64_t row_v = n_slots, row_bar = n_slots + n_nodes, row_s = 2 * n_slots + n_nodes;
+  const int64_t rows = 2 * (n_slots + n_nodes) + 1;  // phi, V, bar, S and a row for padding terms
+  // destinations to warps
+  std::vector<int64_t> weight(n_slots + n_nodes, 0);
+  for (int64_t e = 1; e < tr.n; ++e) ++weight[slot[e]];
+  for (int64_t q = 0; q < n_nodes; ++q)
+    if (nodes[q] != 0) weight[n_slots + q] = kids[nodes[q]];
+  std::vector<int> owner(n_slots + n_nodes, 0);
+  double load[kW] = {0};
+  for (int64_t i : stable_order(n_slots + n_nodes, [&](int64_t q) { return -weight[q]; })) {
+    owner[i] = argmin(load, kW);
+    load[owner[i]] += double(weight[i]);
+  }
+  // entries to chunks: the largest chunks of which four fit beside the rows
+  const std::vector<int64_t> ent =
+      stable_order(K, [&](int64_t i) { return std::make_pair(slot[i + 1], tr.parent[i + 1]); });
+  std::vector<int32_t> perm, off, terms;
+  int64_t E = 0, n_chunks = 0, most = 0;
+  for (int64_t c : {128, 64, 32, 16}) {
+    E = c;
+    n_chunks = (K + E - 1) / E;
+    perm.assign(n_chunks * E, -1);
+    std::vector<std::vector<std::array<int32_t, 3>>> lists(n_chunks * kW);
+    for (int64_t i = 0; i < K; ++i) {
+      const int64_t e = ent[i] + 1, at = i % n_chunks, local = i / n_chunks, n = node_row[tr.parent[e]];
+      perm[at * E + local] = int32_t(e);
+      auto term = [&](int64_t owned, int64_t src, int64_t dst) {
+        lists[at * kW + owner[owned]].push_back({int32_t(src), int32_t(dst), int32_t(local)});
+      };
+      term(slot[e], row_v + n, row_bar + slot[e]);
+      if (tr.parent[e] != 0) term(n_slots + n, slot[e], row_s + n);
+    }
+    // two terms at a time: a pair never has one destination, lists are padded to pairs
+    const std::array<int32_t, 3> none = {0, int32_t(rows - 1), 0};
+    off.clear();
+    terms.clear();
+    most = 0;
+    for (int64_t q = 0; q < n_chunks; ++q) {
+      const size_t begin = terms.size() / 2;
+      for (int w = 0; w < kW; ++w) {
+        off.push_back(int32_t(terms.size() / 2));
+        auto put = [&](const std::array<int32_t, 3>& t) { terms.insert(terms.end(), {t[0] | t[1] << 16, t[2] * 128}); };
+        std::vector<std::array<int32_t, 3>> left = lists[q * kW + w];
+        while (!left.empty()) {
+          const std::array<int32_t, 3> first = left.back();
+          left.pop_back();
+          put(first);
+          size_t other = left.size();
+          for (size_t i = left.size(); i-- > 0;)
+            if (left[i][1] != first[1]) {
+              other = i;
+              break;
+            }
+          if (other == left.size()) {
+            put(none);
+          } else {
+            put(left[other]);
+            left.erase(left.begin() + other);
+          }
+        }
+      }
+      off.push_back(int32_t(terms.size() / 2));
+      most = std::max(most, int64_t(terms.size() / 2 - begin));
+    }
+    if (rows * 128 + 4 * (E * 128 + most * 8) + 256 <= 226 * 1024) break;
+    E = 0;
+  }
+  if (E == 0) return false;
+  auto path_of = [&](int64_t e) {
+    std::vector<uint16_t> p;
+    for (int64_t v = e; v != 0; v = tr.parent[v]) p.push_back(uint16_t(slot[v]));
+    std::reverse(p.begin(), p.end());
+    return p;
+  };
+  auto pack = [](std::vector<int32_t>& to, const std::vector<uint16_t>& p) {
+    uint16_t w[8];
+    for (int i = 0; i < 8; ++i) w[i] = i < int(p.size()) ? p[i] : 0xffff;
+    const size_t at = to.size();
+    to.resize(at + 4);
+    std::memcpy(&to[at], w, 16);
+  };
+  // path factors: by slot, the nodes below it and their other slots
+  std::vector<int32_t> node_path;
+  std::vector<std::vector<std::pair<int32_t, std::vector<uint16_t>>>> rest(n_slots);
+  for (int64_t q = 0; q < n_nodes; ++q) {
+    const std::vector<uint16_t> p = path_of(nodes[q]);
+    pack(node_path, p);
+    for (size_t i = 0; i < p.size(); ++i) {
+      std::vector<uint16_t> others(p);
+      others.erase(others.begin() + i);
+      rest[p[i]].push_back({int32_t(row_s + q), others});
+    }
+  }
+  std::vector<std::vector<int64_t>> mine(kW);
+  std::fill(load, load + kW, 0.0);
+  for (int64_t s : stable_order(n_slots, [&](int64_t q) { return -int64_t(rest[q].size()); })) {
+    const int w = argmin(load, kW);
+    mine[w].push_back(s);
+    load[w] += 2.0 * double(rest[s].size()) + 6.0;
+  }
+  std::vector<int32_t> r_slot, r_warp(1, 0), r_row, r_other;
+  for (int w = 0; w < kW; ++w) {
+    std::sort(mine[w].begin(), mine[w].end());
+    for (int64_t s : mine[w]) {
+      const int32_t t0 = int32_t(r_row.size());
+      for (const auto& tm : rest[s]) {
+        r_row.push_back(tm.first);
+        pack(r_other, tm.second);
+      }
+      r_slot.insert(r_slot.end(), {int32_t(s), t0, int32_t(r_row.size()), 0});
+    }
+    r_warp.push_back(int32_t(r_slot.size() / 4));
+  }
+  out.i32["w_perm"] = perm;
+  out.i32["w_off"] = off;
+  out.i32["w_term"] = terms;
+  out.i32["w_node_path"] = node_path;
+  out.i32["w_slot"] = r_slot;
+  out.i32["w_warp"] = r_warp;
+  out.i32["w_row"] = r_row;
+  out.i32["w_other"] = r_other;
+  out.scalar["w_n_nodes"] = double(n_nodes);
+  out.scalar["w_n_chunks"] = double(n_chunks);
+  out.scalar["w_chunk"] = double(E);
+  out.scalar["w_most"] = double(most);
+  return true;
+}
+
 // Tape of the tensor-core panel (spectral.py build_tape): non-root entries in
 // DFS pre-order; word = basis slot | depth << 16; slots of dimension j with
 // max degree m_j > 0 are dsoff[j] .. dsoff[j] + m_j - 1.
@@ -1114,7 +1278,7 @@ extern "C" int smx_layout_build(int kind, int64_t n, const int32_t* parent, cons
                                 int d_out, const int64_t* maxdeg, int d, const int32_t* fam, const double* fa,
                                 const double* fb, smx_host_tables** out) {
   SMX_REQUIRE(out && n >= 1 && d >= 1 && d_out >= 1 && parent && dim && deg && level && rank && rem && maxdeg && fam &&
-                  fa && fb && (kind == SMX_LAYOUT_TAPE || C),
+                  fa && fb && (kind == SMX_LAYOUT_TAPE || kind == SMX_LAYOUT_WALK || C),
               "smx_layout_build: bad arguments");
   *out = nullptr;
   smx::layout::Tree tr{n, parent, dim, deg, level, rank, rem};
@@ -1130,6 +1294,8 @@ extern "C" int smx_layout_build(int kind, int64_t n, const int32_t* parent, cons
   } else if (kind == SMX_LAYOUT_BLOCKED_TC) {
     SMX_REQUIRE(d_out == 1, "smx_layout_build: the blocked evaluator has one output");
     ok = smx::layout::build_blocked_tc(tr, C, maxdeg, d, fam, fa, fb, h->t);
+  } else if (kind == SMX_LAYOUT_WALK) {
+    ok = smx::layout::build_walk(tr, maxdeg, d, h->t);
   } else if (kind == SMX_LAYOUT_STREAM) {
     ok = smx::layout::build_stream(tr, C, d_out, maxdeg, d, fam, fa, fb, h->t);
   } else {

@@ -47,6 +47,9 @@ bool build_perpoint64(const Tree& tr, const double* C, int d_out, const int64_t*
 template <typename T>
 bool build_stream(const Tree& tr, const T* C, int d_out, const int64_t* maxdeg, int d, const int32_t* fam,
                   const double* fa, const double* fb, Tables& out);
+// Tables of the gradient walk over G^T (struct smx_walk); false for entries
+// deeper than 8 or more slots than 15 bits.
+bool build_walk(const Tree& tr, const int64_t* maxdeg, int d, Tables& out);
 bool build_tape(const Tree& tr, const int64_t* maxdeg, int d, Tables& out);
 bool build_blocked_tc(const Tree& tr, const float* C, const int64_t* maxdeg, int d, const int32_t* fam,
                       const double* fa, const double* fb, Tables& out);

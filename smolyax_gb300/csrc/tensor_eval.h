@@ -26,7 +26,7 @@ struct SplitGemm {
   const float* col_scale;
   int M, N, K;
   float* D;
-  int64_t ldd;
+  int64_t ldd;  // 0: D is [N / 32][M][32], the columns of 32 together
   const float* bias;
   int* err;
   int splits;

@@ -25,6 +25,8 @@ BLOCKED_TC_TABLES = dict(i32=("tc_td", "tc_row", "tc_chunk", "tc_b", "tc_box"), 
                          scalars=("tc_n_td", "tc_n_phi", "tc_n_phi_pad", "tc_n_rows", "tc_max_depth", "tc_n_agen",
                                   "tc_n_chunks", "tc_n_boxes", "tc_lin0", "tc_stages", "tc_td_col", "tc_td_bytes",
                                   "c0"))
+WALK_TABLES = ("w_perm", "w_off", "w_term", "w_node_path", "w_slot", "w_warp", "w_row", "w_other")
+WALK_SCALARS = ("w_n_nodes", "w_n_chunks", "w_chunk", "w_most")
 STREAM_TABLES = dict(i32=("st_hot", "st_vp", "st_desc", "st_warp", "st_chunk"),
                      scalars=("st_pass", "st_row_bytes", "st_n_hb", "st_n_vp", "st_n_rows", "st_n_hot", "st_n_chunks"))
 FP64_TABLES = dict(i32=("node_seg", "cold_seg", "hot_dim", "hot_deg", "hot_soff", "node", "cold", "run"),
@@ -234,10 +236,14 @@ class SpectralPlan:
             return None
         dev = self.fam.device
         K = int(tp["ent"].size)
+        max_deg = max(1, int(np.max(tp["dmax"], initial=1)))
+        m = np.arange(max_deg)
+        rec = np.stack([np.stack([(2 * m + 1) / (m + 1), m / (m + 1)], axis=1),
+                        np.stack([np.sqrt(2.0 / (m + 1)), np.sqrt(m / (m + 1))], axis=1)])
         return dict(dims=T(tp["dims"], torch.int32), dmax=T(tp["dmax"], torch.int32),
                     dsoff=T(tp["dsoff"], torch.int32), n_slots=int(tp["n_slots"]), tape=T(tp["tape"], torch.int32),
                     path=T(tp["path"], torch.int32), K=K, ldk=_round32(max(K, 1)),
-                    max_deg=max(1, int(np.max(tp["dmax"], initial=1))), bias=self.keep["c0"],
+                    max_deg=max_deg, rec=T(rec, torch.float32), bias=self.keep["c0"],
                     err=torch.zeros(1, dtype=torch.int32, device=dev),
                     ent=torch.as_tensor(tp["ent"].astype(np.int64), device=dev), ent_h=tp["ent"].astype(np.int64),
                     # tape positions of the depth-1 entries: where independent segments may start
@@ -255,10 +261,19 @@ class SpectralPlan:
         B = np.zeros((d_out, ldk), dtype=np.float32)
         B[:, :K] = C32[tc["ent_h"][::-1]].T  # the panel stores the entries in reversed pre-order
         tc["Bd"] = T(B, torch.float32)
-        m = np.arange(tc["max_deg"])
-        tc["rec"] = T(np.stack([np.stack([(2 * m + 1) / (m + 1), m / (m + 1)], axis=1),
-                                np.stack([np.sqrt(2.0 / (m + 1)), np.sqrt(m / (m + 1))], axis=1)]), torch.float32)
         self.tc = tc
+
+    def _tensor_struct(self, ops, d_out):
+        """``smx_tensor`` with the tape's shapes and basis tables (no operands)."""
+        s = capi.SmxTensor()
+        s.d_in, s.d_out = int(self.c.d_in), int(d_out)
+        s.n_dims, s.n_slots, s.max_deg = int(ops["dims"].numel()), ops["n_slots"], ops["max_deg"]
+        s.K, s.n_groups = ops["K"], (ops["K"] + 63) // 64
+        for name in ("dims", "dmax", "dsoff", "path", "rec", "bias", "err"):
+            setattr(s, name, ops[name].data_ptr())
+        for name in ("fam_a", "fam_b", "fam"):
+            setattr(s, name, self.keep[name].data_ptr())
+        return s
 
     def _tc_struct(self, bf16=False):
         """``smx_tensor`` of the plan: FP16 operands with scales, or the BF16
@@ -284,15 +299,8 @@ class SpectralPlan:
                 if K:
                     call("smx_tensor_operands", ptr(Bd), d_out, K, tc["ldk"], ptr(tc["tape"]), ptr(k["tape"]),
                          ptr(k["Bh"]), ptr(k["Bl"]), ldb, ptr(k["out_scale"]), st)
-            s = capi.SmxTensor()
-            s.d_in, s.d_out = int(self.c.d_in), d_out
-            s.n_dims, s.n_slots, s.max_deg = int(tc["dims"].numel()), tc["n_slots"], tc["max_deg"]
-            s.K, s.n_groups, s.bf16 = K, n_groups, int(bf16)
-            s.splits, s.chunk, s.ldb = self.tc_splits(), self._tc_step(1 << 40), ldb
-            for name in ("dims", "dmax", "dsoff", "path", "rec", "bias", "err"):
-                setattr(s, name, tc[name].data_ptr())
-            for name in ("fam_a", "fam_b", "fam"):
-                setattr(s, name, self.keep[name].data_ptr())
+            s = self._tensor_struct(tc, d_out)
+            s.bf16, s.splits, s.chunk, s.ldb = int(bf16), self.tc_splits(), self._tc_step(1 << 40), ldb
             for name, t in k.items():
                 setattr(s, name, t.data_ptr())
             tc[key] = (s, k)
@@ -373,7 +381,7 @@ class SpectralPlan:
             Rd = T(rows, torch.float32)
             Rh, Rl = torch.empty_like(Rd), torch.empty_like(Rd)
             call("smx_split_tf32", ptr(Rd), rows.shape[0], ldo, ldo, ptr(Rh), ptr(Rl), ldo, st)
-            ops.update(Rh=Rh, Rl=Rl, ldo=ldo)
+            ops.update(Rh=Rh, Rl=Rl, ldo=ldo, walk=self._build_walk(ops, C32))
             # tape segments of the gradient walk: fixed per plan (a point's dL/dx
             # does not depend on the batch it comes in)
             want = vjp_segment_count(K, ops["lvl1"].size)
@@ -384,6 +392,71 @@ class SpectralPlan:
                 ops["vjp_seg"] = (None, 1)
             self._bwd = ops
         return self._bwd
+
+    def _build_walk(self, ops, C32):
+        """Structs of the gradient walk over G^T (``csrc/tensor_vjp.cu``), or None
+        where its rows do not fit in shared memory."""
+        import ctypes
+
+        tr, _, maxdeg, fam, fa, fb, T, st = self._fwd_args
+        n_lam, d_out = C32.shape
+        if n_lam < 2:
+            return None
+        lay = capi.host_layout("walk", tr, None, d_out, maxdeg, fam, fa, fb, i32=WALK_TABLES, scalars=WALK_SCALARS)
+        n_dims, n_slots = int(ops["dims"].numel()), ops["n_slots"]
+        if lay is None or 33 * n_dims > 32 * (n_slots + int(lay["w_n_nodes"])):
+            return None
+        dev = self.fam.device
+        ldo = (d_out + 63) // 64 * 64
+        dim_index = np.full(int(self.c.d_in), -1, dtype=np.int32)
+        active = np.nonzero(np.asarray(maxdeg) > 0)[0]
+        dim_index[active] = np.arange(active.size)
+        perm = lay.pop("w_perm")
+        k = {name[2:]: T(lay[name], torch.int32) for name in WALK_TABLES[1:]}
+        k["dim_index"] = T(dim_index, torch.int32)
+        t = self._tensor_struct(ops, d_out)
+        b = capi.SmxTensorBwd()
+        w = b.walk
+        w.n_nodes, w.n_chunks, w.chunk, w.most = (int(lay[q]) for q in WALK_SCALARS)
+        for name, v in k.items():
+            setattr(w, name, v.data_ptr() if v.numel() else None)
+        n_rows = int(perm.size)
+        b.n_rows, b.ldo = n_rows, ldo
+        b.chunk = max(128, int(self.memory_limit * 1024**3 // (4 * (n_rows + 2 * n_slots))) // 128 * 128)
+        k["Rh"] = torch.empty(n_rows, ldo, dtype=torch.float16, device=dev)
+        k["Rl"] = torch.empty_like(k["Rh"])
+        k["row_scale"] = torch.empty(ldo // 64, n_rows, dtype=torch.float32, device=dev)
+        k["out_scale"] = torch.empty(d_out, dtype=torch.float32, device=dev)
+        C = T(np.where((perm >= 0)[:, None], C32[np.maximum(perm, 0)], np.float32(0)), torch.float32)
+        call("smx_tensor_bwd_operands", ptr(C), n_rows, d_out, ldo, ptr(k["Rh"]), ptr(k["Rl"]), ptr(k["row_scale"]),
+             ptr(k["out_scale"]), capi.stream_ptr(torch.cuda.current_stream()))
+        for name in ("Rh", "Rl", "row_scale", "out_scale"):
+            setattr(b, name, k[name].data_ptr())
+        return t, b, k
+
+    def vjp_x_workspace(self, P):
+        """Device bytes of scratch of one dL/dx of P points."""
+        import ctypes
+
+        ops = self._backward_ops()
+        if ops["walk"] is not None:
+            t, b, _ = ops["walk"]
+            return capi.size("smx_tensor_vjp_x_workspace", ctypes.byref(t), ctypes.byref(b), int(P))
+        step = min(int(P), max(128, int(self.memory_limit * 1024**3 // (8 * ops["ldk"])) // 128 * 128))
+        return (2 * int(P) * ops["ldo"] * 4 + step * (ops["ldk"] + 31) // 32 * 32 * 4
+                + capi.size("smx_spectral_vjp_x_workspace", ops["n_slots"], ops["vjp_seg"][1], step))
+
+    def _vjp_x_walk(self, x, g):
+        import ctypes
+
+        t, b, _ = self._backward_ops()["walk"]
+        P, d = int(x.shape[0]), int(x.shape[1])
+        dx = torch.empty(P, d, dtype=torch.float64, device=x.device)
+        nws = self.vjp_x_workspace(P)
+        ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=x.device)
+        call("smx_tensor_vjp_x", ctypes.byref(t), ctypes.byref(b), ptr(x), P, d, ptr(g), int(g.shape[1]), ptr(dx), d,
+             ptr(ws), nws, capi.stream_ptr(torch.cuda.current_stream()))
+        return dx
 
     def vjp(self, x, g, need_x=True, need_coef=True, check=True):
         """Vector-Jacobian products of y = c0 + A(x) C at cotangent g [P, d_out]:
@@ -401,14 +474,18 @@ class SpectralPlan:
         seg, n_seg = ops["vjp_seg"]
         walk = (nd, ptr(ops["dims"]), ptr(ops["dmax"]), ptr(ops["dsoff"]), ops["n_slots"], ptr(ops["tape"]), K,
                 ptr(seg), n_seg, ptr(k["fam_a"]), ptr(k["fam_b"]), ptr(k["fam"]))
-        g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
-        g32[:, :d_out] = g.float()
-        gh, gl = torch.empty_like(g32), torch.empty_like(g32)
-        call("smx_split_tf32", ptr(g32), P, ldo, ldo, ptr(gh), ptr(gl), ldo, st)
+        gf = g.float().contiguous()
         err = ops["err"]
         dx = dC = None
         step = max(128, int(self.memory_limit * 1024**3 // (8 * ldk)) // 128 * 128)
+        if need_x and ops["walk"] is not None:
+            dx = self._vjp_x_walk(x, gf)
+            need_x = False
+        g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
+        g32[:, :d_out] = gf
         if need_x:
+            gh, gl = torch.empty_like(g32), torch.empty_like(g32)
+            call("smx_split_tf32", ptr(g32), P, ldo, ldo, ptr(gh), ptr(gl), ldo, st)
             dx = torch.zeros(P, d, dtype=torch.float64, device=dev)
             ldg = _round32(K)  # 128-byte rows
             G = torch.empty(min(step, P), ldg, dtype=torch.float32, device=dev)
