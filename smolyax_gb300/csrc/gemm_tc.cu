@@ -33,8 +33,9 @@ using namespace smx::tc;
 // K-major operand descriptor of this kernel's slices (kRowBytes swizzle)
 __device__ __forceinline__ uint64_t make_desc_k(uint32_t saddr) { return make_desc_sw(saddr, kRowBytes); }
 
-// Tiles: 128 x BN outputs per CTA (BN = 128, or 256 for wide products: A is
-// then read once per 256 columns and B streams past L2 half as often).  The
+// Tiles: 128 x BN outputs per CTA (BN = 64 for narrow products, 128, or 256 for
+// wide ones: A is then read once per 256 columns and B streams past L2 half as
+// often).  The
 // FP32 accumulator of the tensor cores truncates when it adds, so one
 // accumulator must not run over long stretches of K: the MMA thread
 // alternates between two accumulators in tensor memory (columns [0, BN) and
@@ -48,17 +49,20 @@ constexpr int kChunkTf32 = 64 / kBK;
 constexpr int kChunkBf16 = 256 / (2 * kBK);
 constexpr int kChunkF16 = 64 / (2 * kBK);  // scaled FP16: one row scale per 64 products
 
-template <int BN>
+template <int BN, int S = 0>
 struct Tile {
   static constexpr int kN = BN;
-  static constexpr int kDrainWarps = 4 * (BN / 128);
+  static constexpr int kCols = BN < 128 ? BN : 128;  // columns per drain warp
+  static constexpr int kDrainWarps = 4 * (BN / kCols);
   static constexpr int kWarpTMA = kDrainWarps, kWarpMMA = kDrainWarps + 1;
   static constexpr int kThreads = 32 * (kDrainWarps + 2);
-  static constexpr int kStages = BN == 128 ? 3 : 2;  // 64 KB or 96 KB stages in ~192 KB
+  static constexpr int kStages = S ? S : BN == 64 ? 4 : BN == 128 ? 3 : 2;  // 48, 64 or 96 KB stages in ~192 KB
   static constexpr int kA = kBM * kBK * 4;
   static constexpr int kB = BN * kBK * 4;
   static constexpr int kStage = 2 * kA + 2 * kB;
-  static constexpr int kTiles = kStages * kStage;
+  static constexpr int kEpiLd = kCols + 4;  // epilogue staging row stride (floats): 16-byte rows, conflict-free
+  static constexpr int kEpi = kDrainWarps * 32 * kEpiLd * 4;
+  static constexpr int kTiles = kStages * kStage > kEpi ? kStages * kStage : kEpi;
   static constexpr int kTotal = kTiles + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -78,23 +82,19 @@ struct GemmArgs {
   const float* col_scale;  // scaled FP16: by column
 };
 
-constexpr int kEpiLd = 132;  // epilogue staging row stride (floats): 16-byte rows, conflict-free
-static_assert(Tile<128>::kDrainWarps * 32 * kEpiLd * 4 <= Tile<128>::kTiles, "epilogue staging must fit");
-static_assert(Tile<256>::kDrainWarps * 32 * kEpiLd * 4 <= Tile<256>::kTiles, "epilogue staging must fit");
-
 // KIND kTf32: kind::tf32 on FP32 operands (32 per 128-byte slice); kBf16, kF16:
 // kind::f16 on 16-bit operands (64 per slice).  Same slices, stages and MMAs;
 // kF16 multiplies each drained accumulator by its row's scale of the slice and
 // the result by the column's.
-template <int KIND, int BN>
-__global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
+template <int KIND, int BN, int S>
+__global__ void __launch_bounds__(Tile<BN, S>::kThreads, S == 1 ? 2 : 1)
     gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                        const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, GemmArgs g) {
   constexpr bool BF16 = KIND != kTf32;  // 16-bit operands
   constexpr int EK = BF16 ? 2 * kBK : kBK;  // elements per K-tile
   constexpr int kChunk = KIND == kF16 ? kChunkF16 : BF16 ? kChunkBf16 : kChunkTf32;
-  using L = Tile<BN>;
-  constexpr int kBN = BN;
+  using L = Tile<BN, S>;
+  constexpr int kBN = BN, kCols = L::kCols, kEpiLd = L::kEpiLd;
   constexpr int kStages = L::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -218,11 +218,11 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     __syncwarp();
   } else {
     // ---- drain warps: warp w owns TMEM lanes 32 (w % 4) .. +31 (rows m0 + 32 (w % 4) + lane)
-    // and the 128 columns cw .. cw + 127 of the tile
-    const int quad = warp & 3, cw = (warp >> 2) * 128;
-    float acc[128];
+    // and the kCols columns from cw of the tile
+    const int quad = warp & 3, cw = (warp >> 2) * kCols;
+    float acc[kCols];
 #pragma unroll
-    for (int j = 0; j < 128; ++j) acc[j] = 0.f;
+    for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
     bool ok = true;
     const uint32_t lane_base = tmem + (uint32_t(quad * 32) << 16);
     const float* rs = nullptr;  // this row's scale of the next slice
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-      for (int q = 0; q < 128; q += 16) {
+      for (int q = 0; q < kCols; q += 16) {
         uint32_t r[16];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -263,14 +263,15 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     if (ok) {
       // The last accumulator has been read, so every MMA and every copy into the
       // pipeline stages is complete: the warp stages its 32 rows there
-      // (T[row][col], stride kEpiLd) and writes them back row by row, 512
-      // contiguous bytes per store instruction.
+      // (T[row][col], stride kEpiLd) and writes them back by rows, 512 bytes in
+      // one or two contiguous pieces per store instruction.
       float* T = reinterpret_cast<float*>(base) + warp * (32 * kEpiLd);
 #pragma unroll
-      for (int q = 0; q < 128; q += 4)
+      for (int q = 0; q < kCols; q += 4)
         *reinterpret_cast<float4*>(T + lane * kEpiLd + q) = make_float4(acc[q], acc[q + 1], acc[q + 2], acc[q + 3]);
       __syncwarp();
-      const int c0 = n0 + cw + 4 * lane;
+      constexpr int kLanes = kCols / 4;  // lanes per row
+      const int tc = 4 * (lane % kLanes), c0 = n0 + cw + tc;
       const bool blocked = KIND == kF16 && g.ldd == 0;  // D is [N / 32][M][32]
       const bool vec = (g.ldd % 4) == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0 && c0 + 3 < g.N;
       float bv[4];
@@ -281,10 +282,10 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
 #pragma unroll
         for (int i = 0; i < 4; ++i) cs[i] = c0 + i < g.N ? g.col_scale[c0 + i] : 1.f;
       }
-      for (int r = 0; r < 32; ++r) {
+      for (int r = lane / kLanes; r < 32; r += 32 / kLanes) {
         const int row = m0 + quad * 32 + r;
         if (row >= g.M) break;
-        const float4 t = *reinterpret_cast<const float4*>(T + r * kEpiLd + 4 * lane);
+        const float4 t = *reinterpret_cast<const float4*>(T + r * kEpiLd + tc);
         float v[4] = {t.x + bv[0], t.y + bv[1], t.z + bv[2], t.w + bv[3]};
         if constexpr (KIND == kF16)
           v[0] = fmaf(t.x, cs[0], bv[0]), v[1] = fmaf(t.y, cs[1], bv[1]), v[2] = fmaf(t.z, cs[2], bv[2]),
@@ -370,17 +371,17 @@ int make_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64
   return SMX_OK;
 }
 
-template <int KIND, int BN>
+template <int KIND, int BN, int S = 0>
 int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, const void* Bl, int64_t ldb, int M,
                 int N, int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
                 int splits, uint64_t wait_ns, int no_loads, const SplitGemm* sc) {
-  using L = Tile<BN>;
+  using L = Tile<BN, S>;
   CUtensorMap tBh, tBl;
   int rc;
   if ((rc = make_map(&tBh, Bh, N, K, ldb, BN, KIND)) || (rc = make_map(&tBl, Bl, N, K, ldb, BN, KIND))) return rc;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(gemm_tf32x3_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
+    cudaFuncSetAttribute(gemm_tf32x3_kernel<KIND, BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
     attr = true;
   }
   // split-K: slice z runs K-tiles [z * kt_per_z, ...) into D + z * zstride
@@ -392,12 +393,17 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
              wait_ns, no_loads, nullptr, 0,      nullptr};
   if (sc) g.row_scale = sc->row_scale, g.ld_scale = sc->ld_scale, g.col_scale = sc->col_scale;
   dim3 grid((N + BN - 1) / BN, (M + kBM - 1) / kBM, nz);
-  gemm_tf32x3_kernel<KIND, BN><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
+  gemm_tf32x3_kernel<KIND, BN, S><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
   SMX_LAUNCH_CHECK(KIND == kTf32 ? "smx_gemm_tf32x3" : KIND == kBf16 ? "smx_gemm_bf16x3" : "smx_tensor_eval");
   return SMX_OK;
 }
 
-// Products wider than 192 columns use 128 x 256 tiles, the others 128 x 128.
+// Tiles by the product's width: 128 x 64 up to 64 columns (no padding to 128, half
+// the accumulators to drain: 1e5 x 64 outputs over K = 4999 in 394 us, 484 us with
+// 128 x 128), 128 x 128 up to 192, 128 x 256 beyond.  A product of one slice of K
+// has no pipeline to fill, so two single-stage blocks share an SM and one's loads
+// and MMAs run under the other's stores (5120 x 1e5 outputs over K = 64: 791 us,
+// 844 us with 128 x 256 and one block).
 template <int KIND>
 int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const void* Bl, int64_t ldb, int M, int N,
            int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
@@ -405,6 +411,13 @@ int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const vo
   CUtensorMap tAh, tAl;
   int rc;
   if ((rc = make_map(&tAh, Ah, M, K, lda, kBM, KIND)) || (rc = make_map(&tAl, Al, M, K, lda, kBM, KIND))) return rc;
+  if constexpr (KIND == kF16)
+    if (K <= 2 * kBK && N > 64)
+      return launch_tile<KIND, 128, 1>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits,
+                                       wait_ns, no_loads, sc);
+  if (N <= 64)
+    return launch_tile<KIND, 64>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
+                                 no_loads, sc);
   if (N > 192)
     return launch_tile<KIND, 256>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
                                   no_loads, sc);
