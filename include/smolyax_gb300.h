@@ -750,6 +750,15 @@ int smx_tensor_vjp_x(const smx_tensor* plan_host, const smx_tensor_bwd* bwd_host
                      int64_t ldx, const float* g, int64_t ldg, double* dx, int64_t lddx, void* ws, size_t ws_bytes,
                      void* stream);
 
+/* dL/dC = A^T g (FP32) over plan->chunk points at a time (a multiple of 64): rows in the
+ * order of the padded tape, dC[64 n_groups][d_out], with the plan's splits
+ * (smx_tensor_coef_splits) over the points.  Plans with more basis slots than fit in
+ * shared memory (workspace 0) are refused. */
+int smx_tensor_coef_splits(int d_out, int K);
+size_t smx_tensor_vjp_coef_workspace(const smx_tensor* plan_host, int64_t P);
+int smx_tensor_vjp_coef(const smx_tensor* plan_host, const double* x, int64_t P, int64_t ldx, const float* g,
+                        int64_t ldg, float* dC, void* ws, size_t ws_bytes, void* stream);
+
 /* ---- host-side layout builders of the FP32 evaluators ------------------------------
  * The tables of the blocked one-output evaluator (smx_blocked), of the
  * per-point evaluator (smx_spectral) and the entry tape of the tensor-core

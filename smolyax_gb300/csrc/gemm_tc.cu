@@ -80,6 +80,7 @@ struct GemmArgs {
   const float* row_scale;  // scaled FP16: [K-tile][ld_scale], by row
   int64_t ld_scale;
   const float* col_scale;  // scaled FP16: by column
+  int rows_a, rows_b;      // operands stored slice by slice, [K-tile][rows][kRowBytes]; 0: row-major
 };
 
 // KIND kTf32: kind::tf32 on FP32 operands (32 per 128-byte slice); kBf16, kF16:
@@ -152,11 +153,13 @@ __global__ void __launch_bounds__(Tile<BN, S>::kThreads, S == 1 ? 2 : 1)
         }
         uint8_t* st = base + s * L::kStage;
         mbar_expect_tx(&full[s], L::kStage);
-        const int k = (kt_base + kt) * EK;
-        tma_load_2d(st, &tmAh, k, m0, &full[s]);
-        tma_load_2d(st + L::kA, &tmAl, k, m0, &full[s]);
-        tma_load_2d(st + 2 * L::kA, &tmBh, k, n0, &full[s]);
-        tma_load_2d(st + 2 * L::kA + L::kB, &tmBl, k, n0, &full[s]);
+        const int q = kt_base + kt;
+        const int ka = g.rows_a ? 0 : q * EK, ma = m0 + q * g.rows_a;
+        const int kb = g.rows_b ? 0 : q * EK, nb = n0 + q * g.rows_b;
+        tma_load_2d(st, &tmAh, ka, ma, &full[s]);
+        tma_load_2d(st + L::kA, &tmAl, ka, ma, &full[s]);
+        tma_load_2d(st + 2 * L::kA, &tmBh, kb, nb, &full[s]);
+        tma_load_2d(st + 2 * L::kA + L::kB, &tmBl, kb, nb, &full[s]);
         armed_upto = kt + 1;
       }
       *armed_slot = armed_upto;
@@ -371,6 +374,16 @@ int make_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64
   return SMX_OK;
 }
 
+// Map of an operand of `rows` rows: row-major, or slice by slice ([K-tile][rows]
+// rows of kRowBytes; a tile past the last row reads the next slice's rows, whose
+// products are not written).
+int operand_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t K, int64_t ld, int box_rows, int kind,
+                bool sliced) {
+  if (!sliced) return make_map(tm, ptr, rows, K, ld, box_rows, kind);
+  const int ek = kind == kTf32 ? kBK : 2 * kBK;
+  return make_map(tm, ptr, (K + ek - 1) / ek * rows, ek, ek, box_rows, kind);
+}
+
 template <int KIND, int BN, int S = 0>
 int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, const void* Bl, int64_t ldb, int M,
                 int N, int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
@@ -378,7 +391,9 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
   using L = Tile<BN, S>;
   CUtensorMap tBh, tBl;
   int rc;
-  if ((rc = make_map(&tBh, Bh, N, K, ldb, BN, KIND)) || (rc = make_map(&tBl, Bl, N, K, ldb, BN, KIND))) return rc;
+  if ((rc = operand_map(&tBh, Bh, N, K, ldb, BN, KIND, sc && sc->sliced)) ||
+      (rc = operand_map(&tBl, Bl, N, K, ldb, BN, KIND, sc && sc->sliced)))
+    return rc;
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(gemm_tf32x3_kernel<KIND, BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
@@ -390,8 +405,11 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
   const int kt_per_z = splits > 1 ? (KT + splits - 1) / splits : 0;
   const int nz = splits > 1 ? (KT + kt_per_z - 1) / kt_per_z : 1;
   GemmArgs g{M,       N,        K,       D,      ldd, bias, err, accumulate, kt_per_z, int64_t(M) * ldd,
-             wait_ns, no_loads, nullptr, 0,      nullptr};
-  if (sc) g.row_scale = sc->row_scale, g.ld_scale = sc->ld_scale, g.col_scale = sc->col_scale;
+             wait_ns, no_loads, nullptr, 0,      nullptr, 0, 0};
+  if (sc) {
+    g.row_scale = sc->row_scale, g.ld_scale = sc->ld_scale, g.col_scale = sc->col_scale;
+    if (sc->sliced) g.rows_a = M, g.rows_b = N;
+  }
   dim3 grid((N + BN - 1) / BN, (M + kBM - 1) / kBM, nz);
   gemm_tf32x3_kernel<KIND, BN, S><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
   SMX_LAUNCH_CHECK(KIND == kTf32 ? "smx_gemm_tf32x3" : KIND == kBf16 ? "smx_gemm_bf16x3" : "smx_tensor_eval");
@@ -410,7 +428,9 @@ int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const vo
            int splits = 1, uint64_t wait_ns = kWaitNs, int no_loads = 0, const SplitGemm* sc = nullptr) {
   CUtensorMap tAh, tAl;
   int rc;
-  if ((rc = make_map(&tAh, Ah, M, K, lda, kBM, KIND)) || (rc = make_map(&tAl, Al, M, K, lda, kBM, KIND))) return rc;
+  if ((rc = operand_map(&tAh, Ah, M, K, lda, kBM, KIND, sc && sc->sliced)) ||
+      (rc = operand_map(&tAl, Al, M, K, lda, kBM, KIND, sc && sc->sliced)))
+    return rc;
   if constexpr (KIND == kF16)
     if (K <= 2 * kBK && N > 64)
       return launch_tile<KIND, 128, 1>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits,
@@ -575,14 +595,14 @@ int smx::tc::split_gemm(const SplitGemm& g, cudaStream_t st) {
   if (g.K == 0 || g.splits <= 1) {
     if (g.K == 0) {  // the constant alone
       splitk_reduce_kernel<<<smx::grid_for(int64_t(g.M) * g.N, 256), 256, 0, st>>>(nullptr, 0, g.M, g.N, g.D, g.ldd,
-                                                                                  g.bias, 0);
+                                                                                  g.bias, g.accumulate);
       SMX_LAUNCH_CHECK("smx_tensor_eval");
       return SMX_OK;
     }
     return g.bits == kF16 ? launch<kF16>(g.Ah, g.Al, g.lda, g.Bh, g.Bl, g.ldb, g.M, g.N, g.K, g.D, g.ldd, g.bias,
-                                         g.err, 0, st, 1, kWaitNs, 0, &g)
+                                         g.err, g.accumulate, st, 1, kWaitNs, 0, &g)
                           : launch<kBf16>(g.Ah, g.Al, g.lda, g.Bh, g.Bl, g.ldb, g.M, g.N, g.K, g.D, g.ldd, g.bias,
-                                          g.err, 0, st);
+                                          g.err, g.accumulate, st);
   }
   const int kt = (g.K + 2 * kBK - 1) / (2 * kBK), per = (kt + g.splits - 1) / g.splits;
   const int slices = (kt + per - 1) / per;
@@ -592,7 +612,7 @@ int smx::tc::split_gemm(const SplitGemm& g, cudaStream_t st) {
                                       g.err, 0, st, g.splits);
   if (rc) return rc;
   splitk_reduce_kernel<<<smx::grid_for(int64_t(g.M) * g.N, 256), 256, 0, st>>>(g.partial, slices, g.M, g.N, g.D,
-                                                                              g.ldd, g.bias, 0);
+                                                                              g.ldd, g.bias, g.accumulate);
   SMX_LAUNCH_CHECK("smx_tensor_eval");
   return SMX_OK;
 }

@@ -32,10 +32,6 @@ namespace {
 using namespace smx::tc;
 
 constexpr size_t kSmemMax = 227 * 1024;
-// second tape word: the entry's factor 2^f (FP32 bits), the byte offset of its
-// parent on the stack (128 per depth), and flags
-constexpr int kPop = 1, kPush = 2, kStackMask = 0xf80, kFactorMask = 0x7f800000;
-constexpr int kGroup = 64;  // columns per scale and per 128-byte row of 16-bit values
 
 // x coordinate in FP32, infinities as NaN (the point's value is then NaN).
 __device__ __forceinline__ float x32(double v) {
@@ -347,6 +343,12 @@ Layout layout(const smx_tensor* t, int64_t m) {
 
 }  // namespace
 
+void smx::tc::tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, int64_t ldp,
+                           cudaStream_t st) {
+  const dim3 grid(unsigned(ldp / 32), unsigned(std::min((t.n_dims + 31) / 32, 65535)));
+  tensor_basis_kernel<<<grid, 256, 0, st>>>(t, x, P, ldx, grow, ldp);
+}
+
 extern "C" int smx_tensor_operands(const float* B, int N, int K, int64_t ldb, const int32_t* tape, int32_t* tape_out,
                                    uint16_t* Bh, uint16_t* Bl, int64_t ldh, float* out_scale, void* stream) {
   SMX_REQUIRE(N >= 1 && K >= 1 && ldb >= K && ldh >= K && B && tape && tape_out && Bh && Bl && out_scale,
@@ -415,8 +417,7 @@ extern "C" int smx_tensor_eval(const smx_tensor* t, const double* x, int64_t P, 
     float* part = reinterpret_cast<float*>(w + 2 * L.panel + L.scales + L.rows);
     int rc;
     if (t->K > 0) {
-      const dim3 bgrid(unsigned(L.gstride / 32), unsigned(std::min((t->n_dims + 31) / 32, 65535)));
-      tensor_basis_kernel<<<bgrid, 256, 0, st>>>(*t, x + p0 * ldx, m, ldx, grow, L.gstride);
+      tensor_basis(*t, x + p0 * ldx, m, ldx, grow, L.gstride, st);
       CUtensorMap tmH, tmL;
       const int bits = t->bf16 ? kBf16 : kF16;
       if ((rc = panel_map(&tmH, Ah, m, t->K, t->ldb, 32, bits)) ||

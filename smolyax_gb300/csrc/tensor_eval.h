@@ -6,8 +6,20 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "smolyax_gb300.h"
+
 namespace smx {
 namespace tc {
+
+// Second word of a tape entry (first: 128 * slot): the entry's factor 2^f (FP32
+// bits), the byte offset of its parent on a stack of 128 bytes per depth, and flags.
+constexpr int kPop = 1, kPush = 2, kStackMask = 0xf80, kFactorMask = 0x7f800000;
+constexpr int kGroup = 64;  // tape entries (panel columns) per group
+
+// Basis values of all slots, grow[slot][p], p < ldp (a multiple of 32; points past
+// P repeat the last one).
+void tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, int64_t ldp,
+                  cudaStream_t st);
 
 constexpr int kTf32 = 0, kBf16 = 1, kF16 = 2;
 
@@ -31,6 +43,8 @@ struct SplitGemm {
   int* err;
   int splits;
   float* partial;
+  bool sliced;     // kF16: A is [ceil(K / 64)][M][64], B [ceil(K / 64)][N][64] (lda, ldb unused)
+  int accumulate;  // D += instead of D =
 };
 int split_gemm(const SplitGemm& g, cudaStream_t st);
 

@@ -1,8 +1,9 @@
-// Backward of the tensor-core evaluation with respect to x:
+// Backward of the tensor-core evaluation, with respect to x:
 //   G^T[e][p] = sum_o C[e][o] g[p][o]       (tensor cores, scaled FP16 pairs)
 //   dL/dx[p][j] = a_j sum_g phi_g'(z_j) bar[slot (j, g)]
-// with bar the adjoints of the basis values under L = sum_e G_e prod phi.  The
-// reference has the dense Jacobian instead (interpolation.py:306-345).
+// with bar the adjoints of the basis values under L = sum_e G_e prod phi, and
+// dL/dC[e][o] = sum_p A[p][e] g[p][o] further down.  The reference has the dense
+// Jacobian instead (interpolation.py:306-345).
 //
 // G is made transposed in blocks of 32 points, [p / 32][entry][32]: a block of 32
 // warps (lane = point) streams its adjoints once, in order, through shared
@@ -291,6 +292,169 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// ---- dL/dC = A^T g ---------------------------------------------------------------------
+// A^T in slices of 64 points, [p / 64][entry][64] as FP16 pairs with one power of
+// two per entry and slice (times the slice's scale of g).  A block of W warps holds
+// the basis rows of 64 points (two per lane) in shared memory; each warp walks its
+// run of tape groups as tensor_panel_kernel does (tensor_eval.cu), but an entry's 64
+// values are one register pair per lane, so they are scaled and written at once:
+// 128 contiguous bytes per entry and part.  Bound: HBM writes, 4 bytes per value.
+// Leja d_in = 200, |Lambda| = 5000, 1e5 points: 0.34 ms (6.0 TB/s of writes, issue
+// slots 71 % busy) and 0.32 ms for the product with 64 outputs; one thread per point
+// writing TF32 pairs through 400 KB strides took 1.34 ms and its product 0.62 ms.
+template <int W, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB)
+    coef_panel_kernel(smx_tensor t, int groups_per_block, const float* __restrict__ grow, int64_t gstride,
+                      int64_t n_slices, const float* __restrict__ gscale, uint32_t* __restrict__ AH,
+                      uint32_t* __restrict__ AL, float* __restrict__ S) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint8_t* ring = smem + warp * 1024;  // two tape groups
+  uint8_t* stk = smem + W * 1024 + warp * (9 * 256) + lane * 8;  // stk[256 d]: first d factors
+  uint8_t* rows = smem + W * (1024 + 9 * 256) + lane * 8;
+  const int b0 = blockIdx.x * groups_per_block, nb = min(t.n_groups - b0, groups_per_block);
+  const int t0 = b0 + nb * warp / W, t1 = b0 + nb * (warp + 1) / W;
+  const int64_t E = int64_t(t.n_groups) * kGroup;
+  auto f2 = [](uint8_t* q) -> float2& { return *reinterpret_cast<float2*>(q); };
+  for (int64_t sl = blockIdx.y; sl < n_slices; sl += gridDim.y) {
+    __syncthreads();  // the previous slice's walks are done
+    for (int i = warp; i < t.n_slots; i += W)
+      f2(rows + i * 256) = __ldg(reinterpret_cast<const float2*>(grow + i * gstride + sl * 64) + lane);
+    __syncthreads();
+    if (t0 == t1) continue;
+    const float gsc = __ldg(gscale + sl);
+    f2(stk) = make_float2(1.f, 1.f);
+    for (int i = 0; i < 8; ++i) {
+      const int s = __ldg(t.path + t0 * 8 + i);
+      if (s < 0) break;
+      f2(stk + (i + 1) * 256) = __fmul2_rn(f2(stk + i * 256), f2(rows + s * 256));
+    }
+    const int4* tape = reinterpret_cast<const int4*>(t.tape) + t0 * (kGroup / 2) + lane;
+    auto copy_group = [&](int g) {
+      if (g < t1)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(ring + (g & 1) * 512 + lane * 16)),
+                     "l"(tape + (g - t0) * (kGroup / 2))
+                     : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    copy_group(t0);
+    for (int g = t0; g < t1; ++g) {
+      copy_group(g + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      const int4* words = reinterpret_cast<const int4*>(ring + (g & 1) * 512);
+      const int64_t e0 = sl * E + g * kGroup;
+      float2 cur = make_float2(1.f, 1.f);
+      float sc = 0.f;
+#pragma unroll 2
+      for (int k = 0; k < kGroup; k += 4) {
+        const int4 wa = words[k / 2], wb = words[k / 2 + 1];
+        const int wr[4] = {wa.x, wa.z, wb.x, wb.z}, wf[4] = {wa.y, wa.w, wb.y, wb.w};
+        float2 b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) b[u] = f2(rows + wr[u] * 2);
+        unsigned m[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (wf[u] & kPop) cur = f2(stk + (wf[u] & kStackMask) * 2);
+          b[u] = __fmul2_rn(cur, b[u]);
+          if (wf[u] & kPush) {
+            cur = b[u];
+            f2(stk + (wf[u] & kStackMask) * 2 + 256) = cur;
+          }
+          m[u] = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fabsf(b[u].x), fabsf(b[u].y))));
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          // power of two that brings the maximum to [2^14, 2^15)
+          const int e = min(max(int(m[u] >> 23), 27), 254);
+          const float inv = __int_as_float((268 - e) << 23);
+          if (lane == ((k + u) & 31)) sc = __int_as_float((e - 14) << 23);
+          const float2 v = __fmul2_rn(b[u], make_float2(inv, inv));
+          const __half2 h = __float22half2_rn(v);
+          const __half2 l = __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-1.f, -1.f), v));
+          AH[(e0 + k + u) * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
+          AL[(e0 + k + u) * 32 + lane] = *reinterpret_cast<const uint32_t*>(&l);
+        }
+        if ((k & 31) == 28) S[e0 + (k & 32) + lane] = sc * gsc;
+      }
+    }
+  }
+}
+
+// Largest finite |g| of every output (bits; `most` starts at zero) ...
+__global__ void __launch_bounds__(256) output_most_kernel(const float* __restrict__ g, int64_t ldg, int64_t P, int d_out,
+                                                          unsigned* __restrict__ most) {
+  __shared__ float red[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o0 = blockIdx.y * 32; o0 < d_out; o0 += gridDim.y * 32) {
+    const int o = o0 + lane;
+    const int64_t p1 = min(P, (blockIdx.x + 1) * int64_t(512));
+    float m = 0.f;
+    if (o < d_out)
+      for (int64_t p = blockIdx.x * int64_t(512) + warp; p < p1; p += 8) {
+        const float a = fabsf(__ldg(g + p * ldg + o));
+        if (a <= 3.0e38f) m = fmaxf(m, a);
+      }
+    red[warp][lane] = m;
+    __syncthreads();
+    if (warp == 0 && o < d_out) {
+      for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w][lane]);
+      if (m > 0.f) atomicMax(most + o, __float_as_uint(m));
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ float output_scale(unsigned most) {
+  return most ? __int_as_float(min(max(int(most >> 23), 1), 253) << 23) : 1.f;
+}
+
+// ... and g / scale transposed in slices of 64 points, [p / 64][output][64], as FP16
+// pairs with one power of two per slice; points past P are zero.
+__global__ void __launch_bounds__(256) output_slices_kernel(const float* __restrict__ g, int64_t ldg, int64_t P,
+                                                            int d_out, const unsigned* __restrict__ most,
+                                                            uint32_t* __restrict__ hi, uint32_t* __restrict__ lo,
+                                                            float* __restrict__ gscale, float* __restrict__ scale) {
+  __shared__ float tile[64][65];
+  __shared__ float red[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, oc = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+  const int64_t p0 = blockIdx.x * int64_t(64);
+  auto value = [&](int64_t p, int o) {
+    return p < P && o < d_out
+               ? __ldg(g + p * ldg + o) * __int_as_float((254 << 23) - __float_as_int(output_scale(__ldg(most + o))))
+               : 0.f;
+  };
+  if (blockIdx.x == 0)
+    for (int o = threadIdx.x; o < d_out; o += 256) scale[o] = output_scale(most[o]);
+  float m = 0.f;
+  for (int o0 = 0; o0 < d_out; o0 += 64)
+    for (int r = r0; r < 64; r += 4) {
+      const float a = fabsf(value(p0 + r, o0 + oc));
+      if (a <= 3.0e38f) m = fmaxf(m, a);
+    }
+  m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+  if (lane == 0) red[warp] = m;
+  __syncthreads();
+  for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w]);
+  const int e = min(max(__float_as_int(m) >> 23, 27), 254);
+  const float inv = __int_as_float((268 - e) << 23);
+  if (threadIdx.x == 0) gscale[blockIdx.x] = __int_as_float((e - 14) << 23);
+  for (int o0 = 0; o0 < d_out; o0 += 64) {
+    for (int r = r0; r < 64; r += 4) tile[r][oc] = value(p0 + r, o0 + oc) * inv;
+    __syncthreads();
+    for (int o = warp; o < 64 && o0 + o < d_out; o += 8) {
+      const float2 v = make_float2(tile[2 * lane][o], tile[2 * lane + 1][o]);
+      const __half2 h = __float22half2_rn(v);
+      const __half2 l = __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-1.f, -1.f), v));
+      const int64_t at = (blockIdx.x * int64_t(d_out) + o0 + o) * 32 + lane;
+      hi[at] = *reinterpret_cast<const uint32_t*>(&h);
+      lo[at] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+    __syncthreads();
+  }
+}
+
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 size_t walk_smem(const smx_tensor* t, const smx_walk& w) {
@@ -312,7 +476,144 @@ Layout layout(const smx_tensor* t, const smx_tensor_bwd* b, int64_t m) {
   return L;
 }
 
+size_t coef_smem(int warps, int slots) { return size_t(warps) * (1024 + 9 * 256) + size_t(slots) * 256; }
+
+struct CoefLayout {  // workspace of one chunk of m points
+  int64_t gstride, slices, E;
+  size_t panel, scales, rows, cot, gscale, out, partial, total;
+};
+CoefLayout coef_layout(const smx_tensor* t, int64_t m) {
+  CoefLayout L;
+  L.gstride = (m + 127) / 128 * 128;
+  L.slices = (m + 63) / 64;
+  L.E = int64_t(t->n_groups) * kGroup;
+  L.panel = up256(size_t(L.slices) * L.E * 128);
+  L.scales = up256(size_t(L.slices) * L.E * 4);
+  L.rows = up256(size_t(t->n_slots) * L.gstride * 4);
+  L.cot = up256(size_t(L.slices) * t->d_out * 128);
+  L.gscale = up256(size_t(L.slices) * 4);
+  L.out = up256(size_t(t->d_out) * 4);
+  L.partial = t->splits > 1 ? up256(size_t(t->splits) * L.E * t->d_out * 4) : 0;
+  L.total = 2 * L.panel + L.scales + L.rows + 2 * L.cot + L.gscale + 2 * L.out + L.partial;
+  return L;
+}
+
+template <int W, int MINB>
+void launch_coef_panel(const smx_tensor& t, const CoefLayout& L, const float* grow, const float* gscale, uint32_t* AH,
+                       uint32_t* AL, float* S, int sms, cudaStream_t st) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(coef_panel_kernel<W, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax));
+    attr = true;
+  }
+  // the split of the tape with the shortest total of rounds x (groups of a warp +
+  // about 2 groups' time to load the rows and start), as in the evaluation
+  int per = t.n_groups;
+  int64_t best = -1;
+  for (int segs = 1; segs <= 32 && segs * W <= t.n_groups + W - 1; ++segs) {
+    const int p = (t.n_groups + segs - 1) / segs;
+    const int64_t blocks = L.slices * ((t.n_groups + p - 1) / p);
+    const int64_t cost = ((blocks + MINB * sms - 1) / (MINB * sms)) * ((p + W - 1) / W + 2);
+    if (best < 0 || cost < best) best = cost, per = p;
+  }
+  const dim3 grid(unsigned((t.n_groups + per - 1) / per), unsigned(std::min<int64_t>(L.slices, 65535)));
+  coef_panel_kernel<W, MINB><<<grid, 32 * W, coef_smem(W, t.n_slots), st>>>(t, per, grow, L.gstride, L.slices, gscale,
+                                                                            AH, AL, S);
+}
+
 }  // namespace
+
+// Slices of the contraction over the points: the count of up to 16 with the fewest
+// rounds of tiles on the SMs per slice.
+extern "C" int smx_tensor_coef_splits(int d_out, int K) {
+  if (d_out < 1 || K < 1) return 1;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  const int64_t bn = d_out <= 64 ? 64 : d_out <= 192 ? 128 : 256;
+  const int64_t tiles = (K + 127) / 128 * ((d_out + bn - 1) / bn);
+  int best = 1;
+  double cost = 1e30;
+  for (int s = 1; s <= 16; ++s) {
+    const double c = double((tiles * s + sms - 1) / sms) / s;
+    if (c < 0.98 * cost) cost = c, best = s;
+  }
+  return best;
+}
+
+extern "C" size_t smx_tensor_vjp_coef_workspace(const smx_tensor* t, int64_t P) {
+  if (!t || P <= 0 || t->chunk < 1 || t->K < 1 || coef_smem(16, t->n_slots) > kSmemMax) return 0;
+  return coef_layout(t, std::min(P, t->chunk)).total;
+}
+
+extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t P, int64_t ldx, const float* g,
+                                   int64_t ldg, float* dC, void* ws, size_t ws_bytes, void* stream) {
+  SMX_REQUIRE(t != nullptr, "smx_tensor_vjp_coef: null plan");
+  SMX_REQUIRE(t->d_in >= 1 && t->d_out >= 1 && t->K >= 1 && t->n_groups == (t->K + kGroup - 1) / kGroup &&
+                  t->splits >= 1 && t->chunk >= 64 && t->chunk % 64 == 0 &&
+                  (std::min(P, t->chunk) + 63) / 64 * std::max<int64_t>(64 * t->n_groups, t->d_out) < (int64_t(1) << 31),
+              "smx_tensor_vjp_coef: bad plan sizes");
+  SMX_REQUIRE(P >= 1 && ldx >= t->d_in && ldg >= t->d_out, "smx_tensor_vjp_coef: bad sizes");
+  SMX_REQUIRE(x && g && dC && t->err && t->dims && t->dmax && t->dsoff && t->fam && t->fam_a && t->fam_b && t->rec &&
+                  t->tape && t->path,
+              "smx_tensor_vjp_coef: null pointer");
+  SMX_REQUIRE(coef_smem(16, t->n_slots) <= kSmemMax, "smx_tensor_vjp_coef: the basis rows do not fit in shared memory");
+  SMX_REQUIRE(ws && ws_bytes >= smx_tensor_vjp_coef_workspace(t, P) && (reinterpret_cast<uintptr_t>(ws) & 15) == 0,
+              "smx_tensor_vjp_coef: workspace too small or not 16-byte aligned");
+  cudaStream_t st = smx::as_stream(stream);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_coef: no device");
+  for (int64_t p0 = 0; p0 < P; p0 += t->chunk) {
+    const int64_t m = std::min(t->chunk, P - p0);
+    const CoefLayout L = coef_layout(t, m);
+    uint8_t* q = static_cast<uint8_t*>(ws);
+    auto take = [&](size_t bytes) {
+      uint8_t* r = q;
+      q += bytes;
+      return r;
+    };
+    uint32_t* AH = reinterpret_cast<uint32_t*>(take(L.panel));
+    uint32_t* AL = reinterpret_cast<uint32_t*>(take(L.panel));
+    float* S = reinterpret_cast<float*>(take(L.scales));
+    float* grow = reinterpret_cast<float*>(take(L.rows));
+    uint32_t* gh = reinterpret_cast<uint32_t*>(take(L.cot));
+    uint32_t* gl = reinterpret_cast<uint32_t*>(take(L.cot));
+    float* gscale = reinterpret_cast<float*>(take(L.gscale));
+    unsigned* most = reinterpret_cast<unsigned*>(take(L.out));
+    float* scale = reinterpret_cast<float*>(take(L.out));
+    if (cudaMemsetAsync(most, 0, size_t(t->d_out) * 4, st) != cudaSuccess)
+      return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_coef: memset failed");
+    const dim3 ogrid(unsigned((m + 511) / 512), unsigned(std::min((t->d_out + 31) / 32, 65535)));
+    output_most_kernel<<<ogrid, 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most);
+    output_slices_kernel<<<unsigned(L.slices), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, gh, gl, gscale,
+                                                             scale);
+    tensor_basis(*t, x + p0 * ldx, m, ldx, grow, L.gstride, st);
+    // two blocks of 8 warps per SM while their rows fit (up to ~330 slots), else one of 16
+    if (coef_smem(8, t->n_slots) <= (kSmemMax - 2048) / 2)
+      launch_coef_panel<8, 2>(*t, L, grow, gscale, AH, AL, S, sms, st);
+    else
+      launch_coef_panel<16, 1>(*t, L, grow, gscale, AH, AL, S, sms, st);
+    SMX_LAUNCH_CHECK("smx_tensor_vjp_coef");
+    SplitGemm s{};
+    s.bits = kF16;
+    s.sliced = true;
+    s.Ah = AH, s.Al = AL, s.Bh = gh, s.Bl = gl;
+    s.row_scale = S, s.ld_scale = L.E;
+    s.col_scale = scale;
+    s.M = int(L.E), s.N = t->d_out, s.K = int(L.slices * 64);
+    s.D = dC, s.ldd = t->d_out;
+    s.err = t->err, s.splits = t->splits, s.partial = reinterpret_cast<float*>(q);
+    s.accumulate = p0 > 0;
+    const int rc = split_gemm(s, st);
+    if (rc) return rc;
+  }
+  return SMX_OK;
+}
 
 extern "C" int smx_tensor_bwd_operands(const float* C, int64_t n_rows, int d_out, int64_t ldo, uint16_t* Rh,
                                        uint16_t* Rl, float* row_scale, float* out_scale, void* stream) {

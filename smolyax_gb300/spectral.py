@@ -381,7 +381,7 @@ class SpectralPlan:
             Rd = T(rows, torch.float32)
             Rh, Rl = torch.empty_like(Rd), torch.empty_like(Rd)
             call("smx_split_tf32", ptr(Rd), rows.shape[0], ldo, ldo, ptr(Rh), ptr(Rl), ldo, st)
-            ops.update(Rh=Rh, Rl=Rl, ldo=ldo, walk=self._build_walk(ops, C32))
+            ops.update(Rh=Rh, Rl=Rl, ldo=ldo, walk=self._build_walk(ops, C32), coef=self._build_coef(ops, d_out))
             # tape segments of the gradient walk: fixed per plan (a point's dL/dx
             # does not depend on the batch it comes in)
             want = vjp_segment_count(K, ops["lvl1"].size)
@@ -434,6 +434,39 @@ class SpectralPlan:
             setattr(b, name, k[name].data_ptr())
         return t, b, k
 
+    def _build_coef(self, ops, d_out):
+        """``smx_tensor`` of dL/dC (``smx_tensor_vjp_coef``), or None where the basis
+        rows do not fit in shared memory."""
+        import ctypes
+
+        K = ops["K"]
+        if K == 0:
+            return None
+        t = self._tensor_struct(ops, d_out)
+        tape = torch.zeros(2 * 64 * t.n_groups, dtype=torch.int32, device=self.fam.device)
+        call("smx_tensor_tape", ptr(ops["tape"]), K, ptr(tape), capi.stream_ptr(torch.cuda.current_stream()))
+        t.tape = tape.data_ptr()
+        t.splits = capi.size("smx_tensor_coef_splits", d_out, K)
+        per_point = 68 * t.n_groups * 4 + 4 * t.n_slots + 4 * d_out
+        t.chunk = max(128, min(int(self.memory_limit * 1024**3 // per_point), 1 << 22) // 128 * 128)
+        return (t, tape) if capi.size("smx_tensor_vjp_coef_workspace", ctypes.byref(t), 64) else None
+
+    def _vjp_coef(self, x, g):
+        """dL/dC [n_lambda, d_out] FP64 but for the constant's row."""
+        import ctypes
+
+        ops = self._backward_ops()
+        t, _ = ops["coef"]
+        P, d_out, K = int(x.shape[0]), int(g.shape[1]), ops["K"]
+        nws = capi.size("smx_tensor_vjp_coef_workspace", ctypes.byref(t), P)
+        ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
+        rows = torch.empty(64 * t.n_groups, d_out, dtype=torch.float32, device=x.device)
+        call("smx_tensor_vjp_coef", ctypes.byref(t), ptr(x), P, int(x.shape[1]), ptr(g), d_out, ptr(rows), ptr(ws), nws,
+             capi.stream_ptr(torch.cuda.current_stream()))
+        dC = torch.zeros(int(self.C64.shape[0]), d_out, dtype=torch.float64, device=x.device)
+        dC[ops["ent"]] = rows[64 * t.n_groups - K :].double()  # the padding comes first
+        return dC
+
     def vjp_x_workspace(self, P):
         """Device bytes of scratch of one dL/dx of P points."""
         import ctypes
@@ -481,8 +514,13 @@ class SpectralPlan:
         if need_x and ops["walk"] is not None:
             dx = self._vjp_x_walk(x, gf)
             need_x = False
-        g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
-        g32[:, :d_out] = gf
+        if need_coef and ops["coef"] is not None and P:
+            dC = self._vjp_coef(x, gf)
+            dC[0] = g.double().sum(0)
+            need_coef = False
+        if need_x or need_coef:
+            g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
+            g32[:, :d_out] = gf
         if need_x:
             gh, gl = torch.empty_like(g32), torch.empty_like(g32)
             call("smx_split_tf32", ptr(g32), P, ldo, ldo, ptr(gh), ptr(gl), ldo, st)
