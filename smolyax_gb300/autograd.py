@@ -4,7 +4,7 @@
 built interpolant and registers a hand-written backward:
 
 * dL/dx      -- G = g C^T on the tensor cores, then a reverse pass through the
-                basis products per point (``smx_spectral_vjp_x``);
+                basis products per point (``smx_tensor_vjp_x``);
 * dL/dvalues -- dL/dC = A(x)^T g on the tensor cores, the adjoint of the FP64
                 coefficient transform (``smx_spectral_coefficients_adjoint``)
                 and the chain rule through the plan's rows
@@ -19,6 +19,17 @@ from __future__ import annotations
 import torch
 
 
+def _row_factors(keep):
+    """The plan's constants of the chain rule, laid out with its first gradient:
+    zeta of every row, the first row's value and the sum of all zeta (reading them
+    back costs a synchronisation each, which a backward does not repeat)."""
+    if "row_factors" not in keep:
+        eoff = keep["sum_eoff"]
+        zrow = torch.repeat_interleave(keep["sum_zeta"].double(), (eoff[1:] - eoff[:-1]))[:, None]
+        keep["row_factors"] = (zrow, int(keep["umap"][0].item()), float(keep["sum_zeta"].sum().item()))
+    return keep["row_factors"]
+
+
 def _fu_gradient(ip, Fbar, dC_root):
     """Chain rule from dL/dF (plan rows) and dL/d(constant term) to dL/dfu."""
     P = ip._plan
@@ -28,12 +39,9 @@ def _fu_gradient(ip, Fbar, dC_root):
     R = P.c.n_entries
     if R == 0:
         return dfu
-    eoff = keep["sum_eoff"]
-    zrow = torch.repeat_interleave(keep["sum_zeta"].double(), (eoff[1:] - eoff[:-1]))
-    zF = Fbar * zrow[:, None]
+    zrow, u0, zsum = _row_factors(keep)
+    zF = Fbar * zrow
     dfu.index_add_(0, keep["umap"], zF)
-    u0 = int(keep["umap"][0].item())
-    zsum = float(keep["sum_zeta"].sum().item())
     # F = zeta (fu[umap] - c), offset = zeta0 fu[u0] + c sum(zeta), c = fu[u0]
     dfu[u0] += -zF.sum(0) + zsum * dC_root + float(keep["zeta0"]) * dC_root
     return dfu
@@ -52,12 +60,15 @@ class _SmolyakFunction(torch.autograd.Function):
         ip = ctx.ip
         sp = ip.spectral_plan()
         need_x, need_fu = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-        dx, dC = sp.vjp(x.contiguous(), g.contiguous(), need_x=need_x, need_coef=need_fu)
+        # the error flag is read once everything is queued
+        dx, dC = sp.vjp(x.contiguous(), g.contiguous(), need_x=need_x, need_coef=need_fu, check=False)
         dfu = None
         if need_fu:
             Fbar = sp.coefficient_adjoint(dC)
             dfu = _fu_gradient(ip, Fbar, dC[0])
-        return (dx.to(x.dtype) if dx is not None else None), dfu, None
+        dx = dx.to(x.dtype) if dx is not None else None
+        sp.check_vjp()
+        return dx, dfu, None
 
 
 def interpolate(ip, x, nodal_values=None):

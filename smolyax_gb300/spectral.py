@@ -516,7 +516,7 @@ class SpectralPlan:
             need_x = False
         if need_coef and ops["coef"] is not None and P:
             dC = self._vjp_coef(x, gf)
-            dC[0] = g.double().sum(0)
+            dC[0] = g.sum(0, dtype=torch.float64)
             need_coef = False
         if need_x or need_coef:
             g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
@@ -566,9 +566,14 @@ class SpectralPlan:
             ent = ops["ent"]
             dC[ent.flip(0)] = dCrev.double()
             dC[0] = g.double().sum(0)
-        if check and int(err.item()):
-            raise RuntimeError("tensor-core contraction reported a pipeline timeout")
+        if check:
+            self.check_vjp()
         return dx, dC
+
+    def check_vjp(self):
+        """Raise if a tensor-core contraction of a backward ran into its time limit."""
+        if int(self._backward_ops()["err"].item()):
+            raise RuntimeError("tensor-core contraction reported a pipeline timeout")
 
     def coefficient_adjoint(self, dC):
         """dL/d(plan rows F64) [n_entries, d_out] from dL/dC (FP64 adjoint transform)."""
