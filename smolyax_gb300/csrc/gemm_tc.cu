@@ -49,20 +49,20 @@ constexpr int kChunkTf32 = 64 / kBK;
 constexpr int kChunkBf16 = 256 / (2 * kBK);
 constexpr int kChunkF16 = 64 / (2 * kBK);  // scaled FP16: one row scale per 64 products
 
-template <int BN, int S = 0>
+template <int BN>
 struct Tile {
   static constexpr int kN = BN;
   static constexpr int kCols = BN < 128 ? BN : 128;  // columns per drain warp
   static constexpr int kDrainWarps = 4 * (BN / kCols);
   static constexpr int kWarpTMA = kDrainWarps, kWarpMMA = kDrainWarps + 1;
   static constexpr int kThreads = 32 * (kDrainWarps + 2);
-  static constexpr int kStages = S ? S : BN == 64 ? 4 : BN == 128 ? 3 : 2;  // 48, 64 or 96 KB stages in ~192 KB
+  static constexpr int kStages = BN == 64 ? 4 : BN == 128 ? 3 : 2;  // 48, 64 or 96 KB stages in ~192 KB
   static constexpr int kA = kBM * kBK * 4;
   static constexpr int kB = BN * kBK * 4;
   static constexpr int kStage = 2 * kA + 2 * kB;
   static constexpr int kEpiLd = kCols + 4;  // epilogue staging row stride (floats): 16-byte rows, conflict-free
-  static constexpr int kEpi = kDrainWarps * 32 * kEpiLd * 4;
-  static constexpr int kTiles = kStages * kStage > kEpi ? kStages * kStage : kEpi;
+  static constexpr int kTiles = kStages * kStage;
+  static_assert(kDrainWarps * 32 * kEpiLd * 4 <= kTiles, "epilogue staging must fit");
   static constexpr int kTotal = kTiles + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -87,14 +87,14 @@ struct GemmArgs {
 // kind::f16 on 16-bit operands (64 per slice).  Same slices, stages and MMAs;
 // kF16 multiplies each drained accumulator by its row's scale of the slice and
 // the result by the column's.
-template <int KIND, int BN, int S>
-__global__ void __launch_bounds__(Tile<BN, S>::kThreads, S == 1 ? 2 : 1)
+template <int KIND, int BN>
+__global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                        const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, GemmArgs g) {
   constexpr bool BF16 = KIND != kTf32;  // 16-bit operands
   constexpr int EK = BF16 ? 2 * kBK : kBK;  // elements per K-tile
   constexpr int kChunk = KIND == kF16 ? kChunkF16 : BF16 ? kChunkBf16 : kChunkTf32;
-  using L = Tile<BN, S>;
+  using L = Tile<BN>;
   constexpr int kBN = BN, kCols = L::kCols, kEpiLd = L::kEpiLd;
   constexpr int kStages = L::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -384,11 +384,11 @@ int operand_map(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t K, int64
   return make_map(tm, ptr, (K + ek - 1) / ek * rows, ek, ek, box_rows, kind);
 }
 
-template <int KIND, int BN, int S = 0>
+template <int KIND, int BN>
 int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, const void* Bl, int64_t ldb, int M,
                 int N, int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
                 int splits, uint64_t wait_ns, int no_loads, const SplitGemm* sc) {
-  using L = Tile<BN, S>;
+  using L = Tile<BN>;
   CUtensorMap tBh, tBl;
   int rc;
   if ((rc = operand_map(&tBh, Bh, N, K, ldb, BN, KIND, sc && sc->sliced)) ||
@@ -396,7 +396,7 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
     return rc;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(gemm_tf32x3_kernel<KIND, BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
+    cudaFuncSetAttribute(gemm_tf32x3_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
     attr = true;
   }
   // split-K: slice z runs K-tiles [z * kt_per_z, ...) into D + z * zstride
@@ -411,17 +411,14 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
     if (sc->sliced) g.rows_a = M, g.rows_b = N;
   }
   dim3 grid((N + BN - 1) / BN, (M + kBM - 1) / kBM, nz);
-  gemm_tf32x3_kernel<KIND, BN, S><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
+  gemm_tf32x3_kernel<KIND, BN><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
   SMX_LAUNCH_CHECK(KIND == kTf32 ? "smx_gemm_tf32x3" : KIND == kBf16 ? "smx_gemm_bf16x3" : "smx_tensor_eval");
   return SMX_OK;
 }
 
 // Tiles by the product's width: 128 x 64 up to 64 columns (no padding to 128, half
 // the accumulators to drain: 1e5 x 64 outputs over K = 4999 in 394 us, 484 us with
-// 128 x 128), 128 x 128 up to 192, 128 x 256 beyond.  A product of one slice of K
-// has no pipeline to fill, so two single-stage blocks share an SM and one's loads
-// and MMAs run under the other's stores (5120 x 1e5 outputs over K = 64: 791 us,
-// 844 us with 128 x 256 and one block).
+// 128 x 128), 128 x 128 up to 192, 128 x 256 beyond.
 template <int KIND>
 int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const void* Bl, int64_t ldb, int M, int N,
            int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
@@ -431,10 +428,6 @@ int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const vo
   if ((rc = operand_map(&tAh, Ah, M, K, lda, kBM, KIND, sc && sc->sliced)) ||
       (rc = operand_map(&tAl, Al, M, K, lda, kBM, KIND, sc && sc->sliced)))
     return rc;
-  if constexpr (KIND == kF16)
-    if (K <= 2 * kBK && N > 64)
-      return launch_tile<KIND, 128, 1>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits,
-                                       wait_ns, no_loads, sc);
   if (N <= 64)
     return launch_tile<KIND, 64>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
                                  no_loads, sc);

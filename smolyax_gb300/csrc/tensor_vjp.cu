@@ -15,7 +15,7 @@
 // the order of every sum is fixed.  Traffic that has to be: G^T written and read
 // once.  Leja d_in = 200, d_out = 64, |Lambda| = 5000, 1e5 points: the walk takes
 // 1.35 ms (60 % of its issue slots and 58 % of the shared-memory pipe busy, the
-// bound), G^T 0.84 ms, basis and cotangent 0.14 ms; the TF32 product and the walk
+// bound), G^T 0.33 ms, basis and cotangent 0.14 ms; the TF32 product and the walk
 // per path factor through global memory took 0.82 + 3.94 ms.  On the way: terms
 // read from global memory by each warp 1.68 ms, two stages instead of four 1.46 ms.
 #include <cuda_fp16.h>
@@ -143,6 +143,228 @@ __global__ void split_rows_kernel(const float* __restrict__ C, int64_t n, int d_
     hi[e * ldo + o] = h;
     lo[e * ldo + o] = __float2half_rn(v - __half2float(h));
   }
+}
+
+// ---- G^T = C g^T, few outputs -------------------------------------------------------------
+// D[p / 32][entry][32] from R (128 entries a tile) and the cotangents (128 points a
+// tile), up to 128 outputs: the contraction is one or two slices of 64, so the
+// kernel is bound by writing D and runs as a persistent pipeline.  A block takes a
+// run of tiles, entries fastest, so that the points' operand stays in shared
+// memory; warp 8 streams R (three stages of TMA), one thread of warp 9 issues the
+// MMAs into four accumulators of 128 columns, and warps 0 - 7 drain them (row
+// scale per slice, column scale), stage 32 x 32 values and write them by TMA.
+// 5120 x 1e5 values from 64 outputs: 326 us (6.3 TB/s of writes); the general
+// product, a block per tile with nothing to overlap, took 793 us.
+// Every wait is bounded: on timeout the block sets an error code, finishes its own
+// copies and MMAs (bounded) and frees tensor memory.
+constexpr int kAdjStages = 3, kAdjAcc = 4, kAdjDrain = 8;
+constexpr int kAdjThreads = 32 * (kAdjDrain + 2);
+constexpr int kAdjTile = 32 * 1024;  // 128 rows x 64 values, high and low part
+constexpr int kAdjMaxSlices = 2;
+constexpr int kAdjSmem = kAdjStages * kAdjTile + kAdjMaxSlices * kAdjTile + kAdjDrain * 2 * 4096 + 1024 + 256;
+
+struct AdjArgs {
+  int MT, slices, M;
+  int64_t tiles;  // point tiles x MT
+  const float* row_scale;  // [slice][M]
+  const float* col_scale;  // by point, readable to whole tiles of 128
+  int* err;
+};
+
+__global__ void __launch_bounds__(kAdjThreads, 1)
+    adjoint_kernel(const __grid_constant__ CUtensorMap tmRh, const __grid_constant__ CUtensorMap tmRl,
+                   const __grid_constant__ CUtensorMap tmGh, const __grid_constant__ CUtensorMap tmGl,
+                   const __grid_constant__ CUtensorMap tmD, AdjArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* B = base + kAdjStages * kAdjTile;
+  uint8_t* out = B + kAdjMaxSlices * kAdjTile;
+  uint64_t* a_full = reinterpret_cast<uint64_t*>(out + kAdjDrain * 2 * 4096);
+  uint64_t* a_empty = a_full + kAdjStages;
+  uint64_t* b_full = a_empty + kAdjStages;  // [kAdjMaxSlices]
+  uint64_t* b_empty = b_full + kAdjMaxSlices;
+  uint64_t* acc_full = b_empty + kAdjMaxSlices;
+  uint64_t* acc_empty = acc_full + kAdjAcc;
+  uint64_t* flush = acc_empty + kAdjAcc;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(flush + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = a.slices, nb = kAdjMaxSlices / q;  // buffers of the points' operand
+  const int64_t t0 = a.tiles * blockIdx.x / gridDim.x, t1 = a.tiles * (blockIdx.x + 1) / gridDim.x;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kAdjStages; ++i) mbar_init(&a_full[i], 1), mbar_init(&a_empty[i], 1);
+    for (int i = 0; i < kAdjMaxSlices; ++i) mbar_init(&b_full[i], 1), mbar_init(&b_empty[i], 1);
+    for (int i = 0; i < kAdjAcc; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], kAdjDrain);
+    mbar_init(flush, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(kAdjAcc * 128));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == kAdjDrain) {
+    if (lane == 0) {  // ---- copies
+      int64_t last = -1;
+      int u = 0, n = 0;
+      bool ok = true;
+      for (int64_t t = t0; t < t1 && ok; ++t) {
+        const int64_t pt = t / a.MT;
+        const int mt = int(t - pt * a.MT);
+        if (pt != last) {
+          const int b = n % nb;
+          if (n >= nb && !mbar_wait(&b_empty[b], ((n / nb) & 1) ^ 1, abort_flag)) break;
+          mbar_expect_tx(&b_full[b], q * kAdjTile);
+          for (int s = 0; s < q; ++s) {
+            uint8_t* d = B + (b * q + s) * kAdjTile;
+            tma_load_2d(d, &tmGh, s * 64, int(pt * 128), &b_full[b]);
+            tma_load_2d(d + kAdjTile / 2, &tmGl, s * 64, int(pt * 128), &b_full[b]);
+          }
+          last = pt, ++n;
+        }
+        for (int s = 0; s < q; ++s, ++u) {
+          const int i = u % kAdjStages;
+          if (u >= kAdjStages && !mbar_wait(&a_empty[i], ((u / kAdjStages) & 1) ^ 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&a_full[i], kAdjTile);
+          tma_load_2d(base + i * kAdjTile, &tmRh, s * 64, mt * 128, &a_full[i]);
+          tma_load_2d(base + i * kAdjTile + kAdjTile / 2, &tmRl, s * 64, mt * 128, &a_full[i]);
+        }
+      }
+      if (*abort_flag || u < int((t1 - t0) * q)) {  // gave up: wait (bounded) for what was issued
+        atomicExch(a.err, 1);
+        *abort_flag = 1;
+        for (int v = max(0, u - kAdjStages); v < u; ++v)
+          mbar_wait(&a_full[v % kAdjStages], (v / kAdjStages) & 1, nullptr);
+        for (int v = max(0, n - nb); v < n; ++v) mbar_wait(&b_full[v % nb], (v / nb) & 1, nullptr);
+      }
+    }
+    __syncwarp();
+  } else if (warp == kAdjDrain + 1) {
+    if (lane == 0) {  // ---- MMAs
+      constexpr uint32_t idesc = idesc_fmt(128, 128, 0u);
+      int64_t last = -1;
+      int u = 0, n = 0;
+      bool ok = true;
+      for (int64_t t = t0; t < t1 && ok; ++t) {
+        const int64_t pt = t / a.MT;
+        if (pt != last) {
+          if (n > 0) mma_commit(&b_empty[(n - 1) % nb]);
+          ok = mbar_wait(&b_full[n % nb], (n / nb) & 1, abort_flag);
+          last = pt, ++n;
+        }
+        for (int s = 0; s < q && ok; ++s, ++u) {
+          const int i = u % kAdjStages, c = u % kAdjAcc;
+          if ((u >= kAdjAcc && !mbar_wait(&acc_empty[c], ((u / kAdjAcc) & 1) ^ 1, abort_flag)) ||
+              !mbar_wait(&a_full[i], (u / kAdjStages) & 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint32_t ah = smem_u32(base + i * kAdjTile), al = ah + kAdjTile / 2;
+          const uint32_t bh = smem_u32(B + (((n - 1) % nb) * q + s) * kAdjTile), bl = bh + kAdjTile / 2;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {  // 16 values of 64 per MMA
+            const uint64_t dah = make_desc_sw(ah + k * 32, 128), dal = make_desc_sw(al + k * 32, 128);
+            const uint64_t dbh = make_desc_sw(bh + k * 32, 128), dbl = make_desc_sw(bl + k * 32, 128);
+            mma_op<true>(tmem + c * 128, dah, dbh, idesc, k ? 1u : 0u);
+            mma_op<true>(tmem + c * 128, dah, dbl, idesc, 1u);
+            mma_op<true>(tmem + c * 128, dal, dbh, idesc, 1u);
+          }
+          mma_commit(&a_empty[i]);
+          mma_commit(&acc_full[c]);
+        }
+      }
+      if (!ok) {  // finish the MMAs issued (bounded), then let the others stop
+        mma_commit(flush);
+        mbar_wait(flush, 0, nullptr);
+        atomicExch(a.err, 2);
+        *abort_flag = 1;
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- drain: rows 32 (warp % 4) .. + 31 of a tile, two of its four blocks of 32 points
+    const int quad = warp & 3, half = warp >> 2;
+    uint8_t* stage = out + warp * 8192;
+    int u = 0, n = 0;
+    for (int64_t t = t0; t < t1; ++t, u += q) {
+      const int64_t pt = t / a.MT;
+      const int e0 = int(t - pt * a.MT) * 128 + quad * 32;
+      float rs[kAdjMaxSlices];
+      bool ok = true;
+#pragma unroll
+      for (int s = 0; s < kAdjMaxSlices; ++s) {
+        rs[s] = s < q ? __ldg(a.row_scale + int64_t(s) * a.M + min(e0 + lane, a.M - 1)) : 0.f;
+        if (s < q) ok = ok && mbar_wait(&acc_full[(u + s) % kAdjAcc], ((u + s) / kAdjAcc) & 1, abort_flag);
+      }
+      if (!__all_sync(0xffffffffu, ok && !*abort_flag)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int j = 0; j < 2; ++j, ++n) {
+        const int cb = 2 * half + j;
+        float v[32];
+#pragma unroll
+        for (int s = 0; s < kAdjMaxSlices; ++s) {
+          if (s >= q) break;
+          uint32_t r[32];
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+              "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+                "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+                "=r"(r[30]), "=r"(r[31])
+              : "r"(tmem + (uint32_t(quad * 32) << 16) + uint32_t(((u + s) % kAdjAcc) * 128 + cb * 32)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            v[i] = s ? fmaf(rs[s], __uint_as_float(r[i]), v[i]) : rs[0] * __uint_as_float(r[i]);
+        }
+        if (j == 1) {  // the accumulators have been read
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          __syncwarp();
+          if (lane == 0)
+            for (int s = 0; s < q; ++s) mbar_arrive(&acc_empty[(u + s) % kAdjAcc]);
+        }
+        const float4* cs = reinterpret_cast<const float4*>(a.col_scale + pt * 128 + cb * 32);
+        uint8_t* buf = stage + (n & 1) * 4096;
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 c = __ldg(cs + i);
+          *reinterpret_cast<float4*>(buf + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+              make_float4(v[4 * i] * c.x, v[4 * i + 1] * c.y, v[4 * i + 2] * c.z, v[4 * i + 3] * c.w);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          if (e0 < a.M)
+            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
+                             reinterpret_cast<uint64_t>(&tmD)),
+                         "r"(0), "r"(e0), "r"(int(pt * 4 + cb)), "r"(smem_u32(buf))
+                         : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAdjAcc * 128));
 }
 
 // Product of up to 8 slots' values.
@@ -471,9 +693,40 @@ Layout layout(const smx_tensor* t, const smx_tensor_bwd* b, int64_t m) {
   L.rows = up256(size_t(t->n_slots) * L.gstride * 4);
   L.gt = up256(size_t(b->n_rows) * L.gstride * 4);
   L.half = up256(size_t(m) * b->ldo * 2);
-  L.scale = up256(size_t(m) * 4);
+  L.scale = up256(size_t(L.gstride) * 4);
   L.total = 2 * L.rows + L.gt + 2 * L.half + L.scale;
   return L;
+}
+
+// G^T of m points (adjoint_kernel).
+int adjoint_gemm(const smx_tensor& t, const smx_tensor_bwd& b, const __half* gh, const __half* gl, const float* gs,
+                 float* GT, int64_t m, int64_t gstride, int sms, cudaStream_t st) {
+  PFN_cuTensorMapEncodeTiled_v12000 encode;
+  CUtensorMap tRh, tRl, tGh, tGl, tD;
+  int rc = tensor_map_encoder(&encode);
+  if (rc || (rc = panel_map(&tRh, b.Rh, b.n_rows, b.ldo, b.ldo, 128, kF16)) ||
+      (rc = panel_map(&tRl, b.Rl, b.n_rows, b.ldo, b.ldo, 128, kF16)) ||
+      (rc = panel_map(&tGh, gh, m, b.ldo, b.ldo, 128, kF16)) || (rc = panel_map(&tGl, gl, m, b.ldo, b.ldo, 128, kF16)))
+    return rc;
+  const cuuint64_t dims[3] = {32, cuuint64_t(b.n_rows), cuuint64_t(gstride / 32)};
+  const cuuint64_t strides[2] = {128, cuuint64_t(b.n_rows) * 128};
+  const cuuint32_t box[3] = {32, 32, 1}, estr[3] = {1, 1, 1};
+  if (encode(&tD, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, GT, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_x: cuTensorMapEncodeTiled failed");
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdjSmem);
+    attr = true;
+  }
+  AdjArgs a{};
+  a.MT = int((b.n_rows + 127) / 128), a.slices = int(b.ldo / 64), a.M = int(b.n_rows);
+  a.tiles = (m + 127) / 128 * a.MT;
+  a.row_scale = b.row_scale, a.col_scale = gs, a.err = t.err;
+  adjoint_kernel<<<unsigned(std::min<int64_t>(a.tiles, sms)), kAdjThreads, kAdjSmem, st>>>(tRh, tRl, tGh, tGl, tD, a);
+  SMX_LAUNCH_CHECK("smx_tensor_vjp_x adjoints");
+  return SMX_OK;
 }
 
 size_t coef_smem(int warps, int slots) { return size_t(warps) * (1024 + 9 * 256) + size_t(slots) * 256; }
@@ -656,6 +909,10 @@ extern "C" int smx_tensor_vjp_x(const smx_tensor* t, const smx_tensor_bwd* b, co
     cudaFuncSetAttribute(vjp_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax));
     attr = true;
   }
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_x: no device");
   for (int64_t p0 = 0; p0 < P; p0 += b->chunk) {
     const int64_t m = std::min(b->chunk, P - p0);
     const Layout L = layout(t, b, m);
@@ -670,17 +927,21 @@ extern "C" int smx_tensor_vjp_x(const smx_tensor* t, const smx_tensor_bwd* b, co
     vjp_basis_kernel<<<bgrid, 256, 0, st>>>(*t, x + p0 * ldx, m, ldx, grow, drow, L.gstride);
     cotangent_kernel<<<smx::grid_for(m, 8), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, b->ldo, b->out_scale, gh, gl,
                                                           gs);
-    SplitGemm s{};
-    s.bits = kF16;
-    s.Ah = b->Rh, s.Al = b->Rl, s.lda = b->ldo;
-    s.Bh = gh, s.Bl = gl, s.ldb = b->ldo;
-    s.row_scale = b->row_scale, s.ld_scale = b->n_rows;
-    s.col_scale = gs;
-    s.M = int(b->n_rows), s.N = int(m), s.K = t->d_out;
-    s.D = GT, s.ldd = 0;
-    s.err = t->err, s.splits = 1;
-    int rc = split_gemm(s, st);
-    if (rc) return rc;
+    int rc;
+    if (b->ldo <= 64 * kAdjMaxSlices) {
+      if ((rc = adjoint_gemm(*t, *b, gh, gl, gs, GT, m, L.gstride, sms, st))) return rc;
+    } else {
+      SplitGemm s{};
+      s.bits = kF16;
+      s.Ah = b->Rh, s.Al = b->Rl, s.lda = b->ldo;
+      s.Bh = gh, s.Bl = gl, s.ldb = b->ldo;
+      s.row_scale = b->row_scale, s.ld_scale = b->n_rows;
+      s.col_scale = gs;
+      s.M = int(b->n_rows), s.N = int(m), s.K = t->d_out;
+      s.D = GT, s.ldd = 0;
+      s.err = t->err, s.splits = 1;
+      if ((rc = split_gemm(s, st))) return rc;
+    }
     vjp_walk_kernel<<<smx::grid_for(m, 32), kThreads, walk_smem(t, w), st>>>(*t, w, grow, drow, L.gstride, GT, m,
                                                                               t->err, dx + p0 * lddx, lddx);
     SMX_LAUNCH_CHECK("smx_tensor_vjp_x");
