@@ -1097,12 +1097,12 @@ bool build_walk(const Tree& tr, const int64_t* maxdeg, int d, Tables& out) {
     owner[i] = argmin(load, kW);
     load[owner[i]] += double(weight[i]);
   }
-  // entries to chunks: the largest chunks of which four fit beside the rows
+  // entries to chunks: the largest chunks of which three fit beside the rows
   const std::vector<int64_t> ent =
       stable_order(K, [&](int64_t i) { return std::make_pair(slot[i + 1], tr.parent[i + 1]); });
   std::vector<int32_t> perm, off, terms;
   int64_t E = 0, n_chunks = 0, most = 0;
-  for (int64_t c : {128, 64, 32, 16}) {
+  for (int64_t c : {256, 128, 64, 32, 16}) {
     E = c;
     n_chunks = (K + E - 1) / E;
     perm.assign(n_chunks * E, -1);
@@ -1148,7 +1148,7 @@ bool build_walk(const Tree& tr, const int64_t* maxdeg, int d, Tables& out) {
       off.push_back(int32_t(terms.size() / 2));
       most = std::max(most, int64_t(terms.size() / 2 - begin));
     }
-    if (rows * 128 + 4 * (E * 128 + most * 8) + 256 <= 226 * 1024) break;
+    if (rows * 128 + 3 * (E * 128 + most * 8) + 256 <= 226 * 1024) break;
     E = 0;
   }
   if (E == 0) return false;

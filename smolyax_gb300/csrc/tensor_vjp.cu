@@ -14,10 +14,11 @@
 // adjoint is read, updated and written per path factor in global memory, and
 // the order of every sum is fixed.  Traffic that has to be: G^T written and read
 // once.  Leja d_in = 200, d_out = 64, |Lambda| = 5000, 1e5 points: the walk takes
-// 1.35 ms (60 % of its issue slots and 58 % of the shared-memory pipe busy, the
+// 1.17 ms (56 % of its issue slots and 61 % of the shared-memory pipe busy, the
 // bound), G^T 0.33 ms, basis and cotangent 0.14 ms; the TF32 product and the walk
 // per path factor through global memory took 0.82 + 3.94 ms.  On the way: terms
-// read from global memory by each warp 1.68 ms, two stages instead of four 1.46 ms.
+// read from global memory by each warp 1.68 ms, two stages of 128 entries 1.46 ms,
+// four 1.35 ms; three of 256 halve the steps between chunks.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -30,7 +31,7 @@ namespace {
 
 using namespace smx::tc;
 
-constexpr int kStages = 4;  // chunks in flight (layout.cu build_walk sizes them)
+constexpr int kStages = 3;  // chunks in flight (layout.cu build_walk sizes them)
 constexpr int kWarps = 32;  // owners of destination rows (layout.cu build_walk)
 constexpr int kThreads = 32 * kWarps;
 constexpr size_t kSmemMax = 227 * 1024;
@@ -416,7 +417,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int c = 0; c < min(kStages, w.n_chunks); ++c) load_chunk(c);
   }
-  for (int s = warp; s < ns; s += kWarps) row[s * 32] = grow[s * gstride + p];
+#pragma unroll 8
+  for (int s = warp; s < ns; s += kWarps) row[s * 32] = __ldg(grow + s * gstride + p);
   for (int s = row_bar + warp; s < n_rows; s += kWarps) row[s * 32] = 0.f;
   __syncthreads();
   for (int n0 = warp; n0 < nn; n0 += kWarps * 32) {  // a lane's load for each of 32 nodes
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       auto g = [&](int o) { return *reinterpret_cast<const float*>(gs + o); };
       int4 a = term[0];
       float sa = *at(a.x & 0xffff), sb = *at(a.z & 0xffff), ga = g(a.y), gb = g(a.w);
-#pragma unroll 1
+#pragma unroll 2
       for (int i = 1; i <= n; ++i) {
         float *da = at(unsigned(a.x) >> 16), *db = at(unsigned(a.z) >> 16);
         const float va = fmaf(sa, ga, *da), vb = fmaf(sb, gb, *db);
@@ -483,30 +485,44 @@ __global__ void __launch_bounds__(kThreads, 1)
     return;
   }
   // path factors; the slot's adjoint times its derivative in its row of bar
-  for (int i = __ldg(w.warp + warp); i < __ldg(w.warp + warp + 1); ++i) {
-    const int4 s = __ldg(reinterpret_cast<const int4*>(w.slot) + i);
-    float rest = row[(row_bar + s.x) * 32];
-    for (int q0 = s.y; q0 < s.z; q0 += 32) {  // a lane's load for each of 32 factors
-      const int n = min(32, s.z - q0), q = q0 + min(lane, n - 1), r = __ldg(w.row + q);
-      const int4 other = __ldg(reinterpret_cast<const int4*>(w.other) + q);
-      for (int k = 0; k < n; ++k)
-        rest = fmaf(row[__shfl_sync(0xffffffffu, r, k) * 32], slot_product(row, from_lane(other, k)), rest);
+  const int i1 = __ldg(w.warp + warp + 1);
+  for (int i0 = __ldg(w.warp + warp); i0 < i1; i0 += 32) {  // a lane's load for each of 32 slots
+    const int ni = min(32, i1 - i0);
+    const int4 of = __ldg(reinterpret_cast<const int4*>(w.slot) + i0 + min(lane, ni - 1));
+    float next = __ldg(drow + __shfl_sync(0xffffffffu, of.x, 0) * gstride + p);
+    for (int i = 0; i < ni; ++i) {
+      const int4 s = from_lane(of, i);
+      const float d = next;
+      next = __ldg(drow + __shfl_sync(0xffffffffu, of.x, min(i + 1, ni - 1)) * gstride + p);
+      float rest = row[(row_bar + s.x) * 32];
+      for (int q0 = s.y; q0 < s.z; q0 += 32) {  // ... and for each of 32 factors
+        const int n = min(32, s.z - q0), q = q0 + min(lane, n - 1), r = __ldg(w.row + q);
+        const int4 other = __ldg(reinterpret_cast<const int4*>(w.other) + q);
+        for (int k = 0; k < n; ++k)
+          rest = fmaf(row[__shfl_sync(0xffffffffu, r, k) * 32], slot_product(row, from_lane(other, k)), rest);
+      }
+      row[(row_bar + s.x) * 32] = rest * d;
     }
-    row[(row_bar + s.x) * 32] = rest * drow[s.x * gstride + p];
   }
   __syncthreads();
   // per dimension the sum over its degrees, turned in the place of phi and V
   float* turn = reinterpret_cast<float*>(smem);  // [n_dims][33]: ends before bar (checked on the host)
-  for (int h = warp; h < t.n_dims; h += kWarps) {
-    const int so = __ldg(t.dsoff + h), g = __ldg(t.dmax + h);
-    float acc = 0.f;
-    for (int n = 0; n < g; ++n) acc += row[(row_bar + so + n) * 32];
-    turn[h * 33 + lane] = acc;
+  for (int h0 = warp; h0 < t.n_dims; h0 += kWarps * 32) {
+    const int n = min(32, (t.n_dims - h0 + kWarps - 1) / kWarps), at = h0 + min(lane, n - 1) * kWarps;
+    const int so = __ldg(t.dsoff + at), g = __ldg(t.dmax + at);
+    for (int k = 0; k < n; ++k) {
+      const float* bar = row + (row_bar + __shfl_sync(0xffffffffu, so, k)) * 32;
+      const int gk = __shfl_sync(0xffffffffu, g, k);
+      float acc = 0.f;
+      for (int m = 0; m < gk; ++m) acc += bar[m * 32];
+      turn[(h0 + k * kWarps) * 33 + lane] = acc;
+    }
   }
   __syncthreads();
   for (int q = warp; q < 32; q += kWarps) {
     if (p0 + q >= P) break;
     double* out = dx + (p0 + q) * lddx;
+#pragma unroll 4
     for (int j = lane; j < t.d_in; j += 32) {
       const int h = __ldg(w.dim_index + j);
       out[j] = h < 0 ? 0.0 : double(__ldg(t.fam_a + j)) * double(turn[h * 33 + q]);

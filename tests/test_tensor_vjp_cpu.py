@@ -47,7 +47,7 @@ def test_walk_matches_direct_derivative(d, t):
     perm = lay["w_perm"]
     assert perm.size == nc * E and sorted(perm[perm >= 0]) == list(range(1, n))
     rows = np.zeros(2 * (ns + nn) + 1)
-    assert rows.size * 128 + 4 * (E * 128 + most * 8) + 256 <= 226 * 1024
+    assert rows.size * 128 + 3 * (E * 128 + most * 8) + 256 <= 226 * 1024
     rows[:ns] = phi
     for i, v in enumerate(lay["w_node_path"].reshape(-1, 4)[:nn]):
         rows[ns + i] = product(v)
