@@ -39,35 +39,52 @@ __device__ __forceinline__ float x32(double v) {
   return fabsf(f) == __int_as_float(0x7f800000) ? __int_as_float(0x7fc00000) : f;
 }
 
-// Basis rows grow[slot][p] of 32 points x 32 dimensions per block: x is read by
-// rows (32 neighbouring dimensions of a point) and turned in shared memory, then
-// lane = point.  One thread per point ran through all dimensions one after the
-// other before: 69 -> 6 us at 3001 points x 200 dimensions.
+// Basis rows grow[slot][p] (DERIV: and their derivatives in z, drow) of 32 points x
+// 32 dimensions per block: x is read by rows (32 neighbouring dimensions of a
+// point) and turned in shared memory, then lane = point.  The dimensions' table
+// entries are read beside x, not one after the other by the warps that use them.
+// x read and rows written are 160 + 100 MB at 1e5 points x 200 dimensions: 72 us (76
+// with derivatives; issue slots 79 % busy), 98 us (108) with the table entries read
+// where they are used.  One thread per point ran through all dimensions one after
+// the other at first: 69 us at 3001 points x 200 dimensions, now 6.8.
+template <bool DERIV>
 __global__ void __launch_bounds__(256) tensor_basis_kernel(smx_tensor t, const double* __restrict__ x, int64_t P,
-                                                           int64_t ldx, float* __restrict__ grow, int64_t gstride) {
+                                                           int64_t ldx, float* __restrict__ grow,
+                                                           float* __restrict__ drow, int64_t gstride) {
   __shared__ float z[32][33];
+  __shared__ int4 of[32];  // largest degree, first slot, first recurrence pair
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t p0 = blockIdx.x * int64_t(32);
   for (int h0 = blockIdx.y * 32; h0 < t.n_dims; h0 += gridDim.y * 32) {
     const int h = h0 + lane;
     if (h < t.n_dims) {
       const int dim = __ldg(t.dims + h);
+      double v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = __ldg(x + min(p0 + warp + 8 * i, P - 1) * ldx + dim);
       const float fa = __ldg(t.fam_a + dim), fb = __ldg(t.fam_b + dim);
-      for (int r = warp; r < 32; r += 8) z[lane][r] = fmaf(fa, x32(__ldg(x + min(p0 + r, P - 1) * ldx + dim)), fb);
+      if (warp == 0) of[lane] = make_int4(__ldg(t.dmax + h), __ldg(t.dsoff + h), __ldg(t.fam + dim) * t.max_deg, 0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[lane][warp + 8 * i] = fmaf(fa, x32(v[i]), fb);
     }
     __syncthreads();
     for (int q = warp; q < 32 && h0 + q < t.n_dims; q += 8) {
-      const int hq = h0 + q;
-      const int g = __ldg(t.dmax + hq), so = __ldg(t.dsoff + hq);
-      const float2* rec = reinterpret_cast<const float2*>(t.rec) + __ldg(t.fam + __ldg(t.dims + hq)) * t.max_deg;
+      const int4 m = of[q];
+      const float2* rec = reinterpret_cast<const float2*>(t.rec) + m.z;
       const float zv = z[q][lane];
-      float pm1 = 0.f, pc = 1.f;
-      for (int n = 0; n < g; ++n) {
+      float* to = grow + int64_t(m.y) * gstride + p0 + lane;
+      float* td = DERIV ? drow + int64_t(m.y) * gstride + p0 + lane : nullptr;
+      float pm1 = 0.f, pc = 1.f, dm1 = 0.f, dc = 0.f;
+      for (int n = 0; n < m.x; ++n) {
         const float2 ab = __ldg(rec + n);
         const float pn = ab.x * zv * pc - ab.y * pm1;
-        pm1 = pc;
-        pc = pn;
-        grow[int64_t(so + n) * gstride + p0 + lane] = pc;
+        if constexpr (DERIV) {
+          const float dn = ab.x * (pc + zv * dc) - ab.y * dm1;
+          dm1 = dc, dc = dn;
+          td[n * gstride] = dc;
+        }
+        pm1 = pc, pc = pn;
+        to[n * gstride] = pc;
       }
     }
     __syncthreads();
@@ -97,10 +114,12 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, const void* 
 // known, are scaled, split and written as the lane's own 128-byte row of two
 // swizzled tiles, which leave by TMA while the next group is walked; the warps
 // never wait for each other.  Bound: HBM writes, 4 bytes per value.
-// Gauss-Hermite d_in = 100, |Lambda| = 20010, 65536 points: 1.14 ms (4.6 TB/s of
+// Gauss-Hermite d_in = 100, |Lambda| = 20010, 65536 points: 1.13 ms (4.6 TB/s of
 // writes); the TF32 panel it replaces wrote twice the bytes in 3.2 ms.  Measured
 // on the way: basis rows read from global memory 3.2 ms (latency), every product
-// through the stack 1.35 ms, the tape read from global memory 1.3 - 1.8 ms.
+// through the stack 1.35 ms, the tape read from global memory 1.3 - 1.8 ms.  The
+// rows are copied with cp.async (no registers between loads and stores): Leja d_in
+// = 200, |Lambda| = 5000, 1e5 points 524 us, 554 with loads through registers.
 template <bool F16, int W, bool SROWS>
 __global__ void __launch_bounds__(32 * W, 1)
     tensor_panel_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmL, smx_tensor t,
@@ -123,7 +142,9 @@ __global__ void __launch_bounds__(32 * W, 1)
     const int64_t rs = SROWS ? 32 : gstride;
     if constexpr (SROWS) {
       __syncthreads();  // the previous points' walks are done
-      for (int i = warp; i < t.n_slots; i += W) rows[i * 32 + lane] = grow[i * gstride + p0 + lane];
+      for (int i = warp * 4 + (lane >> 3); i < t.n_slots; i += W * 4)
+        copy16(rows + i * 32 + (lane & 7) * 4, grow + i * gstride + p0 + (lane & 7) * 4);
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
     }
     if (t0 == t1) continue;
@@ -343,10 +364,13 @@ Layout layout(const smx_tensor* t, int64_t m) {
 
 }  // namespace
 
-void smx::tc::tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, int64_t ldp,
-                           cudaStream_t st) {
+void smx::tc::tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, float* drow,
+                           int64_t ldp, cudaStream_t st) {
   const dim3 grid(unsigned(ldp / 32), unsigned(std::min((t.n_dims + 31) / 32, 65535)));
-  tensor_basis_kernel<<<grid, 256, 0, st>>>(t, x, P, ldx, grow, ldp);
+  if (drow)
+    tensor_basis_kernel<true><<<grid, 256, 0, st>>>(t, x, P, ldx, grow, drow, ldp);
+  else
+    tensor_basis_kernel<false><<<grid, 256, 0, st>>>(t, x, P, ldx, grow, nullptr, ldp);
 }
 
 extern "C" int smx_tensor_operands(const float* B, int N, int K, int64_t ldb, const int32_t* tape, int32_t* tape_out,
@@ -417,7 +441,7 @@ extern "C" int smx_tensor_eval(const smx_tensor* t, const double* x, int64_t P, 
     float* part = reinterpret_cast<float*>(w + 2 * L.panel + L.scales + L.rows);
     int rc;
     if (t->K > 0) {
-      tensor_basis(*t, x + p0 * ldx, m, ldx, grow, L.gstride, st);
+      tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st);
       CUtensorMap tmH, tmL;
       const int bits = t->bf16 ? kBf16 : kF16;
       if ((rc = panel_map(&tmH, Ah, m, t->K, t->ldb, 32, bits)) ||

@@ -16,9 +16,16 @@ namespace tc {
 constexpr int kPop = 1, kPush = 2, kStackMask = 0xf80, kFactorMask = 0x7f800000;
 constexpr int kGroup = 64;  // tape entries (panel columns) per group
 
-// Basis values of all slots, grow[slot][p], p < ldp (a multiple of 32; points past
-// P repeat the last one).
-void tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, int64_t ldp,
+// 16 bytes global -> shared, asynchronously (cp.async.wait_all).
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+// Basis values of all slots, grow[slot][p], and (drow given) their derivatives,
+// p < ldp (a multiple of 32; points past P repeat the last one).
+void tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, float* drow, int64_t ldp,
                   cudaStream_t st);
 
 constexpr int kTf32 = 0, kBf16 = 1, kF16 = 2;

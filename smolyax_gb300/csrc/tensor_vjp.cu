@@ -14,8 +14,8 @@
 // adjoint is read, updated and written per path factor in global memory, and
 // the order of every sum is fixed.  Traffic that has to be: G^T written and read
 // once.  Leja d_in = 200, d_out = 64, |Lambda| = 5000, 1e5 points: the walk takes
-// 1.17 ms (56 % of its issue slots and 61 % of the shared-memory pipe busy, the
-// bound), G^T 0.33 ms, basis and cotangent 0.14 ms; the TF32 product and the walk
+// 1.12 ms (56 % of its issue slots and 61 % of the shared-memory pipe busy, the
+// bound), G^T 0.32 ms, basis and cotangent 0.10 ms; the TF32 product and the walk
 // per path factor through global memory took 0.82 + 3.94 ms.  On the way: terms
 // read from global memory by each warp 1.68 ms, two stages of 128 entries 1.46 ms,
 // four 1.35 ms; three of 256 halve the steps between chunks.
@@ -35,45 +35,6 @@ constexpr int kStages = 3;  // chunks in flight (layout.cu build_walk sizes them
 constexpr int kWarps = 32;  // owners of destination rows (layout.cu build_walk)
 constexpr int kThreads = 32 * kWarps;
 constexpr size_t kSmemMax = 227 * 1024;
-
-__device__ __forceinline__ float x32(double v) {
-  const float f = static_cast<float>(v);
-  return fabsf(f) == __int_as_float(0x7f800000) ? __int_as_float(0x7fc00000) : f;
-}
-
-// Basis values and their derivatives in z, [slot][p] (as tensor_basis_kernel).
-__global__ void __launch_bounds__(256) vjp_basis_kernel(smx_tensor t, const double* __restrict__ x, int64_t P,
-                                                        int64_t ldx, float* __restrict__ grow,
-                                                        float* __restrict__ drow, int64_t gstride) {
-  __shared__ float z[32][33];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t p0 = blockIdx.x * int64_t(32);
-  for (int h0 = blockIdx.y * 32; h0 < t.n_dims; h0 += gridDim.y * 32) {
-    const int h = h0 + lane;
-    if (h < t.n_dims) {
-      const int dim = __ldg(t.dims + h);
-      const float fa = __ldg(t.fam_a + dim), fb = __ldg(t.fam_b + dim);
-      for (int r = warp; r < 32; r += 8) z[lane][r] = fmaf(fa, x32(__ldg(x + min(p0 + r, P - 1) * ldx + dim)), fb);
-    }
-    __syncthreads();
-    for (int q = warp; q < 32 && h0 + q < t.n_dims; q += 8) {
-      const int hq = h0 + q;
-      const int g = __ldg(t.dmax + hq), so = __ldg(t.dsoff + hq);
-      const float2* rec = reinterpret_cast<const float2*>(t.rec) + __ldg(t.fam + __ldg(t.dims + hq)) * t.max_deg;
-      const float zv = z[q][lane];
-      float pm1 = 0.f, pc = 1.f, dm1 = 0.f, dc = 0.f;
-      for (int n = 0; n < g; ++n) {
-        const float2 ab = __ldg(rec + n);
-        const float pn = ab.x * zv * pc - ab.y * pm1;
-        const float dn = ab.x * (pc + zv * dc) - ab.y * dm1;
-        pm1 = pc, pc = pn, dm1 = dc, dc = dn;
-        grow[int64_t(so + n) * gstride + p0 + lane] = pc;
-        drow[int64_t(so + n) * gstride + p0 + lane] = dc;
-      }
-    }
-    __syncthreads();
-  }
-}
 
 // Cotangent rows as FP16 pairs: warp per point, v = g * out_scale, one power of
 // two per point; columns d_out .. ldo are zero.
@@ -417,9 +378,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int c = 0; c < min(kStages, w.n_chunks); ++c) load_chunk(c);
   }
-#pragma unroll 8
-  for (int s = warp; s < ns; s += kWarps) row[s * 32] = __ldg(grow + s * gstride + p);
+  for (int s = warp * 4 + (lane >> 3); s < ns; s += kWarps * 4)
+    copy16(row - lane + s * 32 + (lane & 7) * 4, grow + s * gstride + p0 + (lane & 7) * 4);
   for (int s = row_bar + warp; s < n_rows; s += kWarps) row[s * 32] = 0.f;
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   for (int n0 = warp; n0 < nn; n0 += kWarps * 32) {  // a lane's load for each of 32 nodes
     const int n = (nn - n0 + kWarps - 1) / kWarps, at = n0 + min(lane, n - 1) * kWarps;
@@ -537,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // run of tape groups as tensor_panel_kernel does (tensor_eval.cu), but an entry's 64
 // values are one register pair per lane, so they are scaled and written at once:
 // 128 contiguous bytes per entry and part.  Bound: HBM writes, 4 bytes per value.
-// Leja d_in = 200, |Lambda| = 5000, 1e5 points: 0.34 ms (6.0 TB/s of writes, issue
+// Leja d_in = 200, |Lambda| = 5000, 1e5 points: 0.33 ms (6.1 TB/s of writes, issue
 // slots 71 % busy) and 0.32 ms for the product with 64 outputs; one thread per point
 // writing TF32 pairs through 400 KB strides took 1.34 ms and its product 0.62 ms.
 template <int W, int MINB>
@@ -556,8 +518,9 @@ __global__ void __launch_bounds__(32 * W, MINB)
   auto f2 = [](uint8_t* q) -> float2& { return *reinterpret_cast<float2*>(q); };
   for (int64_t sl = blockIdx.y; sl < n_slices; sl += gridDim.y) {
     __syncthreads();  // the previous slice's walks are done
-    for (int i = warp; i < t.n_slots; i += W)
-      f2(rows + i * 256) = __ldg(reinterpret_cast<const float2*>(grow + i * gstride + sl * 64) + lane);
+    for (int i = warp * 2 + (lane >> 4); i < t.n_slots; i += W * 2)
+      copy16(rows - lane * 8 + i * 256 + (lane & 15) * 16, grow + i * gstride + sl * 64 + (lane & 15) * 4);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (t0 == t1) continue;
     const float gsc = __ldg(gscale + sl);
@@ -861,7 +824,7 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
     output_most_kernel<<<ogrid, 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most);
     output_slices_kernel<<<unsigned(L.slices), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, gh, gl, gscale,
                                                              scale);
-    tensor_basis(*t, x + p0 * ldx, m, ldx, grow, L.gstride, st);
+    tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st);
     // two blocks of 8 warps per SM while their rows fit (up to ~330 slots), else one of 16
     if (coef_smem(8, t->n_slots) <= (kSmemMax - 2048) / 2)
       launch_coef_panel<8, 2>(*t, L, grow, gscale, AH, AL, S, sms, st);
@@ -939,8 +902,7 @@ extern "C" int smx_tensor_vjp_x(const smx_tensor* t, const smx_tensor_bwd* b, co
     __half* gh = reinterpret_cast<__half*>(q + 2 * L.rows + L.gt);
     __half* gl = reinterpret_cast<__half*>(q + 2 * L.rows + L.gt + L.half);
     float* gs = reinterpret_cast<float*>(q + 2 * L.rows + L.gt + 2 * L.half);
-    const dim3 bgrid(unsigned(L.gstride / 32), unsigned(std::min((t->n_dims + 31) / 32, 65535)));
-    vjp_basis_kernel<<<bgrid, 256, 0, st>>>(*t, x + p0 * ldx, m, ldx, grow, drow, L.gstride);
+    tensor_basis(*t, x + p0 * ldx, m, ldx, grow, drow, L.gstride, st);
     cotangent_kernel<<<smx::grid_for(m, 8), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, b->ldo, b->out_scale, gh, gl,
                                                           gs);
     int rc;
