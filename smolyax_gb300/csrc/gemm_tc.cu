@@ -416,9 +416,30 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
   return SMX_OK;
 }
 
-// Tiles by the product's width: 128 x 64 up to 64 columns (no padding to 128, half
-// the accumulators to drain: 1e5 x 64 outputs over K = 4999 in 394 us, 484 us with
-// 128 x 128), 128 x 128 up to 192, 128 x 256 beyond.
+// Columns per tile: the width with the least rounds of tiles on the SMs x time of a
+// round, which measured 69, 73 and 115 - 140 us for 64, 128 and 256 columns (split
+// BF16, K = 6016: a narrow tile still loads the 128 rows of A).  Columns and rounds that
+// are not filled cost as much as full ones: 10000 x 300 outputs take 136 us with
+// 128 columns (2 rounds) and 212 with 256 (2), 65536 x 400 take 878 (14) and 785
+// (7), 10000 x 100 take 127 with 64 (2) and 76 with 128 (1).
+int tile_columns(int64_t M, int N, int64_t nz) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    sms = 152;
+  }
+  const int64_t rows = (M + kBM - 1) / kBM * nz;
+  int best = 0;
+  int64_t cost = 0;
+  for (int bn : {256, 128, 64}) {
+    const int64_t tiles = rows * ((N + bn - 1) / bn);
+    const int64_t c = (tiles + sms - 1) / sms * (bn == 256 ? 177 : bn == 128 ? 100 : 94);
+    if (!best || c < cost) best = bn, cost = c;
+  }
+  return best;
+}
+
 template <int KIND>
 int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const void* Bl, int64_t ldb, int M, int N,
            int K, float* D, int64_t ldd, const float* bias, int* err, int accumulate, cudaStream_t st,
@@ -428,14 +449,18 @@ int launch(const void* Ah, const void* Al, int64_t lda, const void* Bh, const vo
   if ((rc = operand_map(&tAh, Ah, M, K, lda, kBM, KIND, sc && sc->sliced)) ||
       (rc = operand_map(&tAl, Al, M, K, lda, kBM, KIND, sc && sc->sliced)))
     return rc;
-  if (N <= 64)
-    return launch_tile<KIND, 64>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
-                                 no_loads, sc);
-  if (N > 192)
-    return launch_tile<KIND, 256>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
-                                  no_loads, sc);
-  return launch_tile<KIND, 128>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
-                                no_loads, sc);
+  const int64_t KT = (int64_t(K) + (KIND == kTf32 ? kBK : 2 * kBK) - 1) / (KIND == kTf32 ? kBK : 2 * kBK);
+  switch (tile_columns(M, N, std::min<int64_t>(splits, KT))) {
+    case 64:
+      return launch_tile<KIND, 64>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
+                                   no_loads, sc);
+    case 128:
+      return launch_tile<KIND, 128>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
+                                    no_loads, sc);
+    default:
+      return launch_tile<KIND, 256>(tAh, tAl, Bh, Bl, ldb, M, N, K, D, ldd, bias, err, accumulate, st, splits, wait_ns,
+                                    no_loads, sc);
+  }
 }
 
 // ---- BF16 split: hi = x rounded to BF16 (round to nearest even), lo = BF16(x - hi)
