@@ -117,6 +117,23 @@ __global__ void basis64_kernel(int n_pairs, const int32_t* __restrict__ pdim, co
 }
 
 // --- contraction --------------------------------------------------------------------------
+// Outputs of one row of F (0 past nout): 16-byte loads where the row allows.
+template <int OC>
+__device__ __forceinline__ void load_row(const double* __restrict__ f, int nout, double (&v)[OC]) {
+  if constexpr (OC % 2 == 0) {
+    if (nout == OC && (reinterpret_cast<uintptr_t>(f) & 15) == 0) {
+#pragma unroll
+      for (int q = 0; q < OC; q += 2) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(f + q));
+        v[q] = t.x, v[q + 1] = t.y;
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < OC; ++q) v[q] = q < nout ? __ldg(f + q) : 0.0;
+}
+
 // Level L of a summand with N active pairs: sum over mu_L of l_L[mu_L] * (inner).
 // The innermost level reads rows of F.  `dslot` selects a pair whose basis is
 // replaced by its derivative table (jacobian); -1 for evaluation.
@@ -158,9 +175,7 @@ __device__ inline void clevel(const double* __restrict__ Lt, const double* __res
       const double l = lt[int64_t(j) * P];
       double sub[OC];
       if constexpr (L == N - 1) {
-        const double* fr = Fs + (row * (g + 1) + j) * dout + o0;
-#pragma unroll
-        for (int q = 0; q < OC; ++q) sub[q] = q < nout ? fr[q] : 0.0;
+        load_row<OC>(Fs + (row * (g + 1) + j) * dout + o0, nout, sub);
       } else {
 #pragma unroll
         for (int q = 0; q < OC; ++q) sub[q] = 0.0;
@@ -198,6 +213,20 @@ __device__ inline void cgeneric(const double* __restrict__ Lt, const double* __r
   }
 }
 
+// Up to kMaxN pairs, nested.
+template <int OC>
+__device__ __forceinline__ void contract_nest(const double* __restrict__ Lt, const double* __restrict__ dLt, int dslot,
+                                              int64_t P, int64_t p, const int (&voff)[kMaxN], const int (&deg)[kMaxN],
+                                              int n, const double* __restrict__ Fs, int dout, int o0, int nout,
+                                              double (&acc)[OC]) {
+  switch (n) {
+    case 1: clevel<OC, 0, 1>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
+    case 2: clevel<OC, 0, 2>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
+    case 3: clevel<OC, 0, 3>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
+    default: clevel<OC, 0, 4>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
+  }
+}
+
 template <int OC>
 __device__ inline void contract_summand(const double* __restrict__ Lt, const double* __restrict__ dLt, int dslot,
                                         int64_t P, int64_t p, const int32_t* __restrict__ pairs, int n,
@@ -214,16 +243,11 @@ __device__ inline void contract_summand(const double* __restrict__ Lt, const dou
     voff[i] = i < n ? pvoff[pairs[i]] : 0;
     deg[i] = i < n ? pdeg[pairs[i]] : 0;
   }
-  switch (n) {
-    case 1: clevel<OC, 0, 1>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
-    case 2: clevel<OC, 0, 2>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
-    case 3: clevel<OC, 0, 3>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
-    default: clevel<OC, 0, 4>(Lt, dLt, dslot, P, p, voff, deg, Fs, dout, o0, nout, 0, acc); break;
-  }
+  contract_nest<OC>(Lt, dLt, dslot, P, p, voff, deg, n, Fs, dout, o0, nout, acc);
 }
 
 struct PlanArgs {
-  int n_sum, dout, d_in;
+  int n_sum, dout, d_in, n_values;
   const int32_t* poff;
   const int32_t* pairs;
   const int64_t* eoff;
@@ -234,41 +258,163 @@ struct PlanArgs {
   const double* offset;
 };
 
-// Grid: points along x, chunks of OC outputs along y (from output o_base).
-template <int OC>
-__global__ void __launch_bounds__(128, OC == 1 ? 8 : 5) contract64_kernel(PlanArgs a, const double* __restrict__ Lt,
-                                                                          int64_t P, double* __restrict__ y,
-                                                                          int o_base) {
-  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int o0 = o_base + int(blockIdx.y) * OC;
-  if (p >= P || o0 >= a.dout) return;
-  const int nout = min(OC, a.dout - o0);
-  // Two-level sum: summands accumulate into `blk`, which is folded into `acc`
-  // every 32 summands, so rounding grows with 32 + n_sum/32 instead of n_sum.
-  double acc[OC], blk[OC];
+// Evaluation: y[p][o] = offset[o] + sum over all rows r of F of (product of the
+// row's basis values at p) * F[r][o].  A cluster of `parts` blocks of kWarps warps
+// takes 32 points (lane = point) and up to 8 outputs: the rows are cut into parts x
+// kWarps runs of whole summands, one per warp, so that a few thousand points
+// already fill the GPU and a basis value is read once for all outputs.  The sums of
+// a summand stay nested (pair by pair): with one weight per row its terms lose the
+// cancellation inside each dimension, 3 to 4 times the error (2.6 ms instead of
+// 3.4, not kept).  The basis values of the points sit in shared memory when
+// they fit (SROWS).  Sums are added in a fixed order that does not depend on the
+// batch.  Bound: the FP64 pipe,
+// 2 multiply-adds per SM clock (0.63 T/s).  Gauss-Hermite d_in = 100, |Lambda| =
+// 3545 (19993 rows), 8 outputs: 5000 points 3.4 ms, 50 points 0.36 ms; a thread per
+// point and four outputs that ran through all summands took 10.7 and 10.4 ms.  Leja
+// d_in = 1000 (50610 rows), one output: 10000 points 14.7 -> 3.6 ms, 1e5 points 38.3
+// -> 32.9.  The summands' tables are loaded by lanes, 32 at a time (33 ms; 49 with a
+// chain of loads per summand), and sums over them are compensated every kRun: the
+// same error or less than the two-level sum before (2.2e-13 after 2.3e-13, 7e-15
+// after 1.8e-14); compensated for every summand 5.1 ms.
+constexpr int kWarps = 16;
+constexpr int kRun = 8;  // summands between two compensated additions
+constexpr int kSmemMax = 226 * 1024;
+
+// Blocks per cluster, fixed per plan (a point's value does not depend on its
+// batch): up to 8, while a warp's run has 64 rows.  8 blocks for a plan of 32 rows
+// took 152 us at 3000 points, one 73; for 4282 rows 7.5 ms at 1e5 points and 160 us
+// at 1000, 4 blocks 5.5 ms and 107 us.
+int contract_parts(int64_t rows) {
+  int parts = 1;
+  while (parts < 8 && rows >= int64_t(2 * parts) * kWarps * 64) parts *= 2;
+  return parts;
+}
+
+// The correction of an infinite or undefined sum is left out, so that the sum stays what it is.
+__device__ __forceinline__ double finite_or_zero(double e) {
+  return (__double2hiint(e) & 0x7ff00000) == 0x7ff00000 ? 0.0 : e;
+}
+
+// sum + v exactly as the new sum and an error that is added to `low`.
+__device__ __forceinline__ void two_sum(double& sum, double& low, double v) {
+  const double t = __dadd_rn(sum, v), z = __dadd_rn(t, -sum);
+  const double e = __dadd_rn(__dadd_rn(sum, -__dadd_rn(t, -z)), __dadd_rn(v, -z));
+  low += finite_or_zero(e);
+  sum = t;
+}
+
+// First summand whose rows begin at or after row r, by a warp.
+__device__ __forceinline__ int first_summand(const PlanArgs& a, int64_t r, int lane) {
+  int lo = 0, n = a.n_sum;  // answer in [lo, lo + n]
+  while (n > 0) {
+    const int step = (n + 31) / 32, i = lo + min((lane + 1) * step, n) - 1;
+    const unsigned before = __ballot_sync(0xffffffffu, a.eoff[i] < r);
+    const int k = __popc(before);  // whole steps before the answer
+    if (k == 32) return lo + n;
+    lo += k * step;
+    n = min(step - 1, n - k * step - 1);
+    if (n < 0) n = 0;
+  }
+  return lo;
+}
+
+template <int DO, bool SROWS>
+__global__ void __launch_bounds__(32 * kWarps, DO == 1 ? 2 : 1)
+    contract_kernel(PlanArgs a, const double* __restrict__ Lt, int64_t P, double* __restrict__ y, int o_base,
+                    int parts) {
+  extern __shared__ __align__(16) double sm64[];
+  double* all = sm64;                         // [parts][DO][32][2] at the first block
+  double* rows = all + parts * DO * 64;      // [n_values][32]
+  double* own = rows;                         // [kWarps][DO][32], when the rows are done with
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned part;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(part));
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // all blocks run: their memory may be written
+  const int64_t p0 = (blockIdx.x / parts) * int64_t(32), p = min(p0 + lane, P - 1);
+  const int o0 = o_base + int(blockIdx.y) * DO, nout = min(DO, a.dout - o0);
+  if constexpr (SROWS) {
+#pragma unroll 4
+    for (int v = warp; v < a.n_values; v += kWarps) rows[v * 32 + lane] = __ldg(Lt + int64_t(v) * P + p);
+    __syncthreads();
+  }
+  double acc[DO], comp[DO];
 #pragma unroll
-  for (int q = 0; q < OC; ++q) acc[q] = blk[q] = 0.0;
-  for (int s = 0; s < a.n_sum; ++s) {
-    const int q0 = a.poff[s], n = a.poff[s + 1] - q0;
-    const int64_t e0 = a.eoff[s], K = a.eoff[s + 1] - e0;
-    double one[OC];
+  for (int o = 0; o < DO; ++o) acc[o] = comp[o] = 0.0;
+  const int64_t R = a.n_sum > 0 ? a.eoff[a.n_sum] : 0;
+  const int seg = int(part) * kWarps + warp;
+  const int s1 = first_summand(a, R * (seg + 1) / (parts * kWarps), lane);
+  const int s0 = first_summand(a, R * seg / (parts * kWarps), lane);
+  double run[DO];  // up to kRun summands
 #pragma unroll
-    for (int q = 0; q < OC; ++q) one[q] = 0.0;
-    contract_summand<OC>(Lt, nullptr, -1, P, p, a.pairs + q0, n, a.pvoff, a.pdeg, a.F + e0 * a.dout, K, a.dout, o0, nout,
-                     one);
+  for (int o = 0; o < DO; ++o) run[o] = 0.0;
+  int n_of = 0, voff_of[kMaxN], deg_of[kMaxN];
+  int64_t e_of = 0;
+  for (int s = s0; s < s1; ++s) {
+    const int k = (s - s0) & 31;
+    if (k == 0) {  // a lane's loads for each of the next 32 summands
+      const int mine = min(s + lane, s1 - 1), q0 = __ldg(a.poff + mine);
+      n_of = __ldg(a.poff + mine + 1) - q0;
+      e_of = __ldg(a.eoff + mine);
 #pragma unroll
-    for (int q = 0; q < OC; ++q) blk[q] += one[q];
-    if ((s & 31) == 31) {
+      for (int i = 0; i < kMaxN; ++i) {
+        const int u = i < n_of ? __ldg(a.pairs + q0 + i) : -1;
+        voff_of[i] = u >= 0 ? __ldg(a.pvoff + u) : 0;
+        deg_of[i] = u >= 0 ? __ldg(a.pdeg + u) : 0;
+      }
+    }
+    const int n = __shfl_sync(0xffffffffu, n_of, k);
+    const int64_t e0 = __shfl_sync(0xffffffffu, e_of, k);
+    const double* lt = SROWS ? rows : Lt;
+    const int64_t stride = SROWS ? 32 : P, at = SROWS ? lane : p;
+    if (n <= kMaxN) {
+      int voff[kMaxN], deg[kMaxN];
 #pragma unroll
-      for (int q = 0; q < OC; ++q) {
-        acc[q] += blk[q];
-        blk[q] = 0.0;
+      for (int i = 0; i < kMaxN; ++i) {
+        voff[i] = __shfl_sync(0xffffffffu, voff_of[i], k);
+        deg[i] = __shfl_sync(0xffffffffu, deg_of[i], k);
+      }
+      contract_nest<DO>(lt, nullptr, -1, stride, at, voff, deg, n, a.F + e0 * a.dout, a.dout, o0, nout, run);
+    } else {
+      cgeneric<DO>(lt, nullptr, -1, stride, at, a.pairs + __ldg(a.poff + s), n, a.pvoff, a.pdeg, a.F + e0 * a.dout,
+                   __ldg(a.eoff + s + 1) - e0, a.dout, o0, nout, run);
+    }
+    if ((s - s0) % kRun == kRun - 1 || s + 1 == s1) {
+#pragma unroll
+      for (int o = 0; o < DO; ++o) {  // compensated
+        const double v = __dadd_rn(run[o], -comp[o]), t = __dadd_rn(acc[o], v);
+        comp[o] = finite_or_zero(__dadd_rn(__dadd_rn(t, -acc[o]), -v));
+        acc[o] = t;
+        run[o] = 0.0;
       }
     }
   }
+  // the block's warps, then the cluster's blocks, in order
+  __syncthreads();
 #pragma unroll
-  for (int q = 0; q < OC; ++q)
-    if (q < nout) y[p * a.dout + o0 + q] = a.offset[o0 + q] + (acc[q] + blk[q]);
+  for (int o = 0; o < DO; ++o) own[(warp * DO + o) * 32 + lane] = acc[o];
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  for (int i = threadIdx.x; i < DO * 32; i += 32 * kWarps) {
+    double sum = own[i], low = 0.0;
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) two_sum(sum, low, own[w * DO * 32 + i]);
+    uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(all + 2 * (part * DO * 32 + i)));
+    asm volatile("mapa.shared::cluster.u32 %0, %0, 0;" : "+r"(to));
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(to), "d"(sum), "d"(low) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+  if (part != 0) return;
+  for (int i = threadIdx.x; i < 32 * nout; i += 32 * kWarps) {
+    const int q = i / nout, o = i - q * nout;
+    if (p0 + q >= P) break;
+    double sum = a.offset[o0 + o], low = 0.0;
+    for (int b = 0; b < parts; ++b) {
+      const double2 v = reinterpret_cast<const double2*>(all)[(b * DO + o) * 32 + q];
+      two_sum(sum, low, v.x);
+      low += v.y;
+    }
+    y[(p0 + q) * a.dout + o0 + o] = sum + low;
+  }
 }
 
 // Jacobian: J[p][o][dim] += derivative contraction of every summand and every
@@ -397,6 +543,7 @@ PlanArgs args_of(const smx_plan* pl, const double* F) {
   a.n_sum = pl->n_summands;
   a.dout = pl->d_out;
   a.d_in = pl->d_in;
+  a.n_values = int(pl->n_values);
   a.poff = pl->sum_poff;
   a.pairs = pl->sum_pairs;
   a.eoff = pl->sum_eoff;
@@ -417,6 +564,42 @@ int check_plan(const smx_plan* pl, const char* who) {
     return smx::set_error(SMX_ERR_ARG, std::string(who) + ": null plan array");
   if (!pl->offset) return smx::set_error(SMX_ERR_ARG, std::string(who) + ": null offset");
   return SMX_OK;
+}
+
+template <int DO, bool SROWS>
+int launch_contract(const PlanArgs& a, const double* Lt, int64_t P, double* y, int o_base, int passes, int parts,
+                    size_t smem, cudaStream_t st) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(contract_kernel<DO, SROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    attr = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = unsigned(parts);
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(unsigned((P + 31) / 32 * parts), unsigned(passes));
+  cfg.blockDim = dim3(32 * kWarps);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, contract_kernel<DO, SROWS>, a, Lt, P, y, o_base, parts);
+  SMX_LAUNCH_CHECK("smx_contract_f64");
+  return SMX_OK;
+}
+
+// Basis values in shared memory while they fit (up to 770 with 8 outputs).
+template <int DO>
+int launch_contract(const PlanArgs& a, const double* Lt, int64_t P, double* y, int o_base, int passes, int64_t n_rows,
+                    cudaStream_t st) {
+  const int parts = contract_parts(n_rows);
+  const size_t all = size_t(parts) * DO * 512, own = size_t(kWarps) * DO * 256, rows = size_t(a.n_values) * 256;
+  const size_t room = DO == 1 ? kSmemMax / 2 : kSmemMax;  // one output: two blocks per SM
+  return all + rows <= room
+             ? launch_contract<DO, true>(a, Lt, P, y, o_base, passes, parts, all + std::max(own, rows), st)
+             : launch_contract<DO, false>(a, Lt, P, y, o_base, passes, parts, all + own, st);
 }
 
 constexpr int kPairsPerBlock = 64;
@@ -441,9 +624,12 @@ extern "C" int smx_basis_f64(const smx_plan* pl, const double* x, int64_t P, int
   SMX_REQUIRE(P >= 0 && ldx >= pl->d_in, "smx_basis_f64: bad sizes");
   if (P == 0 || pl->n_pairs == 0) return SMX_OK;
   SMX_REQUIRE(x && Lt && pl->node && pl->bweight, "smx_basis_f64: null pointer");
-  dim3 grid(smx::grid_for(P, 128), (pl->n_pairs + kPairsPerBlock - 1) / kPairsPerBlock);
+  // pairs per block: few enough that a small batch fills the GPU
+  const int64_t blocks = (P + 127) / 128;
+  const int per = int(std::max<int64_t>(1, std::min<int64_t>(kPairsPerBlock, blocks * pl->n_pairs / 1024)));
+  dim3 grid(smx::grid_for(P, 128), (pl->n_pairs + per - 1) / per);
   basis64_kernel<<<grid, 128, 0, smx::as_stream(stream)>>>(pl->n_pairs, pl->pair_dim, pl->pair_deg, pl->pair_voff,
-                                                           pl->node, pl->bweight, x, P, ldx, Lt, dLt, kPairsPerBlock);
+                                                           pl->node, pl->bweight, x, P, ldx, Lt, dLt, per);
   SMX_LAUNCH_CHECK("smx_basis_f64");
   return SMX_OK;
 }
@@ -455,17 +641,22 @@ extern "C" int smx_contract_f64(const smx_plan* pl, const double* Lt, int64_t P,
   if (P == 0) return SMX_OK;
   SMX_REQUIRE(y && (pl->n_summands == 0 || Lt), "smx_contract_f64: null pointer");
   PlanArgs a = args_of(pl, pl->F64);
-  // all output chunks in one launch (blockIdx.y), so few points still fill the GPU
-  // one output: one accumulator per entry (the FP64 pipe is the bound)
-  const int oc = pl->d_out == 1 ? 1 : kOC;
-  const int chunks = (pl->d_out + oc - 1) / oc;
-  for (int c0 = 0; c0 < chunks; c0 += kMaxGridY) {
-    const dim3 grid(smx::grid_for(P, 128), unsigned(std::min(kMaxGridY, chunks - c0)));
-    if (oc == 1)
-      contract64_kernel<1><<<grid, 128, 0, smx::as_stream(stream)>>>(a, Lt, P, y, c0);
-    else
-      contract64_kernel<kOC><<<grid, 128, 0, smx::as_stream(stream)>>>(a, Lt, P, y, c0 * kOC);
-    SMX_LAUNCH_CHECK("smx_contract_f64");
+  // up to 8 outputs per block, as evenly as they divide
+  const int passes = (pl->d_out + 7) / 8, DO = (pl->d_out + passes - 1) / passes;
+  for (int c0 = 0; c0 < passes; c0 += kMaxGridY) {
+    const int n = std::min(kMaxGridY, passes - c0);
+    cudaStream_t st = smx::as_stream(stream);
+    switch (DO) {
+      case 1: rc = launch_contract<1>(a, Lt, P, y, c0, n, pl->n_entries, st); break;
+      case 2: rc = launch_contract<2>(a, Lt, P, y, c0 * 2, n, pl->n_entries, st); break;
+      case 3: rc = launch_contract<3>(a, Lt, P, y, c0 * 3, n, pl->n_entries, st); break;
+      case 4: rc = launch_contract<4>(a, Lt, P, y, c0 * 4, n, pl->n_entries, st); break;
+      case 5: rc = launch_contract<5>(a, Lt, P, y, c0 * 5, n, pl->n_entries, st); break;
+      case 6: rc = launch_contract<6>(a, Lt, P, y, c0 * 6, n, pl->n_entries, st); break;
+      case 7: rc = launch_contract<7>(a, Lt, P, y, c0 * 7, n, pl->n_entries, st); break;
+      default: rc = launch_contract<8>(a, Lt, P, y, c0 * 8, n, pl->n_entries, st); break;
+    }
+    if (rc) return rc;
   }
   return SMX_OK;
 }
