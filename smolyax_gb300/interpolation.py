@@ -478,9 +478,11 @@ class SmolyakBarycentricInterpolator:
     def _coefficients(self):
         """FP64 coefficients of the orthogonal form (built on first use)."""
         if self._coef is None:
-            from .spectral import Coefficients
+            from .spectral import Coefficients, finish_build
 
-            self._coef = Coefficients(self)
+            coef = Coefficients(self)
+            finish_build()
+            self._coef = coef
         return self._coef
 
     def spectral_plan(self):
@@ -554,12 +556,16 @@ class SmolyakBarycentricInterpolator:
         values' rows, which the combination sum does not need twice)."""
         if self._jacobian is None:
             from .jacobian import MAX_DEGREE, JacobianPlan
+            from .spectral import finish_build
 
             c = self._plan.c
             ok = (c.n_entries > 0 and c.n_entries * c.d_out * 8 <= 16 * 1024**3
                   and int(np.max(self._maxdeg, initial=0)) < MAX_DEGREE
                   and all(isinstance(g, (_nodes.Leja1D, _nodes.GaussHermite1D)) for g in self._node_gen))
-            self._jacobian = JacobianPlan(self) if ok else False
+            jac = JacobianPlan(self) if ok else False
+            if ok:
+                finish_build()
+            self._jacobian = jac
         return self._jacobian or None
 
     def gradient(self, x: ArrayLike) -> torch.Tensor:

@@ -13,6 +13,8 @@ then laid out for the FP32 evaluator of ``csrc/spectral.cu``:
 """
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import torch
 
@@ -51,6 +53,13 @@ def stream_tables(struct, tree, coef, d_out, maxdeg, fam, fa, fb, T, fp64):
     for name, t in keep.items():
         setattr(s, name, t.data_ptr() if t.numel() else None)
     return keep
+
+
+def finish_build():
+    """Operands just built on the current stream are read from any stream next:
+    wait for them, once per plan (a capture cannot wait; it is their only reader then)."""
+    if not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream().synchronize()
 
 
 def _phi_table(fam, z, n):
@@ -212,12 +221,13 @@ class SpectralPlan:
         self.c = s
         self.tc = None
         self._bwd = None
+        self._lock = threading.RLock()  # operands built on first use
+        self.memory_limit = ip._memory_limit
         self._fwd_args = (tree_np, C32, np.asarray(ip._maxdeg), fam, fa, fb, T, st)
         self.plan = pl
         stream_fits = (lay["row"] + 4 * (1 if d_out == 1 else 4) * 2) * 128 * 4 <= 220 * 1024
         if d_out >= TC_MIN_DOUT or not stream_fits:
             self._build_tc(*self._fwd_args)
-        self.memory_limit = ip._memory_limit
         self._f64 = None
         self.blocked = None
         self.blocked_tc = None
@@ -262,6 +272,7 @@ class SpectralPlan:
         B[:, :K] = C32[tc["ent_h"][::-1]].T  # the panel stores the entries in reversed pre-order
         tc["Bd"] = T(B, torch.float32)
         self.tc = tc
+        self._tc_struct()
 
     def _tensor_struct(self, ops, d_out):
         """``smx_tensor`` with the tape's shapes and basis tables (no operands)."""
@@ -276,35 +287,39 @@ class SpectralPlan:
         return s
 
     def _tc_struct(self, bf16=False):
-        """``smx_tensor`` of the plan: FP16 operands with scales, or the BF16
-        operands of ``mode="bf16x3"`` (each built on first use)."""
+        """``smx_tensor`` of the plan: FP16 operands with scales (built with the
+        plan), or the BF16 operands of ``mode="bf16x3"`` (built on first use)."""
         tc = self.tc
         key = "bf16" if bf16 else "f16"
-        if key not in tc:
-            Bd = tc["Bd"]
-            d_out, K = int(Bd.shape[0]), tc["K"]
-            n_groups = (K + 63) // 64
-            ldb = max(64, 64 * n_groups)
-            dev = Bd.device
-            st = capi.stream_ptr(torch.cuda.current_stream())
-            k = dict(Bh=torch.zeros(d_out, ldb, dtype=torch.bfloat16 if bf16 else torch.float16, device=dev))
-            k["Bl"] = torch.zeros_like(k["Bh"])
-            k["tape"] = torch.zeros(2 * 64 * n_groups, dtype=torch.int32, device=dev)
-            if bf16:
-                if K:
-                    call("smx_tensor_tape", ptr(tc["tape"]), K, ptr(k["tape"]), st)
-                    call("smx_split_bf16", ptr(Bd), d_out, K, tc["ldk"], ptr(k["Bh"]), ptr(k["Bl"]), ldb, st)
-            else:
-                k["out_scale"] = torch.ones(d_out, dtype=torch.float32, device=dev)
-                if K:
-                    call("smx_tensor_operands", ptr(Bd), d_out, K, tc["ldk"], ptr(tc["tape"]), ptr(k["tape"]),
-                         ptr(k["Bh"]), ptr(k["Bl"]), ldb, ptr(k["out_scale"]), st)
-            s = self._tensor_struct(tc, d_out)
-            s.bf16, s.splits, s.chunk, s.ldb = int(bf16), self.tc_splits(), self._tc_step(1 << 40), ldb
-            for name, t in k.items():
-                setattr(s, name, t.data_ptr())
-            tc[key] = (s, k)
-        return tc[key][0]
+        with self._lock:
+            return self._build_tc_struct(tc, key, bf16) if key not in tc else tc[key][0]
+
+    def _build_tc_struct(self, tc, key, bf16):
+        Bd = tc["Bd"]
+        d_out, K = int(Bd.shape[0]), tc["K"]
+        n_groups = (K + 63) // 64
+        ldb = max(64, 64 * n_groups)
+        dev = Bd.device
+        st = capi.stream_ptr(torch.cuda.current_stream())
+        k = dict(Bh=torch.zeros(d_out, ldb, dtype=torch.bfloat16 if bf16 else torch.float16, device=dev))
+        k["Bl"] = torch.zeros_like(k["Bh"])
+        k["tape"] = torch.zeros(2 * 64 * n_groups, dtype=torch.int32, device=dev)
+        if bf16:
+            if K:
+                call("smx_tensor_tape", ptr(tc["tape"]), K, ptr(k["tape"]), st)
+                call("smx_split_bf16", ptr(Bd), d_out, K, tc["ldk"], ptr(k["Bh"]), ptr(k["Bl"]), ldb, st)
+        else:
+            k["out_scale"] = torch.ones(d_out, dtype=torch.float32, device=dev)
+            if K:
+                call("smx_tensor_operands", ptr(Bd), d_out, K, tc["ldk"], ptr(tc["tape"]), ptr(k["tape"]),
+                     ptr(k["Bh"]), ptr(k["Bl"]), ldb, ptr(k["out_scale"]), st)
+        s = self._tensor_struct(tc, d_out)
+        s.bf16, s.splits, s.chunk, s.ldb = int(bf16), self.tc_splits(), self._tc_step(1 << 40), ldb
+        for name, t in k.items():
+            setattr(s, name, t.data_ptr())
+        finish_build()
+        tc[key] = (s, k)
+        return s
 
     def _build_blocked(self, tr, c, maxdeg, d, fam, fa, fb, T):
         """Tables of the blocked evaluator (one output), if the plan fits it."""
@@ -365,33 +380,37 @@ class SpectralPlan:
     def _backward_ops(self):
         """Tape operands (built as for the forward tensor-core path) plus the
         coefficient rows C[K x ldo] in the panel's reversed order, TF32 hi/lo."""
-        if self._bwd is None:
-            ops = dict(self.tc) if self.tc is not None else self._build_tape(*self._fwd_args)
-            if ops is None:
-                raise RuntimeError("backward needs Smolyak index depth <= 8 (register product stack)")
-            T = self._fwd_args[6]
-            st = self._fwd_args[7]
-            C32 = self._fwd_args[1]
-            K = ops["K"]
-            d_out = C32.shape[1]
-            ldo = _round4(d_out)
-            ent = ops["ent_h"]
-            rows = np.zeros((max(K, 1), ldo), dtype=np.float32)
-            rows[:K, :d_out] = C32[ent[::-1]]
-            Rd = T(rows, torch.float32)
-            Rh, Rl = torch.empty_like(Rd), torch.empty_like(Rd)
-            call("smx_split_tf32", ptr(Rd), rows.shape[0], ldo, ldo, ptr(Rh), ptr(Rl), ldo, st)
-            ops.update(Rh=Rh, Rl=Rl, ldo=ldo, walk=self._build_walk(ops, C32), coef=self._build_coef(ops, d_out))
-            # tape segments of the gradient walk: fixed per plan (a point's dL/dx
-            # does not depend on the batch it comes in)
-            want = vjp_segment_count(K, ops["lvl1"].size)
-            if want > 1:
-                b = T(segment_bounds(ops["lvl1"], K, want), torch.int32)
-                ops["vjp_seg"] = (b, int(b.numel()) - 1)
-            else:
-                ops["vjp_seg"] = (None, 1)
-            self._bwd = ops
-        return self._bwd
+        with self._lock:
+            return self._bwd if self._bwd is not None else self._build_backward_ops()
+
+    def _build_backward_ops(self):
+        ops = dict(self.tc) if self.tc is not None else self._build_tape(*self._fwd_args)
+        if ops is None:
+            raise RuntimeError("backward needs Smolyak index depth <= 8 (register product stack)")
+        T = self._fwd_args[6]
+        st = capi.stream_ptr(torch.cuda.current_stream())
+        C32 = self._fwd_args[1]
+        K = ops["K"]
+        d_out = C32.shape[1]
+        ldo = _round4(d_out)
+        ent = ops["ent_h"]
+        rows = np.zeros((max(K, 1), ldo), dtype=np.float32)
+        rows[:K, :d_out] = C32[ent[::-1]]
+        Rd = T(rows, torch.float32)
+        Rh, Rl = torch.empty_like(Rd), torch.empty_like(Rd)
+        call("smx_split_tf32", ptr(Rd), rows.shape[0], ldo, ldo, ptr(Rh), ptr(Rl), ldo, st)
+        ops.update(Rh=Rh, Rl=Rl, ldo=ldo, walk=self._build_walk(ops, C32), coef=self._build_coef(ops, d_out))
+        # tape segments of the gradient walk: fixed per plan (a point's dL/dx
+        # does not depend on the batch it comes in)
+        want = vjp_segment_count(K, ops["lvl1"].size)
+        if want > 1:
+            b = T(segment_bounds(ops["lvl1"], K, want), torch.int32)
+            ops["vjp_seg"] = (b, int(b.numel()) - 1)
+        else:
+            ops["vjp_seg"] = (None, 1)
+        finish_build()
+        self._bwd = ops
+        return ops
 
     def _build_walk(self, ops, C32):
         """Structs of the gradient walk over G^T (``csrc/tensor_vjp.cu``), or None
