@@ -373,28 +373,27 @@ def tensor_workload(name, steps, warmup, points=None):
                 "note": "3 kind::f16 BF16 passes (hi*hi + hi*lo + lo*hi), FP32 accumulation"}
     K = sp.tc["K"] if sp.tc is not None else None
     # algorithmic flops: one multiply-add per (point, entry, output); the
-    # kernel executes 3 TF32 passes (hi*hi + hi*lo + lo*hi) for them
+    # kernel executes 3 FP16 passes (hi*hi + hi*lo + lo*hi) for them
     tensor_flops = 2.0 * P * d_out * K if K else None
     try:
         peak = float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops"])
         pk = "measured bf16 dense"
     except Exception:
         peak, pk = 1900.0, "fallback bf16 dense"
-    tf32_peak = peak / 2  # kind::tf32 issues at half the bf16 dense rate
     line = {
         "metric": METRIC, "workload": name, "value": P * d_out / (ms * 1e-3), "unit": "evals/s",
         "n_gpus": 1, "steps": steps, "warmup": warmup, "ms_per_step": ms, "higher_is_better": True,
-        "dtype": "fp32 (3xTF32 tensor contraction)", "data": "synthetic",
+        "dtype": "fp32 (tensor contraction of scaled FP16 pairs)", "data": "synthetic",
         "config": {"workload": desc, "points": P, "d_in": d, "d_out": d_out, "lambda": K + 1 if K else None},
         "error": {"fp32_per_point_normwise_vs_fp64": err, "fp32_elementwise_max_rel_vs_fp64": err_ew,
                   "points_checked": sub, "bound": 1e-6, "bound_norm": "per-point norm-wise"},
         "tflops_algorithmic": tensor_flops / (ms * 1e-3) / 1e12 if K else None,
-        "frac_of_tf32_peak": tensor_flops / (ms * 1e-3) / 1e12 / tf32_peak if K else None,
+        "frac_of_three_pass_peak": 3 * tensor_flops / (ms * 1e-3) / 1e12 / peak if K else None,
         "roofline": {"bound": "tensor", "achieved": tensor_flops / (ms * 1e-3) / 1e12 if K else None, "peak": peak,
                      "unit": "TFLOP/s", "frac": tensor_flops / (ms * 1e-3) / 1e12 / peak if K else None,
                      "peak_kind": pk, "flops_per_step": tensor_flops,
-                     "tf32x3_bound": peak / 2 / 3,
-                     "note": "3 kind::tf32 passes per product; kind::tf32 runs at half the bf16 dense rate"},
+                     "three_pass_bound": peak / 3,
+                     "note": "3 kind::f16 passes per product, at the bf16 dense rate"},
         "bf16x3": bf16,
         "setup_s": setup_s, "clocks": clk.summary(),
         # per step: per chunk of points a panel (+ its basis rows) and a tensor-core GEMM, or one
@@ -469,7 +468,7 @@ def backward_workload(steps, warmup, points=None):
     line = {
         "metric": METRIC, "workload": "leja64bwd", "value": P * d_out / (ms * 1e-3), "unit": "evals/s",
         "n_gpus": 1, "steps": steps, "warmup": warmup, "ms_per_step": ms, "higher_is_better": True,
-        "dtype": "fp32 (3xTF32 tensor contractions, FP64 coefficient adjoint)", "data": "synthetic",
+        "dtype": "fp32 (tensor contractions of scaled FP16 pairs, FP64 coefficient adjoint)", "data": "synthetic",
         "config": {"workload": "Leja d_in=200 d_out=64 |Lambda|=5000 (t=7.853604) rational f, 1e5 points U[-1,1]^200,"
                                " forward + backward (dL/dx and dL/d nodal values), FP32 cotangent N(0,1)",
                    "points": P, "d_in": d, "d_out": d_out},
@@ -483,7 +482,7 @@ def backward_workload(steps, warmup, points=None):
 def fp64_workload(steps, warmup, points=None):
     """FP64 evaluation at the headline configuration (Leja d_in=1000, d_out=1,
     |Lambda|=9999, rational f): the default FP64 evaluator of this plan (the
-    orthogonal form, csrc/spectral64.cu) and the reference's combination sum
+    orthogonal form, csrc/stream_eval.cuh) and the reference's combination sum
     (precision="fp64_barycentric"), one JSON line."""
     import torch
 
@@ -525,7 +524,7 @@ def fp64_workload(steps, warmup, points=None):
         "data": "synthetic",
         "config": {"workload": WORKLOAD + ", FP64 evaluation", "points": P, "d_in": D_IN, "d_out": D_OUT,
                    "lambda": int(ip._tree.size)},
-        "form": "orthogonal polynomials in FP64 (csrc/spectral64.cu)",
+        "form": "orthogonal polynomials in FP64 (csrc/stream_eval.cuh)",
         "barycentric_ms": ms_b, "max_rel_diff_vs_barycentric": diff,
         "roofline": {"bound": "fp64", "achieved": P * terms / (ms * 1e-3), "peak": peak, "unit": "DFMA/s",
                      "frac": P * terms / (ms * 1e-3) / peak, "peak_kind": "nominal (2 per SM clock at 2070 MHz)"},
@@ -650,7 +649,7 @@ def fleet_workload(P, steps, warmup):
                          max_rel_err_vs_fp64=err))
     return {"workload": "fleet", "points": P, "steps": steps, "warmup": warmup, "unit": "ms", "data": "synthetic",
             "config": {"workload": "tensor-core plans of the 16-interpolant serving fleet (seed 0) with |Lambda| >= "
-                                   "1e4, each alone, FP32 (3xTF32 contraction)"},
+                                   "1e4, each alone, FP32 (contraction of FP16 pairs)"},
             "plans": rows}
 
 
@@ -838,7 +837,7 @@ def run_ours(args):
         "config": headline_config(world, P),
         "latency_ms": {"p50": statistics.median(per32), "p99": p99, "max": max(per32)},
         "fp64": {"value": world * P * D_OUT / (ms64 * 1e-3), "ms_per_step": ms64, "steps": fp64_steps,
-                 "form": "orthogonal polynomials, FP64 (csrc/spectral64.cu)"},
+                 "form": "orthogonal polynomials, FP64 (csrc/stream_eval.cuh)"},
         "fp64_barycentric": {"value": world * P * D_OUT / (ms64b * 1e-3), "ms_per_step": ms64b, "steps": 3,
                              "max_rel_diff_vs_fp64": err64},
         "speedup_vs_fp64": ms64 / ms32,
