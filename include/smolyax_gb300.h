@@ -750,14 +750,24 @@ int smx_tensor_vjp_x(const smx_tensor* plan_host, const smx_tensor_bwd* bwd_host
                      int64_t ldx, const float* g, int64_t ldg, double* dx, int64_t lddx, void* ws, size_t ws_bytes,
                      void* stream);
 
-/* dL/dC = A^T g (FP32) over plan->chunk points at a time (a multiple of 64): rows in the
- * order of the padded tape, dC[64 n_groups][d_out], with the plan's splits
- * (smx_tensor_coef_splits) over the points.  Plans with more basis slots than fit in
- * shared memory (workspace 0) are refused. */
+/* dL/dC [n_lambda][d_out] (FP64) of y = c0 + A C: A^T g in FP32 over plan->chunk points at
+ * a time (a multiple of 64) with the plan's splits (smx_tensor_coef_splits) over the
+ * points, written to the rows ent[K] of the tape's entries; row 0 (the constant) is the
+ * sum of g.  Plans with more basis slots than fit in shared memory (workspace 0) are
+ * refused. */
 int smx_tensor_coef_splits(int d_out, int K);
 size_t smx_tensor_vjp_coef_workspace(const smx_tensor* plan_host, int64_t P);
 int smx_tensor_vjp_coef(const smx_tensor* plan_host, const double* x, int64_t P, int64_t ldx, const float* g,
-                        int64_t ldg, float* dC, void* ws, size_t ws_bytes, void* stream);
+                        int64_t ldg, const int64_t* ent, double* dC, void* ws, size_t ws_bytes, void* stream);
+/* dL/d(nodal values) out[n_values][d_out] from dL/dF Fbar[rows][d_out] of the rows
+ * F[r] = zeta_r (f[u(r)] - f[first]): `row` lists the rows by value, run i is row[run_begin[i]]
+ * .. row[run_begin[i+1]) (of one value, a few dozen rows), value u has the runs value_run[u]
+ * .. value_run[u+1); the sums go in order, and the first value gets root_factor * root[d_out]
+ * less the sum over all rows. */
+size_t smx_nodal_adjoint_workspace(int64_t n_values, int64_t n_runs, int d_out);
+int smx_nodal_adjoint(const double* Fbar, const double* zeta, int64_t n_values, int64_t n_runs, int d_out,
+                      const int64_t* value_run, const int64_t* run_begin, const int64_t* row, const double* root,
+                      double root_factor, int64_t first, double* out, void* ws, size_t ws_bytes, void* stream);
 
 /* ---- host-side layout builders of the FP32 evaluators ------------------------------
  * The tables of the blocked one-output evaluator (smx_blocked), of the

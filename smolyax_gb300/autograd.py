@@ -18,32 +18,52 @@ from __future__ import annotations
 
 import torch
 
+from . import _capi as capi
+
+
+def _value_runs(umap, n):
+    """Rows by nodal value in runs of at most 64 rows of one value: (value_run
+    [n + 1], run_begin [runs + 1], rows)."""
+    zero = torch.zeros(1, dtype=torch.int64, device=umap.device)
+    count = torch.bincount(umap, minlength=n)
+    runs = (count + 63) // 64
+    value_run = torch.cat([zero, runs.cumsum(0)])
+    value = torch.repeat_interleave(torch.arange(n, device=umap.device), runs)
+    first = torch.cat([zero, count.cumsum(0)])  # the first row of each value
+    begin = first[value] + 64 * (torch.arange(value.numel(), device=umap.device) - value_run[value])
+    return value_run, torch.cat([begin, first[n:]]), torch.argsort(umap, stable=True)
+
 
 def _row_factors(keep):
     """The plan's constants of the chain rule, laid out with its first gradient:
-    zeta of every row, the first row's value and the sum of all zeta (reading them
-    back costs a synchronisation each, which a backward does not repeat)."""
+    zeta of every row, the rows of each nodal value, the first row's value and the
+    factor of the constant term (reading them back costs a synchronisation each,
+    which a backward does not repeat)."""
     if "row_factors" not in keep:
-        eoff = keep["sum_eoff"]
-        zrow = torch.repeat_interleave(keep["sum_zeta"].double(), (eoff[1:] - eoff[:-1]))[:, None]
-        keep["row_factors"] = (zrow, int(keep["umap"][0].item()), float(keep["sum_zeta"].sum().item()))
+        eoff, umap = keep["sum_eoff"], keep["umap"]
+        zrow = torch.repeat_interleave(keep["sum_zeta"].double(), (eoff[1:] - eoff[:-1]))
+        runs = _value_runs(umap, int(keep["fu"].shape[0]))
+        factor = float(keep["sum_zeta"].sum().item()) + float(keep["zeta0"])
+        keep["row_factors"] = (zrow, runs, int(umap[0].item()), factor)
     return keep["row_factors"]
 
 
 def _fu_gradient(ip, Fbar, dC_root):
-    """Chain rule from dL/dF (plan rows) and dL/d(constant term) to dL/dfu."""
+    """Chain rule from dL/dF (plan rows) and dL/d(constant term) to dL/dfu:
+    F = zeta (fu[umap] - c), offset = zeta0 fu[u0] + c sum(zeta), c = fu[u0]."""
     P = ip._plan
     keep = P.keep
     fu = keep["fu"]
-    dfu = torch.zeros_like(fu)
-    R = P.c.n_entries
-    if R == 0:
-        return dfu
-    zrow, u0, zsum = _row_factors(keep)
-    zF = Fbar * zrow
-    dfu.index_add_(0, keep["umap"], zF)
-    # F = zeta (fu[umap] - c), offset = zeta0 fu[u0] + c sum(zeta), c = fu[u0]
-    dfu[u0] += -zF.sum(0) + zsum * dC_root + float(keep["zeta0"]) * dC_root
+    if P.c.n_entries == 0:
+        return torch.zeros_like(fu)
+    zrow, (value_run, begin, rows), u0, factor = _row_factors(keep)
+    dfu = torch.empty_like(fu)
+    n, n_runs, d_out = int(fu.shape[0]), int(begin.numel()) - 1, int(fu.shape[1])
+    nws = capi.size("smx_nodal_adjoint_workspace", n, n_runs, d_out)
+    ws = torch.empty(nws, dtype=torch.uint8, device=fu.device)
+    ptr = capi.ptr
+    capi.call("smx_nodal_adjoint", ptr(Fbar), ptr(zrow), n, n_runs, d_out, ptr(value_run), ptr(begin), ptr(rows),
+              ptr(dC_root), factor, u0, ptr(dfu), ptr(ws), nws, capi.stream_ptr(torch.cuda.current_stream()))
     return dfu
 
 

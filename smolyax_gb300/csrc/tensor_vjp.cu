@@ -656,6 +656,107 @@ __global__ void __launch_bounds__(256) output_slices_kernel(const float* __restr
   }
 }
 
+// ---- the adjoints' way back to coefficients and nodal values ----------------------------
+// Column sums in FP64 in a fixed order: blocks of kSumRows rows (a warp reads whole
+// lines: 2^to_log columns by 256 >> to_log row lanes), then the blocks' sums.
+constexpr int kSumRows = 512, kSumThreads = 256;
+
+__device__ __forceinline__ double sum_lanes(double v, int to_log, double* red) {
+  const int t = threadIdx.x;
+  red[t] = v;
+  __syncthreads();
+  for (int n = kSumThreads >> 1; n >= (1 << to_log); n >>= 1) {
+    if (t < n) red[t] += red[t + n];
+    __syncthreads();
+  }
+  return red[t];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads) column_partial_kernel(const T* __restrict__ A, int64_t n, int64_t ld,
+                                                                     int d, int to_log, double* __restrict__ part) {
+  __shared__ double red[kSumThreads];
+  const int t = threadIdx.x, o = (int(blockIdx.y) << to_log) + (t & ((1 << to_log) - 1));
+  const int64_t r0 = blockIdx.x * int64_t(kSumRows), r1 = min(n, r0 + kSumRows);
+  double acc = 0.0;
+  if (o < d) {
+#pragma unroll 8
+    for (int64_t r = r0 + (t >> to_log); r < r1; r += kSumThreads >> to_log) acc += double(__ldg(A + r * ld + o));
+  }
+  acc = sum_lanes(acc, to_log, red);
+  if (t < (1 << to_log) && o < d) part[blockIdx.x * int64_t(d) + o] = acc;
+}
+
+// out[o] = sum, or (extra given) out[o] + factor * extra[o] - sum.
+__global__ void __launch_bounds__(kSumThreads) column_final_kernel(const double* __restrict__ part, int64_t blocks, int d,
+                                                                   int to_log, const double* __restrict__ extra,
+                                                                   double factor, double* __restrict__ out) {
+  __shared__ double red[kSumThreads];
+  const int t = threadIdx.x, o = (int(blockIdx.x) << to_log) + (t & ((1 << to_log) - 1));
+  double acc = 0.0;
+  if (o < d) {
+#pragma unroll 8
+    for (int64_t b = t >> to_log; b < blocks; b += kSumThreads >> to_log) acc += __ldg(part + b * d + o);
+  }
+  acc = sum_lanes(acc, to_log, red);
+  if (t < (1 << to_log) && o < d) out[o] = extra ? out[o] + factor * extra[o] - acc : acc;
+}
+
+int sum_log(int d) {
+  int l = 0;
+  while (l < 8 && (1 << l) < d) ++l;
+  return l;
+}
+
+size_t sum_bytes(int64_t n, int d) { return size_t((n + kSumRows - 1) / kSumRows) * d * sizeof(double); }
+
+template <typename T>
+void column_sums(const T* A, int64_t n, int64_t ld, int d, double* part, const double* extra, double factor, double* out,
+                 cudaStream_t st) {
+  const int l = sum_log(d);
+  const int64_t blocks = (n + kSumRows - 1) / kSumRows;
+  const unsigned tiles = unsigned((d + (1 << l) - 1) >> l);
+  column_partial_kernel<<<dim3(unsigned(blocks), tiles), kSumThreads, 0, st>>>(A, n, ld, d, l, part);
+  column_final_kernel<<<tiles, kSumThreads, 0, st>>>(part, blocks, d, l, extra, factor, out);
+}
+
+// Rows of dL/dC from the tape's order (pad rows first) to the entries', in FP64.
+__global__ void coef_rows_kernel(const float* __restrict__ rows, int64_t pad, int64_t K, int d,
+                                 const int64_t* __restrict__ ent, double* __restrict__ dC) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= K * d) return;
+  const int64_t j = i / d;
+  dC[__ldg(ent + j) * d + (i - j * d)] = double(rows[(pad + j) * d + (i - j * d)]);
+}
+
+// Sums of runs [begin[i], begin[i + 1]) of A (rows row[..] of it, each times its
+// weight; or A's rows as they are), in order.  dL/d(nodal values) is two of them:
+// runs of at most 64 rows, then the runs of each value, because with nested nodes one
+// value may stand in half of all rows.  Leja |Lambda| = 5000, 5000 values x 64
+// outputs: 25 + 15 us; a thread through all rows of a value 2.4 ms.  The chain rule
+// as a dozen tensor operations (multiply, index_add, sums, ...) cost the host more
+// than the GPU: a training step of 1e3 points 0.9 ms, 0.68 with these kernels.
+template <bool ROWS>
+__global__ void run_sum_kernel(const double* __restrict__ A, const double* __restrict__ weight,
+                               const int64_t* __restrict__ row, const int64_t* __restrict__ begin, int64_t n, int d,
+                               double* __restrict__ out) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= n * d) return;
+  const int64_t u = i / d, q1 = __ldg(begin + u + 1);
+  const int o = int(i - u * d);
+  double acc = 0.0;
+#pragma unroll 8
+  for (int64_t q = __ldg(begin + u); q < q1; ++q) {
+    if constexpr (ROWS) {
+      const int64_t r = __ldg(row + q);
+      acc = fma(__ldg(weight + r), __ldg(A + r * d + o), acc);
+    } else {
+      acc += __ldg(A + q * d + o);
+    }
+  }
+  out[i] = acc;
+}
+
 size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 size_t walk_smem(const smx_tensor* t, const smx_walk& w) {
@@ -712,7 +813,7 @@ size_t coef_smem(int warps, int slots) { return size_t(warps) * (1024 + 9 * 256)
 
 struct CoefLayout {  // workspace of one chunk of m points
   int64_t gstride, slices, E;
-  size_t panel, scales, rows, cot, gscale, out, partial, total;
+  size_t panel, scales, rows, cot, gscale, out, dC, partial, total;
 };
 CoefLayout coef_layout(const smx_tensor* t, int64_t m) {
   CoefLayout L;
@@ -725,8 +826,9 @@ CoefLayout coef_layout(const smx_tensor* t, int64_t m) {
   L.cot = up256(size_t(L.slices) * t->d_out * 128);
   L.gscale = up256(size_t(L.slices) * 4);
   L.out = up256(size_t(t->d_out) * 4);
+  L.dC = up256(size_t(L.E) * t->d_out * 4);
   L.partial = t->splits > 1 ? up256(size_t(t->splits) * L.E * t->d_out * 4) : 0;
-  L.total = 2 * L.panel + L.scales + L.rows + 2 * L.cot + L.gscale + 2 * L.out + L.partial;
+  L.total = 2 * L.panel + L.scales + L.rows + 2 * L.cot + L.gscale + 2 * L.out + L.dC + L.partial;
   return L;
 }
 
@@ -778,18 +880,19 @@ extern "C" int smx_tensor_coef_splits(int d_out, int K) {
 
 extern "C" size_t smx_tensor_vjp_coef_workspace(const smx_tensor* t, int64_t P) {
   if (!t || P <= 0 || t->chunk < 1 || t->K < 1 || coef_smem(16, t->n_slots) > kSmemMax) return 0;
-  return coef_layout(t, std::min(P, t->chunk)).total;
+  return up256(sum_bytes(P, t->d_out)) + coef_layout(t, std::min(P, t->chunk)).total;
 }
 
 extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t P, int64_t ldx, const float* g,
-                                   int64_t ldg, float* dC, void* ws, size_t ws_bytes, void* stream) {
+                                   int64_t ldg, const int64_t* ent, double* dC, void* ws, size_t ws_bytes,
+                                   void* stream) {
   SMX_REQUIRE(t != nullptr, "smx_tensor_vjp_coef: null plan");
   SMX_REQUIRE(t->d_in >= 1 && t->d_out >= 1 && t->K >= 1 && t->n_groups == (t->K + kGroup - 1) / kGroup &&
                   t->splits >= 1 && t->chunk >= 64 && t->chunk % 64 == 0 &&
                   (std::min(P, t->chunk) + 63) / 64 * std::max<int64_t>(64 * t->n_groups, t->d_out) < (int64_t(1) << 31),
               "smx_tensor_vjp_coef: bad plan sizes");
   SMX_REQUIRE(P >= 1 && ldx >= t->d_in && ldg >= t->d_out, "smx_tensor_vjp_coef: bad sizes");
-  SMX_REQUIRE(x && g && dC && t->err && t->dims && t->dmax && t->dsoff && t->fam && t->fam_a && t->fam_b && t->rec &&
+  SMX_REQUIRE(x && g && ent && dC && t->err && t->dims && t->dmax && t->dsoff && t->fam && t->fam_a && t->fam_b && t->rec &&
                   t->tape && t->path,
               "smx_tensor_vjp_coef: null pointer");
   SMX_REQUIRE(coef_smem(16, t->n_slots) <= kSmemMax, "smx_tensor_vjp_coef: the basis rows do not fit in shared memory");
@@ -800,10 +903,15 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_coef: no device");
+  // the constant's row, then the others chunk by chunk
+  double* sums = static_cast<double*>(ws);
+  column_sums(g, P, ldg, t->d_out, sums, nullptr, 0.0, dC, st);
+  const size_t first = up256(sum_bytes(P, t->d_out)), dC_bytes = coef_layout(t, 1).dC;
+  float* rows = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + first);
   for (int64_t p0 = 0; p0 < P; p0 += t->chunk) {
     const int64_t m = std::min(t->chunk, P - p0);
     const CoefLayout L = coef_layout(t, m);
-    uint8_t* q = static_cast<uint8_t*>(ws);
+    uint8_t* q = static_cast<uint8_t*>(ws) + first + dC_bytes;
     auto take = [&](size_t bytes) {
       uint8_t* r = q;
       q += bytes;
@@ -838,12 +946,42 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
     s.row_scale = S, s.ld_scale = L.E;
     s.col_scale = scale;
     s.M = int(L.E), s.N = t->d_out, s.K = int(L.slices * 64);
-    s.D = dC, s.ldd = t->d_out;
+    s.D = rows, s.ldd = t->d_out;
     s.err = t->err, s.splits = t->splits, s.partial = reinterpret_cast<float*>(q);
     s.accumulate = p0 > 0;
     const int rc = split_gemm(s, st);
     if (rc) return rc;
   }
+  coef_rows_kernel<<<smx::grid_for(int64_t(t->K) * t->d_out, 256), 256, 0, st>>>(
+      rows, int64_t(t->n_groups) * kGroup - t->K, t->K, t->d_out, ent, dC);
+  SMX_LAUNCH_CHECK("smx_tensor_vjp_coef");
+  return SMX_OK;
+}
+
+extern "C" size_t smx_nodal_adjoint_workspace(int64_t n_values, int64_t n_runs, int d_out) {
+  return n_values > 0 && n_runs >= 0 && d_out > 0 ? sum_bytes(n_values, d_out) + size_t(n_runs) * d_out * sizeof(double)
+                                                  : 0;
+}
+
+extern "C" int smx_nodal_adjoint(const double* Fbar, const double* zeta, int64_t n_values, int64_t n_runs, int d_out,
+                                 const int64_t* value_run, const int64_t* run_begin, const int64_t* row,
+                                 const double* root, double root_factor, int64_t first, double* out, void* ws,
+                                 size_t ws_bytes, void* stream) {
+  SMX_REQUIRE(n_values >= 1 && n_runs >= 0 && d_out >= 1 && first >= 0 && first < n_values,
+              "smx_nodal_adjoint: bad sizes");
+  SMX_REQUIRE(Fbar && zeta && value_run && run_begin && row && root && out, "smx_nodal_adjoint: null pointer");
+  SMX_REQUIRE(ws && ws_bytes >= smx_nodal_adjoint_workspace(n_values, n_runs, d_out) &&
+                  (reinterpret_cast<uintptr_t>(ws) & 7) == 0,
+              "smx_nodal_adjoint: workspace too small or not 8-byte aligned");
+  cudaStream_t st = smx::as_stream(stream);
+  double* runs = static_cast<double*>(ws);
+  if (n_runs)
+    run_sum_kernel<true><<<smx::grid_for(n_runs * d_out, 256), 256, 0, st>>>(Fbar, zeta, row, run_begin, n_runs, d_out,
+                                                                             runs);
+  run_sum_kernel<false><<<smx::grid_for(n_values * d_out, 256), 256, 0, st>>>(runs, nullptr, nullptr, value_run,
+                                                                              n_values, d_out, out);
+  column_sums(out, n_values, d_out, d_out, runs + n_runs * d_out, root, root_factor, out + first * d_out, st);
+  SMX_LAUNCH_CHECK("smx_nodal_adjoint");
   return SMX_OK;
 }
 

@@ -471,19 +471,17 @@ class SpectralPlan:
         return (t, tape) if capi.size("smx_tensor_vjp_coef_workspace", ctypes.byref(t), 64) else None
 
     def _vjp_coef(self, x, g):
-        """dL/dC [n_lambda, d_out] FP64 but for the constant's row."""
+        """dL/dC [n_lambda, d_out] FP64 by the sliced FP16 panel."""
         import ctypes
 
         ops = self._backward_ops()
         t, _ = ops["coef"]
-        P, d_out, K = int(x.shape[0]), int(g.shape[1]), ops["K"]
+        P, d_out = int(x.shape[0]), int(g.shape[1])
         nws = capi.size("smx_tensor_vjp_coef_workspace", ctypes.byref(t), P)
         ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
-        rows = torch.empty(64 * t.n_groups, d_out, dtype=torch.float32, device=x.device)
-        call("smx_tensor_vjp_coef", ctypes.byref(t), ptr(x), P, int(x.shape[1]), ptr(g), d_out, ptr(rows), ptr(ws), nws,
-             capi.stream_ptr(torch.cuda.current_stream()))
-        dC = torch.zeros(int(self.C64.shape[0]), d_out, dtype=torch.float64, device=x.device)
-        dC[ops["ent"]] = rows[64 * t.n_groups - K :].double()  # the padding comes first
+        dC = torch.empty(int(self.C64.shape[0]), d_out, dtype=torch.float64, device=x.device)
+        call("smx_tensor_vjp_coef", ctypes.byref(t), ptr(x), P, int(x.shape[1]), ptr(g), d_out, ptr(ops["ent"]), ptr(dC),
+             ptr(ws), nws, capi.stream_ptr(torch.cuda.current_stream()))
         return dC
 
     def vjp_x_workspace(self, P):
@@ -535,7 +533,8 @@ class SpectralPlan:
             need_x = False
         if need_coef and ops["coef"] is not None and P:
             dC = self._vjp_coef(x, gf)
-            dC[0] = g.sum(0, dtype=torch.float64)
+            if g.dtype == torch.float64:
+                dC[0] = g.sum(0)
             need_coef = False
         if need_x or need_coef:
             g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
