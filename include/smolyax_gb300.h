@@ -753,12 +753,15 @@ int smx_tensor_vjp_x(const smx_tensor* plan_host, const smx_tensor_bwd* bwd_host
 /* dL/dC [n_lambda][d_out] (FP64) of y = c0 + A C: A^T g in FP32 over plan->chunk points at
  * a time (a multiple of 64) with the plan's splits (smx_tensor_coef_splits) over the
  * points, written to the rows ent[K] of the tape's entries; row 0 (the constant) is the
- * sum of g.  Plans with more basis slots than fit in shared memory (workspace 0) are
+ * sum of g.  `rows`: the basis values of the same points as smx_tensor_vjp_x leaves them at
+ * the start of its workspace, [n_slots][P rounded up to 128], or NULL (used where P points
+ * are one pass).  Plans with more basis slots than fit in shared memory (workspace 0) are
  * refused. */
 int smx_tensor_coef_splits(int d_out, int K);
 size_t smx_tensor_vjp_coef_workspace(const smx_tensor* plan_host, int64_t P);
 int smx_tensor_vjp_coef(const smx_tensor* plan_host, const double* x, int64_t P, int64_t ldx, const float* g,
-                        int64_t ldg, const int64_t* ent, double* dC, void* ws, size_t ws_bytes, void* stream);
+                        int64_t ldg, const int64_t* ent, const float* rows, double* dC, void* ws, size_t ws_bytes,
+                        void* stream);
 /* dL/d(nodal values) out[n_values][d_out] from dL/dF Fbar[rows][d_out] of the rows
  * F[r] = zeta_r (f[u(r)] - f[first]): `row` lists the rows by value, run i is row[run_begin[i]]
  * .. row[run_begin[i+1]) (of one value, a few dozen rows), value u has the runs value_run[u]

@@ -376,7 +376,7 @@ SIGNATURES = {
     "smx_tensor_vjp_x": (_int, [_p, _p, _p, _i64, _i64, _p, _i64, _p, _i64, _p, _sz, _p]),
     "smx_tensor_coef_splits": (_int, [_int, _int]),
     "smx_tensor_vjp_coef_workspace": (_sz, [_p, _i64]),
-    "smx_tensor_vjp_coef": (_int, [_p, _p, _i64, _i64, _p, _i64, _p, _p, _p, _sz, _p]),
+    "smx_tensor_vjp_coef": (_int, [_p, _p, _i64, _i64, _p, _i64, _p, _p, _p, _p, _sz, _p]),
     "smx_nodal_adjoint_workspace": (_sz, [_i64, _i64, _int]),
     "smx_nodal_adjoint": (_int, [_p, _p, _i64, _i64, _int, _p, _p, _p, _p, _dbl, _i64, _p, _p, _sz, _p]),
     "smx_tensor_workspace": (_sz, [_p, _i64]),

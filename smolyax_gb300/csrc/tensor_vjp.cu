@@ -583,25 +583,34 @@ __global__ void __launch_bounds__(32 * W, MINB)
   }
 }
 
-// Largest finite |g| of every output (bits; `most` starts at zero) ...
+// Per output the largest finite |g| (bits; `most` starts at zero) and the sum of
+// each block's kSumRows points in FP64 ...
+constexpr int kSumRows = 512;
 __global__ void __launch_bounds__(256) output_most_kernel(const float* __restrict__ g, int64_t ldg, int64_t P, int d_out,
-                                                          unsigned* __restrict__ most) {
+                                                          unsigned* __restrict__ most, double* __restrict__ part) {
   __shared__ float red[8][33];
+  __shared__ double sum[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int o0 = blockIdx.y * 32; o0 < d_out; o0 += gridDim.y * 32) {
     const int o = o0 + lane;
-    const int64_t p1 = min(P, (blockIdx.x + 1) * int64_t(512));
+    const int64_t p1 = min(P, (blockIdx.x + 1) * int64_t(kSumRows));
     float m = 0.f;
-    if (o < d_out)
-      for (int64_t p = blockIdx.x * int64_t(512) + warp; p < p1; p += 8) {
-        const float a = fabsf(__ldg(g + p * ldg + o));
+    double acc = 0.0;
+    if (o < d_out) {
+#pragma unroll 8
+      for (int64_t p = blockIdx.x * int64_t(kSumRows) + warp; p < p1; p += 8) {
+        const float v = __ldg(g + p * ldg + o), a = fabsf(v);
         if (a <= 3.0e38f) m = fmaxf(m, a);
+        acc += double(v);
       }
+    }
     red[warp][lane] = m;
+    sum[warp][lane] = acc;
     __syncthreads();
     if (warp == 0 && o < d_out) {
-      for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w][lane]);
+      for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w][lane]), acc += sum[w][lane];
       if (m > 0.f) atomicMax(most + o, __float_as_uint(m));
+      part[blockIdx.x * int64_t(d_out) + o] = acc;
     }
     __syncthreads();
   }
@@ -659,7 +668,7 @@ __global__ void __launch_bounds__(256) output_slices_kernel(const float* __restr
 // ---- the adjoints' way back to coefficients and nodal values ----------------------------
 // Column sums in FP64 in a fixed order: blocks of kSumRows rows (a warp reads whole
 // lines: 2^to_log columns by 256 >> to_log row lanes), then the blocks' sums.
-constexpr int kSumRows = 512, kSumThreads = 256;
+constexpr int kSumThreads = 256;
 
 __device__ __forceinline__ double sum_lanes(double v, int to_log, double* red) {
   const int t = threadIdx.x;
@@ -672,16 +681,15 @@ __device__ __forceinline__ double sum_lanes(double v, int to_log, double* red) {
   return red[t];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSumThreads) column_partial_kernel(const T* __restrict__ A, int64_t n, int64_t ld,
-                                                                     int d, int to_log, double* __restrict__ part) {
+__global__ void __launch_bounds__(kSumThreads) column_partial_kernel(const double* __restrict__ A, int64_t n, int d,
+                                                                     int to_log, double* __restrict__ part) {
   __shared__ double red[kSumThreads];
   const int t = threadIdx.x, o = (int(blockIdx.y) << to_log) + (t & ((1 << to_log) - 1));
   const int64_t r0 = blockIdx.x * int64_t(kSumRows), r1 = min(n, r0 + kSumRows);
   double acc = 0.0;
   if (o < d) {
 #pragma unroll 8
-    for (int64_t r = r0 + (t >> to_log); r < r1; r += kSumThreads >> to_log) acc += double(__ldg(A + r * ld + o));
+    for (int64_t r = r0 + (t >> to_log); r < r1; r += kSumThreads >> to_log) acc += __ldg(A + r * d + o);
   }
   acc = sum_lanes(acc, to_log, red);
   if (t < (1 << to_log) && o < d) part[blockIdx.x * int64_t(d) + o] = acc;
@@ -710,14 +718,11 @@ int sum_log(int d) {
 
 size_t sum_bytes(int64_t n, int d) { return size_t((n + kSumRows - 1) / kSumRows) * d * sizeof(double); }
 
-template <typename T>
-void column_sums(const T* A, int64_t n, int64_t ld, int d, double* part, const double* extra, double factor, double* out,
-                 cudaStream_t st) {
+// Sums of the blocks' column sums.
+void column_finish(const double* part, int64_t blocks, int d, const double* extra, double factor, double* out,
+                   cudaStream_t st) {
   const int l = sum_log(d);
-  const int64_t blocks = (n + kSumRows - 1) / kSumRows;
-  const unsigned tiles = unsigned((d + (1 << l) - 1) >> l);
-  column_partial_kernel<<<dim3(unsigned(blocks), tiles), kSumThreads, 0, st>>>(A, n, ld, d, l, part);
-  column_final_kernel<<<tiles, kSumThreads, 0, st>>>(part, blocks, d, l, extra, factor, out);
+  column_final_kernel<<<unsigned((d + (1 << l) - 1) >> l), kSumThreads, 0, st>>>(part, blocks, d, l, extra, factor, out);
 }
 
 // Rows of dL/dC from the tape's order (pad rows first) to the entries', in FP64.
@@ -832,6 +837,12 @@ CoefLayout coef_layout(const smx_tensor* t, int64_t m) {
   return L;
 }
 
+// Sums of g by blocks of kSumRows points, in each chunk.
+size_t coef_sum_bytes(const smx_tensor* t, int64_t P) {
+  const int64_t whole = P / t->chunk;
+  return size_t(whole) * sum_bytes(t->chunk, t->d_out) + sum_bytes(P - whole * t->chunk, t->d_out);
+}
+
 template <int W, int MINB>
 void launch_coef_panel(const smx_tensor& t, const CoefLayout& L, const float* grow, const float* gscale, uint32_t* AH,
                        uint32_t* AL, float* S, int sms, cudaStream_t st) {
@@ -880,12 +891,12 @@ extern "C" int smx_tensor_coef_splits(int d_out, int K) {
 
 extern "C" size_t smx_tensor_vjp_coef_workspace(const smx_tensor* t, int64_t P) {
   if (!t || P <= 0 || t->chunk < 1 || t->K < 1 || coef_smem(16, t->n_slots) > kSmemMax) return 0;
-  return up256(sum_bytes(P, t->d_out)) + coef_layout(t, std::min(P, t->chunk)).total;
+  return up256(coef_sum_bytes(t, P)) + coef_layout(t, std::min(P, t->chunk)).total;
 }
 
 extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t P, int64_t ldx, const float* g,
-                                   int64_t ldg, const int64_t* ent, double* dC, void* ws, size_t ws_bytes,
-                                   void* stream) {
+                                   int64_t ldg, const int64_t* ent, const float* rows_given, double* dC, void* ws,
+                                   size_t ws_bytes, void* stream) {
   SMX_REQUIRE(t != nullptr, "smx_tensor_vjp_coef: null plan");
   SMX_REQUIRE(t->d_in >= 1 && t->d_out >= 1 && t->K >= 1 && t->n_groups == (t->K + kGroup - 1) / kGroup &&
                   t->splits >= 1 && t->chunk >= 64 && t->chunk % 64 == 0 &&
@@ -896,17 +907,17 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
                   t->tape && t->path,
               "smx_tensor_vjp_coef: null pointer");
   SMX_REQUIRE(coef_smem(16, t->n_slots) <= kSmemMax, "smx_tensor_vjp_coef: the basis rows do not fit in shared memory");
-  SMX_REQUIRE(ws && ws_bytes >= smx_tensor_vjp_coef_workspace(t, P) && (reinterpret_cast<uintptr_t>(ws) & 15) == 0,
+  SMX_REQUIRE(ws && ws_bytes >= smx_tensor_vjp_coef_workspace(t, P) && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 &&
+                  (reinterpret_cast<uintptr_t>(rows_given) & 15) == 0,
               "smx_tensor_vjp_coef: workspace too small or not 16-byte aligned");
   cudaStream_t st = smx::as_stream(stream);
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_coef: no device");
-  // the constant's row, then the others chunk by chunk
-  double* sums = static_cast<double*>(ws);
-  column_sums(g, P, ldg, t->d_out, sums, nullptr, 0.0, dC, st);
-  const size_t first = up256(sum_bytes(P, t->d_out)), dC_bytes = coef_layout(t, 1).dC;
+  double* sums = static_cast<double*>(ws);  // of g, for the constant's row
+  int64_t sum_blocks = 0;
+  const size_t first = up256(coef_sum_bytes(t, P)), dC_bytes = coef_layout(t, 1).dC;
   float* rows = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + first);
   for (int64_t p0 = 0; p0 < P; p0 += t->chunk) {
     const int64_t m = std::min(t->chunk, P - p0);
@@ -928,11 +939,15 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
     float* scale = reinterpret_cast<float*>(take(L.out));
     if (cudaMemsetAsync(most, 0, size_t(t->d_out) * 4, st) != cudaSuccess)
       return smx::set_error(SMX_ERR_CUDA, "smx_tensor_vjp_coef: memset failed");
-    const dim3 ogrid(unsigned((m + 511) / 512), unsigned(std::min((t->d_out + 31) / 32, 65535)));
-    output_most_kernel<<<ogrid, 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most);
+    const dim3 ogrid(unsigned((m + kSumRows - 1) / kSumRows), unsigned(std::min((t->d_out + 31) / 32, 65535)));
+    output_most_kernel<<<ogrid, 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, sums + sum_blocks * t->d_out);
+    sum_blocks += ogrid.x;
     output_slices_kernel<<<unsigned(L.slices), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, gh, gl, gscale,
                                                              scale);
-    tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st);
+    if (rows_given && P <= t->chunk)
+      grow = const_cast<float*>(rows_given);
+    else
+      tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st);
     // two blocks of 8 warps per SM while their rows fit (up to ~330 slots), else one of 16
     if (coef_smem(8, t->n_slots) <= (kSmemMax - 2048) / 2)
       launch_coef_panel<8, 2>(*t, L, grow, gscale, AH, AL, S, sms, st);
@@ -952,6 +967,7 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
     const int rc = split_gemm(s, st);
     if (rc) return rc;
   }
+  column_finish(sums, sum_blocks, t->d_out, nullptr, 0.0, dC, st);
   coef_rows_kernel<<<smx::grid_for(int64_t(t->K) * t->d_out, 256), 256, 0, st>>>(
       rows, int64_t(t->n_groups) * kGroup - t->K, t->K, t->d_out, ent, dC);
   SMX_LAUNCH_CHECK("smx_tensor_vjp_coef");
@@ -980,7 +996,12 @@ extern "C" int smx_nodal_adjoint(const double* Fbar, const double* zeta, int64_t
                                                                              runs);
   run_sum_kernel<false><<<smx::grid_for(n_values * d_out, 256), 256, 0, st>>>(runs, nullptr, nullptr, value_run,
                                                                               n_values, d_out, out);
-  column_sums(out, n_values, d_out, d_out, runs + n_runs * d_out, root, root_factor, out + first * d_out, st);
+  double* part = runs + n_runs * d_out;
+  const int l = sum_log(d_out);
+  const int64_t blocks = (n_values + kSumRows - 1) / kSumRows;
+  column_partial_kernel<<<dim3(unsigned(blocks), unsigned((d_out + (1 << l) - 1) >> l)), kSumThreads, 0, st>>>(
+      out, n_values, d_out, l, part);
+  column_finish(part, blocks, d_out, root, root_factor, out + first * d_out, st);
   SMX_LAUNCH_CHECK("smx_nodal_adjoint");
   return SMX_OK;
 }

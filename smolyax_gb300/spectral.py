@@ -470,7 +470,7 @@ class SpectralPlan:
         t.chunk = max(128, min(int(self.memory_limit * 1024**3 // per_point), 1 << 22) // 128 * 128)
         return (t, tape) if capi.size("smx_tensor_vjp_coef_workspace", ctypes.byref(t), 64) else None
 
-    def _vjp_coef(self, x, g):
+    def _vjp_coef(self, x, g, rows=None):
         """dL/dC [n_lambda, d_out] FP64 by the sliced FP16 panel."""
         import ctypes
 
@@ -480,8 +480,8 @@ class SpectralPlan:
         nws = capi.size("smx_tensor_vjp_coef_workspace", ctypes.byref(t), P)
         ws = torch.empty(nws, dtype=torch.uint8, device=x.device)
         dC = torch.empty(int(self.C64.shape[0]), d_out, dtype=torch.float64, device=x.device)
-        call("smx_tensor_vjp_coef", ctypes.byref(t), ptr(x), P, int(x.shape[1]), ptr(g), d_out, ptr(ops["ent"]), ptr(dC),
-             ptr(ws), nws, capi.stream_ptr(torch.cuda.current_stream()))
+        call("smx_tensor_vjp_coef", ctypes.byref(t), ptr(x), P, int(x.shape[1]), ptr(g), d_out, ptr(ops["ent"]),
+             ptr(rows), ptr(dC), ptr(ws), nws, capi.stream_ptr(torch.cuda.current_stream()))
         return dC
 
     def vjp_x_workspace(self, P):
@@ -506,7 +506,7 @@ class SpectralPlan:
         ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=x.device)
         call("smx_tensor_vjp_x", ctypes.byref(t), ctypes.byref(b), ptr(x), P, d, ptr(g), int(g.shape[1]), ptr(dx), d,
              ptr(ws), nws, capi.stream_ptr(torch.cuda.current_stream()))
-        return dx
+        return dx, ws if P <= b.chunk else None
 
     def vjp(self, x, g, need_x=True, need_coef=True, check=True):
         """Vector-Jacobian products of y = c0 + A(x) C at cotangent g [P, d_out]:
@@ -526,13 +526,13 @@ class SpectralPlan:
                 ptr(seg), n_seg, ptr(k["fam_a"]), ptr(k["fam_b"]), ptr(k["fam"]))
         gf = g.float().contiguous()
         err = ops["err"]
-        dx = dC = None
+        dx = dC = rows = None
         step = max(128, int(self.memory_limit * 1024**3 // (8 * ldk)) // 128 * 128)
         if need_x and ops["walk"] is not None:
-            dx = self._vjp_x_walk(x, gf)
+            dx, rows = self._vjp_x_walk(x, gf)  # the basis rows of all points, if one pass
             need_x = False
         if need_coef and ops["coef"] is not None and P:
-            dC = self._vjp_coef(x, gf)
+            dC = self._vjp_coef(x, gf, rows)
             if g.dtype == torch.float64:
                 dC[0] = g.sum(0)
             need_coef = False

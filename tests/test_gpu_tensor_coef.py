@@ -73,3 +73,17 @@ def test_plans_with_many_slots_keep_their_path():
     dC = sp.vjp(torch.as_tensor(x, device="cuda"), torch.as_tensor(g, device="cuda"), need_x=False)[1].cpu().numpy()
     ref = _direct(sp, x, g.astype(np.float64))
     assert np.abs(dC - ref).max() < 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("P", [1, 129, 700])
+def test_basis_rows_of_the_walk_are_shared(P):
+    """dL/dx and dL/dC together (one set of basis rows) are what they are alone."""
+    ip, sp = _plan(40, 5, 900)
+    rng = np.random.default_rng(P)
+    x = torch.as_tensor(rng.uniform(-1, 1, (P, 40)), device="cuda")
+    g = torch.as_tensor(rng.normal(size=(P, 5)).astype(np.float32), device="cuda")
+    dx, dC = sp.vjp(x, g)
+    assert torch.equal(dx, sp.vjp(x, g, need_coef=False)[0]) and torch.equal(dC, sp.vjp(x, g, need_x=False)[1])
+    sp._backward_ops()["walk"][1].chunk = 128  # several passes of the walk: its rows are of the last
+    many = sp.vjp(x, g)
+    assert torch.equal(many[0], dx) and torch.equal(many[1], dC)
