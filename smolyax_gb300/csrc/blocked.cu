@@ -421,11 +421,14 @@ struct TabOff {
   int n_ent16, n_w, n_items;  // 16-byte words of hot_ent, rows of W, work items
 };
 
+// (asynchronously: all tables are in flight at once, not one after the other: 1e5
+// points x 1000 dimensions 255.2 -> 252.5 us, one cold point 31.5 -> 28.6)
 template <typename T>
 __device__ __forceinline__ const T* tab_copy(uint8_t* base, int off, const T* src, int n16) {
-  int4* d = reinterpret_cast<int4*>(base + off);
-  const int4* s = reinterpret_cast<const int4*>(src);
-  for (int i = threadIdx.x; i < n16; i += kThr) d[i] = __ldg(s + i);
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(base + off));
+  const char* s = reinterpret_cast<const char*>(src);
+  for (int i = threadIdx.x; i < n16; i += kThr)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + i * 16), "l"(s + int64_t(i) * 16) : "memory");
   return reinterpret_cast<const T*>(base + off);
 }
 
@@ -445,12 +448,14 @@ __global__ void __launch_bounds__(kThr, 1)
     a.grp_ab = tab_copy(tb, to.grp_ab, a.grp_ab, (to.W - to.grp_ab) / 16);
     a.W = tab_copy(tb, to.W, a.W, to.n_w);
     {
-      int32_t* d = reinterpret_cast<int32_t*>(tb + to.items);
-      for (int i = threadIdx.x; i < to.n_items; i += kThr) d[i] = __ldg(a.items + i);
-      a.items = d;
-      int32_t* w = reinterpret_cast<int32_t*>(tb + to.warp_off);
-      if (threadIdx.x <= kW) w[threadIdx.x] = __ldg(a.warp_off + threadIdx.x);
-      a.warp_off = w;
+      auto copy4 = [&](int off, const int32_t* src, int n) {
+        const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(tb + off));
+        for (int i = threadIdx.x; i < n; i += kThr)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + i * 4), "l"(src + i) : "memory");
+        return reinterpret_cast<const int32_t*>(tb + off);
+      };
+      a.items = copy4(to.items, a.items, to.n_items);
+      a.warp_off = copy4(to.warp_off, a.warp_off, kW + 1);
       int4* hd = reinterpret_cast<int4*>(tb + to.hd);
       float2* hab = reinterpret_cast<float2*>(tb + to.hab);
       for (int h = threadIdx.x; h < a.n_hot_dims; h += kThr) {
@@ -461,6 +466,7 @@ __global__ void __launch_bounds__(kThr, 1)
       a.hd = hd;
       a.hab = hab;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
   }
   const int64_t n_tiles = (P + 32 * NP - 1) / (32 * NP);
