@@ -243,11 +243,31 @@ __device__ __forceinline__ void blocked_tile(const BArgs& a, const double* __res
     float ys[NP], yc[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) ys[i] = yc[i] = 0.f;
-    // hot items come first in every warp's list, cold groups after them
-    int it = it0 + split_c;
-    for (; it < it1; it += split_S) {
-      const int code = tl<TS>(a.items + it);
-      if (code & kColdBit) break;
+    // hot items come first in every warp's list, cold groups after them.  The x
+    // values of group n + 1 are loaded while group n is contracted and turned into
+    // basis values an iteration later; the short groups at the end of the list each
+    // wait for theirs behind a hot item (1e5 points x 1000 dimensions: 252.5 -> 246.6
+    // us).
+    int hot = it0 + split_c, cold = hot;
+    for (int i0 = it0; i0 < it1; i0 += 32) {
+      const int code = tl<TS>(a.items + min(i0 + lane, it1 - 1));
+      const int n = __popc(__ballot_sync(0xffffffffu, i0 + lane < it1 && !(code & kColdBit)));
+      while (cold < i0 + n) cold += split_S;
+      if (n < 32) break;
+    }
+    int n_hot = (cold - hot) / split_S;
+    int n_cold = cold < it1 ? (it1 - cold + split_S - 1) / split_S : 0;
+    int g = 0;
+    int4 gd = make_int4(0, 0, 0, 0), gdim = gd;
+    double xv[NP][4];
+    if (n_cold) {
+      g = tl<TS>(a.items + cold) & (kColdBit - 1);
+      gd = tl<TS>(a.grp + 3 * g), gdim = tl<TS>(a.grp + 3 * g + 1);
+      load_x<NP>(x, prow, fastx, gd, gdim, xv);
+    }
+    for (;; --n_cold, cold += split_S) {
+      for (; n_hot > 0 && n_hot >= n_cold; --n_hot, hot += split_S) {
+        const int code = tl<TS>(a.items + hot);
         // hot node: gather over its hot entries, times the path product
         const int4 h0 = tl<TS>(a.node + 3 * code), pa = tl<TS>(a.node + 3 * code + 1),
                    pb = tl<TS>(a.node + 3 * code + 2);
@@ -271,17 +291,9 @@ __device__ __forceinline__ void blocked_tile(const BArgs& a, const double* __res
         const float va[4] = {p01.x, p01.y, p23.x, p23.y};
 #pragma unroll
         for (int i = 0; i < NP; ++i) kahan_add(ys[i], yc[i], va[i]);
-    }
-
-    // cold groups, software-pipelined: the x values of group n + 1 are loaded
-    // while group n is contracted; they are turned into basis values at the
-    // start of the next iteration.
-    if (it < it1) {
-      int g = tl<TS>(a.items + it) & (kColdBit - 1);
-      int4 gd = tl<TS>(a.grp + 3 * g), gdim = tl<TS>(a.grp + 3 * g + 1);
-      double xv[NP][4];
-      load_x<NP>(x, prow, fastx, gd, gdim, xv);
-      for (; it < it1; it += split_S) {
+      }
+      if (n_cold == 0) break;
+      {
         // basis values of this group from the x values that have arrived
         // (ph2[h][j]: slot j of points 2h, 2h + 1)
         float2 ph2[2][4];
@@ -321,8 +333,8 @@ __device__ __forceinline__ void blocked_tile(const BArgs& a, const double* __res
         }
         // next group: descriptors and x loads in flight during this contraction
         const int4 gdc = gd;
-        if (it + split_S < it1) {
-          g = tl<TS>(a.items + it + split_S) & (kColdBit - 1);
+        if (n_cold > 1) {
+          g = tl<TS>(a.items + cold + split_S) & (kColdBit - 1);
           gd = tl<TS>(a.grp + 3 * g);
           gdim = tl<TS>(a.grp + 3 * g + 1);
           load_x<NP>(x, prow, fastx, gd, gdim, xv);
