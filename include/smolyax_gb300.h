@@ -738,7 +738,7 @@ typedef struct smx_tensor_bwd {
   const uint16_t* Rh;        /* [n_rows][ldo]                                           */
   const uint16_t* Rl;
   const float* row_scale;    /* [ldo / 64][n_rows]                                      */
-  const float* out_scale;    /* [d_out]                                                 */
+  const float* out_scale;    /* [d_out], 0 for an output without coefficients           */
   smx_walk walk;
 } smx_tensor_bwd;
 /* From FP32 coefficient rows C[n_rows][d_out]. */

@@ -61,7 +61,9 @@ __global__ void __launch_bounds__(256) cotangent_kernel(const float* __restrict_
   if (lane == 0) scale[p] = __int_as_float((e - 14) << 23);
 }
 
-// Rows of C: per output the power of two of its largest finite coefficient ...
+// Rows of C: per output the power of two of its largest finite coefficient, 0 for an
+// output without any (a constant: its cotangent contributes nothing and must not set
+// the scale of its point's cotangents) ...
 __global__ void col_scale_kernel(const float* __restrict__ C, int64_t n, int d_out, float* __restrict__ scale) {
   __shared__ float red[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -76,7 +78,7 @@ __global__ void col_scale_kernel(const float* __restrict__ C, int64_t n, int d_o
   __syncthreads();
   if (warp == 0 && o < d_out) {
     for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w][lane]);
-    scale[o] = m > 0.f ? __int_as_float(min(max(__float_as_int(m) >> 23, 1), 253) << 23) : 1.f;
+    scale[o] = m > 0.f ? __int_as_float(min(max(__float_as_int(m) >> 23, 1), 253) << 23) : 0.f;
   }
 }
 
