@@ -697,8 +697,8 @@ typedef struct smx_tensor {
 int smx_tensor_splits(int d_out, int K);
 /* FP16 operands from the FP32 coefficients B[N][K] (column k = tape entry K-1-k):
  * high and low parts, the output scales, and the padded tape: ceil(K/64)*64 - K
- * entries of padding, then per entry {128 * slot, FP32 bits of 2^f | 128 * (depth - 1)
- * | 1 where the parent's product is read back from the stack | 2 where the entry has
+ * entries of padding, then per entry {128 * slot, FP32 bits of 2^f (0 for an entry
+ * without coefficients) | 128 * (depth - 1) | 1 where the parent's product is read back from the stack | 2 where the entry has
  * children}.  smx_tensor_tape: the padded tape alone, f = 0 (bf16). */
 int smx_tensor_operands(const float* B, int N, int K, int64_t ldb, const int32_t* tape, int32_t* tape_out,
                         uint16_t* B_hi, uint16_t* B_lo, int64_t ldh, float* out_scale, void* stream);

@@ -10,6 +10,7 @@
 //   u_n  per output       max_k |C[k][n]| 2^-u_n in [1, 2)
 //   f_k  per entry        max_n |C[k][n]| 2^(-u_n - f_k) in [2^13, 2^14), so that
 //                         A[p][k] 2^f_k is the size of the entry's largest term
+//                         (factor 0 for an entry without coefficients)
 //   s    per point and group of 64 columns: max |A 2^f| / s in [2^14, 2^15)
 // B = C 2^(-u - f) and A 2^f / s are split; the contraction multiplies each
 // 64-column partial sum by s as it leaves tensor memory (where it was added
@@ -305,29 +306,32 @@ __device__ __forceinline__ float scaled(float b, float scale) {
   return b * __int_as_float((254 << 23) - __float_as_int(scale));  // b / scale, scale a power of two
 }
 
-// The padded tape: per column k (tape entry j = K - 1 - k) the exponent f (0
-// without coefficients) and the stack flags.
+// The padded tape: per column k (tape entry j = K - 1 - k) the factor 2^f (1 without
+// a B) and the stack flags.  An entry whose coefficients are all zero gets the factor
+// 0: its product must not set the scale of its point's group.
 __global__ void tape_kernel(const float* __restrict__ B, int N, int K, int64_t ldb, const float* __restrict__ scale,
                             const int32_t* __restrict__ tape, int pad, int2* __restrict__ tape_out) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   // padding in front: depth 1, factor 0 (its columns are past K)
   if (k < pad) tape_out[k] = make_int2(0, k == 0 ? kPop : 0);
   if (k >= K) return;
-  int f = 0;
+  int factor = 127 << 23;
   if (B) {
     float m = 0.f;
+    bool any = false;
     for (int n = 0; n < N; ++n) {
-      const float a = fabsf(scaled(B[n * ldb + k], scale[n]));
+      const float b = B[n * ldb + k], a = fabsf(scaled(b, scale[n]));
+      any = any || !(b == 0.f);
       if (a <= 3.0e38f) m = fmaxf(m, a);
     }
     const int e = m > 0.f ? (__float_as_int(m) >> 23) - 127 : 13;
-    f = min(max(e - 13, -100), 100);
+    factor = any ? (min(max(e - 13, -100), 100) + 127) << 23 : 0;
   }
   const int j = K - 1 - k;
   const int w = tape[j], d = w >> 16;
   const int before = j ? tape[j - 1] >> 16 : 0, after = j + 1 < K ? tape[j + 1] >> 16 : 0;
   const int flags = ((pad + j) % kGroup == 0 || before > d ? kPop : 0) | (after == d + 1 ? kPush : 0);
-  tape_out[pad + j] = make_int2((w & 0xffff) * 128, ((f + 127) << 23) | ((d - 1) * 128) | flags);
+  tape_out[pad + j] = make_int2((w & 0xffff) * 128, factor | ((d - 1) * 128) | flags);
 }
 
 __global__ void split_f16_kernel(const float* __restrict__ B, int N, int K, int64_t ldb,

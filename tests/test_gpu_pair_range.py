@@ -37,3 +37,49 @@ def test_a_constant_output_does_not_hide_small_ones(d_out, size):
     dx, _ = sp.vjp(x, g, need_coef=False)
     ref = torch.einsum("po,poi->pi", g.double(), ip.gradient(x))
     assert float((dx - ref).abs().max()) < 1e-5 * float(ref.abs().max())
+
+
+def _products(sp, x):
+    """A [P, entries] in FP64, from the index set and the recurrences alone."""
+    from smolyax_gb300.spectral import _phi_table
+
+    tr, _, maxdeg, fam, fa, fb = sp._fwd_args[:6]
+    A = np.ones((tr["parent"].size, x.shape[0]))
+    table = {j: _phi_table(int(fam[j]), fa[j] * x[:, j] + fb[j], int(maxdeg[j])) for j in np.nonzero(maxdeg)[0]}
+    for e in range(1, A.shape[0]):
+        A[e] = A[tr["parent"][e]] * table[int(tr["dim"][e])][int(tr["deg"][e])]
+    return A.T
+
+
+def _set_coefficients(sp, C):
+    """The plan's tensor-core operands from other coefficients (row 0 stays)."""
+    tc = sp.tc
+    tc["Bd"][:, : tc["K"]] = torch.as_tensor(C[tc["ent_h"][::-1]].T.astype(np.float32), device="cuda")
+    tc.pop("f16")
+
+
+def _term_error(sp, C, x):
+    """Per output: largest error over the points, relative to sum |terms|."""
+    y = torch.empty(x.shape[0], C.shape[1], dtype=torch.float32, device="cuda")
+    sp.evaluate(torch.as_tensor(x, device="cuda"), y)
+    A, C32 = _products(sp, x), C.astype(np.float32).astype(float)
+    return np.max(np.abs(y.cpu().numpy() - A @ C32) / (np.abs(A) @ np.abs(C32)), axis=0)
+
+
+@pytest.mark.parametrize("far", [1.0, 30.0, 3000.0])
+@pytest.mark.parametrize("j", [0, 2, 8])
+def test_entries_without_coefficients_do_not_hide_the_others(j, far):
+    """Values where the target ignores a coordinate that lies far outside its box:
+    the entries of that coordinate have no coefficients, whatever their products."""
+    d = 20
+    ip = _plan(d, 900, 24, fns.rational_vec(d, 24, seed=3))
+    sp = ip.spectral_plan()
+    tr = sp._fwd_args[0]
+    uses = np.zeros(tr["parent"].size, dtype=bool)
+    for e in range(1, uses.size):
+        uses[e] = uses[tr["parent"][e]] or tr["dim"][e] == j
+    C = np.where(uses[:, None], 0.0, sp.C64.cpu().numpy())
+    _set_coefficients(sp, C)
+    x = np.random.default_rng(0).uniform(-1, 1, (200, d))
+    x[:, j] = far
+    assert _term_error(sp, C, x).max() <= 1e-6
