@@ -85,8 +85,8 @@ struct GemmArgs {
 
 // KIND kTf32: kind::tf32 on FP32 operands (32 per 128-byte slice); kBf16, kF16:
 // kind::f16 on 16-bit operands (64 per slice).  Same slices, stages and MMAs;
-// kF16 multiplies each drained accumulator by its row's scale of the slice and
-// the result by the column's.
+// kF16 (pairs hi + 2^-11 lo, tc_util.cuh) multiplies each drained accumulator by its
+// row's scale of the slice and the result by the column's.
 template <int KIND, int BN>
 __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
@@ -192,15 +192,20 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
           const uint32_t a_lo = a_hi + L::kA;
           const uint32_t b_hi = a_hi + 2 * L::kA;
           const uint32_t b_lo = b_hi + L::kB;
+          if constexpr (KIND == kF16) {
+            static_assert(kRowBytes == 128 && kChunkF16 == 1, "an accumulator holds one slice");
+            mma_pair_slice(acc, a_hi, a_lo, b_hi, b_lo, idesc);
+          } else {
 #pragma unroll
-          for (int k8 = 0; k8 < kRowBytes / 32; ++k8) {  // 32 bytes (8 tf32 or 16 bf16) of K per MMA
-            const uint32_t off = k8 * 32;
-            const uint64_t dah = make_desc_k(a_hi + off), dal = make_desc_k(a_lo + off);
-            const uint64_t dbh = make_desc_k(b_hi + off), dbl = make_desc_k(b_lo + off);
-            mma_op<BF16>(acc, dah, dbh, idesc, first ? 0u : 1u);
-            first = false;
-            mma_op<BF16>(acc, dah, dbl, idesc, 1u);
-            mma_op<BF16>(acc, dal, dbh, idesc, 1u);
+            for (int k8 = 0; k8 < kRowBytes / 32; ++k8) {  // 32 bytes (8 tf32 or 16 bf16) of K per MMA
+              const uint32_t off = k8 * 32;
+              const uint64_t dah = make_desc_k(a_hi + off), dal = make_desc_k(a_lo + off);
+              const uint64_t dbh = make_desc_k(b_hi + off), dbl = make_desc_k(b_lo + off);
+              mma_op<BF16>(acc, dah, dbh, idesc, first ? 0u : 1u);
+              first = false;
+              mma_op<BF16>(acc, dah, dbl, idesc, 1u);
+              mma_op<BF16>(acc, dal, dbh, idesc, 1u);
+            }
           }
           mma_commit(&empty[s]);  // frees the stage once these MMAs have read it
         }

@@ -122,6 +122,41 @@ __device__ __forceinline__ void mma_op(uint32_t tmem_d, uint64_t adesc, uint64_t
   }
 }
 
+// Pairs of FP16 values x = hi + 2^-kPairShift lo: the low part is stored scaled up, so
+// that it keeps its 11 bits down to hi's smallest normal number.  With the group's
+// largest value in [2^14, 2^15) an element has 22 significant bits down to 2^-29 of
+// the largest and errs by 2^-51 of it below (16 bits less range without the shift).
+// The products of a high and a low part are added first; the first product of high
+// parts then scales the accumulator down by 2^-kPairShift (mma_pair_head).
+constexpr int kPairShift = 11;
+constexpr float kPairScale = float(1 << kPairShift);
+
+// kind::f16 MMA that multiplies the accumulator by 2^-kPairShift before it adds.
+__device__ __forceinline__ void mma_pair_head(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.eq.b32 p, 0, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "n"(kPairShift));
+}
+
+// One 64-column slice of (Ah + Al)(Bh + Bl) into a fresh accumulator, rows of 128 bytes.
+__device__ __forceinline__ void mma_pair_slice(uint32_t tmem_d, uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl,
+                                               uint32_t idesc) {
+#pragma unroll
+  for (int k = 0; k < 128; k += 32) {  // 16 values per MMA
+    mma_op<true>(tmem_d, make_desc_sw(ah + k, 128), make_desc_sw(bl + k, 128), idesc, k ? 1u : 0u);
+    mma_op<true>(tmem_d, make_desc_sw(al + k, 128), make_desc_sw(bh + k, 128), idesc, 1u);
+  }
+#pragma unroll
+  for (int k = 0; k < 128; k += 32) {
+    const uint64_t da = make_desc_sw(ah + k, 128), db = make_desc_sw(bh + k, 128);
+    if (k == 0)
+      mma_pair_head(tmem_d, da, db, idesc);
+    else
+      mma_op<true>(tmem_d, da, db, idesc, 1u);
+  }
+}
+
 // Arrives on `bar` once every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))

@@ -2,11 +2,11 @@
 // A[p][k] = prod_j phi(z_j), the basis products of the entries of Lambda
 // (interpolation.py:264-304 re-expressed over the index set).
 //
-// Operands are split into two 16-bit parts, x ~= scale (hi + lo): FP16 with
-// scales (the default) or BF16 (the caller's faster, less precise choice).  FP16
-// keeps 11 + 11 significant bits, as the TF32 pair of the 3xTF32 product does,
-// at twice the tensor rate and half the bytes; its narrow exponent range is
-// covered by exact powers of two:
+// Operands are split into two 16-bit parts: FP16 with scales (the default), x ~=
+// scale (hi + 2^-11 lo), or BF16 (the caller's faster, less precise choice), x ~=
+// hi + lo.  FP16 keeps 11 + 11 significant bits, as the TF32 pair of the 3xTF32
+// product does, at twice the tensor rate and half the bytes; its narrow exponent
+// range is covered by exact powers of two:
 //   u_n  per output       max_k |C[k][n]| 2^-u_n in [1, 2)
 //   f_k  per entry        max_n |C[k][n]| 2^(-u_n - f_k) in [2^13, 2^14), so that
 //                         A[p][k] 2^f_k is the size of the entry's largest term
@@ -14,8 +14,12 @@
 //   s    per point and group of 64 columns: max |A 2^f| / s in [2^14, 2^15)
 // B = C 2^(-u - f) and A 2^f / s are split; the contraction multiplies each
 // 64-column partial sum by s as it leaves tensor memory (where it was added
-// before) and the result by 2^u_n.  An element below 2^-16 of its group's
-// largest term loses bits only below 2^-39 of that term.
+// before) and the result by 2^u_n.  With the low parts scaled (tc_util.cuh) an
+// element keeps 22 bits down to 2^-29 of the largest of its group and errs by 2^-51 of
+// that one below.  So an output's value has the accuracy of the TF32 pairs as long as
+// the largest term of any output at the point (each output's coefficients counted in
+// units of its largest) is below 2^29 times the output's own largest term; beyond, its
+// relative error grows with that ratio, to 1e-6 at 2^31.
 //
 // Kernels: basis values of all (dimension, degree) slots [slot][point]; the panel
 // A in groups of 64 columns; the contraction (gemm_tc.cu).
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(32 * W, 1)
           const float2 ab = __fmul2_rn(make_float2(v[63 - 8 * i - 2 * k], v[62 - 8 * i - 2 * k]), make_float2(inv, inv));
           if constexpr (F16) {
             const __half2 hh = __float22half2_rn(ab);
-            const __half2 ll = __float22half2_rn(__ffma2_rn(__half22float2(hh), make_float2(-1.f, -1.f), ab));
+            const __half2 ll = pair_low(ab, hh);
             h[k] = *reinterpret_cast<const uint32_t*>(&hh);
             l[k] = *reinterpret_cast<const uint32_t*>(&ll);
           } else {
@@ -345,7 +349,7 @@ __global__ void split_f16_kernel(const float* __restrict__ B, int N, int K, int6
     const float v = scaled(B[n * ldb + k], scale[n]) * __int_as_float((254 << 23) - factor);
     const __half h = __float2half_rn(v);
     Bh[n * ldh + k] = h;
-    Bl[n * ldh + k] = __float2half_rn(v - __half2float(h));
+    Bl[n * ldh + k] = pair_low(v, h);
   }
 }
 

@@ -3,10 +3,12 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "smolyax_gb300.h"
+#include "tc_util.cuh"
 
 namespace smx {
 namespace tc {
@@ -15,6 +17,15 @@ namespace tc {
 // bits), the byte offset of its parent on a stack of 128 bytes per depth, and flags.
 constexpr int kPop = 1, kPush = 2, kStackMask = 0xf80, kFactorMask = 0x7f800000;
 constexpr int kGroup = 64;  // tape entries (panel columns) per group
+
+// Low parts of the pairs (tc_util.cuh): (v - h) 2^kPairShift.
+__device__ __forceinline__ __half pair_low(float v, __half h) {
+  return __float2half_rn((v - __half2float(h)) * kPairScale);
+}
+__device__ __forceinline__ __half2 pair_low(float2 v, __half2 h) {
+  return __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-kPairScale, -kPairScale),
+                                      __fmul2_rn(v, make_float2(kPairScale, kPairScale))));
+}
 
 // 16 bytes global -> shared, asynchronously (cp.async.wait_all).
 __device__ __forceinline__ void copy16(void* dst, const void* src) {

@@ -5,6 +5,11 @@
 // dL/dC[e][o] = sum_p A[p][e] g[p][o] further down.  The reference has the dense
 // Jacobian instead (interpolation.py:306-345).
 //
+// Range of G's FP16 pairs (tc_util.cuh): one power of two per point for g (in units of
+// the outputs' largest coefficients) and one per entry and 64 outputs for C, so that
+// G[e][p] has the accuracy of the TF32 pairs while max |C[e]| max |g[p]| is below 2^29
+// times the largest of its terms (outputs in disjoint inputs, 2^29 apart in C g).
+//
 // G is made transposed in blocks of 32 points, [p / 32][entry][32]: a block of 32
 // warps (lane = point) streams its adjoints once, in order, through shared
 // memory.  Each entry is two terms, row value * G added to a destination row
@@ -56,7 +61,7 @@ __global__ void __launch_bounds__(256) cotangent_kernel(const float* __restrict_
     const float v = o < d_out ? gp[o] * out_scale[o] * inv : 0.f;
     const __half h = __float2half_rn(v);
     hi[p * ldo + o] = h;
-    lo[p * ldo + o] = __float2half_rn(v - __half2float(h));
+    lo[p * ldo + o] = pair_low(v, h);
   }
   if (lane == 0) scale[p] = __int_as_float((e - 14) << 23);
 }
@@ -105,7 +110,7 @@ __global__ void split_rows_kernel(const float* __restrict__ C, int64_t n, int d_
     const float v = value(o) * inv;
     const __half h = __float2half_rn(v);
     hi[e * ldo + o] = h;
-    lo[e * ldo + o] = __float2half_rn(v - __half2float(h));
+    lo[e * ldo + o] = pair_low(v, h);
   }
 }
 
@@ -235,14 +240,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint32_t ah = smem_u32(base + i * kAdjTile), al = ah + kAdjTile / 2;
           const uint32_t bh = smem_u32(B + (((n - 1) % nb) * q + s) * kAdjTile), bl = bh + kAdjTile / 2;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {  // 16 values of 64 per MMA
-            const uint64_t dah = make_desc_sw(ah + k * 32, 128), dal = make_desc_sw(al + k * 32, 128);
-            const uint64_t dbh = make_desc_sw(bh + k * 32, 128), dbl = make_desc_sw(bl + k * 32, 128);
-            mma_op<true>(tmem + c * 128, dah, dbh, idesc, k ? 1u : 0u);
-            mma_op<true>(tmem + c * 128, dah, dbl, idesc, 1u);
-            mma_op<true>(tmem + c * 128, dal, dbh, idesc, 1u);
-          }
+          mma_pair_slice(tmem + c * 128, ah, al, bh, bl, idesc);
           mma_commit(&a_empty[i]);
           mma_commit(&acc_full[c]);
         }
@@ -575,7 +573,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
           if (lane == ((k + u) & 31)) sc = __int_as_float((e - 14) << 23);
           const float2 v = __fmul2_rn(b[u], make_float2(inv, inv));
           const __half2 h = __float22half2_rn(v);
-          const __half2 l = __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-1.f, -1.f), v));
+          const __half2 l = pair_low(v, h);
           AH[(e0 + k + u) * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
           AL[(e0 + k + u) * 32 + lane] = *reinterpret_cast<const uint32_t*>(&l);
         }
@@ -658,7 +656,7 @@ __global__ void __launch_bounds__(256) output_slices_kernel(const float* __restr
     for (int o = warp; o < 64 && o0 + o < d_out; o += 8) {
       const float2 v = make_float2(tile[2 * lane][o], tile[2 * lane + 1][o]);
       const __half2 h = __float22half2_rn(v);
-      const __half2 l = __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-1.f, -1.f), v));
+      const __half2 l = pair_low(v, h);
       const int64_t at = (blockIdx.x * int64_t(d_out) + o0 + o) * 32 + lane;
       hi[at] = *reinterpret_cast<const uint32_t*>(&h);
       lo[at] = *reinterpret_cast<const uint32_t*>(&l);

@@ -83,3 +83,45 @@ def test_entries_without_coefficients_do_not_hide_the_others(j, far):
     x = np.random.default_rng(0).uniform(-1, 1, (200, d))
     x[:, j] = far
     assert _term_error(sp, C, x).max() <= 1e-6
+
+
+@pytest.mark.parametrize("j,far", [(0, 1.0), (0, 30.0), (8, 1e5)])
+def test_small_terms_beside_large_ones(j, far):
+    """Values of outputs without a coordinate beside outputs of that coordinate alone,
+    whose terms are up to 1e8 times larger."""
+    d = 20
+    ip = _plan(d, 900, 24, fns.rational_vec(d, 24, seed=3))
+    sp = ip.spectral_plan()
+    tr = sp._fwd_args[0]
+    uses = np.zeros(tr["parent"].size, dtype=bool)
+    for e in range(1, uses.size):
+        uses[e] = uses[tr["parent"][e]] or tr["dim"][e] == j
+    C = sp.C64.cpu().numpy().copy()
+    C[1:, 0::2][uses[1:]] = 0.0
+    C[1:, 1::2][~uses[1:]] = 0.0
+    _set_coefficients(sp, C)
+    x = np.random.default_rng(0).uniform(-1, 1, (200, d))
+    x[:, j] = far
+    assert _term_error(sp, C, x).max() <= 1e-6
+
+
+@pytest.mark.parametrize("size", [1.0, 1e-4, 1e-6, 1e-8])
+@pytest.mark.parametrize("d_out", [2, 130])
+def test_derivatives_of_small_outputs_in_their_own_inputs(d_out, size):
+    """dL/dx in the inputs that only the small outputs use, beside large outputs of
+    other inputs, relative to their own size."""
+    d, half = 20, d_out // 2
+    h = fns.rational_vec(10, d_out, seed=3)
+
+    def f(x):
+        return np.concatenate([h(x[0::2])[:half], size * h(x[1::2])[half:]])
+
+    ip = _plan(d, 400, d_out, f)
+    sp = ip.spectral_plan()
+    assert sp._backward_ops()["walk"] is not None
+    x = _x(100, d)
+    g = torch.as_tensor(np.random.default_rng(1).normal(size=(100, d_out)).astype(np.float32), device="cuda")
+    dx, _ = sp.vjp(x, g, need_coef=False)
+    ref = torch.einsum("po,poi->pi", g.double(), ip.gradient(x))
+    for i in (0, 1):
+        assert float((dx - ref)[:, i::2].abs().max()) < 1e-5 * float(ref[:, i::2].abs().max())
