@@ -494,7 +494,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // ---- dL/dC = A^T g ---------------------------------------------------------------------
 // A^T in slices of 64 points, [p / 64][entry][64] as FP16 pairs with one power of
-// two per entry and slice (times the slice's scale of g).  A block of W warps holds
+// two per entry and slice.  Each point's products are multiplied by the power of two of
+// its largest cotangent (in units of each output's largest), and the cotangents divided
+// by it: the pairs' range (2^29 below the slice's largest at full precision, tc_util.cuh)
+// then counts the points' terms A g and not A and g by themselves, which may run against
+// each other over the points, and points without a cotangent weigh nothing.  A block of
+// W warps holds
 // the basis rows of 64 points (two per lane) in shared memory; each warp walks its
 // run of tape groups as tensor_panel_kernel does (tensor_eval.cu), but an entry's 64
 // values are one register pair per lane, so they are scaled and written at once:
@@ -502,10 +507,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Leja d_in = 200, |Lambda| = 5000, 1e5 points: 0.33 ms (6.1 TB/s of writes, issue
 // slots 71 % busy) and 0.32 ms for the product with 64 outputs; one thread per point
 // writing TF32 pairs through 400 KB strides took 1.34 ms and its product 0.62 ms.
+constexpr float kPointScale = 1.f / 16384.f;
 template <int W, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB)
     coef_panel_kernel(smx_tensor t, int groups_per_block, const float* __restrict__ grow, int64_t gstride,
-                      int64_t n_slices, const float* __restrict__ gscale, uint32_t* __restrict__ AH,
+                      int64_t n_slices, const float2* __restrict__ pscale, uint32_t* __restrict__ AH,
                       uint32_t* __restrict__ AL, float* __restrict__ S) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -523,8 +529,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (t0 == t1) continue;
-    const float gsc = __ldg(gscale + sl);
-    f2(stk) = make_float2(1.f, 1.f);
+    f2(stk) = __ldg(pscale + sl * 32 + lane);  // every product starts with its point's scale
     for (int i = 0; i < 8; ++i) {
       const int s = __ldg(t.path + t0 * 8 + i);
       if (s < 0) break;
@@ -577,7 +582,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
           AH[(e0 + k + u) * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
           AL[(e0 + k + u) * 32 + lane] = *reinterpret_cast<const uint32_t*>(&l);
         }
-        if ((k & 31) == 28) S[e0 + (k & 32) + lane] = sc * gsc;
+        if ((k & 31) == 28) S[e0 + (k & 32) + lane] = sc * kPointScale;
       }
     }
   }
@@ -621,13 +626,14 @@ __device__ __forceinline__ float output_scale(unsigned most) {
 }
 
 // ... and g / scale transposed in slices of 64 points, [p / 64][output][64], as FP16
-// pairs with one power of two per slice; points past P are zero.
+// pairs, each point's largest brought to [2^14, 2^15); pscale: what that divided by, times
+// kPointScale^-1 (0 for points without a cotangent and past P).
 __global__ void __launch_bounds__(256) output_slices_kernel(const float* __restrict__ g, int64_t ldg, int64_t P,
                                                             int d_out, const unsigned* __restrict__ most,
                                                             uint32_t* __restrict__ hi, uint32_t* __restrict__ lo,
-                                                            float* __restrict__ gscale, float* __restrict__ scale) {
+                                                            float* __restrict__ pscale, float* __restrict__ scale) {
   __shared__ float tile[64][65];
-  __shared__ float red[8];
+  __shared__ float red[64][2], inv[64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, oc = threadIdx.x & 63, r0 = threadIdx.x >> 6;
   const int64_t p0 = blockIdx.x * int64_t(64);
   auto value = [&](int64_t p, int o) {
@@ -637,21 +643,25 @@ __global__ void __launch_bounds__(256) output_slices_kernel(const float* __restr
   };
   if (blockIdx.x == 0)
     for (int o = threadIdx.x; o < d_out; o += 256) scale[o] = output_scale(most[o]);
-  float m = 0.f;
-  for (int o0 = 0; o0 < d_out; o0 += 64)
-    for (int r = r0; r < 64; r += 4) {
+  for (int r = r0; r < 64; r += 4) {  // two warps per point
+    float m = 0.f;
+    for (int o0 = 0; o0 < d_out; o0 += 64) {
       const float a = fabsf(value(p0 + r, o0 + oc));
       if (a <= 3.0e38f) m = fmaxf(m, a);
     }
-  m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-  if (lane == 0) red[warp] = m;
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    if (lane == 0) red[r][warp & 1] = m;
+  }
   __syncthreads();
-  for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w]);
-  const int e = min(max(__float_as_int(m) >> 23, 27), 254);
-  const float inv = __int_as_float((268 - e) << 23);
-  if (threadIdx.x == 0) gscale[blockIdx.x] = __int_as_float((e - 14) << 23);
+  if (threadIdx.x < 64) {
+    const float m = fmaxf(red[threadIdx.x][0], red[threadIdx.x][1]);
+    const int e = min(max(__float_as_int(m) >> 23, 27), 254);
+    inv[threadIdx.x] = __int_as_float((268 - e) << 23);
+    pscale[p0 + threadIdx.x] = m > 0.f ? __int_as_float(e << 23) : 0.f;
+  }
+  __syncthreads();
   for (int o0 = 0; o0 < d_out; o0 += 64) {
-    for (int r = r0; r < 64; r += 4) tile[r][oc] = value(p0 + r, o0 + oc) * inv;
+    for (int r = r0; r < 64; r += 4) tile[r][oc] = value(p0 + r, o0 + oc) * inv[r];
     __syncthreads();
     for (int o = warp; o < 64 && o0 + o < d_out; o += 8) {
       const float2 v = make_float2(tile[2 * lane][o], tile[2 * lane + 1][o]);
@@ -818,7 +828,7 @@ size_t coef_smem(int warps, int slots) { return size_t(warps) * (1024 + 9 * 256)
 
 struct CoefLayout {  // workspace of one chunk of m points
   int64_t gstride, slices, E;
-  size_t panel, scales, rows, cot, gscale, out, dC, partial, total;
+  size_t panel, scales, rows, cot, pscale, out, dC, partial, total;
 };
 CoefLayout coef_layout(const smx_tensor* t, int64_t m) {
   CoefLayout L;
@@ -829,11 +839,11 @@ CoefLayout coef_layout(const smx_tensor* t, int64_t m) {
   L.scales = up256(size_t(L.slices) * L.E * 4);
   L.rows = up256(size_t(t->n_slots) * L.gstride * 4);
   L.cot = up256(size_t(L.slices) * t->d_out * 128);
-  L.gscale = up256(size_t(L.slices) * 4);
+  L.pscale = up256(size_t(L.slices) * 256);
   L.out = up256(size_t(t->d_out) * 4);
   L.dC = up256(size_t(L.E) * t->d_out * 4);
   L.partial = t->splits > 1 ? up256(size_t(t->splits) * L.E * t->d_out * 4) : 0;
-  L.total = 2 * L.panel + L.scales + L.rows + 2 * L.cot + L.gscale + 2 * L.out + L.dC + L.partial;
+  L.total = 2 * L.panel + L.scales + L.rows + 2 * L.cot + L.pscale + 2 * L.out + L.dC + L.partial;
   return L;
 }
 
@@ -844,7 +854,7 @@ size_t coef_sum_bytes(const smx_tensor* t, int64_t P) {
 }
 
 template <int W, int MINB>
-void launch_coef_panel(const smx_tensor& t, const CoefLayout& L, const float* grow, const float* gscale, uint32_t* AH,
+void launch_coef_panel(const smx_tensor& t, const CoefLayout& L, const float* grow, const float* pscale, uint32_t* AH,
                        uint32_t* AL, float* S, int sms, cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
@@ -862,8 +872,8 @@ void launch_coef_panel(const smx_tensor& t, const CoefLayout& L, const float* gr
     if (best < 0 || cost < best) best = cost, per = p;
   }
   const dim3 grid(unsigned((t.n_groups + per - 1) / per), unsigned(std::min<int64_t>(L.slices, 65535)));
-  coef_panel_kernel<W, MINB><<<grid, 32 * W, coef_smem(W, t.n_slots), st>>>(t, per, grow, L.gstride, L.slices, gscale,
-                                                                            AH, AL, S);
+  coef_panel_kernel<W, MINB><<<grid, 32 * W, coef_smem(W, t.n_slots), st>>>(t, per, grow, L.gstride, L.slices,
+                                                                            reinterpret_cast<const float2*>(pscale), AH, AL, S);
 }
 
 }  // namespace
@@ -934,7 +944,7 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
     float* grow = reinterpret_cast<float*>(take(L.rows));
     uint32_t* gh = reinterpret_cast<uint32_t*>(take(L.cot));
     uint32_t* gl = reinterpret_cast<uint32_t*>(take(L.cot));
-    float* gscale = reinterpret_cast<float*>(take(L.gscale));
+    float* pscale = reinterpret_cast<float*>(take(L.pscale));
     unsigned* most = reinterpret_cast<unsigned*>(take(L.out));
     float* scale = reinterpret_cast<float*>(take(L.out));
     if (cudaMemsetAsync(most, 0, size_t(t->d_out) * 4, st) != cudaSuccess)
@@ -942,7 +952,7 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
     const dim3 ogrid(unsigned((m + kSumRows - 1) / kSumRows), unsigned(std::min((t->d_out + 31) / 32, 65535)));
     output_most_kernel<<<ogrid, 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, sums + sum_blocks * t->d_out);
     sum_blocks += ogrid.x;
-    output_slices_kernel<<<unsigned(L.slices), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, gh, gl, gscale,
+    output_slices_kernel<<<unsigned(L.slices), 256, 0, st>>>(g + p0 * ldg, ldg, m, t->d_out, most, gh, gl, pscale,
                                                              scale);
     if (rows_given && P <= t->chunk)
       grow = const_cast<float*>(rows_given);
@@ -950,9 +960,9 @@ extern "C" int smx_tensor_vjp_coef(const smx_tensor* t, const double* x, int64_t
       tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st);
     // two blocks of 8 warps per SM while their rows fit (up to ~330 slots), else one of 16
     if (coef_smem(8, t->n_slots) <= (kSmemMax - 2048) / 2)
-      launch_coef_panel<8, 2>(*t, L, grow, gscale, AH, AL, S, sms, st);
+      launch_coef_panel<8, 2>(*t, L, grow, pscale, AH, AL, S, sms, st);
     else
-      launch_coef_panel<16, 1>(*t, L, grow, gscale, AH, AL, S, sms, st);
+      launch_coef_panel<16, 1>(*t, L, grow, pscale, AH, AL, S, sms, st);
     SMX_LAUNCH_CHECK("smx_tensor_vjp_coef");
     SplitGemm s{};
     s.bits = kF16;

@@ -125,3 +125,38 @@ def test_derivatives_of_small_outputs_in_their_own_inputs(d_out, size):
     ref = torch.einsum("po,poi->pi", g.double(), ip.gradient(x))
     for i in (0, 1):
         assert float((dx - ref)[:, i::2].abs().max()) < 1e-5 * float(ref[:, i::2].abs().max())
+
+
+def _coef_error(sp, x, g):
+    """Largest error of dL/dC relative to sum |A g| of the entry and output."""
+    _, dC = sp.vjp(torch.as_tensor(x, device="cuda"), torch.as_tensor(g, device="cuda"), need_x=False)
+    A, g = _products(sp, x).T, g.astype(float)
+    return np.max(np.abs(dC.cpu().numpy() - A @ g) / np.maximum(np.abs(A) @ np.abs(g), 1e-300))
+
+
+@pytest.mark.parametrize("spread", [1.0, 2.0**20, 2.0**30, 2.0**45])
+@pytest.mark.parametrize("d_out", [3, 70])
+def test_products_and_cotangents_of_opposite_spread(d_out, spread):
+    """dL/dC over points whose products grow as their cotangents fall."""
+    ip = _plan(20, 900, d_out, fns.rational_vec(20, d_out, seed=3))
+    sp = ip.spectral_plan()
+    assert sp._backward_ops()["coef"] is not None
+    rng = np.random.default_rng(0)
+    P, deg = 200, int(np.max(ip._maxdeg))
+    x = rng.uniform(-1, 1, (P, 20))
+    w = spread ** rng.uniform(0, 1, P)  # the largest products of the points, about
+    x[:, 0] = np.maximum(w ** (1 / deg), np.abs(x[:, 0]))
+    g = (rng.normal(size=(P, d_out)) / w[:, None]).astype(np.float32)
+    assert _coef_error(sp, x, g) <= 1e-5
+
+
+def test_points_without_a_cotangent_weigh_nothing():
+    """dL/dC where points far outside the box are masked out by a zero cotangent."""
+    ip = _plan(20, 900, 5, fns.rational_vec(20, 5, seed=3))
+    sp = ip.spectral_plan()
+    rng = np.random.default_rng(0)
+    x = rng.uniform(-1, 1, (200, 20))
+    g = rng.normal(size=(200, 5)).astype(np.float32)
+    x[::7] *= 1e4
+    g[::7] = 0.0
+    assert _coef_error(sp, x, g) <= 1e-5
