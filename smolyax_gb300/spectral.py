@@ -57,9 +57,13 @@ def stream_tables(struct, tree, coef, d_out, maxdeg, fam, fa, fb, T, fp64):
 
 def finish_build():
     """Operands just built on the current stream are read from any stream next:
-    wait for them, once per plan (a capture cannot wait; it is their only reader then)."""
-    if not torch.cuda.is_current_stream_capturing():
-        torch.cuda.current_stream().synchronize()
+    wait for them, once per plan.  False under capture: the kernels that build them
+    are only recorded, so that the operands belong to the graph and nobody may keep
+    them."""
+    if torch.cuda.is_current_stream_capturing():
+        return False
+    torch.cuda.current_stream().synchronize()
+    return True
 
 
 def _phi_table(fam, z, n):
@@ -288,7 +292,8 @@ class SpectralPlan:
 
     def _tc_struct(self, bf16=False):
         """``smx_tensor`` of the plan: FP16 operands with scales (built with the
-        plan), or the BF16 operands of ``mode="bf16x3"`` (built on first use)."""
+        plan), or the BF16 operands of ``mode="bf16x3"`` (built on first use; a call
+        under capture before that records their construction into its graph)."""
         tc = self.tc
         key = "bf16" if bf16 else "f16"
         with self._lock:
@@ -317,8 +322,9 @@ class SpectralPlan:
         s.bf16, s.splits, s.chunk, s.ldb = int(bf16), self.tc_splits(), self._tc_step(1 << 40), ldb
         for name, t in k.items():
             setattr(s, name, t.data_ptr())
-        finish_build()
-        tc[key] = (s, k)
+        s.keep = k
+        if finish_build():
+            tc[key] = (s, k)
         return s
 
     def _build_blocked(self, tr, c, maxdeg, d, fam, fa, fb, T):
@@ -408,8 +414,8 @@ class SpectralPlan:
             ops["vjp_seg"] = (b, int(b.numel()) - 1)
         else:
             ops["vjp_seg"] = (None, 1)
-        finish_build()
-        self._bwd = ops
+        if finish_build():
+            self._bwd = ops
         return ops
 
     def _build_walk(self, ops, C32):
@@ -734,7 +740,8 @@ class SpectralPlan:
         points, each contracted with the coefficient matrix (``smx_tensor_eval``)."""
         import ctypes
 
-        ref = ctypes.byref(self._tc_struct(bf16))
+        struct = self._tc_struct(bf16)  # holds its operands
+        ref = ctypes.byref(struct)
         P = int(x.shape[0])
         nws = capi.size("smx_tensor_workspace", ref, P)
         ws = torch.empty(max(nws, 16), dtype=torch.uint8, device=x.device)
