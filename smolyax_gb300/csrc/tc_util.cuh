@@ -65,6 +65,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// Copies go round `stages` buffers, copy c into buffer c % stages in the phase of
+// parity (c / stages) & 1.  Calls wait(buffer, parity) for every copy that may be in
+// flight after `issued` of them: the last into each buffer (a buffer is filled again
+// only once its copy has been read).
+template <typename Wait>
+__host__ __device__ __forceinline__ void for_pending_copies(int issued, int stages, Wait wait) {
+  for (int c = issued > stages ? issued - stages : 0; c < issued; ++c) wait(c % stages, (c / stages) & 1);
+}
+
 // 2-D tiled TMA load into shared memory, completion counted on `bar`.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar) {
   asm volatile(

@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* full = reinterpret_cast<uint64_t*>(stage + kStages * stage_bytes);
   uint64_t* empty = full + kStages;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + kStages);
+  int issued = 0;  // chunks, by thread 0
   const uint8_t* G = reinterpret_cast<const uint8_t*>(GT) + blockIdx.x * (int64_t(w.n_chunks) * E * 128);
   auto load_chunk = [&](int c) {
     const int s = c % kStages, t0 = __ldg(w.off + c * 33), n = __ldg(w.off + c * 33 + 32) - t0;
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int c = 0; c < min(kStages, w.n_chunks); ++c) load_chunk(c);
+    for (; issued < min(kStages, w.n_chunks); ++issued) load_chunk(issued);
   }
   for (int s = warp * 4 + (lane >> 3); s < ns; s += kWarps * 4)
     copy16(row - lane + s * 32 + (lane & 7) * 4, grow + s * gstride + p0 + (lane & 7) * 4);
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   __syncthreads();
   // terms of this warp, chunk by chunk; a destination row is only ever touched by
-  // its warp, so the warps need not keep step beyond the two stages
+  // its warp, so the warps need not keep step beyond the stages
   uint8_t* rb = smem + lane * 4;
   int t0 = __ldg(w.off + warp), t1 = __ldg(w.off + warp + 1), first = __ldg(w.off);
   bool ok = true;
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) mbar_arrive(&empty[s]);
     if (threadIdx.x == 0 && c + kStages < w.n_chunks) {
       if (mbar_wait(&empty[s], parity, abort_flag)) {
-        load_chunk(c + kStages);
+        load_chunk(issued++);  // chunk c + kStages
       } else {
         *abort_flag = 1;  // no further chunk comes: every warp's next wait ends
       }
@@ -439,10 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (*abort_flag) {  // leave no copy behind: wait (bounded) for what was issued
     if (threadIdx.x == 0) {
       atomicExch(err, 3);
-      for (int s = 0; s < kStages; ++s)
-        if (s < w.n_chunks)
-          for (uint32_t ph = 0; ph < 2 && !mbar_wait(&full[s], ph, nullptr); ++ph) {
-          }
+      for_pending_copies(issued, kStages, [&](int s, uint32_t parity) { mbar_wait(&full[s], parity, nullptr); });
     }
     return;
   }
