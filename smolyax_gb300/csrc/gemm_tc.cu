@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;  // [2] MMA -> drain
   uint64_t* acc_empty = acc_full + 2;    // [2] drain -> MMA
-  uint64_t* flush = acc_empty + 2;       // MMA thread, on failure: its own MMAs complete
+  uint64_t* flush = acc_empty + 2;       // after an abort: all MMAs complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(flush + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* armed_slot = abort_flag + 1;
@@ -213,12 +213,8 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
       }
       if (!ok) {
         // A wait ran out (or the producer gave up): the abandoned accumulator
-        // is never signalled, so no drain warp reads it; this thread waits
-        // (bounded) until its own MMAs have completed, then raises the abort
-        // flag, on which the other warps stop waiting, skip the epilogue and
-        // the block frees its tensor memory.
-        mma_commit(flush);
-        mbar_wait(flush, 0, nullptr);
+        // is never signalled, so no drain warp reads it; on the abort flag the
+        // other warps stop waiting and skip the epilogue.
         atomicExch(g.err, 2);
         *abort_flag = 1;
       }
@@ -244,7 +240,13 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
       }
       ok = __all_sync(0xffffffffu,
                       ok && mbar_wait(&acc_full[b], (c >> 1) & 1, abort_flag, g.wait_ns) && !*abort_flag);
-      if (!ok) break;
+      if (!ok) {
+        if (lane == 0) {
+          atomicCAS(g.err, 0, 3);
+          *abort_flag = 1;
+        }
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
       for (int q = 0; q < kCols; q += 16) {
@@ -313,14 +315,19 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
       }
     }
   }
-  // after an abort, wait (bounded) for the last copy armed on every stage
-  if (warp == L::kWarpTMA && lane == 0 && *abort_flag) {
-    const int armed = *armed_slot;
-    for (int kt = max(0, armed - kStages); kt < armed; ++kt)
-      mbar_wait(&full[kt % kStages], (kt / kStages) & 1, nullptr);
-  }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  if (*abort_flag) {
+    // all roles have stopped, and the block gives nothing up before its copies and
+    // MMAs have ended (bounded)
+    if (warp == L::kWarpTMA && lane == 0)
+      for_pending_copies(*armed_slot, kStages, [&](int s, uint32_t ph) { mbar_wait(&full[s], ph, nullptr); });
+    if (warp == L::kWarpMMA && lane == 0) {
+      mma_commit(flush);
+      mbar_wait(flush, 0, nullptr);
+    }
+    __syncthreads();
+  }
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kBN));
   }

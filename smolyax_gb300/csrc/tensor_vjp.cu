@@ -124,8 +124,8 @@ __global__ void split_rows_kernel(const float* __restrict__ C, int64_t n, int d_
 // scale per slice, column scale), stage 32 x 32 values and write them by TMA.
 // 5120 x 1e5 values from 64 outputs: 326 us (6.3 TB/s of writes); the general
 // product, a block per tile with nothing to overlap, took 793 us.
-// Every wait is bounded: on timeout the block sets an error code, finishes its own
-// copies and MMAs (bounded) and frees tensor memory.
+// Every wait is bounded: on timeout the block sets an error code, and once all its
+// roles have stopped it waits (bounded) for its copies and MMAs and frees tensor memory.
 constexpr int kAdjStages = 3, kAdjAcc = 4, kAdjDrain = 8;
 constexpr int kAdjThreads = 32 * (kAdjDrain + 2);
 constexpr int kAdjTile = 32 * 1024;  // 128 rows x 64 values, high and low part
@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   uint64_t* flush = acc_empty + kAdjAcc;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(flush + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* issued = abort_flag + 1;  // slices of R, points' operands
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = a.slices, nb = kAdjMaxSlices / q;  // buffers of the points' operand
   const int64_t t0 = a.tiles * blockIdx.x / gridDim.x, t1 = a.tiles * (blockIdx.x + 1) / gridDim.x;
@@ -208,13 +209,11 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           tma_load_2d(base + i * kAdjTile + kAdjTile / 2, &tmRl, s * 64, mt * 128, &a_full[i]);
         }
       }
-      if (*abort_flag || u < int((t1 - t0) * q)) {  // gave up: wait (bounded) for what was issued
+      if (u < int((t1 - t0) * q)) {  // gave up
         atomicExch(a.err, 1);
         *abort_flag = 1;
-        for (int v = max(0, u - kAdjStages); v < u; ++v)
-          mbar_wait(&a_full[v % kAdjStages], (v / kAdjStages) & 1, nullptr);
-        for (int v = max(0, n - nb); v < n; ++v) mbar_wait(&b_full[v % nb], (v / nb) & 1, nullptr);
       }
+      issued[0] = u, issued[1] = n;
     }
     __syncwarp();
   } else if (warp == kAdjDrain + 1) {
@@ -245,9 +244,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
           mma_commit(&acc_full[c]);
         }
       }
-      if (!ok) {  // finish the MMAs issued (bounded), then let the others stop
-        mma_commit(flush);
-        mbar_wait(flush, 0, nullptr);
+      if (!ok) {
         atomicExch(a.err, 2);
         *abort_flag = 1;
       }
@@ -268,7 +265,13 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
         rs[s] = s < q ? __ldg(a.row_scale + int64_t(s) * a.M + min(e0 + lane, a.M - 1)) : 0.f;
         if (s < q) ok = ok && mbar_wait(&acc_full[(u + s) % kAdjAcc], ((u + s) / kAdjAcc) & 1, abort_flag);
       }
-      if (!__all_sync(0xffffffffu, ok && !*abort_flag)) break;
+      if (!__all_sync(0xffffffffu, ok && !*abort_flag)) {
+        if (lane == 0) {
+          atomicCAS(a.err, 0, 3);
+          *abort_flag = 1;
+        }
+        break;
+      }
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll 1
       for (int j = 0; j < 2; ++j, ++n) {
@@ -325,6 +328,17 @@ __global__ void __launch_bounds__(kAdjThreads, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  if (*abort_flag) {  // all roles have stopped: wait (bounded) for the copies and MMAs issued
+    if (warp == kAdjDrain && lane == 0) {
+      for_pending_copies(issued[0], kAdjStages, [&](int s, uint32_t ph) { mbar_wait(&a_full[s], ph, nullptr); });
+      for_pending_copies(issued[1], nb, [&](int b, uint32_t ph) { mbar_wait(&b_full[b], ph, nullptr); });
+    }
+    if (warp == kAdjDrain + 1 && lane == 0) {
+      mma_commit(flush);
+      mbar_wait(flush, 0, nullptr);
+    }
+    __syncthreads();
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAdjAcc * 128));
 }
