@@ -695,6 +695,9 @@ typedef struct smx_tensor {
   int32_t* err;               /* set when a pipeline wait runs out                     */
 } smx_tensor;
 int smx_tensor_splits(int d_out, int K);
+/* `chunk` of a plan (its other sizes set): the most points whose panel fits the memory
+ * limit, at most 65535 * 128. */
+int64_t smx_tensor_chunk(const smx_tensor* plan_host, double memory_limit_gib);
 /* FP16 operands from the FP32 coefficients B[N][K] (column k = tape entry K-1-k):
  * high and low parts, the output scales, and the padded tape: ceil(K/64)*64 - K
  * entries of padding, then per entry {128 * slot, FP32 bits of 2^f (0 for an entry

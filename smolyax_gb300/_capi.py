@@ -369,6 +369,7 @@ SIGNATURES = {
     "smx_serve_destroy": (None, [_p]),
     "smx_eval_f64_noalloc": (_int, [_p, _p, _i64, _i64, _p, _p]),
     "smx_tensor_splits": (_int, [_int, _int]),
+    "smx_tensor_chunk": (_i64, [_p, _dbl]),
     "smx_tensor_operands": (_int, [_p, _int, _int, _i64, _p, _p, _p, _p, _i64, _p, _p]),
     "smx_tensor_tape": (_int, [_p, _int, _p, _p]),
     "smx_tensor_bwd_operands": (_int, [_p, _i64, _int, _i64, _p, _p, _p, _p, _p]),

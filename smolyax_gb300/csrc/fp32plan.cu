@@ -387,7 +387,7 @@ extern "C" int smx_fp32_plan_create(const smx_plan* pl, const smx_tree* tree, co
       t.K = h->K, t.n_groups = (h->K + 63) / 64;
       t.ldb = std::max(64, 64 * t.n_groups);
       t.splits = smx_tensor_splits(dout, h->K);
-      t.chunk = std::max<int64_t>(128, int64_t(memory_limit_gib * 1073741824.0 / double(4 * t.ldb)) / 128 * 128);
+      t.chunk = smx_tensor_chunk(&t, memory_limit_gib);
       t.max_deg = 1;
       for (int64_t m : maxdeg) t.max_deg = std::max(t.max_deg, int32_t(m));
       std::vector<float> rec(size_t(4) * t.max_deg);

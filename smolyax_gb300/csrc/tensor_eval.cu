@@ -414,6 +414,18 @@ extern "C" int smx_tensor_splits(int d_out, int K) {
   return std::max(1, std::min({8, K / 1024, K / (8 * d_out)}));
 }
 
+// Points per pass: the panel within the memory limit, and at most 65535 tiles of 128
+// rows (the contraction's second grid dimension).
+namespace {
+constexpr int64_t kMaxPass = int64_t(65535) * 128;
+}
+
+extern "C" int64_t smx_tensor_chunk(const smx_tensor* t, double memory_limit_gib) {
+  if (!t || t->ldb < 1) return 128;
+  const int64_t fit = int64_t(std::min(memory_limit_gib * 1073741824.0 / double(4 * t->ldb), double(kMaxPass)));
+  return std::max<int64_t>(128, fit / 128 * 128);
+}
+
 extern "C" size_t smx_tensor_workspace(const smx_tensor* t, int64_t P) {
   if (!t || P <= 0 || t->chunk < 1) return 0;
   return layout(t, std::min(P, t->chunk)).total;
@@ -426,6 +438,7 @@ extern "C" int smx_tensor_eval(const smx_tensor* t, const double* x, int64_t P, 
                   t->splits >= 1 && t->chunk >= 1 && t->ldb >= t->K && t->ldb % kGroup == 0,
               "smx_tensor_eval: bad plan sizes");
   SMX_REQUIRE(P >= 0 && ldx >= t->d_in, "smx_tensor_eval: bad sizes");
+  SMX_REQUIRE(std::min(P, t->chunk) <= kMaxPass, "smx_tensor_eval: more points per pass than smx_tensor_chunk allows");
   if (P == 0) return SMX_OK;
   SMX_REQUIRE(x && y && t->bias && t->err, "smx_tensor_eval: null pointer");
   SMX_REQUIRE(t->K == 0 || (t->dims && t->dmax && t->dsoff && t->fam && t->fam_a && t->fam_b && t->rec && t->tape &&

@@ -300,6 +300,8 @@ class SpectralPlan:
             return self._build_tc_struct(tc, key, bf16) if key not in tc else tc[key][0]
 
     def _build_tc_struct(self, tc, key, bf16):
+        import ctypes
+
         Bd = tc["Bd"]
         d_out, K = int(Bd.shape[0]), tc["K"]
         n_groups = (K + 63) // 64
@@ -319,7 +321,8 @@ class SpectralPlan:
                 call("smx_tensor_operands", ptr(Bd), d_out, K, tc["ldk"], ptr(tc["tape"]), ptr(k["tape"]),
                      ptr(k["Bh"]), ptr(k["Bl"]), ldb, ptr(k["out_scale"]), st)
         s = self._tensor_struct(tc, d_out)
-        s.bf16, s.splits, s.chunk, s.ldb = int(bf16), self.tc_splits(), self._tc_step(1 << 40), ldb
+        s.bf16, s.splits, s.ldb = int(bf16), self.tc_splits(), ldb
+        s.chunk = capi.size("smx_tensor_chunk", ctypes.byref(s), float(self.memory_limit))
         for name, t in k.items():
             setattr(s, name, t.data_ptr())
         s.keep = k
@@ -696,9 +699,8 @@ class SpectralPlan:
         return y
 
     def _tc_step(self, P):
-        """Points per panel chunk (the 16-bit hi/lo panel of one chunk fits the memory limit)."""
-        step = max(128, int(self.memory_limit * 1024**3 // (4 * max(64, (self.tc["K"] + 63) // 64 * 64))) // 128 * 128)
-        return max(1, min(step, P))
+        """Points per panel chunk (``smx_tensor_chunk``)."""
+        return max(1, min(int(self._tc_struct().chunk), P))
 
     def tc_splits(self):
         """K slices of the forward contraction (``smx_tensor_splits``): a plan
