@@ -676,7 +676,7 @@ typedef struct smx_tensor {
   int32_t splits;             /* K slices of the contraction (smx_tensor_splits)       */
   int32_t bf16;
   int32_t reserved;
-  int64_t chunk;              /* points per pass (the panel of one pass: 4 ldb bytes a point) */
+  int64_t chunk;              /* points per pass (smx_tensor_chunk)                   */
   int64_t ldb;                /* row pitch of Bh, Bl and the panel: K rounded up to 64  */
   const int32_t* dims;        /* [n_dims], with dmax (largest degree), dsoff (first slot) */
   const int32_t* dmax;
@@ -696,7 +696,7 @@ typedef struct smx_tensor {
 } smx_tensor;
 int smx_tensor_splits(int d_out, int K);
 /* `chunk` of a plan (its other sizes set): the most points whose panel fits the memory
- * limit, at most 65535 * 128. */
+ * limit, with all scratch in 9/8 of it, at most 65535 * 128. */
 int64_t smx_tensor_chunk(const smx_tensor* plan_host, double memory_limit_gib);
 /* FP16 operands from the FP32 coefficients B[N][K] (column k = tape entry K-1-k):
  * high and low parts, the output scales, and the padded tape: ceil(K/64)*64 - K

@@ -414,15 +414,18 @@ extern "C" int smx_tensor_splits(int d_out, int K) {
   return std::max(1, std::min({8, K / 1024, K / (8 * d_out)}));
 }
 
-// Points per pass: the panel within the memory limit, and at most 65535 tiles of 128
-// rows (the contraction's second grid dimension).
+// Points per pass: the panel within the memory limit, all scratch (basis rows, scales
+// and partial sums too) within 9/8 of it, and at most 65535 tiles of 128 rows (the
+// contraction's second grid dimension).
 namespace {
 constexpr int64_t kMaxPass = int64_t(65535) * 128;
 }
 
 extern "C" int64_t smx_tensor_chunk(const smx_tensor* t, double memory_limit_gib) {
   if (!t || t->ldb < 1) return 128;
-  const int64_t fit = int64_t(std::min(memory_limit_gib * 1073741824.0 / double(4 * t->ldb), double(kMaxPass)));
+  const double limit = memory_limit_gib * 1073741824.0, panel = 4.0 * double(t->ldb);
+  const double all = panel + 4.0 * t->n_groups + 4.0 * t->n_slots + (t->splits > 1 ? 4.0 * t->splits * t->d_out : 0.0);
+  const int64_t fit = int64_t(std::min({limit / panel, 1.125 * limit / all, double(kMaxPass)}));
   return std::max<int64_t>(128, fit / 128 * 128);
 }
 
