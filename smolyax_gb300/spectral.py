@@ -650,38 +650,43 @@ class SpectralPlan:
         first use from the same tree and the FP64 coefficients; None where that
         evaluator does not apply (hot nodes deeper than 8, or a per-point row
         beyond shared memory)."""
-        if self._f64 is None:
-            self._f64 = False
-            tr, _, maxdeg, fam, fa, fb, T, _ = self._fwd_args
-            d = int(self.c.d_in)
-            C64 = self.C64.cpu().numpy()
-            lay = capi.host_layout("perpoint", tr, C64, int(C64.shape[1]), maxdeg, fam, fa, fb, fp64=True,
-                                   **FP64_TABLES)
-            if lay is None:
-                return None
-            row = int(lay["row"])
-            DO = 1 if int(lay["d_out"]) == 1 else 4
-            if (row + 4 * DO) * 64 * 8 <= 227 * 1024 and int(lay["max_depth"]) <= 8:
-                k = {}
-                for name in ("hot_dim", "hot_deg", "hot_soff", "node", "cold", "run"):
-                    k[name] = T(lay[name], torch.int32)
-                for name in ("node_c", "cold_ab", "terms", "coef"):
-                    k[name] = T(lay[name], torch.float64)
-                k["c0"] = self.C64[0].contiguous()
-                st = capi.SmxSpectral64()
-                st.d_in, st.row = d, row
-                for name in ("d_out", "dstride", "n_hb", "n_vp", "n_hot_dims", "n_nodes", "n_cold_groups", "max_depth",
-                             "n_terms"):
-                    setattr(st, name, int(lay[name]))
-                for i in range(5):
-                    st.node_seg[i] = int(lay["node_seg"][i])
-                    st.cold_seg[i] = int(lay["cold_seg"][i])
-                for name, t in k.items():
-                    setattr(st, name, t.data_ptr() if t.numel() else None)
-                st.fam_a, st.fam_b, st.fam = self.fa64.data_ptr(), self.fb64.data_ptr(), self.fam.data_ptr()
-                k["stream"] = stream_tables(st, tr, C64, int(lay["d_out"]), maxdeg, fam, fa, fb, T, True)
-                self._f64 = (st, k)
-        return self._f64 or None
+        with self._lock:
+            if self._f64 is None:
+                self._f64 = self._build_fp64_form() or False
+            return self._f64 or None
+
+    def _build_fp64_form(self):
+        tr, _, maxdeg, fam, fa, fb, T, _ = self._fwd_args
+        d = int(self.c.d_in)
+        C64 = self.C64.cpu().numpy()
+        lay = capi.host_layout("perpoint", tr, C64, int(C64.shape[1]), maxdeg, fam, fa, fb, fp64=True,
+                               **FP64_TABLES)
+        if lay is None:
+            return None
+        row = int(lay["row"])
+        DO = 1 if int(lay["d_out"]) == 1 else 4
+        if (row + 4 * DO) * 64 * 8 > 227 * 1024 or int(lay["max_depth"]) > 8:
+            return None
+        k = {}
+        for name in ("hot_dim", "hot_deg", "hot_soff", "node", "cold", "run"):
+            k[name] = T(lay[name], torch.int32)
+        for name in ("node_c", "cold_ab", "terms", "coef"):
+            k[name] = T(lay[name], torch.float64)
+        k["c0"] = self.C64[0].contiguous()
+        st = capi.SmxSpectral64()
+        st.d_in, st.row = d, row
+        for name in ("d_out", "dstride", "n_hb", "n_vp", "n_hot_dims", "n_nodes", "n_cold_groups", "max_depth",
+                     "n_terms"):
+            setattr(st, name, int(lay[name]))
+        for i in range(5):
+            st.node_seg[i] = int(lay["node_seg"][i])
+            st.cold_seg[i] = int(lay["cold_seg"][i])
+        for name, t in k.items():
+            setattr(st, name, t.data_ptr() if t.numel() else None)
+        st.fam_a, st.fam_b, st.fam = self.fa64.data_ptr(), self.fb64.data_ptr(), self.fam.data_ptr()
+        k["stream"] = stream_tables(st, tr, C64, int(lay["d_out"]), maxdeg, fam, fa, fb, T, True)
+        finish_build()
+        return st, k
 
     def evaluate64(self, x, y):
         """y[P, d_out] (FP64, contiguous) at x[P, d_in] (FP64, rows contiguous, on
