@@ -485,6 +485,11 @@ class SmolyakBarycentricInterpolator:
             self._coef = coef
         return self._coef
 
+    def _coefficient_bytes(self):
+        """Device bytes that building the coefficients takes: the rows of the nodal
+        values once more, and the coefficients."""
+        return 8 * self._d_out * (int(self._plan.c.n_entries) + int(self._tree.size))
+
     def spectral_plan(self):
         """The FP32 orthogonal-polynomial form of this interpolant (built on first use)."""
         assert self._plan is not None, "The operator has not yet been set up for a target function via `set_f`."
@@ -552,15 +557,16 @@ class SmolyakBarycentricInterpolator:
         sum serves ``gradient``: other rules than Leja and Gauss-Hermite (their
         polynomial families are the form's), degrees of 24 and more (the basis
         change of the form is a host computation there), interpolants without
-        summands, and coefficient workspaces beyond 16 GB (as large as the nodal
-        values' rows, which the combination sum does not need twice)."""
+        summands, and coefficients that are still to be built where that takes more
+        scratch than the memory limit (the combination sum needs none of it)."""
+        if self._coef is None and self._coefficient_bytes() > self._memory_limit * 1024**3:
+            return None
         if self._jacobian is None:
             from .jacobian import MAX_DEGREE, JacobianPlan
             from .spectral import finish_build
 
             c = self._plan.c
-            ok = (c.n_entries > 0 and c.n_entries * c.d_out * 8 <= 16 * 1024**3
-                  and int(np.max(self._maxdeg, initial=0)) < MAX_DEGREE
+            ok = (c.n_entries > 0 and int(np.max(self._maxdeg, initial=0)) < MAX_DEGREE
                   and all(isinstance(g, (_nodes.Leja1D, _nodes.GaussHermite1D)) for g in self._node_gen))
             jac = JacobianPlan(self) if ok else False
             if ok:
