@@ -569,10 +569,11 @@ int check_plan(const smx_plan* pl, const char* who) {
 template <int DO, bool SROWS>
 int launch_contract(const PlanArgs& a, const double* Lt, int64_t P, double* y, int o_base, int passes, int parts,
                     size_t smem, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(contract_kernel<DO, SROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-    attr = true;
+  // (with every launch: the attribute belongs to the current device, and the call is cheap)
+  if (cudaFuncSetAttribute(contract_kernel<DO, SROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return smx::set_error(SMX_ERR_CUDA, "smx_contract_f64: shared memory of a block refused");
   }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
