@@ -387,7 +387,8 @@ class SpectralPlan:
 
     # ------------------------------------------------------------------ backward
     def _backward_ops(self):
-        """Tape operands (built as for the forward tensor-core path) plus the
+        """Tape operands (built as for the forward tensor-core path) and those of the
+        gradient walk and of dL/dC; plans outside the walk's limits have the
         coefficient rows C[K x ldo] in the panel's reversed order, TF32 hi/lo."""
         with self._lock:
             return self._bwd if self._bwd is not None else self._build_backward_ops()
@@ -402,13 +403,14 @@ class SpectralPlan:
         K = ops["K"]
         d_out = C32.shape[1]
         ldo = _round4(d_out)
-        ent = ops["ent_h"]
-        rows = np.zeros((max(K, 1), ldo), dtype=np.float32)
-        rows[:K, :d_out] = C32[ent[::-1]]
-        Rd = T(rows, torch.float32)
-        Rh, Rl = torch.empty_like(Rd), torch.empty_like(Rd)
-        call("smx_split_tf32", ptr(Rd), rows.shape[0], ldo, ldo, ptr(Rh), ptr(Rl), ldo, st)
-        ops.update(Rh=Rh, Rl=Rl, ldo=ldo, walk=self._build_walk(ops, C32), coef=self._build_coef(ops, d_out))
+        ops.update(ldo=ldo, walk=self._build_walk(ops, C32), coef=self._build_coef(ops, d_out))
+        if ops["walk"] is None:
+            rows = np.zeros((max(K, 1), ldo), dtype=np.float32)
+            rows[:K, :d_out] = C32[ops["ent_h"][::-1]]
+            Rd = T(rows, torch.float32)
+            Rh, Rl = torch.empty_like(Rd), torch.empty_like(Rd)
+            call("smx_split_tf32", ptr(Rd), rows.shape[0], ldo, ldo, ptr(Rh), ptr(Rl), ldo, st)
+            ops.update(Rh=Rh, Rl=Rl)
         # tape segments of the gradient walk: fixed per plan (a point's dL/dx
         # does not depend on the batch it comes in)
         want = vjp_segment_count(K, ops["lvl1"].size)
@@ -424,8 +426,6 @@ class SpectralPlan:
     def _build_walk(self, ops, C32):
         """Structs of the gradient walk over G^T (``csrc/tensor_vjp.cu``), or None
         where its rows do not fit in shared memory."""
-        import ctypes
-
         tr, _, maxdeg, fam, fa, fb, T, st = self._fwd_args
         n_lam, d_out = C32.shape
         if n_lam < 2:
@@ -527,12 +527,6 @@ class SpectralPlan:
         P, d = int(x.shape[0]), int(x.shape[1])
         d_out = int(g.shape[1])
         K, ldk, ldo = ops["K"], ops["ldk"], ops["ldo"]
-        nd = int(ops["dims"].numel())
-        common = (nd, ptr(ops["dims"]), ptr(ops["dmax"]), ptr(ops["dsoff"]), ops["n_slots"], ptr(ops["tape"]), K,
-                  ptr(k["fam_a"]), ptr(k["fam_b"]), ptr(k["fam"]))
-        seg, n_seg = ops["vjp_seg"]
-        walk = (nd, ptr(ops["dims"]), ptr(ops["dmax"]), ptr(ops["dsoff"]), ops["n_slots"], ptr(ops["tape"]), K,
-                ptr(seg), n_seg, ptr(k["fam_a"]), ptr(k["fam_b"]), ptr(k["fam"]))
         gf = g.float().contiguous()
         err = ops["err"]
         dx = dC = rows = None
@@ -545,10 +539,14 @@ class SpectralPlan:
             if g.dtype == torch.float64:
                 dC[0] = g.sum(0)
             need_coef = False
-        if need_x or need_coef:
+        if need_x or need_coef:  # plans outside the limits of the above
             g32 = torch.zeros(P, ldo, dtype=torch.float32, device=dev)
             g32[:, :d_out] = gf
+            tape = (int(ops["dims"].numel()), ptr(ops["dims"]), ptr(ops["dmax"]), ptr(ops["dsoff"]), ops["n_slots"],
+                    ptr(ops["tape"]), K)
+            maps = (ptr(k["fam_a"]), ptr(k["fam_b"]), ptr(k["fam"]))
         if need_x:
+            seg, n_seg = ops["vjp_seg"]
             gh, gl = torch.empty_like(g32), torch.empty_like(g32)
             call("smx_split_tf32", ptr(g32), P, ldo, ldo, ptr(gh), ptr(gl), ldo, st)
             dx = torch.zeros(P, d, dtype=torch.float64, device=dev)
@@ -560,8 +558,8 @@ class SpectralPlan:
                 p1 = min(P, p0 + step)
                 call("smx_gemm_tf32x3", ptr(gh[p0:p1]), ptr(gl[p0:p1]), ldo, ptr(ops["Rh"]), ptr(ops["Rl"]), ldo,
                      p1 - p0, K, ldo, ptr(G), ldg, None, 0, ptr(err), st)
-                call("smx_spectral_vjp_x", *walk, ptr(x[p0:p1]), p1 - p0, d, ptr(G), ldg, ptr(dx[p0:p1]), d,
-                     ptr(ws), nws, st)
+                call("smx_spectral_vjp_x", *tape, ptr(seg), n_seg, *maps, ptr(x[p0:p1]), p1 - p0, d, ptr(G), ldg,
+                     ptr(dx[p0:p1]), d, ptr(ws), nws, st)
         if need_coef:
             ldp = _round32(min(step, P))  # 128-byte rows
             ATh = torch.empty(K, ldp, dtype=torch.float32, device=dev)
@@ -582,8 +580,8 @@ class SpectralPlan:
                 n = p1 - p0
                 # the contraction runs over the chunk's n points: the columns past n
                 # are outside the operands' tensor maps and need no zeros
-                call("smx_spectral_panel_t_tf32", *common, ptr(x[p0:p1]), n, d, ptr(ATh), ptr(ATl), ldp, ptr(ws), nws,
-                     st)
+                call("smx_spectral_panel_t_tf32", *tape, *maps, ptr(x[p0:p1]), n, d, ptr(ATh), ptr(ATl), ldp, ptr(ws),
+                     nws, st)
                 gT[:, :n] = g32[p0:p1].t()
                 call("smx_split_tf32", ptr(gT), ldo, n, ldp, ptr(gTh), ptr(gTl), ldp, st)
                 call("smx_gemm_tf32x3_splitk", ptr(ATh), ptr(ATl), ldp, ptr(gTh), ptr(gTl), ldp, K, d_out, n,
