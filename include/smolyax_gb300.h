@@ -693,6 +693,13 @@ typedef struct smx_tensor {
   const float* out_scale;     /* [d_out] (bf16 = 0)                                    */
   const float* bias;          /* [d_out] c0                                            */
   int32_t* err;               /* set when a pipeline wait runs out                     */
+  const float* B;             /* [d_out][ldk] the coefficients in FP32 (16-byte aligned rows,
+                                 zero from K to a multiple of 4) and the slots of every
+                                 column ("col_path" of the tape tables: 8 uint16, 0xffff past
+                                 the last), for points whose terms exceed the range of the
+                                 FP16 pairs; NULL: no such evaluation                   */
+  int64_t ldk;
+  const int32_t* col_path;    /* [K][4], 16-byte aligned                               */
 } smx_tensor;
 int smx_tensor_splits(int d_out, int K);
 /* `chunk` of a plan (its other sizes set): the most points whose panel fits the memory
@@ -785,7 +792,7 @@ int smx_nodal_adjoint(const double* Fbar, const double* zeta, int64_t n_values, 
  * reference's evaluation (interpolation.py:264-304) as the smx_spectral /
  * smx_blocked comments describe; smx_fp32_plan_create uses them.  Tables are
  * read back by name (the field names of smx_blocked / smx_spectral, plus
- * "dims", "dmax", "dsoff", "tape", "ent", "lvl1", "path" of the tape; the int32 tables
+ * "dims", "dmax", "dsoff", "tape", "ent", "lvl1", "path", "col_path" of the tape; the int32 tables
  * "st_hot", "st_vp", "st_desc", "st_warp", "st_chunk" and the scalars "st_pass",
  * "st_row_bytes", "st_n_hb", "st_n_vp", "st_n_rows", "st_n_hot", "st_n_chunks" of the stream). */
 #define SMX_LAYOUT_BLOCKED 0

@@ -192,6 +192,9 @@ class SmxTensor(C.Structure):
         ("out_scale", _p),
         ("bias", _p),
         ("err", _p),
+        ("B", _p),
+        ("ldk", _i64),
+        ("col_path", _p),
     ]
 
 

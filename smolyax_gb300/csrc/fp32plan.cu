@@ -127,9 +127,9 @@ struct smx_fp32_plan {
   bool have_tape = false;
   int K = 0, ldk = 0, ldo = 0, n_slots = 0, n_dims = 0;
   DevBuf<int32_t> dims, dmax, dsoff, tape, ent, segs, err;
-  DevBuf<float> bias, Rh, Rl, out_scale, rec;
+  DevBuf<float> bias, Rh, Rl, out_scale, rec, B;
   DevBuf<uint16_t> Bh, Bl;
-  DevBuf<int32_t> tape_pad, path;
+  DevBuf<int32_t> tape_pad, path, col_path;
   smx_tensor tensor{};
   std::vector<int32_t> lvl1;
   std::vector<int> seg_off, seg_n;  // per wanted segment count: offset into segs, number of segments
@@ -373,7 +373,7 @@ extern "C" int smx_fp32_plan_create(const smx_plan* pl, const smx_tree* tree, co
         Rrows[size_t(j) * h->ldo + o] = v;
       }
     for (int o = 0; o < dout; ++o) c0[o] = C32[o];
-    DevBuf<float> Bd, Rd;
+    DevBuf<float> Rd;
     if ((rc = h->dims.upload(tp.i32["dims"], st)) || (rc = h->dmax.upload(tp.i32["dmax"], st)) ||
         (rc = h->dsoff.upload(tp.i32["dsoff"], st)) || (rc = h->tape.upload(tp.i32["tape"], st)) ||
         (rc = h->ent.upload(ent, st)) || (rc = h->bias.upload(c0, st)) || (rc = Rd.upload(Rrows, st)) ||
@@ -401,17 +401,19 @@ extern "C" int smx_fp32_plan_create(const smx_plan* pl, const smx_tree* tree, co
       const size_t nb = size_t(dout) * t.ldb;
       if ((rc = h->rec.upload(rec, st)) || (rc = h->path.upload(tp.i32["path"], st)) ||
           (rc = h->tape_pad.alloc(size_t(128) * t.n_groups)) || (rc = h->Bh.alloc(nb)) || (rc = h->Bl.alloc(nb)) ||
-          (rc = h->out_scale.alloc(dout)) || (rc = Bd.upload(B, st)))
+          (rc = h->out_scale.alloc(dout)) || (rc = h->B.upload(B, st)) ||
+          (rc = h->col_path.upload(tp.i32["col_path"], st)))
         return rc;
       cudaMemsetAsync(h->Bh.p, 0, nb * sizeof(uint16_t), st);
       cudaMemsetAsync(h->Bl.p, 0, nb * sizeof(uint16_t), st);
-      if (h->K > 0 && (rc = smx_tensor_operands(Bd.p, dout, h->K, h->ldk, h->tape.p, h->tape_pad.p, h->Bh.p, h->Bl.p,
+      if (h->K > 0 && (rc = smx_tensor_operands(h->B.p, dout, h->K, h->ldk, h->tape.p, h->tape_pad.p, h->Bh.p, h->Bl.p,
                                                 t.ldb, h->out_scale.p, stream)))
         return rc;
       t.dims = h->dims.p, t.dmax = h->dmax.p, t.dsoff = h->dsoff.p;
       t.fam_a = h->fam_a.p, t.fam_b = h->fam_b.p, t.fam = h->fam.p, t.rec = h->rec.p;
       t.tape = h->tape_pad.p, t.path = h->path.p, t.Bh = h->Bh.p, t.Bl = h->Bl.p;
       t.out_scale = h->out_scale.p, t.bias = h->bias.p, t.err = h->err.p;
+      t.B = h->B.p, t.ldk = h->ldk, t.col_path = h->col_path.p;
     }
     // segment bounds of the panel for every wanted count (spectral.py segment_bounds):
     // near-equal splits of the tape, every bound but the last at a depth-1 entry

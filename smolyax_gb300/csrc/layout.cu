@@ -1251,6 +1251,15 @@ bool build_tape(const Tree& tr, const int64_t* maxdeg, int d, Tables& out) {
       for (int q = 1; q < depth; ++q) path[(pad + i) / 64 * 8 + q - 1] = above[q];
     above[depth] = tape[i] & 0xffff;
   }
+  // the slots of every entry, by column of the panel (reversed tape): 8 uint16 words
+  std::vector<int32_t> col_path(ent.size() * 4, -1);
+  for (size_t i = 0; i < ent.size(); ++i) {
+    const int depth = int(tr.level[ent[i]]);
+    above[depth] = tape[i] & 0xffff;
+    uint16_t s[8];
+    for (int q = 0; q < depth; ++q) s[q] = uint16_t(above[q + 1]);
+    std::memcpy(&col_path[(ent.size() - 1 - i) * 4], s, depth * sizeof(uint16_t));
+  }
   out.i32["dims"] = dims;
   out.i32["dmax"] = dmax;
   out.i32["dsoff"] = dsoff;
@@ -1258,6 +1267,7 @@ bool build_tape(const Tree& tr, const int64_t* maxdeg, int d, Tables& out) {
   out.i32["ent"] = ent32;
   out.i32["lvl1"] = lvl1;
   out.i32["path"] = path;
+  out.i32["col_path"] = col_path;
   out.scalar["n_slots"] = double(n_slots);
   out.scalar["K"] = double(ent.size());
   out.scalar["ldk"] = double(round32(std::max<int64_t>(int64_t(ent.size()), 1)));

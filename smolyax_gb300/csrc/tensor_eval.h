@@ -35,11 +35,29 @@ __device__ __forceinline__ void copy16(void* dst, const void* src) {
 }
 
 // Basis values of all slots, grow[slot][p], and (drow given) their derivatives,
-// p < ldp (a multiple of 32; points past P repeat the last one).
+// p < ldp (a multiple of 32; points past P repeat the last one).  `far` given: the list
+// of far points, emptied.
 void tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, float* drow, int64_t ldp,
-                  cudaStream_t st);
+                  cudaStream_t st, int32_t* far = nullptr);
 
 constexpr int kTf32 = 0, kBf16 = 1, kF16 = 2;
+
+// Far points (far_points.cuh): the lists of a pass (the count, then from kFarHead on a
+// mark per point and, gstride further, the points) and what their products are made of.
+struct FarPoints {
+  const int32_t* list;  // NULL: none
+  const float* rows;    // basis values [slot][gstride]
+  int64_t gstride;
+  const int32_t* col_path;  // [K][4]
+  const float* B;           // [N][ldk], zero from K to a multiple of 4
+  int64_t ldk;
+};
+constexpr int kFarHead = 64;
+constexpr int kFarPts = 8, kFarCols = 512;
+
+inline __host__ __device__ size_t far_bytes(int64_t gstride) {
+  return (kFarHead + 2 * size_t(gstride)) * sizeof(int32_t);
+}
 
 // D [M x N] = sum over 64-column groups q of row_scale[q][m] * (A_q B_q^T), times
 // col_scale[n], plus bias[n].  A = Ah + Al, B = Bh + Bl, 16-bit, row-major
@@ -63,6 +81,7 @@ struct SplitGemm {
   float* partial;
   bool sliced;     // kF16: A is [ceil(K / 64)][M][64], B [ceil(K / 64)][N][64] (lda, ldb unused)
   int accumulate;  // D += instead of D =
+  FarPoints far;   // kF16, row-major: rows of D evaluated apart
 };
 int split_gemm(const SplitGemm& g, cudaStream_t st);
 

@@ -245,7 +245,8 @@ class SpectralPlan:
         evaluation and the backward, or None (entries deeper than 8: the panel's
         product stack)."""
         tp = capi.host_layout("tape", tr, None, int(C32.shape[1]), maxdeg, fam, fa, fb,
-                              i32=("dims", "dmax", "dsoff", "tape", "ent", "lvl1", "path"), scalars=("n_slots",))
+                              i32=("dims", "dmax", "dsoff", "tape", "ent", "lvl1", "path", "col_path"),
+                              scalars=("n_slots",))
         if tp is None:
             return None
         dev = self.fam.device
@@ -256,7 +257,7 @@ class SpectralPlan:
                         np.stack([np.sqrt(2.0 / (m + 1)), np.sqrt(m / (m + 1))], axis=1)])
         return dict(dims=T(tp["dims"], torch.int32), dmax=T(tp["dmax"], torch.int32),
                     dsoff=T(tp["dsoff"], torch.int32), n_slots=int(tp["n_slots"]), tape=T(tp["tape"], torch.int32),
-                    path=T(tp["path"], torch.int32), K=K, ldk=_round32(max(K, 1)),
+                    path=T(tp["path"], torch.int32), col_path=T(tp["col_path"], torch.int32), K=K, ldk=_round32(max(K, 1)),
                     max_deg=max_deg, rec=T(rec, torch.float32), bias=self.keep["c0"],
                     err=torch.zeros(1, dtype=torch.int32, device=dev),
                     ent=torch.as_tensor(tp["ent"].astype(np.int64), device=dev), ent_h=tp["ent"].astype(np.int64),
@@ -311,6 +312,9 @@ class SpectralPlan:
         k = dict(Bh=torch.zeros(d_out, ldb, dtype=torch.bfloat16 if bf16 else torch.float16, device=dev))
         k["Bl"] = torch.zeros_like(k["Bh"])
         k["tape"] = torch.zeros(2 * 64 * n_groups, dtype=torch.int32, device=dev)
+        s = self._tensor_struct(tc, d_out)
+        s.bf16, s.splits, s.ldb = int(bf16), self.tc_splits(), ldb
+        s.chunk = capi.size("smx_tensor_chunk", ctypes.byref(s), float(self.memory_limit))
         if bf16:
             if K:
                 call("smx_tensor_tape", ptr(tc["tape"]), K, ptr(k["tape"]), st)
@@ -320,9 +324,8 @@ class SpectralPlan:
             if K:
                 call("smx_tensor_operands", ptr(Bd), d_out, K, tc["ldk"], ptr(tc["tape"]), ptr(k["tape"]),
                      ptr(k["Bh"]), ptr(k["Bl"]), ldb, ptr(k["out_scale"]), st)
-        s = self._tensor_struct(tc, d_out)
-        s.bf16, s.splits, s.ldb = int(bf16), self.tc_splits(), ldb
-        s.chunk = capi.size("smx_tensor_chunk", ctypes.byref(s), float(self.memory_limit))
+            s.B, s.ldk = Bd.data_ptr(), tc["ldk"]
+            s.col_path = tc["col_path"].data_ptr() if K else None
         for name, t in k.items():
             setattr(s, name, t.data_ptr())
         s.keep = k

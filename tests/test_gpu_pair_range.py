@@ -85,10 +85,10 @@ def test_entries_without_coefficients_do_not_hide_the_others(j, far):
     assert _term_error(sp, C, x).max() <= 1e-6
 
 
-@pytest.mark.parametrize("j,far", [(0, 1.0), (0, 30.0), (8, 1e5)])
+@pytest.mark.parametrize("j,far", [(0, 1.0), (0, 30.0), (2, 1e3), (2, 1e4), (8, 1e5)])
 def test_small_terms_beside_large_ones(j, far):
     """Values of outputs without a coordinate beside outputs of that coordinate alone,
-    whose terms are up to 1e8 times larger."""
+    whose terms are up to 1e16 times larger."""
     d = 20
     ip = _plan(d, 900, 24, fns.rational_vec(d, 24, seed=3))
     sp = ip.spectral_plan()
@@ -160,3 +160,35 @@ def test_points_without_a_cotangent_weigh_nothing():
     x[::7] *= 1e4
     g[::7] = 0.0
     assert _coef_error(sp, x, g) <= 1e-5
+
+
+@pytest.mark.parametrize("n,d_out", [(900, 24), (900, 130), (900, 300), (3000, 17), (3000, 70)])
+def test_far_points_among_others(n, d_out):
+    """Points far outside the box between points inside, with one slice of K and several:
+    term-relative errors, and every value the same in other batches and passes."""
+    from smolyax_gb300 import _capi as capi
+
+    import ctypes
+
+    d, P = 20, 333
+    ip = _plan(d, n, d_out, fns.rational_vec(d, d_out, seed=3))
+    sp = ip.spectral_plan()
+    assert (sp.tc_splits() > 1) == (n > 2048)
+    C = sp.C64.cpu().numpy()
+    x = np.random.default_rng(0).uniform(-1, 1, (P, d))
+    x[::5, 1] = 1e3
+    x[7::50] *= 1e2
+    assert _term_error(sp, C, x).max() <= 1e-6
+    xd = torch.as_tensor(x, device="cuda")
+    y, got = (torch.empty(P, d_out, dtype=torch.float32, device="cuda") for _ in range(2))
+    sp.evaluate(xd, y)
+    for part in (slice(5, 6), slice(100, 201), slice(330, 333)):
+        alone = torch.empty(xd[part].shape[0], d_out, dtype=torch.float32, device="cuda")
+        assert torch.equal(sp.evaluate(xd[part].contiguous(), alone), y[part])
+    s = type(sp._tc_struct()).from_buffer_copy(sp._tc_struct())
+    s.chunk = 128
+    nws = capi.size("smx_tensor_workspace", ctypes.byref(s), P)
+    ws = torch.empty(nws, dtype=torch.uint8, device="cuda")
+    capi.call("smx_tensor_eval", ctypes.byref(s), capi.ptr(xd), P, d, capi.ptr(got), capi.ptr(ws), nws,
+              capi.stream_ptr(torch.cuda.current_stream()))
+    assert torch.equal(got, y)
