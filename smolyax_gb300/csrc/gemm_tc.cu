@@ -20,6 +20,7 @@
 #include "far_points.cuh"
 #include "tc_util.cuh"
 #include "tensor_eval.h"
+#include "tile_rule.h"
 
 namespace {
 
@@ -451,12 +452,7 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
   return SMX_OK;
 }
 
-// Columns per tile: the width with the least rounds of tiles on the SMs x time of a
-// round, which measured 69, 73 and 115 - 140 us for 64, 128 and 256 columns (split
-// BF16, K = 6016: a narrow tile still loads the 128 rows of A).  Columns and rounds that
-// are not filled cost as much as full ones: 10000 x 300 outputs take 136 us with
-// 128 columns (2 rounds) and 212 with 256 (2), 65536 x 400 take 878 (14) and 785
-// (7), 10000 x 100 take 127 with 64 (2) and 76 with 128 (1).
+// Columns per tile (tile_rule.h).
 int tile_columns(int64_t M, int N, int64_t nz) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -464,15 +460,7 @@ int tile_columns(int64_t M, int N, int64_t nz) {
     cudaGetLastError();
     sms = 152;
   }
-  const int64_t rows = (M + kBM - 1) / kBM * nz;
-  int best = 0;
-  int64_t cost = 0;
-  for (int bn : {256, 128, 64}) {
-    const int64_t tiles = rows * ((N + bn - 1) / bn);
-    const int64_t c = (tiles + sms - 1) / sms * (bn == 256 ? 177 : bn == 128 ? 100 : 94);
-    if (!best || c < cost) best = bn, cost = c;
-  }
-  return best;
+  return choose_tile((M + kBM - 1) / kBM * nz, N, sms).columns;
 }
 
 template <int KIND>

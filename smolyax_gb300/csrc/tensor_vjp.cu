@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "tc_util.cuh"
 #include "tensor_eval.h"
+#include "tile_rule.h"
 
 namespace {
 
@@ -510,7 +511,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 // its largest cotangent (in units of each output's largest), and the cotangents divided
 // by it: the pairs' range (2^29 below the slice's largest at full precision, tc_util.cuh)
 // then counts the points' terms A g and not A and g by themselves, which may run against
-// each other over the points, and points without a cotangent weigh nothing.  A block of
+// each other over the points, and points without a cotangent weigh nothing.  An element
+// of dL/dC has the accuracy of the TF32 pairs while its own largest term of a slice is
+// within 2^29 of its entry's largest over the outputs (in units of their largest g).  A block of
 // W warps holds
 // the basis rows of 64 points (two per lane) in shared memory; each warp walks its
 // run of tape groups as tensor_panel_kernel does (tensor_eval.cu), but an entry's 64
@@ -890,8 +893,7 @@ void launch_coef_panel(const smx_tensor& t, const CoefLayout& L, const float* gr
 
 }  // namespace
 
-// Slices of the contraction over the points: the count of up to 16 with the fewest
-// rounds of tiles on the SMs per slice.
+// Slices of the contraction over the points (tile_rule.h).
 extern "C" int smx_tensor_coef_splits(int d_out, int K) {
   if (d_out < 1 || K < 1) return 1;
   int dev = 0, sms = 0;
@@ -900,15 +902,7 @@ extern "C" int smx_tensor_coef_splits(int d_out, int K) {
     cudaGetLastError();
     return 1;
   }
-  const int64_t bn = d_out <= 64 ? 64 : d_out <= 192 ? 128 : 256;
-  const int64_t tiles = (K + 127) / 128 * ((d_out + bn - 1) / bn);
-  int best = 1;
-  double cost = 1e30;
-  for (int s = 1; s <= 16; ++s) {
-    const double c = double((tiles * s + sms - 1) / sms) / s;
-    if (c < 0.98 * cost) cost = c, best = s;
-  }
-  return best;
+  return choose_slices(K, d_out, sms);
 }
 
 extern "C" size_t smx_tensor_vjp_coef_workspace(const smx_tensor* t, int64_t P) {
