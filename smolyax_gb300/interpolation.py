@@ -269,7 +269,10 @@ class SmolyakBarycentricInterpolator:
     def set_nodal_values(self, fu) -> None:
         """Rebuild the interpolant from new values at the same nodes (no calls of f)."""
         dev = indices.device()
-        fu = torch.as_tensor(fu, dtype=torch.float64, device=dev)
+        if isinstance(fu, torch.Tensor):  # a copy: the caller's tensor may change in place (optimizers)
+            fu = fu.detach().to(dtype=torch.float64, device=dev, copy=True)
+        else:
+            fu = torch.as_tensor(fu, dtype=torch.float64, device=dev)
         assert tuple(fu.shape) == tuple(self.nodal_values.shape), "nodal values must keep their shape"
         if self._plan.keep["zeta0"] != 0 and self._plan.c.n_entries:
             # the constant term follows the zero point's value in fu
