@@ -1,6 +1,7 @@
-// Points whose terms exceed the range of the FP16 pairs (tensor_eval.cu): the panel
-// lists them, and the kernel that writes the values evaluates them once more, in FP32
-// from the coefficients as they are.  With an empty list that is one load per block.
+// Rows of the scaled FP16 product whose terms exceed the range of the pairs
+// (tensor_eval.cu): the drain warps see each row's scale of every 64-column group, and
+// a block evaluates the rows that reach kFarScale once more, over its columns of K, in
+// FP32 from the coefficients as they are.
 #pragma once
 
 #include <stdint.h>
@@ -10,22 +11,29 @@
 namespace smx {
 namespace tc {
 
-// D[p][o] = bias[o] + sum_k A[p][k] B[o][k] for points p[0 .. kFarPts) and outputs
-// [o0, o1), by all threads of a block: the products of kFarCols columns in shared memory
-// (each along its column's slots), a thread per output, sums of 64 columns in FP32 and
-// those added in FP64, so that a value depends on its point alone.
-static __device__ __noinline__ void far_batch(const FarPoints& f, const int (&p)[kFarPts], int K, int o0, int o1,
-                                              const float* __restrict__ bias, float* __restrict__ D, int64_t ldd,
-                                              float* a) {
+// Scale of a group whose largest product times its factor 2^f, which brings the entry's
+// largest coefficient to [2^13, 2^14), reaches 64 (scale: 2^14 below its power of two).
+constexpr float kFarScale = 1.f / 256.f;
+constexpr int kFarPts = 8, kFarCols = 512;
+constexpr int kFarBytes = kFarPts * kFarCols * 4;  // of shared memory
+
+// D[p][o] = bias[o] + sum of A[p][k] B[o][k] over columns [K0, K1) (K0 a multiple of 4)
+// for points p[0 .. kFarPts) and outputs [o0, o1), by all threads of a block: the
+// products of kFarCols columns in shared memory (each along its column's slots), a thread
+// per output, sums of 64 columns in FP32 and those added in FP64, so that a value depends
+// on its point alone.
+static __device__ __noinline__ void far_batch(const FarPoints& f, const int (&p)[kFarPts], int K0, int K1, int o0,
+                                              int o1, const float* __restrict__ bias, float* __restrict__ D,
+                                              int64_t ldd, float* a) {
   for (int o = o0 + int(threadIdx.x); o - int(threadIdx.x) < o1; o += blockDim.x) {
     const float4* b = reinterpret_cast<const float4*>(f.B + int64_t(min(o, o1 - 1)) * f.ldk);
     double sum[kFarPts] = {};
-    for (int k0 = 0; k0 < K; k0 += kFarCols) {
-      const int nk = min(kFarCols, (K - k0 + 3) / 4 * 4);
+    for (int k0 = K0; k0 < K1; k0 += kFarCols) {
+      const int nk = min(kFarCols, (K1 - k0 + 3) / 4 * 4);
       __syncthreads();
       for (int k = threadIdx.x; k < nk; k += blockDim.x) {
         float v[kFarPts];
-        const bool in = k0 + k < K;
+        const bool in = k0 + k < K1;
 #pragma unroll
         for (int i = 0; i < kFarPts; ++i) v[i] = in ? 1.f : 0.f;
         const int4 s4 = in ? __ldg(reinterpret_cast<const int4*>(f.col_path) + k0 + k) : make_int4(-1, -1, -1, -1);
@@ -60,7 +68,8 @@ static __device__ __noinline__ void far_batch(const FarPoints& f, const int (&p)
     }
     if (o < o1)
 #pragma unroll
-      for (int i = 0; i < kFarPts; ++i) D[int64_t(p[i]) * ldd + o] = float(sum[i] + double(__ldg(bias + o)));
+      for (int i = 0; i < kFarPts; ++i)
+        D[int64_t(p[i]) * ldd + o] = float(sum[i] + (bias ? double(__ldg(bias + o)) : 0.0));
   }
 }
 

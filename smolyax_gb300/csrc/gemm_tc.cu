@@ -83,18 +83,18 @@ struct GemmArgs {
   int64_t ld_scale;
   const float* col_scale;  // scaled FP16: by column
   int rows_a, rows_b;      // operands stored slice by slice, [K-tile][rows][kRowBytes]; 0: row-major
-  FarPoints far;           // scaled FP16, one slice of K: rows to evaluate apart
+  FarPoints far;           // scaled FP16: far rows (far_points.cuh)
 };
 
-// Far points among the rows [m0, m1) of a tile (far_points.cuh), by all threads of the block.
-__device__ __noinline__ void far_rows(const FarPoints& f, int K, int m0, int m1, int n0, int n1, const GemmArgs& g,
-                                      uint8_t* shared) {
+// The far rows of a tile (mask: a bit per row), by all threads of the block.
+__device__ __noinline__ void far_rows(const GemmArgs& g, const unsigned* mask, int K0, int K1, int m0, int n0,
+                                      int n1, float* D, uint8_t* shared) {
   int p[kFarPts], n = 0;
-  for (int r = m0; r <= m1; ++r) {  // marks are read by all threads alike
-    if (r < m1 && __ldg(f.list + kFarHead + r)) p[n++] = r;
-    if (n == kFarPts || (r == m1 && n)) {
+  for (int r = 0; r <= kBM; ++r) {
+    if (r < kBM && (mask[r >> 5] >> (r & 31) & 1)) p[n++] = m0 + r;
+    if (n == kFarPts || (r == kBM && n)) {
       for (int i = n; i < kFarPts; ++i) p[i] = p[0];
-      far_batch(f, p, K, n0, n1, g.bias, g.D, g.ldd, reinterpret_cast<float*>(shared));
+      far_batch(g.far, p, K0, K1, n0, n1, g.bias, D, g.ldd, reinterpret_cast<float*>(shared));
       n = 0;
     }
   }
@@ -157,9 +157,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
-  int n_far = 0;
-  if constexpr (KIND == kF16)
-    if (g.far.list) n_far = __ldg(g.far.list);
+  float largest = 0.f;  // scale of a drain lane's row
 
   if (warp == L::kWarpTMA) {
     if (lane == 0) {  // ---- TMA producer
@@ -287,6 +285,7 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
             acc[q + j] += __uint_as_float(r[j]);
         }
       }
+      if constexpr (KIND == kF16) largest = fmaxf(largest, scale);
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
@@ -337,7 +336,11 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
+  int far = 0;
+  if constexpr (KIND == kF16)
+    far = __syncthreads_or(largest >= kFarScale);
+  else
+    __syncthreads();
   if (*abort_flag) {
     // all roles have stopped, and the block gives nothing up before its copies and
     // MMAs have ended (bounded)
@@ -353,7 +356,13 @@ __global__ void __launch_bounds__(Tile<BN>::kThreads, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kBN));
   }
   if constexpr (KIND == kF16)  // the stages are free: copies, MMAs and the staged rows are done with
-    if (n_far > 0 && !*abort_flag) far_rows(g.far, g.K, m0, min(m0 + kBM, g.M), n0, min(n0 + kBN, g.N), g, base);
+    if (far && g.far.rows && !*abort_flag) {
+      unsigned* mask = reinterpret_cast<unsigned*>(base + kFarBytes);
+      const unsigned rows = __ballot_sync(0xffffffffu, largest >= kFarScale && m0 + warp % 4 * 32 + lane < g.M);
+      if (warp < 4 && lane == 0) mask[warp] = rows;
+      __syncthreads();
+      far_rows(g, mask, kt_base * EK, min(g.K, (kt_base + KT) * EK), m0, n0, min(n0 + kBN, g.N), D, base);
+    }
 }
 
 // ---- TF32 split: hi = x rounded to TF32 (10-bit mantissa, round to nearest), lo = TF32(x - hi)
@@ -444,7 +453,7 @@ int launch_tile(const CUtensorMap& tAh, const CUtensorMap& tAl, const void* Bh, 
   if (sc) {
     g.row_scale = sc->row_scale, g.ld_scale = sc->ld_scale, g.col_scale = sc->col_scale;
     if (sc->sliced) g.rows_a = M, g.rows_b = N;
-    if (splits <= 1) g.far = sc->far;
+    g.far = sc->far;
   }
   dim3 grid((N + BN - 1) / BN, (M + kBM - 1) / kBM, nz);
   gemm_tf32x3_kernel<KIND, BN><<<grid, L::kThreads, L::kTotal, st>>>(tAh, tAl, tBh, tBl, g);
@@ -575,33 +584,6 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int nz, int
   }
 }
 
-// The sum of the slices, D = sum + bias, and the far points among its rows (few registers:
-// at one block per SM the sum of 3001 x 64 values took 8.5 us, 4.2 otherwise).
-__global__ void __launch_bounds__(256, 5) splitk_reduce_far_kernel(const float* __restrict__ part, int nz, int M, int N,
-                                                                int K, float* __restrict__ D, int64_t ldd,
-                                                                const float* __restrict__ bias,
-                                                                const __grid_constant__ FarPoints f) {
-  __shared__ __align__(16) float a[kFarPts * kFarCols];
-  const int64_t n = int64_t(M) * N;
-  const int n_far = __ldg(f.list);
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t r = i / N, c = i - r * N;
-    if (n_far && __ldg(f.list + kFarHead + r)) continue;
-    float v = 0.f;
-    for (int z = 0; z < nz; ++z) v += part[z * n + r * N + c];
-    if (bias) v += bias[c];
-    D[r * ldd + c] = v;
-  }
-  const int nt = (N + 255) / 256;
-  const int64_t work = int64_t((n_far + kFarPts - 1) / kFarPts) * nt;
-  for (int64_t w = blockIdx.x; w < work; w += gridDim.x) {
-    const int b0 = int(w / nt) * kFarPts, o0 = int(w % nt) * 256;
-    int p[kFarPts];
-    for (int i = 0; i < kFarPts; ++i) p[i] = __ldg(f.list + kFarHead + f.gstride + min(b0 + i, n_far - 1));
-    far_batch(f, p, K, o0, min(o0 + 256, N), bias, D, ldd, a);
-  }
-}
-
 int splitk_slices(int K, int splits) {
   const int KT = (K + kBK - 1) / kBK;
   const int per = (KT + splits - 1) / splits;
@@ -680,10 +662,7 @@ int smx::tc::split_gemm(const SplitGemm& g, cudaStream_t st) {
                                       g.err, 0, st, g.splits);
   if (rc) return rc;
   const unsigned blocks = smx::grid_for(int64_t(g.M) * g.N, 256);
-  if (g.far.list)
-    splitk_reduce_far_kernel<<<blocks, 256, 0, st>>>(g.partial, slices, g.M, g.N, g.K, g.D, g.ldd, g.bias, g.far);
-  else
-    splitk_reduce_kernel<<<blocks, 256, 0, st>>>(g.partial, slices, g.M, g.N, g.D, g.ldd, g.bias, g.accumulate);
+  splitk_reduce_kernel<<<blocks, 256, 0, st>>>(g.partial, slices, g.M, g.N, g.D, g.ldd, g.bias, g.accumulate);
   SMX_LAUNCH_CHECK("smx_tensor_eval");
   return SMX_OK;
 }

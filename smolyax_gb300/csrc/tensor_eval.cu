@@ -17,14 +17,13 @@
 // before) and the result by 2^u_n.  With the low parts scaled (tc_util.cuh) an
 // element keeps 22 bits down to 2^-29 of the largest of its group and errs by 2^-51 of
 // that one below.  A point's group may serve outputs of very different terms (inputs
-// far outside the box that some outputs do not use), so the panel lists the points with
-// a term of 2^19 and more, in units of its output's largest coefficient, and those are
-// evaluated in FP32 from the coefficients as they are.  For the others the pairs err by
-// less than 2^-26 of an output's largest coefficient.
+// far outside the box that some outputs do not use), so where a point has a term of 2^19
+// and more, in units of its output's largest coefficient, the contraction evaluates its
+// slice of K in FP32 from the coefficients as they are (far_points.cuh).  For the others
+// the pairs err by less than 2^-26 of an output's largest coefficient.
 //
 // Kernels: basis values of all (dimension, degree) slots [slot][point]; the panel
-// A in groups of 64 columns; the contraction (gemm_tc.cu), with the far points
-// (far_points.cuh).
+// A in groups of 64 columns; the contraction (gemm_tc.cu).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -39,10 +38,6 @@ namespace {
 using namespace smx::tc;
 
 constexpr size_t kSmemMax = 227 * 1024;
-
-// A point is far when a product times its factor 2^f, which brings the entry's largest
-// coefficient to [2^13, 2^14), reaches kFar.
-constexpr float kFar = 64.f;
 
 // x coordinate in FP32, infinities as NaN (the point's value is then NaN).
 __device__ __forceinline__ float x32(double v) {
@@ -61,8 +56,7 @@ __device__ __forceinline__ float x32(double v) {
 template <bool DERIV>
 __global__ void __launch_bounds__(256) tensor_basis_kernel(smx_tensor t, const double* __restrict__ x, int64_t P,
                                                            int64_t ldx, float* __restrict__ grow,
-                                                           float* __restrict__ drow, int64_t gstride,
-                                                           int32_t* __restrict__ far) {
+                                                           float* __restrict__ drow, int64_t gstride) {
   __shared__ float z[32][33];
   __shared__ int4 of[32];  // largest degree, first slot, first recurrence pair
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -101,11 +95,6 @@ __global__ void __launch_bounds__(256) tensor_basis_kernel(smx_tensor t, const d
     }
     __syncthreads();
   }
-  // (at the end: at the start the marks hold up the loads of x, 0.9 us of 58)
-  if (!DERIV && far && blockIdx.y == 0 && warp == 0) {
-    far[kFarHead + p0 + lane] = 0;
-    if (blockIdx.x == 0 && lane == 0) far[0] = 0;
-  }
 }
 
 // One bulk tensor store of a 64-column x 128-row tile.
@@ -141,7 +130,7 @@ template <bool F16, int W, bool SROWS>
 __global__ void __launch_bounds__(32 * W, 1)
     tensor_panel_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmL, smx_tensor t,
                         int groups_per_block, const float* __restrict__ grow, int64_t gstride, int64_t P,
-                        float* __restrict__ S, int64_t lds, int32_t* __restrict__ far) {
+                        float* __restrict__ S, int64_t lds) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -181,7 +170,6 @@ __global__ void __launch_bounds__(32 * W, 1)
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     copy_group(t0);
-    float largest = 0.f;
     const char* rowb = reinterpret_cast<const char*>(row);
     char* stkb = reinterpret_cast<char*>(stk);
     for (int g = t0; g < t1; ++g) {
@@ -220,7 +208,6 @@ __global__ void __launch_bounds__(32 * W, 1)
         const int e = min(max(__float_as_int(m) >> 23, 27), 254);
         inv = __int_as_float((268 - e) << 23);
         S[int64_t(q) * lds + p0 + lane] = __int_as_float((e - 14) << 23);
-        largest = fmaxf(largest, m);
       }
       if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tiles' previous stores
       __syncwarp();
@@ -229,10 +216,11 @@ __global__ void __launch_bounds__(32 * W, 1)
         uint32_t h[4], l[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const float2 ab = __fmul2_rn(make_float2(v[63 - 8 * i - 2 * k], v[62 - 8 * i - 2 * k]), make_float2(inv, inv));
+          const float2 vv = make_float2(v[63 - 8 * i - 2 * k], v[62 - 8 * i - 2 * k]);
+          const float2 ab = __fmul2_rn(vv, make_float2(inv, inv));
           if constexpr (F16) {
             const __half2 hh = __float22half2_rn(ab);
-            const __half2 ll = pair_low(ab, hh);
+            const __half2 ll = pair_low_scaled(__fmul2_rn(vv, make_float2(inv * kPairScale, inv * kPairScale)), hh);
             h[k] = *reinterpret_cast<const uint32_t*>(&hh);
             l[k] = *reinterpret_cast<const uint32_t*>(&ll);
           } else {
@@ -255,9 +243,6 @@ __global__ void __launch_bounds__(32 * W, 1)
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
     }
-    if constexpr (F16)
-      if (largest >= kFar && far && p0 + lane < P && atomicExch(far + kFarHead + p0 + lane, 1) == 0)
-        far[kFarHead + lds + atomicAdd(far, 1)] = int(p0 + lane);
   }
   if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
@@ -266,7 +251,7 @@ size_t panel_smem(int warps, int slots) { return 1024 + size_t(warps) * (9216 + 
 
 template <bool F16, int W, bool SROWS>
 void launch_panel(const CUtensorMap& tmH, const CUtensorMap& tmL, const smx_tensor& t, const float* grow,
-                  int64_t gstride, int64_t m, float* S, int32_t* far, int sms, cudaStream_t st) {
+                  int64_t gstride, int64_t m, float* S, int sms, cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(tensor_panel_kernel<F16, W, SROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -287,20 +272,20 @@ void launch_panel(const CUtensorMap& tmH, const CUtensorMap& tmL, const smx_tens
   }
   const dim3 grid(unsigned((t.n_groups + per - 1) / per), unsigned(std::min<int64_t>(n_pb, 65535)));
   tensor_panel_kernel<F16, W, SROWS><<<grid, 32 * W, panel_smem(W, SROWS ? t.n_slots : 0), st>>>(
-      tmH, tmL, t, per, grow, gstride, m, S, gstride, far);
+      tmH, tmL, t, per, grow, gstride, m, S, gstride);
 }
 
 // 16 warps with the basis rows in shared memory up to ~510 slots, 8 warps up to
 // ~1160; beyond, the rows are read through L1.
 template <bool F16>
 void launch_panel(const CUtensorMap& tmH, const CUtensorMap& tmL, const smx_tensor& t, const float* grow,
-                  int64_t gstride, int64_t m, float* S, int32_t* far, int sms, cudaStream_t st) {
+                  int64_t gstride, int64_t m, float* S, int sms, cudaStream_t st) {
   if (panel_smem(16, t.n_slots) <= kSmemMax)
-    launch_panel<F16, 16, true>(tmH, tmL, t, grow, gstride, m, S, far, sms, st);
+    launch_panel<F16, 16, true>(tmH, tmL, t, grow, gstride, m, S, sms, st);
   else if (panel_smem(8, t.n_slots) <= kSmemMax)
-    launch_panel<F16, 8, true>(tmH, tmL, t, grow, gstride, m, S, far, sms, st);
+    launch_panel<F16, 8, true>(tmH, tmL, t, grow, gstride, m, S, sms, st);
   else
-    launch_panel<F16, 16, false>(tmH, tmL, t, grow, gstride, m, S, far, sms, st);
+    launch_panel<F16, 16, false>(tmH, tmL, t, grow, gstride, m, S, sms, st);
 }
 
 // ---- operands -------------------------------------------------------------------------------
@@ -374,7 +359,7 @@ size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
 struct Layout {  // workspace of one chunk of m points
   int64_t gstride;
-  size_t panel, scales, rows, partial, far, total;
+  size_t panel, scales, rows, partial, total;
 };
 Layout layout(const smx_tensor* t, int64_t m) {
   Layout L;
@@ -383,20 +368,19 @@ Layout layout(const smx_tensor* t, int64_t m) {
   L.scales = up256(size_t(t->n_groups) * L.gstride * 4);
   L.rows = up256(size_t(t->n_slots) * L.gstride * 4);
   L.partial = t->splits > 1 ? up256(size_t(t->splits) * m * t->d_out * 4) : 0;
-  L.far = t->B ? up256(far_bytes(L.gstride)) : 0;
-  L.total = 2 * L.panel + L.scales + L.rows + L.partial + L.far;
+  L.total = 2 * L.panel + L.scales + L.rows + L.partial;
   return L;
 }
 
 }  // namespace
 
 void smx::tc::tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, float* drow,
-                           int64_t ldp, cudaStream_t st, int32_t* far) {
+                           int64_t ldp, cudaStream_t st) {
   const dim3 grid(unsigned(ldp / 32), unsigned(std::min((t.n_dims + 31) / 32, 65535)));
   if (drow)
-    tensor_basis_kernel<true><<<grid, 256, 0, st>>>(t, x, P, ldx, grow, drow, ldp, far);
+    tensor_basis_kernel<true><<<grid, 256, 0, st>>>(t, x, P, ldx, grow, drow, ldp);
   else
-    tensor_basis_kernel<false><<<grid, 256, 0, st>>>(t, x, P, ldx, grow, nullptr, ldp, far);
+    tensor_basis_kernel<false><<<grid, 256, 0, st>>>(t, x, P, ldx, grow, nullptr, ldp);
 }
 
 extern "C" int smx_tensor_operands(const float* B, int N, int K, int64_t ldb, const int32_t* tape, int32_t* tape_out,
@@ -442,7 +426,7 @@ constexpr int64_t kMaxPass = int64_t(65535) * 128;
 extern "C" int64_t smx_tensor_chunk(const smx_tensor* t, double memory_limit_gib) {
   if (!t || t->ldb < 1) return 128;
   const double limit = memory_limit_gib * 1073741824.0, panel = 4.0 * double(t->ldb);
-  const double all = panel + 4.0 * t->n_groups + 4.0 * t->n_slots + 8.0 + (t->splits > 1 ? 4.0 * t->splits * t->d_out : 0.0);
+  const double all = panel + 4.0 * t->n_groups + 4.0 * t->n_slots + (t->splits > 1 ? 4.0 * t->splits * t->d_out : 0.0);
   const int64_t fit = int64_t(std::min({limit / panel, 1.125 * limit / all, double(kMaxPass)}));
   return std::max<int64_t>(128, fit / 128 * 128);
 }
@@ -482,21 +466,18 @@ extern "C" int smx_tensor_eval(const smx_tensor* t, const double* x, int64_t P, 
     float* S = reinterpret_cast<float*>(w + 2 * L.panel);
     float* grow = reinterpret_cast<float*>(w + 2 * L.panel + L.scales);
     float* part = reinterpret_cast<float*>(w + 2 * L.panel + L.scales + L.rows);
-    int32_t* far = L.far && !t->bf16 && t->K > 0
-                       ? reinterpret_cast<int32_t*>(w + 2 * L.panel + L.scales + L.rows + L.partial)
-                       : nullptr;
     int rc;
     if (t->K > 0) {
-      tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st, far);
+      tensor_basis(*t, x + p0 * ldx, m, ldx, grow, nullptr, L.gstride, st);
       CUtensorMap tmH, tmL;
       const int bits = t->bf16 ? kBf16 : kF16;
       if ((rc = panel_map(&tmH, Ah, m, t->K, t->ldb, 32, bits)) ||
           (rc = panel_map(&tmL, Al, m, t->K, t->ldb, 32, bits)))
         return rc;
       if (t->bf16)
-        launch_panel<false>(tmH, tmL, *t, grow, L.gstride, m, nullptr, nullptr, sms, st);
+        launch_panel<false>(tmH, tmL, *t, grow, L.gstride, m, nullptr, sms, st);
       else
-        launch_panel<true>(tmH, tmL, *t, grow, L.gstride, m, S, far, sms, st);
+        launch_panel<true>(tmH, tmL, *t, grow, L.gstride, m, S, sms, st);
       SMX_LAUNCH_CHECK("smx_tensor_eval panel");
     }
     SplitGemm g{};
@@ -509,7 +490,7 @@ extern "C" int smx_tensor_eval(const smx_tensor* t, const double* x, int64_t P, 
     g.D = y + p0 * t->d_out, g.ldd = t->d_out;
     g.bias = t->bias, g.err = t->err;
     g.splits = t->splits, g.partial = part;
-    if (far) g.far = FarPoints{far, grow, L.gstride, t->col_path, t->B, t->ldk};
+    if (t->B && !t->bf16) g.far = FarPoints{grow, L.gstride, t->col_path, t->B, t->ldk};
     if ((rc = split_gemm(g, st))) return rc;
   }
   return SMX_OK;

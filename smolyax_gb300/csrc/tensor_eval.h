@@ -18,13 +18,15 @@ namespace tc {
 constexpr int kPop = 1, kPush = 2, kStackMask = 0xf80, kFactorMask = 0x7f800000;
 constexpr int kGroup = 64;  // tape entries (panel columns) per group
 
-// Low parts of the pairs (tc_util.cuh): (v - h) 2^kPairShift.
+// Low parts of the pairs (tc_util.cuh): (v - h) 2^kPairShift, or from v 2^kPairShift.
 __device__ __forceinline__ __half pair_low(float v, __half h) {
   return __float2half_rn((v - __half2float(h)) * kPairScale);
 }
+__device__ __forceinline__ __half2 pair_low_scaled(float2 v, __half2 h) {
+  return __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-kPairScale, -kPairScale), v));
+}
 __device__ __forceinline__ __half2 pair_low(float2 v, __half2 h) {
-  return __float22half2_rn(__ffma2_rn(__half22float2(h), make_float2(-kPairScale, -kPairScale),
-                                      __fmul2_rn(v, make_float2(kPairScale, kPairScale))));
+  return pair_low_scaled(__fmul2_rn(v, make_float2(kPairScale, kPairScale)), h);
 }
 
 // 16 bytes global -> shared, asynchronously (cp.async.wait_all).
@@ -35,29 +37,20 @@ __device__ __forceinline__ void copy16(void* dst, const void* src) {
 }
 
 // Basis values of all slots, grow[slot][p], and (drow given) their derivatives,
-// p < ldp (a multiple of 32; points past P repeat the last one).  `far` given: the list
-// of far points, emptied.
+// p < ldp (a multiple of 32; points past P repeat the last one).
 void tensor_basis(const smx_tensor& t, const double* x, int64_t P, int64_t ldx, float* grow, float* drow, int64_t ldp,
-                  cudaStream_t st, int32_t* far = nullptr);
+                  cudaStream_t st);
 
 constexpr int kTf32 = 0, kBf16 = 1, kF16 = 2;
 
-// Far points (far_points.cuh): the lists of a pass (the count, then from kFarHead on a
-// mark per point and, gstride further, the points) and what their products are made of.
+// What far rows are evaluated from (far_points.cuh).
 struct FarPoints {
-  const int32_t* list;  // NULL: none
-  const float* rows;    // basis values [slot][gstride]
+  const float* rows;  // basis values [slot][gstride]; NULL: no such evaluation
   int64_t gstride;
   const int32_t* col_path;  // [K][4]
   const float* B;           // [N][ldk], zero from K to a multiple of 4
   int64_t ldk;
 };
-constexpr int kFarHead = 64;
-constexpr int kFarPts = 8, kFarCols = 512;
-
-inline __host__ __device__ size_t far_bytes(int64_t gstride) {
-  return (kFarHead + 2 * size_t(gstride)) * sizeof(int32_t);
-}
 
 // D [M x N] = sum over 64-column groups q of row_scale[q][m] * (A_q B_q^T), times
 // col_scale[n], plus bias[n].  A = Ah + Al, B = Bh + Bl, 16-bit, row-major
