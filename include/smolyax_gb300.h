@@ -664,9 +664,10 @@ int smx_split_tf32(const float* src, int64_t rows, int64_t cols, int64_t lds, fl
  * y = A C + c0 with the basis products A of all non-root entries (reversed DFS
  * pre-order) and the coefficients C, both as pairs of 16-bit values
  * (interpolation.py:264-304 over the index set, as smx_spectral_eval).  bf16 = 0:
- * FP16 pairs with exact power-of-two scales per output, entry, and point and
- * 64-column group: 22 significant bits per operand, FP32 accumulation, as the
- * 3xTF32 product.  bf16 = 1: BF16 pairs (16 bits).  All pointers are device
+ * FP16 pairs hi + 2^-11 lo with exact power-of-two scales per output, entry, and
+ * point and 64-column group: 22 significant bits per operand, FP32 accumulation, as
+ * the 3xTF32 product; points whose terms leave the pairs' range are evaluated in FP32
+ * where B is given.  bf16 = 1: BF16 pairs hi + lo (16 bits).  All pointers are device
  * pointers; the struct is read on the host. */
 typedef struct smx_tensor {
   int32_t d_in, d_out;
@@ -739,8 +740,8 @@ typedef struct smx_walk {
   const int32_t* dim_index;  /* [d_in] position of a dimension in smx_tensor.dims, or -1 */
 } smx_walk;
 
-/* Operands of the backward: rows of C / scale in the walk's order as FP16 pairs with a
- * scale per row and group of 64 outputs. */
+/* Operands of the backward: rows of C / scale in the walk's order as FP16 pairs (hi +
+ * 2^-11 lo) with a scale per row and group of 64 outputs. */
 typedef struct smx_tensor_bwd {
   int64_t n_rows;            /* walk.n_chunks * walk.chunk                              */
   int64_t ldo;               /* pitch of Rh, Rl: d_out rounded up to 64                 */
@@ -827,8 +828,8 @@ void smx_layout_free(smx_host_tables* tables);
  * (coefficients in FP64 on the device: smx_spectral_pairs and
  * smx_spectral_coefficients; pair degrees up to 23) and the tables of the
  * evaluator that serves it: the blocked evaluator for one output, the
- * per-point evaluator for 2..15 outputs, the tcgen05 3xTF32 contraction for
- * 16 or more outputs (or rows too large for the per-point evaluator).  It is
+ * per-point evaluator for 2..15 outputs, the tcgen05 contraction of scaled FP16
+ * pairs for 16 or more outputs (or rows too large for the per-point evaluator).  It is
  * what the Python package builds for precision="fp32" (the same host layout
  * builders), replacing interpolation.py:264-304 in FP32.  The tree is the
  * index set built by smx_lambda_* in SMX_MODE_NONZERO (device arrays); fam /

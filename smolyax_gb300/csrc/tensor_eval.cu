@@ -120,12 +120,13 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, const void* 
 // known, are scaled, split and written as the lane's own 128-byte row of two
 // swizzled tiles, which leave by TMA while the next group is walked; the warps
 // never wait for each other.  Bound: HBM writes, 4 bytes per value.
-// Gauss-Hermite d_in = 100, |Lambda| = 20010, 65536 points: 1.13 ms (4.6 TB/s of
+// Gauss-Hermite d_in = 100, |Lambda| = 20010, 65536 points: 1.15 ms (4.6 TB/s of
 // writes); the TF32 panel it replaces wrote twice the bytes in 3.2 ms.  Measured
 // on the way: basis rows read from global memory 3.2 ms (latency), every product
 // through the stack 1.35 ms, the tape read from global memory 1.3 - 1.8 ms.  The
 // rows are copied with cp.async (no registers between loads and stores): Leja d_in
-// = 200, |Lambda| = 5000, 1e5 points 524 us, 554 with loads through registers.
+// = 200, |Lambda| = 5000, 1e5 points 524 us, 554 with loads through registers; the
+// scaled low parts are 2 % more issue slots (534 us).
 template <bool F16, int W, bool SROWS>
 __global__ void __launch_bounds__(32 * W, 1)
     tensor_panel_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmL, smx_tensor t,

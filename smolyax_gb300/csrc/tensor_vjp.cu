@@ -19,7 +19,7 @@
 // adjoint is read, updated and written per path factor in global memory, and
 // the order of every sum is fixed.  Traffic that has to be: G^T written and read
 // once.  Leja d_in = 200, d_out = 64, |Lambda| = 5000, 1e5 points: the walk takes
-// 1.12 ms (56 % of its issue slots and 61 % of the shared-memory pipe busy, the
+// 1.13 ms (56 % of its issue slots and 61 % of the shared-memory pipe busy, the
 // bound), G^T 0.32 ms, basis and cotangent 0.10 ms; the TF32 product and the walk
 // per path factor through global memory took 0.82 + 3.94 ms.  On the way: terms
 // read from global memory by each warp 1.68 ms, two stages of 128 entries 1.46 ms,
@@ -123,7 +123,7 @@ __global__ void split_rows_kernel(const float* __restrict__ C, int64_t n, int d_
 // memory; warp 8 streams R (three stages of TMA), one thread of warp 9 issues the
 // MMAs into four accumulators of 128 columns, and warps 0 - 7 drain them (row
 // scale per slice, column scale), stage 32 x 32 values and write them by TMA.
-// 5120 x 1e5 values from 64 outputs: 326 us (6.3 TB/s of writes); the general
+// 5120 x 1e5 values from 64 outputs: 331 us (6.2 TB/s of writes); the general
 // product, a block per tile with nothing to overlap, took 793 us.
 // Every wait is bounded: on timeout the block sets an error code, and once all its
 // roles have stopped it waits (bounded) for its copies and MMAs and frees tensor memory.
