@@ -192,3 +192,28 @@ def test_far_points_among_others(n, d_out):
     capi.call("smx_tensor_eval", ctypes.byref(s), capi.ptr(xd), P, d, capi.ptr(got), capi.ptr(ws), nws,
               capi.stream_ptr(torch.cuda.current_stream()))
     assert torch.equal(got, y)
+
+
+def test_far_points_of_the_c_plan():
+    """The C plan carries the FP32 coefficients and column paths too: the same values."""
+    from smolyax_gb300 import _capi as capi
+    from test_gpu_capi_fp32 import _fp32_plan
+
+    d, P, d_out = 20, 100, 24
+    ip = _plan(d, 900, d_out, fns.rational_vec(d, d_out, seed=3))
+    sp = ip.spectral_plan()
+    x = np.random.default_rng(0).uniform(-1, 1, (P, d))
+    x[::5, 1] = 1e3
+    xd = torch.as_tensor(x, device="cuda")
+    want, got = (torch.empty(P, d_out, dtype=torch.float32, device="cuda") for _ in range(2))
+    sp.evaluate(xd, want)
+    lib, h = _fp32_plan(ip)
+    try:
+        nws = lib.smx_fp32_workspace(h, P)
+        ws = torch.empty(nws, dtype=torch.uint8, device="cuda")
+        capi.call("smx_fp32_eval", h, capi.ptr(xd), P, d, capi.ptr(got), capi.ptr(ws), nws,
+                  capi.stream_ptr(torch.cuda.current_stream()))
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and _term_error(sp, sp.C64.cpu().numpy(), x).max() <= 1e-6
+    finally:
+        lib.smx_fp32_plan_destroy(h)
