@@ -490,8 +490,10 @@ class SmolyakBarycentricInterpolator:
 
     def _coefficient_bytes(self):
         """Device bytes that building the coefficients takes: the rows of the nodal
-        values once more, and the coefficients."""
-        return 8 * self._d_out * (int(self._plan.c.n_entries) + int(self._tree.size))
+        values once more, the coefficients, and the scratch of their sums."""
+        pl = self._plan
+        return (8 * self._d_out * (int(pl.c.n_entries) + int(self._tree.size))
+                + capi.size("smx_spectral_coefficients_workspace", pl.ref()))
 
     def spectral_plan(self):
         """The FP32 orthogonal-polynomial form of this interpolant (built on first use)."""

@@ -37,3 +37,20 @@ def test_a_jacobian_stays_within_the_limit():
     assert float((J - ref).abs().max()) <= 1e-10 * float(ref.abs().max())
     ip.spectral_plan()  # an evaluation needs the coefficients all the same
     assert torch.equal(ip.gradient(x), ref)
+
+
+@pytest.mark.parametrize("d_out", [1, 64])
+def test_the_coefficients_take_what_is_counted(d_out):
+    """The bytes that the limit is compared with cover what building them allocates."""
+    from smolyax_gb300 import SmolyakBarycentricInterpolator, nodes
+
+    d = 40
+    k = np.log((2 + np.arange(d)) / np.log(2))
+    f = fns.rational_vec(d, d_out, seed=3)
+    f.vectorized = True
+    ip = SmolyakBarycentricInterpolator(node_gen=nodes.Leja(dim=d), k=k, t=7.0, d_out=d_out, f=f)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    ip._coefficients()
+    assert torch.cuda.max_memory_allocated() - before <= 1.1 * ip._coefficient_bytes() + (1 << 18)
